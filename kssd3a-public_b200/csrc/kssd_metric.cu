@@ -15,6 +15,7 @@
 //   - the value itself is derived from them (Naive, Mash or AAF metrics) and lies
 //     within kTolValue of a rounding boundary of the six printed decimals (or of zero);
 // such cells are listed for the host, which recomputes them with its own libm.
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -165,17 +166,13 @@ __device__ bool near(double v, double t) { return fabs(v - t) <= kTol * fmax(1.0
 // the 9- and 10-coden builds carry no calibration model (raw ANI)
 constexpr bool kCalibrate = KSSD_NUM_CODENS >= 11;
 
-// refaf_hgb_predict_ani (src/model_refaf_hgb.h:7593-7628).  *path_unc: a feature derived
-// from log / log1p / pow (or from an inexact raw ANI) came within kTol of a threshold on
-// the path, so another leaf is possible; *val_unc: the result is the inexact raw ANI
-// itself (no calibration), a few ulps from the host's at most.
-__device__ double hgb_predict(const MetricParams &P, double raw_ani, bool raw_unc, double ref_af, const Feat &f,
-                              bool *path_unc, bool *val_unc)
+// The calibration trees' features of a cell (refaf_hgb_predict_ani,
+// src/model_refaf_hgb.h:7593-7628): x[0..10], and the mask of those derived from log /
+// log1p or from an inexact raw ANI, whose thresholds are compared with a tolerance.
+constexpr int kFeatures = 11;
+__device__ uint32_t hgb_features(const MetricParams &P, double raw_ani, bool raw_unc, double ref_af, const Feat &f,
+                                 double *x, int stride)
 {
-    if (!kCalibrate || f.xny == 0) {
-        *val_unc = raw_unc;
-        return raw_ani;
-    }
     raw_ani = clamp01(raw_ani);
     if (ref_af < 1e-12)
         ref_af = 1e-12;
@@ -183,115 +180,170 @@ __device__ double hgb_predict(const MetricParams &P, double raw_ani, bool raw_un
         ref_af = 1.0;
     const double xd = (double)f.xny;
     const double ref_aaf_ani = clamp01(1.0 + log(ref_af) / 11.0);
-    double x[11];
-    bool xu[11];
-    x[0] = raw_ani;
-    xu[0] = raw_unc;
-    x[1] = ref_af;
-    xu[1] = false;
-    x[2] = log1p(xd * fold_scale(P.drfold));
-    xu[2] = true;
-    x[3] = (double)f.diff / xd;
-    x[4] = (double)f.section / xd;
-    x[5] = (double)f.mut2 / xd;
-    xu[3] = xu[4] = xu[5] = false;
-    x[6] = ref_aaf_ani;
-    xu[6] = true;
-    x[7] = raw_ani - ref_aaf_ani;
-    xu[7] = true;
-    x[8] = ref_af < 0.2 ? 1.0 : 0.0;
-    x[9] = (ref_af >= 0.2 && ref_af < 0.5) ? 1.0 : 0.0;
-    x[10] = ref_af >= 0.5 ? 1.0 : 0.0;
-    xu[8] = xu[9] = xu[10] = false;
-    double pred = P.baseline;
-    for (int t = 0; t < P.ntrees; ++t) {
-        const uint32_t begin = __ldg(P.tree_begin + t);
-        uint32_t node = begin;
-        for (int depth = 0; depth < 64; ++depth) {  // trees are far shallower; the bound ends any walk
-            if (node >= P.nnodes)  // a malformed model: the cell is left to the host below
-                break;
-            const HgbNode nd = P.nodes[node];
-            if (nd.flags & 1u)
-                break;
-            const int fi = nd.feature;
-            const double v = x[fi];
-            if (xu[fi] && near(v, nd.x))
-                *path_unc = true;
-            const int left = isnan(v) ? (nd.flags >> 1) & 1u : (v <= nd.x);
-            node = begin + (left ? nd.left : nd.right);
-        }
-        if (node >= P.nnodes || !(P.nodes[node].flags & 1u)) {
-            *path_unc = true;  // the walk did not end on a leaf
-            continue;
-        }
-        pred += P.nodes[node].x;
+    x[0 * stride] = raw_ani;
+    x[1 * stride] = ref_af;
+    x[2 * stride] = log1p(xd * fold_scale(P.drfold));
+    x[3 * stride] = (double)f.diff / xd;
+    x[4 * stride] = (double)f.section / xd;
+    x[5 * stride] = (double)f.mut2 / xd;
+    x[6 * stride] = ref_aaf_ani;
+    x[7 * stride] = raw_ani - ref_aaf_ani;
+    x[8 * stride] = ref_af < 0.2 ? 1.0 : 0.0;
+    x[9 * stride] = (ref_af >= 0.2 && ref_af < 0.5) ? 1.0 : 0.0;
+    x[10 * stride] = ref_af >= 0.5 ? 1.0 : 0.0;
+    return (1u << 2) | (1u << 6) | (1u << 7) | (raw_unc ? 1u : 0u);
+}
+
+// The trees' node records, from the CTA's copy in shared memory or from global memory.
+template <bool SHARED>
+__device__ __forceinline__ HgbNode load_node(const uint4 *nodes, uint32_t i)
+{
+    const uint4 w = SHARED ? nodes[i] : __ldg(nodes + i);
+    HgbNode n;
+    n.x = __longlong_as_double((long long)(((unsigned long long)w.y << 32) | w.x));
+    n.feature = (signed char)(w.z & 0xFFu);
+    n.flags = (unsigned char)((w.z >> 8) & 0xFFu);
+    n.left = (unsigned short)(w.z >> 16);
+    n.right = (unsigned short)(w.w & 0xFFFFu);
+    return n;
+}
+
+// Walks kWays trees side by side, t0, t0 + step, ...: every round loads one node of each,
+// and those loads are independent.  leaf[k] receives the leaf's node number (of a tree
+// below P.ntrees).  Returns true when a feature of `unc` came within kTol of a threshold
+// on a path, or a walk did not end on a leaf (a malformed model): another leaf is
+// possible, the cell is left to the host.
+template <bool SHARED, int kWays>
+__device__ __forceinline__ bool walk_trees(const MetricParams &P, const uint4 *nodes, int t0, int step,
+                                           const double *x, int stride, uint32_t unc, uint32_t (&leaf)[kWays])
+{
+    uint32_t begin[kWays];
+    uint32_t open = 0;
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < kWays; ++k) {
+        const int t = t0 + k * step;
+        begin[k] = t < P.ntrees ? __ldg(P.tree_begin + t) : 0u;
+        leaf[k] = begin[k];
+        open |= t < P.ntrees ? 1u << k : 0u;
     }
-    return clamp01(pred);
+    for (int depth = 0; open && depth <= 64; ++depth) {  // trees are far shallower; the bound ends any walk
+        HgbNode nd[kWays];
+#pragma unroll
+        for (int k = 0; k < kWays; ++k) {
+            if (leaf[k] >= P.nnodes) {  // a malformed model
+                bad = true;
+                leaf[k] = 0;
+                open &= ~(1u << k);
+            }
+            nd[k] = load_node<SHARED>(nodes, leaf[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kWays; ++k) {
+            if (nd[k].flags & 1u)
+                open &= ~(1u << k);
+            if ((open >> k) & 1u) {
+                const double v = x[nd[k].feature * stride];
+                if (((unc >> nd[k].feature) & 1u) && near(v, nd[k].x))
+                    bad = true;
+                const int left = isnan(v) ? (nd[k].flags >> 1) & 1u : (v <= nd[k].x);
+                leaf[k] = begin[k] + (left ? nd[k].left : nd[k].right);
+            }
+        }
+    }
+    return bad || open;
 }
 
 __device__ bool value_available(double v) { return v > 0.0 && v <= 1.0; }
 
+// The calibrated ANI of a cell, once its trees have been walked.
+struct Calibrated {
+    double ani;
+    bool path_unc;
+};
+
+// What a cell needs before its trees (raw ANI, AF of the reference side).
+struct RawAni {
+    double ani, af_r;
+    bool unc;
+};
+
 // kssd_pair_metric for a matrix cell (ani_matrix_pair_value / ani_indexed_self_pair_metric,
-// src/command_ani.c:1458-1496, 1627-1655, with make_selected_output_row :1349-1379)
-__device__ double pair_metric(const MetricParams &P, const Feat &f0, uint32_t qctx, uint32_t rctx, bool *unc)
+// src/command_ani.c:1458-1496, 1627-1655, with make_selected_output_row :1349-1379), each
+// intermediate evaluated only where the selected metric reads it.  A cell whose value
+// depends on the calibration trees returns with *raw filled and *trees set when cal is
+// null; the caller walks the trees and calls again with their sum.
+__device__ __forceinline__ double pair_metric(const MetricParams &P, const Feat &f0, uint32_t qctx, uint32_t rctx,
+                              const Calibrated *cal, RawAni *raw, bool *trees, bool *unc)
 {
     if (qctx == 0 || rctx == 0)
         return P.s < 0 ? 1.0 - P.e : (double)P.e;
     const double af_q = (double)f0.xny / (double)qctx;
     const double af_r = (double)f0.xny / (double)rctx;
     const bool af_pass = (af_q > af_r ? af_q : af_r) >= (double)P.afcut;
-    double moe = P.e, naive = P.e, pd = P.e;
-    bool naive_unc = false;
-    if (af_pass) {
-        moe = lm3ways_dist(f0, P.drfold);
-        naive = naive_dist(f0);
-        naive_unc = true;
-        pd = p_dist(f0, P.obj_bits);
-    }
-    const uint32_t K = (uint32_t)(P.ctx_bits / 2);
-    const double mash = mash_d(K, rctx, qctx, f0.xny);
-    const double aaf = aaf_d(K, rctx, qctx, f0.xny);
-    const double ani = 1.0 - (P.v ? naive : moe);
-    const bool ani_unc = P.v && naive_unc;
-    // fill_calibration (src/command_ani.c:1129-1184); matrix outputs never take the
-    // assembly best-ANI guard (detail output only), so best ANI = calibrated ANI
-    double calibrated = 0, best = 0;
-    bool path_unc = false, cal_unc = false;
-    if (!P.raw_output && af_pass) {
-        if (P.unassembled) {
-            calibrated = best = ani;
-            cal_unc = ani_unc;
-        } else if (f0.xny > 0 && f0.diff == 0 && f0.section == 0 && f0.mut2 == 0 && af_q == 1.0 && af_r == 1.0) {
-            calibrated = best = 1.0;
-        } else {
-            calibrated = hgb_predict(P, ani, ani_unc, af_r, f0, &path_unc, &cal_unc);
-            best = calibrated;
-        }
-    }
     // effective metric (src/command_ani.c:1186-1347)
     int s = P.s < 0 ? -P.s : P.s;
     if (s < 1 || s > 9)
         s = 1;
     if (P.unassembled && !P.unified_metric && s <= 4)
         s = 4;
-    if (s <= 2 && (path_unc || (cal_unc && (near(best, 0.0) || near(best, 1.0)))))
-        *unc = true;  // another leaf, or value_available() of an inexact calibrated value
-    if (s == 1 && !(!P.raw_output && !P.unassembled && value_available(best)))
-        s = 2;
-    if (s == 2 && !(!P.raw_output && !P.unassembled && value_available(calibrated)))
+    const bool calibrates = s <= 2 && !P.raw_output && af_pass && !P.unassembled;
+    double moe = P.e, naive = P.e;
+    if (af_pass && !(P.v && calibrates) && (s <= 3 || s == 7 || s == 8))
+        moe = lm3ways_dist(f0, P.drfold);
+    const bool naive_unc = af_pass;
+    if (af_pass && (s == 4 || (P.v && calibrates)))
+        naive = naive_dist(f0);
+    // fill_calibration (src/command_ani.c:1129-1184); matrix outputs never take the
+    // assembly best-ANI guard (detail output only), so best ANI = calibrated ANI
+    double calibrated = 0;
+    bool cal_unc = false;
+    if (calibrates) {
+        const double ani = 1.0 - (P.v ? naive : moe);
+        const bool ani_unc = P.v && naive_unc;
+        if (f0.xny > 0 && f0.diff == 0 && f0.section == 0 && f0.mut2 == 0 && af_q == 1.0 && af_r == 1.0) {
+            calibrated = 1.0;
+        } else if (!kCalibrate || f0.xny == 0) {  // no calibration model, or nothing to calibrate: the raw ANI
+            calibrated = ani;
+            cal_unc = ani_unc;
+        } else if (!cal) {
+            *raw = RawAni{ani, af_r, ani_unc};
+            *trees = true;
+            return 0;
+        } else {
+            calibrated = cal->ani;
+            if (cal->path_unc)
+                *unc = true;  // another leaf is possible
+        }
+        if (cal_unc && (near(calibrated, 0.0) || near(calibrated, 1.0)))
+            *unc = true;  // value_available() of an inexact calibrated value
+    }
+    if (s <= 2 && P.unassembled && P.v && af_pass && !P.raw_output) {
+        // --qraw with the unified metric: the naive ANI stands in for the calibrated one, and
+        // the selection below asks whether it lies in (0, 1]
+        const double ani = 1.0 - naive_dist(f0);
+        if (near(ani, 0.0) || near(ani, 1.0))
+            *unc = true;
+    }
+    const bool available = calibrates && value_available(calibrated);
+    if (s <= 2 && !available) {
         s = 3;
+        if (P.v && af_pass && calibrates)  // moe was not needed until here
+            moe = lm3ways_dist(f0, P.drfold);
+    }
+    const uint32_t K = (uint32_t)(P.ctx_bits / 2);
     double metric;
     bool vu = false;
     switch (s) {
-    case 1: metric = 1.0 - best; vu = cal_unc; break;
+    case 1:
     case 2: metric = 1.0 - calibrated; vu = cal_unc; break;
     case 3: metric = moe; break;
     case 4: metric = naive; vu = naive_unc; break;
-    case 5: metric = mash; vu = true; break;
-    case 6: metric = aaf; vu = true; break;
-    case 7: metric = af_pass ? moe : mash; vu = !af_pass; break;
-    case 8: metric = af_pass ? moe : aaf; vu = !af_pass; break;
-    default: metric = pd; break;
+    case 5: metric = mash_d(K, rctx, qctx, f0.xny); vu = true; break;
+    case 6: metric = aaf_d(K, rctx, qctx, f0.xny); vu = true; break;
+    case 7: metric = af_pass ? moe : mash_d(K, rctx, qctx, f0.xny); vu = !af_pass; break;
+    case 8: metric = af_pass ? moe : aaf_d(K, rctx, qctx, f0.xny); vu = !af_pass; break;
+    default: metric = af_pass ? p_dist(f0, P.obj_bits) : (double)P.e; break;
     }
     const double value = P.s < 0 ? 1.0 - metric : metric;
     if (vu) {
@@ -306,9 +358,90 @@ __device__ double pair_metric(const MetricParams &P, const Feat &f0, uint32_t qc
     return value;
 }
 
-// One CTA per triangle row q; threads stride over r < q.  Exact cells get their value;
-// the others get NaN and are listed (cell, counters) for the host, up to cap entries.
-__global__ void __launch_bounds__(256) k_lower_metric(MetricParams P, int n, int row0, int row1,
+// Row of triangle cell c: the largest q with q (q - 1) / 2 <= c (c < 2^39).
+__device__ __forceinline__ uint32_t cell_row(size_t c)
+{
+    uint32_t q = (uint32_t)((1.0 + sqrt(1.0 + 8.0 * (double)c)) * 0.5);
+    while ((size_t)q * (q - 1) / 2 > c)
+        --q;
+    while ((size_t)(q + 1) * q / 2 <= c)
+        ++q;
+    return q;
+}
+
+__device__ __forceinline__ Feat cell_feat(unsigned long long c, unsigned long long o)
+{
+    Feat f;
+    f.xny = (uint32_t)c;
+    f.mut2 = (uint32_t)(c >> 32);
+    f.diff = (uint32_t)o;
+    f.section = (uint32_t)(o >> 32);
+    return f;
+}
+
+constexpr int kMetricThreads = 512;    // one CTA per SM
+constexpr int kMetricWarps = kMetricThreads / 32;
+constexpr uint32_t kMetricMost = 8;    // rounds of 32 cells in a warp's tile, at most; their loads are in flight together
+constexpr int kWarpWays = 5;           // trees a lane walks side by side: 160 trees are one round of a warp
+constexpr int kWarpCells = 12;         // from this many tree cells among 32 on, every lane walks its own
+constexpr int kWarpSlots = 8;          // tree cells of a warp in flight
+constexpr size_t kMetricSmem = 220 * 1024;
+
+// Dynamic shared memory: the trees' nodes (SHARED), then each warp's area: per slot the
+// features and the leaf numbers of one cell, or the features of 32 cells, one column a
+// lane (a lane reads a feature that its node names: any choice of rows is free of bank
+// conflicts, where an array of the thread would lie in local memory).
+__host__ __device__ __forceinline__ size_t metric_slot_bytes(int ntrees)
+{
+    return kFeatures * 8 + ((size_t)ntrees * 2 + 7) / 8 * 8;
+}
+__host__ __device__ __forceinline__ size_t metric_warp_bytes(int ntrees)
+{
+    const size_t slots = kWarpSlots * metric_slot_bytes(ntrees), columns = kFeatures * 32 * 8;
+    return slots > columns ? slots : columns;
+}
+__host__ __device__ __forceinline__ size_t metric_smem(int ntrees, uint32_t nnodes, bool shared)
+{
+    return (shared ? (size_t)nnodes * 16 : 0) + kMetricWarps * metric_warp_bytes(ntrees);
+}
+
+// The calibrated value of a cell whose trees sum to cal.
+__device__ __noinline__ double calibrated_value(const MetricParams &P, const Feat &f, uint32_t qc, uint32_t rc,
+                                                const Calibrated &cal, bool *unc)
+{
+    if (value_available(cal.ani)) {  // the selected metric is 1 - calibrated
+        *unc = cal.path_unc;
+        const double metric = 1.0 - cal.ani;
+        return P.s < 0 ? 1.0 - metric : metric;
+    }
+    RawAni raw;
+    bool trees = false;
+    return pair_metric(P, f, qc, rc, &cal, &raw, &trees, unc);
+}
+
+// The value of every cell of a triangle.  Work unit: a warp takes a tile of consecutive
+// cells, 32 of them at a time (256 a tile in a large triangle, fewer when that would leave
+// warps without work, down to 32); warps do not wait for one another.
+//
+// A cell that needs no calibration tree is valued by its lane at once: most cells of a
+// matrix of several species share no context, and that part is a stream of the counters.
+// A cell's 160 trees are independent walks of dependent loads, and the cells of one
+// species lie far apart in a row, so a lane that walks them alone leaves its warp idle
+// for all of them.  Up to kWarpCells of 32 cells the warp takes them one after another,
+// every lane walking five trees side by side, and each cell's lane then adds its leaf
+// values in tree order (the sum's roundings are the reference's).  Above that (a matrix of
+// one species) every lane walks its own cell's trees.  A walk's loads depend on one
+// another, so the model (156 KB) is copied into shared memory first: read through L1, a
+// triangle of a few thousand cells waits for L2 at most levels of every walk.
+//
+// Measured (B200, one call with its launch; before: a CTA per row, a thread per cell):
+// 3,000 genomes of 300 species (4.5 M cells, 13,500 through the trees) 460 -> 57 us,
+// 8,000 genomes of 800 species (32 M cells) 1,346 -> 304 us, 60 genomes of six species
+// 335 -> 45 us (the latency of one warp's cells), 900 genomes of one species (404,550
+// cells, all through the trees) 1,702 -> 1,530 us (issue and shared-memory conflicts).
+template <bool SHARED>
+__global__ void __launch_bounds__(kMetricThreads, 1) k_lower_metric(const __grid_constant__ MetricParams P, size_t cells, uint32_t rounds,
+                                                     int warp_cells,
                                                      const unsigned long long *__restrict__ lc,
                                                      const unsigned long long *__restrict__ lo,
                                                      const uint32_t *__restrict__ qcnt,
@@ -316,30 +449,156 @@ __global__ void __launch_bounds__(256) k_lower_metric(MetricParams P, int n, int
                                                      RecheckCell *__restrict__ recheck, unsigned long long cap,
                                                      unsigned long long *__restrict__ nrecheck)
 {
-    for (int q = row0 + blockIdx.x; q < row1; q += gridDim.x) {
-        const size_t base = (size_t)q * (q - 1) / 2;
-        const uint32_t qc = __ldg(qcnt + q);
-        for (int r = threadIdx.x; r < q; r += blockDim.x) {
-            const unsigned long long c = __ldg(lc + base + r), o = __ldg(lo + base + r);
-            const uint32_t rc = __ldg(rcnt + r);
-            Feat f;
-            f.xny = (uint32_t)c;
-            f.mut2 = (uint32_t)(c >> 32);
-            f.diff = (uint32_t)o;
-            f.section = (uint32_t)(o >> 32);
-            double v;
-            bool unc = false;
-            if (P.zero_const && f.xny == 0 && qc && rc)
-                v = P.zero_value;
-            else
-                v = pair_metric(P, f, qc, rc, &unc);
-            if (unc) {
-                out[base + r] = __longlong_as_double(0x7FF8000000000000ll);
-                const unsigned long long slot = atomicAdd(nrecheck, 1ull);
-                if (slot < cap)
-                    recheck[slot] = RecheckCell{(unsigned long long)(base + r), c, o};
-            } else {
-                out[base + r] = v;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint4 *nodes = reinterpret_cast<const uint4 *>(P.nodes);
+    unsigned char *slots = smem;
+    if (SHARED) {
+        uint4 *copy = reinterpret_cast<uint4 *>(smem);
+        for (uint32_t i = threadIdx.x; i < P.nnodes; i += kMetricThreads)
+            __pipeline_memcpy_async(copy + i, nodes + i, 16);
+        __pipeline_commit();
+        __pipeline_wait_prior(0);
+        nodes = copy;
+        slots += (size_t)P.nnodes * 16;
+        __syncthreads();
+    }
+    const size_t slot_bytes = metric_slot_bytes(P.ntrees);
+    slots += warp * metric_warp_bytes(warp_cells ? P.ntrees : 0);
+    auto put = [&](size_t cell, unsigned long long c, unsigned long long o, double v, bool unc) {
+        if (unc) {
+            out[cell] = __longlong_as_double(0x7FF8000000000000ll);
+            const unsigned long long slot = atomicAdd(nrecheck, 1ull);
+            if (slot < cap)
+                recheck[slot] = RecheckCell{(unsigned long long)cell, c, o};
+        } else {
+            out[cell] = v;
+        }
+    };
+    const size_t tile = (size_t)rounds * 32;
+    // consecutive tiles on different SMs, so that a small triangle uses all of them
+    for (size_t base = ((size_t)warp * gridDim.x + blockIdx.x) * tile; base < cells;
+         base += (size_t)gridDim.x * kMetricWarps * tile) {
+        const size_t end = min(base + tile, cells);
+        // the tile's context words, and every cell that takes the constant (no shared
+        // context between samples with sketches; its object word is not read)
+        unsigned rest = 0;  // rounds with another cell
+        {
+            const size_t first = min(base + lane, cells - 1);
+            uint32_t q = cell_row(first), r = (uint32_t)(first - (size_t)q * (q - 1) / 2);
+            unsigned long long w[kMetricMost];
+#pragma unroll
+            for (uint32_t j = 0; j < kMetricMost; ++j) {
+                const size_t cell = base + 32 * j + lane;
+                w[j] = cell < end ? __ldcs(lc + cell) : 0;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kMetricMost; ++j) {
+                const size_t cell = base + 32 * j + lane;
+                if (cell < end) {
+                    if (P.zero_const && (uint32_t)w[j] == 0 && __ldg(qcnt + q) && __ldg(rcnt + r))
+                        __stcs(out + cell, P.zero_value);
+                    else
+                        rest |= 1u << j;
+                }
+                r += 32;
+                while (r >= q) {  // past the row's end: row q holds q cells
+                    r -= q;
+                    ++q;
+                }
+            }
+        }
+        for (unsigned rounds_left = __reduce_or_sync(0xFFFFFFFFu, rest); rounds_left; rounds_left &= rounds_left - 1) {
+            const int j = __ffs(rounds_left) - 1;
+            const bool in = (rest >> j) & 1u;
+            const size_t cell = base + 32 * j + lane;
+            unsigned long long c = 0, o = 0;
+            uint32_t qc = 0, rc = 0;
+            bool trees = false;
+            RawAni raw{};
+            Feat f{};
+            if (in) {
+                c = __ldg(lc + cell);
+                o = __ldg(lo + cell);
+                const uint32_t q = cell_row(cell), r = (uint32_t)(cell - (size_t)q * (q - 1) / 2);
+                qc = __ldg(qcnt + q);
+                rc = __ldg(rcnt + r);
+                f = cell_feat(c, o);
+                bool unc = false;
+                const double v = pair_metric(P, f, qc, rc, nullptr, &raw, &trees, &unc);
+                if (!trees)
+                    put(cell, c, o, v, unc);
+            }
+            unsigned todo = __ballot_sync(0xFFFFFFFFu, trees);
+            if (__popc(todo) >= warp_cells) {
+                if (trees) {
+                    double *x = reinterpret_cast<double *>(slots) + lane;
+                    const uint32_t fu = hgb_features(P, raw.ani, raw.unc, raw.af_r, f, x, 32);
+                    Calibrated cal{P.baseline, false};
+                    for (int t = 0; t < P.ntrees; t += kWarpWays) {
+                        uint32_t leaf[kWarpWays];
+                        cal.path_unc |= walk_trees<SHARED, kWarpWays>(P, nodes, t, 1, x, 32, fu, leaf);
+#pragma unroll
+                        for (int k = 0; k < kWarpWays; ++k)
+                            if (t + k < P.ntrees)
+                                cal.ani += load_node<SHARED>(nodes, leaf[k]).x;
+                    }
+                    cal.ani = clamp01(cal.ani);
+                    bool unc = false;
+                    const double v = calibrated_value(P, f, qc, rc, cal, &unc);
+                    put(cell, c, o, v, unc);
+                }
+                todo = 0;
+                __syncwarp();  // the columns are rewritten by the next cells
+            }
+            while (todo) {
+                // the next kWarpSlots cells, the lane of rank i among them in slot i
+                unsigned group = 0;
+                for (int i = 0; i < kWarpSlots && todo; ++i) {
+                    group |= todo & (0u - todo);
+                    todo &= todo - 1;
+                }
+                const bool mine = (group >> lane) & 1u;
+                const int rank = __popc(group & ((1u << lane) - 1u));
+                uint32_t fu = 0;
+                if (mine)
+                    fu = hgb_features(P, raw.ani, raw.unc, raw.af_r, f,
+                                      reinterpret_cast<double *>(slots + rank * slot_bytes), 1);
+                __syncwarp();
+                bool bad = false;
+                unsigned left = group;
+                for (int i = 0; left; ++i, left &= left - 1) {
+                    const int src = __ffs(left) - 1;
+                    const uint32_t cu = __shfl_sync(0xFFFFFFFFu, fu, src);
+                    const double *x = reinterpret_cast<const double *>(slots + i * slot_bytes);
+                    unsigned short *leaves = reinterpret_cast<unsigned short *>(slots + i * slot_bytes + kFeatures * 8);
+                    bool b = false;
+                    for (int t = (int)lane; t < P.ntrees; t += 32 * kWarpWays) {
+                        uint32_t leaf[kWarpWays];
+                        b |= walk_trees<SHARED, kWarpWays>(P, nodes, t, 32, x, 1, cu, leaf);
+#pragma unroll
+                        for (int k = 0; k < kWarpWays; ++k)
+                            if (t + 32 * k < P.ntrees)
+                                leaves[t + 32 * k] = (unsigned short)leaf[k];
+                    }
+                    const bool any = __any_sync(0xFFFFFFFFu, b) != 0;
+                    if ((int)lane == src)
+                        bad = any;
+                }
+                __syncwarp();
+                if (mine) {
+                    const unsigned short *leaves =
+                        reinterpret_cast<const unsigned short *>(slots + rank * slot_bytes + kFeatures * 8);
+                    Calibrated cal{P.baseline, bad};
+#pragma unroll 8
+                    for (int t = 0; t < P.ntrees; ++t)
+                        cal.ani += load_node<SHARED>(nodes, leaves[t]).x;
+                    cal.ani = clamp01(cal.ani);
+                    bool unc = false;
+                    const double v = calibrated_value(P, f, qc, rc, cal, &unc);
+                    put(cell, c, o, v, unc);
+                }
+                __syncwarp();  // the slots are rewritten by the next cells
             }
         }
     }
@@ -354,8 +613,28 @@ cudaError_t lower_metric_launch(const MetricParams &P, int n, const unsigned lon
 {
     if (n < 2)
         return cudaSuccess;
-    const int grid = n - 1 < sms * 8 ? n - 1 : sms * 8;
-    k_lower_metric<<<grid, 256, 0, st>>>(P, n, 1, n, lc, lo, qcnt, rcnt, out, recheck, cap, nrecheck);
+    const size_t cells = (size_t)n * (n - 1) / 2;
+    const size_t warps = (size_t)sms * kMetricWarps;
+    const size_t even = cells / (warps * 32);
+    const uint32_t rounds = (uint32_t)(even < 1 ? 1 : even < kMetricMost ? even : kMetricMost);
+    const size_t tiles = (cells + (size_t)rounds * 32 - 1) / ((size_t)rounds * 32);
+    const unsigned grid = (unsigned)(tiles < (size_t)sms ? tiles : (size_t)sms);
+    // the trees matter where the selected metric may be calibrated; a model too large for
+    // shared memory is read from global memory
+    const int s = P.s < 0 ? -P.s : P.s;
+    MetricParams Q = P;
+    if (s >= 3 && s <= 9)
+        Q.ntrees = 0;
+    const bool shared = Q.ntrees > 0 && !P.raw_output && !P.unassembled && Q.nnodes <= 65536 &&
+                        metric_smem(Q.ntrees, Q.nnodes, true) <= kMetricSmem;
+    // a model whose leaf numbers do not fit the slots: every lane walks its own cells
+    const bool slots = metric_smem(Q.ntrees, Q.nnodes, shared) <= kMetricSmem && Q.nnodes <= 65536;
+    const size_t smem = metric_smem(slots ? Q.ntrees : 0, Q.nnodes, shared);
+    auto kern = shared ? k_lower_metric<true> : k_lower_metric<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess)
+        return e;
+    kern<<<grid, kMetricThreads, smem, st>>>(Q, cells, rounds, slots ? kWarpCells : 0, lc, lo, qcnt, rcnt, out, recheck, cap, nrecheck);
     return cudaGetLastError();
 }
 
