@@ -490,13 +490,10 @@ def leg_dense(args, timer, dev, stream, peak_tc):
     alleles = idx.dense_alleles()
     ms_scan = timer(lambda: idx.self_lower_dev(b_c, b_o, flags=kssdgpu.SELF_SCAN, stream=stream), 3, 1)
     same = bool(torch.equal(a_c, b_c) and torch.equal(a_o, b_o))
-    kpad = (alleles + 127) // 128 * 128
-    # int8 multiply-adds x 2 the GEMMs perform: from 6 blocks of 128 genomes on, one GEMM
-    # per block of 128 genomes r over the rows q at or below it, else the whole square
+    # what one operand row per allele would cost over the square: the join's Gram products
+    # of distances stand in for it
     npad = (n + 15) // 16 * 16
-    bw = 128 if (npad + 127) // 128 >= 6 else npad
-    ops = sum(2 * (npad - bw * j) * 4 * min(bw, npad - bw * j) * kpad for j in range((npad + bw - 1) // bw))
-    square_ops = 2 * npad * 4 * npad * kpad
+    square_ops = 2 * npad * 4 * npad * ((alleles + 127) // 128 * 128)
     del a_c, a_o, b_c, b_o
     # the batched probe on the same dense index: 256 new members of the species against
     # it (context groups of hundreds of postings, walked by whole warps), counters of a
@@ -532,11 +529,7 @@ def leg_dense(args, timer, dev, stream, peak_tc):
             "density": density, "default_path": ["scan", "dense", "plan"][path],
             "dense_step_ms": ms_dense, "scan_step_ms": ms_scan, "dense_vs_scan": ms_scan / ms_dense,
             "genome_pairs_s": n * n / (ms_dense / 1e3),
-            "tensor": {"bound": "tensor", "int8_ops": ops, "square_int8_ops": square_ops,
-                       "achieved_tops": ops / ms_dense / 1e9, "peak_tops": peak_tc,
-                       "frac_of_step": ops / ms_dense / 1e9 / peak_tc,
-                       "what": "int8 ops the GEMMs perform (blocks at or below the diagonal) over the whole "
-                               "dense step (allele build + operand rows + GEMMs + epilogue)"},
+            "allele_rows_int8_ops": square_ops,  # of a join with one operand row per allele
             "parity": {"dense_eq_scan": same},
             "batched_probe_256_queries": {"ms": ms_probe, "query_keys": qkeys, "credits": walked,
                                           "genome_pairs_s": qry.n * n / (ms_probe / 1e3),

@@ -255,12 +255,13 @@ int kssdgpu_self_votes(kssdgpu_index_t *idx, const uint64_t *keys, const uint64_
  * (kssdgpu_self_choice).  The one-pass scan (KSSDGPU_SELF_SCAN) zero-fills the packed
  * lower triangle (unless KSSDGPU_NO_ZERO), reads every context group's bounds and
  * joins each group of >= 2 postings as it finds it.  The dense join
- * (KSSDGPU_SELF_DENSE) lists the shared contexts, sorts their postings into alleles
- * (distinct objects per context), builds two int8 operand matrices and computes all
- * four counters of every pair with one exact int8 GEMM on the tensor cores (int32
- * accumulation), then writes every cell of the triangle; it needs a conflict-free
- * index (KSSDGPU_ERR_ARG otherwise) and synchronizes the stream once (for the
- * allele count).
+ * (KSSDGPU_SELF_DENSE) computes the counters of the contexts that many genomes share as
+ * exact int8 Gram products of the genomes' distances to each context's most frequent
+ * object on the tensor cores (int32 accumulation), corrects the pairs that these
+ * misjudge, and scans the other contexts; where minor objects are common it numbers every
+ * context's distinct objects (alleles) and takes one operand row per allele instead,
+ * which synchronizes the stream once (for the allele count).  It writes every cell of the
+ * triangle and needs a conflict-free index (KSSDGPU_ERR_ARG otherwise).
  *
  * With KSSDGPU_SELF_PLAN: the first call builds a set-major plan of the index's
  * shared contexts (kept on the handle; later calls only join over it).  Where the
@@ -359,15 +360,16 @@ int kssdgpu_self_plan_info(kssdgpu_index_t *idx, uint64_t *groups, uint64_t *pos
  * GEMM's multiply-adds up to a constant (the allele count -- distinct objects per
  * shared context -- is estimated at index build from up to 65,536 sampled context
  * groups).  Without a path flag the dense tensor-core join is taken when the index is
- * conflict-free, the density is at least 1/2048 and its operands fit in half of the
- * free device memory; else the one-pass scan.  No reference counterpart.
+ * conflict-free, its estimated time (from the shared contexts' sizes and pairs) is below
+ * the scan's and its operands fit in half of the free device memory; else the one-pass
+ * scan.  No reference counterpart.
  */
 #define KSSDGPU_PATH_SCAN 0
 #define KSSDGPU_PATH_DENSE 1
 #define KSSDGPU_PATH_PLAN 2
 int kssdgpu_self_choice(kssdgpu_index_t *idx, unsigned flags, int *path, double *density);
-/* Allele rows (distinct objects of the shared contexts: the GEMM's K before padding to
- * 128) of the last dense self join on this index; 0 before one ran. */
+/* Alleles (distinct objects of the shared contexts) of an index that a dense self join
+ * ran on; 0 before one ran.  Counted by this call when the join had no use for them. */
 int kssdgpu_self_dense_alleles(kssdgpu_index_t *idx, uint64_t *alleles);
 
 /*

@@ -51,23 +51,29 @@ using Gemm = cutlass::gemm::device::GemmUniversalAdapter<Kernel>;
 
 // lda / ldb: elements between consecutive k rows of A (K x M) and B (K x N); ldd:
 // elements between consecutive rows of D, so that a block of a larger matrix can be
-// one GEMM.
-typename Gemm::Arguments make_args(const int8_t *A, const int8_t *B, int32_t *D, int M, int N, int K, int64_t lda,
-                                   int64_t ldb, int64_t ldd)
+// one GEMM.  batch GEMMs of the same shape lie bsa / bsb / bsd elements apart.
+typename Gemm::Arguments make_args(const int8_t *A, const int8_t *B, int32_t *D, int M, int N, int K, int batch,
+                                   int64_t lda, int64_t ldb, int64_t ldd, int64_t bsa, int64_t bsb, int64_t bsd)
 {
     using SA = typename Gemm::GemmKernel::StrideA;
     using SB = typename Gemm::GemmKernel::StrideB;
     using SC = typename Gemm::GemmKernel::StrideC;
     using SD = typename Gemm::GemmKernel::StrideD;
-    SA sa = cutlass::make_cute_packed_stride(SA{}, cute::make_shape(M, K, 1));
-    SB sb = cutlass::make_cute_packed_stride(SB{}, cute::make_shape(N, K, 1));
-    SC sc = cutlass::make_cute_packed_stride(SC{}, cute::make_shape(M, N, 1));
-    SD sd = cutlass::make_cute_packed_stride(SD{}, cute::make_shape(M, N, 1));
+    SA sa = cutlass::make_cute_packed_stride(SA{}, cute::make_shape(M, K, batch));
+    SB sb = cutlass::make_cute_packed_stride(SB{}, cute::make_shape(N, K, batch));
+    SC sc = cutlass::make_cute_packed_stride(SC{}, cute::make_shape(M, N, batch));
+    SD sd = cutlass::make_cute_packed_stride(SD{}, cute::make_shape(M, N, batch));
     cute::get<1>(sa) = lda;  // A: (m, k) at m + k lda
     cute::get<1>(sb) = ldb;  // B: (n, k) at n + k ldb
     cute::get<0>(sc) = ldd;  // C (not read: beta = 0) and D: (m, n) at m ldd + n
     cute::get<0>(sd) = ldd;
-    typename Gemm::Arguments args{cutlass::gemm::GemmUniversalMode::kGemm, {M, N, K, 1}, {A, sa, B, sb},
+    if (batch > 1) {
+        cute::get<2>(sa) = bsa;
+        cute::get<2>(sb) = bsb;
+        cute::get<2>(sc) = bsd;
+        cute::get<2>(sd) = bsd;
+    }
+    typename Gemm::Arguments args{cutlass::gemm::GemmUniversalMode::kGemm, {M, N, K, batch}, {A, sa, B, sb},
                                   {{1, 0}, D, sc, D, sd}};
 #if KSSD_GEMM_SCHED
     // Fewer output tiles than SMs (up to about 770 genomes): split K evenly over
@@ -79,7 +85,7 @@ typename Gemm::Arguments make_args(const int8_t *A, const int8_t *B, int32_t *D,
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
-    const int tiles = ((M + 127) / 128) * ((N + KSSD_GEMM_TILE_N - 1) / KSSD_GEMM_TILE_N);
+    const int tiles = ((M + 127) / 128) * ((N + KSSD_GEMM_TILE_N - 1) / KSSD_GEMM_TILE_N) * batch;
     if (tiles < sms) {
         args.scheduler.splits = sms / tiles;
         args.scheduler.decomposition_mode = decltype(Sched::decomposition_mode)::SplitK;
@@ -95,20 +101,21 @@ typename Gemm::Arguments make_args(const int8_t *A, const int8_t *B, int32_t *D,
 
 namespace kssd {
 
-// Bytes of device workspace the GEMM of this shape needs (0 or more).
-size_t dense_gemm_s8_workspace(int M, int N, int K)
+// Bytes of device workspace the GEMMs of this shape need (0 or more).
+size_t dense_gemm_s8_workspace(int M, int N, int K, int batch)
 {
-    return Gemm::get_workspace_size(make_args(nullptr, nullptr, nullptr, M, N, K, M, N, N));
+    return Gemm::get_workspace_size(make_args(nullptr, nullptr, nullptr, M, N, K, batch, M, N, N, (int64_t)M * K,
+                                              (int64_t)N * K, (int64_t)M * N));
 }
 
 // D = A^T B for A stored K x M (row stride lda) and B stored K x N (row stride ldb), D
-// row-major with row stride ldd; M, N, lda, ldb multiples of 16 and every base address
-// 16-byte aligned.  Returns 0, or 1 when the shape is not supported, 2 when the launch
-// failed.
-int dense_gemm_s8(const int8_t *A, const int8_t *B, int32_t *D, int M, int N, int K, int64_t lda, int64_t ldb,
-                  int64_t ldd, void *workspace, cudaStream_t st)
+// row-major with row stride ldd; M, N, lda, ldb, bsa, bsb multiples of 16 and every base
+// address 16-byte aligned.  batch of them in one launch, at strides bsa, bsb, bsd.
+// Returns 0, or 1 when the shape is not supported, 2 when the launch failed.
+int dense_gemm_s8(const int8_t *A, const int8_t *B, int32_t *D, int M, int N, int K, int batch, int64_t lda,
+                  int64_t ldb, int64_t ldd, int64_t bsa, int64_t bsb, int64_t bsd, void *workspace, cudaStream_t st)
 {
-    const auto args = make_args(A, B, D, M, N, K, lda, ldb, ldd);
+    const auto args = make_args(A, B, D, M, N, K, batch, lda, ldb, ldd, bsa, bsb, bsd);
     Gemm gemm;
     if (gemm.can_implement(args) != cutlass::Status::kSuccess)
         return 1;

@@ -29,9 +29,9 @@
 using namespace kssd;
 
 namespace kssd {
-size_t dense_gemm_s8_workspace(int M, int N, int K);
-int dense_gemm_s8(const int8_t *A, const int8_t *B, int32_t *D, int M, int N, int K, int64_t lda, int64_t ldb,
-                  int64_t ldd, void *workspace, cudaStream_t st);
+size_t dense_gemm_s8_workspace(int M, int N, int K, int batch);
+int dense_gemm_s8(const int8_t *A, const int8_t *B, int32_t *D, int M, int N, int K, int batch, int64_t lda,
+                  int64_t ldb, int64_t ldd, int64_t bsa, int64_t bsb, int64_t bsd, void *workspace, cudaStream_t st);
 }  // namespace kssd
 
 namespace {
@@ -1760,7 +1760,8 @@ __device__ __forceinline__ void scan_load_bounds(const uint32_t *__restrict__ gb
 // tile), so every lane runs the same short sequence per pair and no thread walks a
 // whole large group while the others wait; with conflicts every thread walks whole
 // groups (run cross products).  Groups of more than kScanLaneMax postings are taken by
-// the whole CTA.
+// the whole CTA.  NARROW: groups of more than kmax postings are left to the caller (a
+// kernel of its own: the comparison costs the join of a 2,000-genome index 7 %).
 #ifndef KSSD_SCAN_PAIR_TABLE
 #define KSSD_SCAN_PAIR_TABLE 1
 #endif
@@ -1774,10 +1775,10 @@ static_assert(kScanPerThread % 4 == 0, "contiguous bounds are loaded 4 at a time
 #ifndef KSSD_SCAN_MINB
 #define KSSD_SCAN_MINB 4
 #endif
-template <bool PAIRS>
+template <bool PAIRS, bool NARROW>
 __global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(const uint32_t *__restrict__ gbeg, uint64_t u,
                                                             const uint64_t *__restrict__ post, int ignoreconflict,
-                                                            CellTable table,
+                                                            uint32_t kmax, CellTable table,
                                                             unsigned long long *__restrict__ oc,
                                                             unsigned long long *__restrict__ oo)
 {
@@ -1814,9 +1815,9 @@ __global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(cons
         for (uint32_t j = 0; j < kScanPerThread; ++j) {
             const uint32_t k = bnd[j + 1] - bnd[j];
             cnt[j] = k;
-            const bool small = k >= 2 && k <= kScanLaneMax;
+            const bool small = k >= 2 && k <= (NARROW ? min(kScanLaneMax, kmax) : kScanLaneMax);
             mine += small ? (1ull | ((unsigned long long)(k * (k - 1) / 2) << 32))
-                          : (k > kScanLaneMax ? 0x10000ull : 0ull);
+                          : (k > kScanLaneMax && (!NARROW || k <= kmax) ? 0x10000ull : 0ull);
         }
         unsigned long long off, tot;
         Scan(scan_tmp).ExclusiveSum(mine, off, tot);
@@ -1826,14 +1827,14 @@ __global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(cons
         for (uint32_t j = 0; j < kScanPerThread; ++j) {
             const uint32_t k = cnt[j];
             const unsigned long long item = (unsigned long long)bnd[j] | ((unsigned long long)k << 32);
-            if (k >= 2 && k <= kScanLaneMax) {
+            if (k >= 2 && k <= (NARROW ? min(kScanLaneMax, kmax) : kScanLaneMax)) {
                 S.queue[sl] = item;
                 if (PAIRS) {
                     S.prefix[sl] = poff;
                     poff += k * (k - 1) / 2;
                 }
                 ++sl;
-            } else if (k > kScanLaneMax) {
+            } else if (k > kScanLaneMax && (!NARROW || k <= kmax)) {
                 S.queue[kScanTile - 1 - ll] = item;
                 ++ll;
             }
@@ -1918,40 +1919,51 @@ __global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(cons
     }
 }
 
-// Facts of the self join: groups of >= 2 postings, postings in them, their pairs,
-// and whether any gid holds several objects of one context (a conflict).
-__global__ void k_self_stats(const uint32_t *__restrict__ gbeg, uint64_t u, const uint64_t *__restrict__ post,
-                             unsigned long long *__restrict__ tot)
+// Facts of the self join: tot[0..2] groups of >= 2 postings, postings in them, their
+// pairs; tot[3] whether any gid holds several objects of one context (a conflict);
+// tot[4..6] the groups of at least `wide` postings, their postings and pairs.  Sums meet in
+// shared memory first: one atomic per warp and fact onto seven global words made this
+// kernel wait on those words (an index of 64 small genomes: 100 us for 0.5 MB of bounds).
+constexpr int kStatFacts = 7;
+__global__ void __launch_bounds__(256) k_self_stats(const uint32_t *__restrict__ gbeg, uint64_t u,
+                                                    const uint64_t *__restrict__ post, uint32_t wide,
+                                                    unsigned long long *__restrict__ tot)
 {
-    unsigned long long g2 = 0, p2 = 0, pairs = 0, conf = 0;
+    __shared__ unsigned long long sum[kStatFacts];
+    if (threadIdx.x < kStatFacts)
+        sum[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long f[kStatFacts] = {};
     for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < u; g += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t b = gbeg[g];
         const unsigned long long k = gbeg[g + 1] - b;
         if (k >= 2) {
-            ++g2;
-            p2 += k;
-            pairs += k * (k - 1) / 2;
+            f[0] += 1;
+            f[1] += k;
+            f[2] += k * (k - 1) / 2;
+            if (k >= wide) {
+                f[4] += 1;
+                f[5] += k;
+                f[6] += k * (k - 1) / 2;
+            }
             uint32_t prev = (uint32_t)(post[b] >> 32);
-            for (uint32_t i = 1; i < k && !conf; ++i) {
+            for (uint32_t i = 1; i < k && !f[3]; ++i) {
                 const uint32_t gid = (uint32_t)(post[b + i] >> 32);
-                conf |= gid == prev;
+                f[3] |= gid == prev;
                 prev = gid;
             }
         }
     }
-    for (int o = 16; o; o >>= 1) {
-        g2 += __shfl_down_sync(0xffffffffu, g2, o);
-        p2 += __shfl_down_sync(0xffffffffu, p2, o);
-        pairs += __shfl_down_sync(0xffffffffu, pairs, o);
-        conf |= __shfl_down_sync(0xffffffffu, conf, o);
+#pragma unroll
+    for (int i = 0; i < kStatFacts; ++i) {
+        for (int o = 16; o; o >>= 1)
+            f[i] += __shfl_down_sync(0xffffffffu, f[i], o);
+        if ((threadIdx.x & 31) == 0 && f[i])
+            atomicAdd(&sum[i], f[i]);
     }
-    if ((threadIdx.x & 31) == 0 && (g2 || conf)) {
-        atomicAdd(tot + 0, g2);
-        atomicAdd(tot + 1, p2);
-        atomicAdd(tot + 2, pairs);
-        if (conf)
-            atomicOr(tot + 3, 1ull);
-    }
+    __syncthreads();
+    if (threadIdx.x < kStatFacts && sum[threadIdx.x])
+        atomicAdd(tot + threadIdx.x, sum[threadIdx.x]);
 }
 
 // ------------------------------------------------------------------ dense self join (tensor cores)
@@ -1968,11 +1980,16 @@ __global__ void k_self_stats(const uint32_t *__restrict__ gbeg, uint64_t u, cons
 // the counters of count_lower (src/command_ani.h:694-716; one object per gid run, so
 // the minimum over the run cross product is that one difference).
 
+#include "kssd_wide.cuh"
+
 // Alleles of a sample of the shared groups (groups g = i * stride, one warp each):
 // tot[0] += distinct objects, tot[1] += postings.  Scales the shared postings to the
-// dense join's allele count (its GEMM's K) for the density rule.
+// dense join's allele count (its GEMM's K) for the density rule.  tot[2] += the pairs of
+// groups of at least `wide` postings that k_wide_rows would correct, estimated from 32
+// of the group's postings.
 __global__ void k_allele_sample(const uint32_t *__restrict__ gbeg, uint64_t u, uint64_t stride, uint32_t samples,
-                                const uint64_t *__restrict__ post, unsigned long long *__restrict__ tot)
+                                const uint64_t *__restrict__ post, uint32_t wide,
+                                unsigned long long *__restrict__ tot)
 {
     const uint32_t lane = threadIdx.x & 31;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < samples; i += (gridDim.x * blockDim.x) >> 5) {
@@ -1992,16 +2009,34 @@ __global__ void k_allele_sample(const uint32_t *__restrict__ gbeg, uint64_t u, u
         }
         for (int o = 16; o; o >>= 1)
             firsts += __shfl_down_sync(0xffffffffu, firsts, o);
+        unsigned long long corr = 0;
+        if (k >= wide) {
+            const uint32_t ns = min(k, 32u);
+            uint32_t o = 0;
+            const uint32_t major = wide_major(post, b, k, lane, o);
+            uint32_t hits = 0;  // ordered pairs of the sample
+            for (uint32_t d = 1; d < 32; ++d) {
+                const uint32_t other = (lane + d) & 31u;
+                const uint32_t p = __shfl_sync(0xffffffffu, o, other);
+                if (lane < ns && other < ns && o != major && p != major)
+                    hits += wide_correction(o, p, major) != 0;
+            }
+            for (int x = 16; x; x >>= 1)
+                hits += __shfl_down_sync(0xffffffffu, hits, x);
+            corr = (unsigned long long)((double)hits * k * (k - 1.0) / (2.0 * ns * (ns - 1.0)));
+        }
         if (lane == 0) {
             atomicAdd(tot + 0, (unsigned long long)firsts);
             atomicAdd(tot + 1, (unsigned long long)k);
+            if (corr)
+                atomicAdd(tot + 2, corr);
         }
     }
 }
 
-// Shared groups (>= 2 postings) as (begin | k << 32), appended in any order.
-__global__ void k_dense_list(const uint32_t *__restrict__ gbeg, uint64_t u, unsigned long long *__restrict__ list,
-                             unsigned int *__restrict__ n_list)
+// Groups of at least kmin postings as (begin | k << 32), appended in any order.
+__global__ void k_dense_list(const uint32_t *__restrict__ gbeg, uint64_t u, uint32_t kmin,
+                             unsigned long long *__restrict__ list, unsigned int *__restrict__ n_list)
 {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -2012,7 +2047,7 @@ __global__ void k_dense_list(const uint32_t *__restrict__ gbeg, uint64_t u, unsi
             b = gbeg[g];
             k = gbeg[g + 1] - b;
         }
-        const bool want = k >= 2;
+        const bool want = k >= kmin;
         const uint32_t at = warp_slot(n_list, want, lane);
         if (want)
             list[at] = (unsigned long long)b | ((unsigned long long)k << 32);
@@ -2572,6 +2607,10 @@ struct kssdgpu_index {
     // postings and pairs, whether any gid run holds several objects (a conflict)
     unsigned long long f_groups = 0, f_postings = 0, f_pairs = 0;
     unsigned long long f_alleles = 0;       // distinct objects of the shared contexts (sampled estimate)
+    // wide groups (at least wide_min postings): count, postings, pairs, and the pairs that
+    // the wide join corrects one by one (sampled estimate)
+    uint32_t wide_min = 2;
+    unsigned long long f_wgroups = 0, f_wpostings = 0, f_wpairs = 0, f_wcorr = 0;
     bool f_conflict = false;
     // dense self join scratch
     DevBuf<unsigned long long> d_list;
@@ -2581,6 +2620,12 @@ struct kssdgpu_index {
     DevBuf<int32_t> d_d;
     DevBuf<unsigned char> d_tmp, d_ws;
     unsigned long long d_alleles = 0;       // alleles of the last dense join (its GEMM's K before padding)
+    // wide join scratch: the wide groups, their rows, the Gram matrices, the pair corrections
+    DevBuf<unsigned long long> w_list, w_corr;
+    DevBuf<unsigned int> w_count;
+    DevBuf<int8_t> w_x;
+    DevBuf<int32_t> w_g;
+    bool w_ran = false;                     // the last dense join was a wide join (kssdgpu_self_dense_alleles)
 };
 
 namespace {
@@ -2667,12 +2712,19 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
     CUDA_TRY(cudaMemcpy(&herr, ix->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!herr && ix->u) {
         // facts of the shared contexts (sizes of the self joins; the dense path's conditions)
-        unsigned long long *d = nullptr, h[4] = {0, 0, 0, 0};
+        ix->wide_min = wide_min_postings(ix->nref);
+        unsigned long long *d = nullptr, h[kStatFacts + 3] = {};
         CUDA_TRY(cudaMalloc(&d, sizeof h));
         cudaError_t e = cudaMemsetAsync(d, 0, sizeof h, st);
         if (e == cudaSuccess) {
-            k_self_stats<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->post, d);
-            count_launch();
+            k_self_stats<<<std::min(grid_for(ix->u), ix->sms * 8), 256, 0, st>>>(ix->gbeg, ix->u, ix->post,
+                                                                                 ix->wide_min, d);
+            // the dense join's allele count, estimated from up to 65,536 sampled groups
+            const uint32_t samples = (uint32_t)std::min<uint64_t>(ix->u, 65536);
+            const uint64_t stride = ix->u / samples;
+            k_allele_sample<<<(samples * 32 + 255) / 256, 256, 0, st>>>(ix->gbeg, ix->u, stride, samples, ix->post,
+                                                                       ix->wide_min, d + kStatFacts);
+            count_launch(2);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, st);
@@ -2684,28 +2736,15 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
         ix->f_postings = h[1];
         ix->f_pairs = h[2];
         ix->f_conflict = h[3] != 0;
-        // the dense join's allele count, estimated from up to 65,536 sampled groups
+        ix->f_wgroups = h[4];
+        ix->f_wpostings = h[5];
+        ix->f_wpairs = h[6];
+        const unsigned long long *sampled = h + kStatFacts;
         ix->f_alleles = ix->f_postings;
-        if (ix->f_groups) {
-            const uint32_t samples = (uint32_t)std::min<uint64_t>(ix->u, 65536);
-            const uint64_t stride = ix->u / samples;
-            unsigned long long *d2 = nullptr, h2[2] = {0, 0};
-            CUDA_TRY(cudaMalloc(&d2, sizeof h2));
-            e = cudaMemsetAsync(d2, 0, sizeof h2, st);
-            if (e == cudaSuccess) {
-                k_allele_sample<<<(samples * 32 + 255) / 256, 256, 0, st>>>(ix->gbeg, ix->u, stride, samples, ix->post,
-                                                                           d2);
-                count_launch();
-                e = cudaGetLastError();
-            }
-            if (e == cudaSuccess) e = cudaMemcpyAsync(h2, d2, sizeof h2, cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            cudaFree(d2);
-            if (e != cudaSuccess)
-                return fail(KSSDGPU_ERR_CUDA, std::string("index facts: ") + cudaGetErrorString(e));
-            if (h2[1])
-                ix->f_alleles = std::max<unsigned long long>(
-                    1, (unsigned long long)((double)ix->f_postings * (double)h2[0] / (double)h2[1]));
+        if (sampled[1]) {
+            const double scale = (double)ix->f_postings / (double)sampled[1];
+            ix->f_alleles = std::max<unsigned long long>(1, (unsigned long long)((double)sampled[0] * scale));
+            ix->f_wcorr = (unsigned long long)((double)sampled[2] * scale);
         }
     }
     if (herr == kDevUnsorted)
@@ -3838,7 +3877,10 @@ int self_plan(kssdgpu_index *ix, cudaStream_t st)
 // the scan join over the whole index.  When the fill stays in L2 the scan launches
 // programmatically after it and waits for it only before its first atomic, so its
 // first tiles' gbeg loads overlap the fill.
-int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, unsigned long long *oo, cudaStream_t st)
+// kmax: larger groups of a conflict-free index are left out (the wide join takes them).
+constexpr uint32_t kScanAll = 0xFFFFFFFFu;
+int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, unsigned long long *oo, cudaStream_t st,
+                   uint32_t kmax = kScanAll)
 {
     const size_t cells = (size_t)ix->nref * (ix->nref - 1) / 2;
     if (!cells)
@@ -3870,13 +3912,14 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
     }
     if (!ix->u)
         return KSSDGPU_OK;
-    auto kern = pairs ? k_self_scan<true> : k_self_scan<false>;
+    auto kern = !pairs ? k_self_scan<false, false> : kmax == kScanAll ? k_self_scan<true, false> : k_self_scan<true, true>;
     const size_t smem = sizeof(ScanSmem);
     if (!ix->scan_grid) {
-        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_self_scan<true>, kScanThreads, smem));
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_self_scan<true, false>, kScanThreads, smem));
         ix->scan_grid = std::max(1, per_sm) * ix->sms;
     }
     const uint64_t ntiles = (ix->u + kScanTile - 1) / kScanTile;
@@ -3893,7 +3936,7 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
         cfg.numAttrs = 1;
     }
     CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const uint32_t *)ix->gbeg, ix->u, (const uint64_t *)ix->post,
-                                (flags & KSSDGPU_IGNORECONFLICT) ? 1 : 0, table, oc, oo));
+                                (flags & KSSDGPU_IGNORECONFLICT) ? 1 : 0, kmax, table, oc, oo));
     count_launch();
     CUDA_TRY(cudaGetLastError());
     if (table.key) {
@@ -3914,12 +3957,175 @@ uint64_t dense_bytes(const kssdgpu_index *ix, uint64_t kpad)
 
 uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 
-// Dense self join (see k_dense_list): list the shared groups, count their alleles
+// Columns of the Gram products one GEMM launch covers: the whole square up to
+// kWideSquare genomes (one launch fills the GPU), else blocks of kWideBlock columns over
+// the rows at or below them (the products are symmetric).
+constexpr uint64_t kWideSquare = 1536, kWideBlock = 512;
+
+uint64_t wide_pass(const kssdgpu_index *ix) { return std::min<uint64_t>(ix->f_wgroups, kWidePass); }
+
+// Device bytes of a wide self join: operand rows, Gram matrices, corrections.
+uint64_t wide_bytes(const kssdgpu_index *ix)
+{
+    const uint64_t np = dense_npad(ix);
+    return (uint64_t)kWideRows * np * (wide_pass(ix) + 4 * np) + 4ull * ix->nref * (ix->nref - 1);
+}
+
+// Estimated times in ms of the three self joins (B200): the scan's pair credits (6.22 G
+// pairs: 45.8 ms), or where few genomes share much the credits that queue up on one cell
+// (14 ns each, one per warp where a group has fewer pairs than a warp lanes: 30 genomes of
+// one species 232 us, two genomes 8 us); the wide join, whose products run near 2.0 P int8 ops/s (six of n^2 a
+// group), whose corrections cost an atomic each and whose narrow groups are scanned; the
+// join with a row per allele (1,024 genomes of one species, 643,817 alleles: products
+// 1.15 ms, rows 0.54 ms, numbering 0.24 ms).  The first terms are launches and gaps.
+double scan_ms(const kssdgpu_index *ix)
+{
+    const double cells = std::max(1.0, 0.5 * (double)ix->nref * (double)(ix->nref - 1));
+    const double merged = std::max(1.0, 32.0 * (double)ix->f_groups / std::max(1.0, (double)ix->f_pairs));
+    return std::max(7.4e-9 * (double)ix->f_pairs, 14e-6 * (double)ix->f_pairs / cells / merged);
+}
+double wide_ms(const kssdgpu_index *ix)
+{
+    const double n = (double)ix->nref;
+    return 0.02 + 7.4e-9 * (double)(ix->f_pairs - ix->f_wpairs + ix->f_wcorr) +
+           (double)ix->f_wgroups * (12 * n * n / 2.0e12 + 6 * n / 4e9);
+}
+double allele_ms(const kssdgpu_index *ix)
+{
+    const double n = (double)ix->nref;
+    return 0.1 + 15e-9 * (double)ix->f_postings +
+           (double)ix->f_alleles * ((ix->nref >= 700 ? 4.5 : 8.0) * n * n / 2.6e12 + 5 * n / 6e9);
+}
+
+// Room for `need` more bytes in half of the free device memory, `have` of which the index
+// holds already (no query of the free memory once it holds them all).
+bool dense_fits(uint64_t need, uint64_t have)
+{
+    if (need <= have)
+        return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return need <= free_b / 2;
+}
+bool wide_fits(const kssdgpu_index *ix)
+{
+    return dense_fits(wide_bytes(ix), ix->w_x.cap + 4 * (uint64_t)ix->w_g.cap + 8 * (uint64_t)ix->w_corr.cap);
+}
+
+// Alleles (distinct objects) of the shared groups, listed and numbered on the device; S =
+// the shared groups.  d_list, d_poff and d_aval hold the groups, their allele counts and
+// values afterwards, d_allele the groups' first allele rows.
+int dense_alleles_impl(kssdgpu_index *ix, uint32_t S, cudaStream_t st, uint32_t &alleles)
+{
+    const int n = ix->nref;
+    const size_t group_smem = dense_group_smem((uint32_t)n);
+    CUDA_TRY(cudaFuncSetAttribute(k_dense_alleles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem));
+    CUDA_TRY(ix->d_list.ensure(S));
+    CUDA_TRY(ix->d_poff.ensure((size_t)S + 1));   // alleles per group, then the fill counter
+    CUDA_TRY(ix->d_allele.ensure((size_t)S + 1)); // first allele row of every group
+    CUDA_TRY(ix->d_aval.ensure(std::max<uint64_t>(ix->n, 1)));
+    unsigned int *d_count = reinterpret_cast<unsigned int *>(ix->d_poff.p + S);
+    size_t tb = 0;
+    CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, ix->d_poff.p, ix->d_allele.p, (int)S + 1, st));
+    CUDA_TRY(ix->d_tmp.ensure(tb));
+    CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));
+    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, 2, ix->d_list.p, d_count);
+    // persistent CTAs over the groups: as many as fit on an SM at once (the group's
+    // barriers and dependent loads leave one CTA mostly waiting)
+    int per_sm_al = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_al, k_dense_alleles, kDenseThreads, group_smem));
+    const int grid_al = ix->sms * std::max(1, per_sm_al);
+    k_dense_alleles<<<grid_al, kDenseThreads, group_smem, st>>>(ix->d_list.p, S, ix->post, (uint32_t)n, ix->d_poff.p,
+                                                                ix->d_aval.p);
+    CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));  // poff[S] = 0: the scan's last term
+    tb = ix->d_tmp.cap;
+    CUDA_TRY(cub::DeviceScan::ExclusiveSum(ix->d_tmp.p, tb, ix->d_poff.p, ix->d_allele.p, (int)S + 1, st));
+    count_launch(4);
+    CUDA_TRY(cudaMemcpyAsync(&alleles, ix->d_allele.p + S, 4, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaStreamSynchronize(st));
+    return KSSDGPU_OK;
+}
+
+// Wide self join (kssd_wide.cuh): zero fill, the narrow groups' pairs by the scan, then per
+// pass of kWidePass wide groups their operand rows and corrections, the six Gram products
+// in one batched GEMM, and the counters from them.  No synchronization.
+int self_wide_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long long *oo, cudaStream_t st)
+{
+    const uint32_t n = (uint32_t)ix->nref;
+    const size_t cells = (size_t)n * (n - 1) / 2;
+    const uint32_t npad = (uint32_t)dense_npad(ix);
+    ix->w_ran = true;
+    if (ix->f_groups > ix->f_wgroups) {
+        const int rc = self_scan_impl(ix, 0, oc, oo, st, ix->wide_min - 1);
+        if (rc)
+            return rc;
+    } else {
+        CUDA_TRY(cudaMemsetAsync(oc, 0, cells * 8, st));
+        CUDA_TRY(cudaMemsetAsync(oo, 0, cells * 8, st));
+    }
+    if (!ix->f_wgroups)
+        return KSSDGPU_OK;
+    if (!wide_fits(ix))
+        return fail(KSSDGPU_ERR_NOMEM, "dense self join: operands of " + std::to_string(wide_bytes(ix)) +
+                                           " bytes exceed half of the free device memory");
+    const uint64_t pass = wide_pass(ix);
+    const size_t gs = (size_t)npad * npad, xs = (size_t)pass * npad;
+    CUDA_TRY(ix->w_list.ensure(ix->f_wgroups));
+    CUDA_TRY(ix->w_count.ensure(1));
+    CUDA_TRY(ix->w_corr.ensure(cells));
+    CUDA_TRY(ix->w_x.ensure(kWideRows * xs));
+    CUDA_TRY(ix->w_g.ensure(kWideRows * gs));
+    const uint64_t bw = npad <= kWideSquare ? npad : kWideBlock;
+    size_t ws = 0;
+    for (uint64_t j = 0; j < npad; j += bw)
+        ws = std::max(ws, kssd::dense_gemm_s8_workspace((int)(npad - j), (int)std::min<uint64_t>(bw, npad - j),
+                                                        (int)pass, kWideRows));
+    CUDA_TRY(ix->d_ws.ensure(ws));
+    CUDA_TRY(cudaMemsetAsync(ix->w_count.p, 0, sizeof(unsigned int), st));
+    CUDA_TRY(cudaMemsetAsync(ix->w_corr.p, 0, cells * 8, st));
+    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->wide_min, ix->w_list.p, ix->w_count.p);
+    count_launch();
+    // warps of a CTA: as many as its shared memory holds, at most 8
+    const size_t per_warp = wide_warp_smem(npad, n);
+    const int warps = (int)std::min<size_t>(8, kWideSmem / per_warp);
+    CUDA_TRY(cudaFuncSetAttribute(k_wide_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(warps * per_warp)));
+    int per_sm = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_rows, warps * 32, warps * per_warp));
+    for (uint64_t c0 = 0; c0 < ix->f_wgroups; c0 += pass) {
+        const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
+        const int grid = std::min<int>(ix->sms * std::max(1, per_sm), (int)((cn + warps - 1) / warps));
+        k_wide_rows<<<grid, warps * 32, warps * per_warp, st>>>(ix->w_list.p + c0, cn, ix->post, n, npad, ix->w_x.p, xs,
+                                                               ix->w_corr.p);
+        count_launch();
+        CUDA_TRY(cudaGetLastError());
+        for (uint64_t j = 0; j < npad; j += bw) {
+            const int grc = kssd::dense_gemm_s8(ix->w_x.p + j, ix->w_x.p + j, ix->w_g.p + j * npad + j,
+                                                (int)(npad - j), (int)std::min<uint64_t>(bw, npad - j), (int)cn,
+                                                kWideRows, npad, npad, npad, (int64_t)xs, (int64_t)xs, (int64_t)gs,
+                                                ix->d_ws.p, st);
+            count_launch();
+            if (grc)
+                return fail(KSSDGPU_ERR_CUDA, grc == 1 ? "dense self join: GEMM shape not supported"
+                                                       : "dense self join: GEMM launch failed");
+            CUDA_TRY(cudaGetLastError());
+        }
+        k_wide_lower<<<grid_for(cells), 256, 0, st>>>(ix->w_g.p, gs, npad, cells, ix->w_corr.p, oc, oo);
+        count_launch();
+        CUDA_TRY(cudaGetLastError());
+    }
+    return KSSDGPU_OK;
+}
+
+// Dense self join, conflict-free indexes of at most kDenseMaxGroup references only: the
+// wide join, or where a row per allele is estimated cheaper (see kssd_wide.cuh): list the
+// shared groups, count their alleles
 // (distinct objects, from a hash of each group's objects in shared memory), build
 // every allele's operand rows, the tensor-core GEMM (per block of genomes below the
 // diagonal from kDenseBlocks blocks on), and the packed lower triangle
-// (every cell written, so no zero fill).  Conflict-free indexes of at most
-// kDenseMaxGroup references only; the operands must fit in half of the free memory.
+// (every cell written, so no zero fill); the operands must fit in half of the free memory.
 int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long long *oo, cudaStream_t st)
 {
     const int n = ix->nref;
@@ -3940,37 +4146,20 @@ int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long lon
         CUDA_TRY(cudaMemsetAsync(oo, 0, cells * 8, st));
         return KSSDGPU_OK;
     }
+    if (wide_ms(ix) <= allele_ms(ix))
+        return self_wide_impl(ix, oc, oo, st);
+    ix->w_ran = false;
     const uint32_t npad = (uint32_t)dense_npad(ix);
-    const size_t group_smem = dense_group_smem((uint32_t)n);
     const size_t rows_smem = dense_rows_smem(npad);
-    CUDA_TRY(cudaFuncSetAttribute(k_dense_alleles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem));
     CUDA_TRY(cudaFuncSetAttribute(k_dense_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem));
-    CUDA_TRY(ix->d_list.ensure(S));
-    CUDA_TRY(ix->d_poff.ensure((size_t)S + 1));   // alleles per group, then the fill counter
-    CUDA_TRY(ix->d_allele.ensure((size_t)S + 1)); // first allele row of every group
-    CUDA_TRY(ix->d_aval.ensure(std::max<uint64_t>(ix->n, 1)));
-    unsigned int *d_count = reinterpret_cast<unsigned int *>(ix->d_poff.p + S);
-    size_t tb = 0;
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, ix->d_poff.p, ix->d_allele.p, (int)S + 1, st));
-    CUDA_TRY(ix->d_tmp.ensure(tb));
     // 1. the shared groups, their allele counts and first allele rows
-    CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));
-    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->d_list.p, d_count);
-    // persistent CTAs over the groups: as many as fit on an SM at once (the group's
-    // barriers and dependent loads leave one CTA mostly waiting)
-    int per_sm_al = 0, per_sm_rows = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_al, k_dense_alleles, kDenseThreads, group_smem));
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rows, k_dense_rows, kDenseThreads, rows_smem));
-    const int grid_al = ix->sms * std::max(1, per_sm_al), grid = ix->sms * std::max(1, per_sm_rows);
-    k_dense_alleles<<<grid_al, kDenseThreads, group_smem, st>>>(ix->d_list.p, S, ix->post, (uint32_t)n, ix->d_poff.p,
-                                                                ix->d_aval.p);
-    CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));  // poff[S] = 0: the scan's last term
-    tb = ix->d_tmp.cap;
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(ix->d_tmp.p, tb, ix->d_poff.p, ix->d_allele.p, (int)S + 1, st));
-    count_launch(4);
     uint32_t alleles = 0;
-    CUDA_TRY(cudaMemcpyAsync(&alleles, ix->d_allele.p + S, 4, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    const int arc = dense_alleles_impl(ix, S, st, alleles);
+    if (arc)
+        return arc;
+    int per_sm_rows = 0;
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_rows, k_dense_rows, kDenseThreads, rows_smem));
+    const int grid = ix->sms * std::max(1, per_sm_rows);
     ix->d_alleles = alleles;
     const uint64_t kpad = round_up(std::max<uint32_t>(alleles, 1), 128);
     size_t free_b = 0, total_b = 0;
@@ -4005,13 +4194,14 @@ int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long lon
     size_t ws = 0;
     for (uint64_t j = 0; j < ngemm; ++j)
         ws = std::max(ws, kssd::dense_gemm_s8_workspace((int)(npad - bw * j),
-                                                        (int)(4 * std::min<uint64_t>(bw, npad - bw * j)), (int)kpad));
+                                                        (int)(4 * std::min<uint64_t>(bw, npad - bw * j)), (int)kpad, 1));
     CUDA_TRY(ix->d_ws.ensure(ws));
     for (uint64_t j = 0; j < ngemm; ++j) {
         const uint64_t m = npad - bw * j, nc = 4 * std::min<uint64_t>(bw, npad - bw * j);
         const int grc = kssd::dense_gemm_s8(ix->d_a.p + bw * j, ix->d_f.p + 4 * bw * j,
-                                            ix->d_d.p + bw * j * 4 * npad + 4 * bw * j, (int)m, (int)nc, (int)kpad,
-                                            (int64_t)npad, (int64_t)(4 * npad), (int64_t)(4 * npad), ix->d_ws.p, st);
+                                            ix->d_d.p + bw * j * 4 * npad + 4 * bw * j, (int)m, (int)nc, (int)kpad, 1,
+                                            (int64_t)npad, (int64_t)(4 * npad), (int64_t)(4 * npad), 0, 0, 0, ix->d_ws.p,
+                                            st);
         count_launch();
         if (grc)
             return fail(KSSDGPU_ERR_CUDA, grc == 1 ? "dense self join: GEMM shape not supported"
@@ -4025,31 +4215,29 @@ int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long lon
     return KSSDGPU_OK;
 }
 
-// The density rule of the self join: the dense path does at most 4 n^2 K multiply-adds (K
-// alleles of the shared contexts), the scan one counter update per pair of postings of
-// a shared context.  density = pairs / (n^2 K); the dense join is taken when it is
-// above kDenseRatio, on a conflict-free index whose operands fit in half of the free
-// device memory.
-constexpr double kDenseRatio = 1.0 / 2048.0;
-
+// density = pairs / (n^2 K), K alleles of the shared contexts (kssdgpu_self_choice).
 double self_density(const kssdgpu_index *ix)
 {
     const double n = (double)ix->nref, k = (double)std::max<unsigned long long>(ix->f_alleles, 1);
     return (double)ix->f_pairs / (n * n * k);
 }
 
+// The rule of the self join: a dense join where the estimates above put it below the
+// scan, on a conflict-free index whose operands fit in half of the free device memory.
+// (A fixed density of 1/2048 sent 64 genomes of eight species, 0.6 M pairs, to the dense
+// join: 290 us of kernels against 12 us by the scan.)
 bool dense_chosen(const kssdgpu_index *ix)
 {
-    if (ix->f_conflict || ix->f_pairs == 0 || ix->nref < 2 || (uint32_t)ix->nref > kDenseMaxGroup ||
-        self_density(ix) < kDenseRatio)
+    if (ix->f_conflict || ix->f_pairs == 0 || ix->nref < 2 || (uint32_t)ix->nref > kDenseMaxGroup)
         return false;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
+    const double wide = wide_ms(ix), allele = allele_ms(ix);
+    if (std::min(wide, allele) >= scan_ms(ix))
         return false;
-    }
+    if (wide <= allele)
+        return wide_fits(ix);
     // the estimate's margin: operands for twice the sampled allele count
-    return dense_bytes(ix, round_up(2 * ix->f_alleles, 128)) <= free_b / 2;
+    return dense_fits(dense_bytes(ix, round_up(2 * ix->f_alleles, 128)),
+                      ix->d_a.cap + ix->d_f.cap + 4 * (uint64_t)ix->d_d.cap);
 }
 
 int self_lower_dev_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, unsigned long long *oo, cudaStream_t st)
@@ -4620,6 +4808,25 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     ix->j_fheads.release();
     ix->j_big.release();
     ix->j_conf.release();
+    ix->s_qcnt.release();
+    ix->s_rcnt.release();
+    ix->s_dcount.release();
+    ix->s_dprefix.release();
+    ix->s_hits.release();
+    ix->d_list.release();
+    ix->d_poff.release();
+    ix->d_allele.release();
+    ix->d_aval.release();
+    ix->d_a.release();
+    ix->d_f.release();
+    ix->d_d.release();
+    ix->d_tmp.release();
+    ix->d_ws.release();
+    ix->w_list.release();
+    ix->w_corr.release();
+    ix->w_count.release();
+    ix->w_x.release();
+    ix->w_g.release();
     delete ix;
 }
 
@@ -5063,6 +5270,16 @@ int kssdgpu_self_dense_alleles(kssdgpu_index_t *ix, uint64_t *alleles)
 {
     if (!ix || !alleles)
         return fail(KSSDGPU_ERR_ARG, "null argument");
+    if (ix->w_ran && ix->f_groups) {  // the wide join has no use for the count: made here
+        CUDA_TRY(cudaSetDevice(ix->device));
+        CUDA_TRY(cudaDeviceSynchronize());
+        uint32_t a = 0;
+        const int rc = dense_alleles_impl(ix, (uint32_t)ix->f_groups, 0, a);
+        if (rc)
+            return rc;
+        ix->d_alleles = a;
+        ix->w_ran = false;
+    }
     *alleles = ix->d_alleles;
     return KSSDGPU_OK;
 }
