@@ -22,6 +22,11 @@
 // (643,817 rows against 17,000 groups of six).  Which is cheaper depends on the data: where
 // minor alleles are common their pairs to correct are many and the alleles few, and the
 // join with a row per allele takes over (dense_chosen compares the two).
+//
+// Measured (B200, whole calls): the self join of 1,024 genomes of one species 1,748 (rows
+// per allele) -> 241 us, of 3,000 genomes of ten species 16.4 -> 3.0 ms; a block of 200
+// queries against 1,024 genomes of their species 6.82 ms (postings walked per query, 1.9 G
+// atomics) -> 0.24 ms, of one query 2.23 -> 0.17 ms.
 #pragma once
 
 // Groups of at least this many postings are wide.  A group costs six rows of the products
@@ -36,6 +41,8 @@ inline uint32_t wide_min_postings(int nref)
 // pair and context a pass's corrections fit the fields of one 64-bit word.
 constexpr uint64_t kWidePass = 131072;
 constexpr int kWideRows = 6;
+constexpr uint32_t kWideMaxRefs = 4096;               // a warp's map and list stay in shared memory
+constexpr uint64_t kWideBlockBytes = 8ull << 30;      // scratch of a block join, at most
 constexpr uint32_t kWideLoads = 4;  // postings of a lane in flight
 constexpr uint32_t kWidePairs = 4;  // genomes compared with a lane's at a time
 constexpr size_t kWideSmem = 220 * 1024;  // dynamic shared memory of a CTA, at most
@@ -108,12 +115,26 @@ __host__ __device__ __forceinline__ size_t wide_warp_smem(uint32_t npad, uint32_
 // group: one pass over its postings fills a byte map of the genomes' distances in shared
 // memory, from which the rows are written in 16-byte pieces, and lists the genomes away
 // from the major object (a tenth of them at 1 % divergence); their pairs are compared
-// with the first of the pair broadcast and lanes on consecutive others.  Bound by the
-// rows' 6 n bytes and the corrections' atomics (L2).
+// with kWidePairs of them broadcast and lanes on consecutive others.  Bound by issue (the
+// pairs) and the corrections' atomics (L2); the rows are 6 n bytes.
+//
+// BLOCK: the pairs are those of a query with the group's genomes instead.  qobj[c * nqpad
+// + q] is the object of query q at group c (kWideNone: it does not hold it), written by
+// the counting kernel; the queries' operand rows go to Y, the corrections to corr[q * nref
+// + r].
+struct WideBlock {
+    const uint32_t *qobj;
+    uint32_t nq, nqpad;
+    int8_t *Y;
+    size_t ys;
+};
+constexpr uint32_t kWideNone = 0xFFFFFFFFu;  // not an object: the block join takes objects below 32 bits
+
+template <bool BLOCK>
 __global__ void __launch_bounds__(256) k_wide_rows(const unsigned long long *__restrict__ list, uint32_t n_list,
                                                    const uint64_t *__restrict__ post, uint32_t nref, uint32_t npad,
                                                    int8_t *__restrict__ X, size_t xs,
-                                                   unsigned long long *__restrict__ corr)
+                                                   unsigned long long *__restrict__ corr, const WideBlock Q)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
     const uint32_t lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
@@ -156,6 +177,43 @@ __global__ void __launch_bounds__(256) k_wide_rows(const unsigned long long *__r
 #pragma unroll
             for (int m = 0; m < kWideRows; ++m)
                 reinterpret_cast<uint4 *>(X + m * xs + (size_t)s * npad)[i] = make_uint4(a.w[m], c.w[m], d.w[m], f.w[m]);
+        }
+        if (BLOCK) {
+            for (uint32_t q0 = 0; q0 < Q.nqpad; q0 += 128) {
+                const uint32_t q = q0 + 4 * lane;
+                uint4 oq = make_uint4(kWideNone, kWideNone, kWideNone, kWideNone);
+                if (q < Q.nqpad)
+                    oq = __ldcs(reinterpret_cast<const uint4 *>(Q.qobj + (size_t)s * Q.nqpad + q));
+                const uint32_t ob[4] = {oq.x, oq.y, oq.z, oq.w};
+                uint32_t e4 = 0;
+#pragma unroll
+                for (int x = 0; x < 4; ++x)
+                    e4 |= (ob[x] == kWideNone ? 0xFFu : wide_e(ob[x], major)) << (8 * x);
+                if (q < Q.nqpad) {
+                    const WideWords w = wide_words(e4);
+#pragma unroll
+                    for (int m = 0; m < kWideRows; ++m)
+                        *reinterpret_cast<uint32_t *>(Q.Y + m * Q.ys + (size_t)s * Q.nqpad + q) = w.w[m];
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const uint32_t ex = (e4 >> (8 * x)) & 0xFFu;
+                    for (unsigned away = __ballot_sync(0xffffffffu, ex != 0 && ex != 0xFFu); away; away &= away - 1) {
+                        const int src = __ffs(away) - 1;
+                        const uint32_t oa = __shfl_sync(0xffffffffu, ob[x], src), ea = __shfl_sync(0xffffffffu, ex, src);
+                        unsigned long long *row = corr + (size_t)(q0 + 4 * src + x) * nref;
+                        for (uint32_t j = lane; j < nm; j += 32) {
+                            const unsigned long long c = minor[j];
+                            const uint32_t rc = (uint32_t)(c >> 32);
+                            const unsigned long long w = wide_correction(oa, (uint32_t)c, ea, rc >> kGidBits);
+                            if (w)
+                                atomicAdd(row + (rc & ((1u << kGidBits) - 1)), w);
+                        }
+                    }
+                }
+            }
+            __syncwarp();  // the warp's shared memory is reused by its next group
+            continue;
         }
         // pairs (i, j), j < i: kWidePairs genomes i against lanes on consecutive j (postings
         // ascend by gid, so i is the pair's higher genome)
@@ -215,6 +273,20 @@ __global__ void __launch_bounds__(256) k_wide_lower(const int32_t *__restrict__ 
         while ((size_t)(q + 1) * q / 2 <= c)
             ++q;
         const uint32_t r = (uint32_t)(c - (size_t)q * (q - 1) / 2);
+        wide_credit(G + (size_t)q * npad + r, gs, corr[c], oc + c, oo + c);
+        corr[c] = 0;
+    }
+}
+
+// The same for a block of queries: cell (q, r) of rows of nref references.
+__global__ void __launch_bounds__(256) k_wide_block(const int32_t *__restrict__ G, size_t gs, uint32_t npad,
+                                                    uint32_t nq, uint32_t nref, unsigned long long *__restrict__ corr,
+                                                    unsigned long long *__restrict__ oc,
+                                                    unsigned long long *__restrict__ oo)
+{
+    const size_t cells = (size_t)nq * nref;
+    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < cells; c += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t q = (uint32_t)(c / nref), r = (uint32_t)(c - (size_t)q * nref);
         wide_credit(G + (size_t)q * npad + r, gs, corr[c], oc + c, oo + c);
         corr[c] = 0;
     }

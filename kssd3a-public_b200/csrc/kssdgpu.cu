@@ -281,6 +281,12 @@ struct CountParams {
     int bloom_stripes;             // its key-range stripes (a power of two)
     const unsigned long long *bloom_bounds;  // first context of each stripe (stripes + 1 words)
     const uint32_t *nitems_dev;    // stripe-major mode: count of P.items (built on the device), may be null
+    // wide groups left to the tensor cores (kssd_wide.cuh), or null: a query's object at a
+    // group of at least wide_min postings goes to wide_obj[number * wide_stride + query], the
+    // group's number at wide_at[its first posting]
+    uint32_t *wide_obj;
+    const uint32_t *wide_at;
+    uint32_t wide_min, wide_stride;
 };
 
 
@@ -649,8 +655,9 @@ __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ p
 // takes one entry per round (the warp's rounds are the same for all its lanes).  Only the
 // first entry of a context run works (src/command_ani.h:498-505); the filter rules out
 // most absent contexts; one hash probe finds the context; the inline single posting is
-// credited at once, short groups are walked by their lane, long ones by the warp.
-template <bool LOWER, bool UNIQUE, class Acc>
+// credited at once, short groups are walked by their lane, long ones by the warp, or
+// (WIDE) left to the tensor cores.
+template <bool LOWER, bool UNIQUE, bool WIDE, class Acc>
 __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, uint64_t e, uint64_t cb, uint64_t ce,
                                               int qgid, uint64_t objmask, const Acc &acc, const Acc &uacc,
                                               const FilterView &fv, uint64_t t0, uint64_t T)
@@ -695,7 +702,10 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
                 const bool single = (sl.x & kInlineBit) != 0;
                 pb = (uint32_t)sl.y;
                 pc = (uint32_t)(sl.y >> 32);
-                if (!single && pc >= kWarpWalk)
+                if (WIDE && !single && s == 1 && pc >= P.wide_min)
+                    P.wide_obj[(size_t)__ldg(P.wide_at + pb) * P.wide_stride + (uint32_t)(qgid - P.qgid_offset)] =
+                        (uint32_t)(__ldg(P.qkeys + i) & objmask);
+                else if (!single && pc >= kWarpWalk)
                     wide = true;
                 else
                     credit_context<LOWER, UNIQUE>(P, i, s, sl.y, single, qgid, objmask, acc, uacc);
@@ -718,7 +728,7 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
 // memory and written once, coalesced; without, counters go to the zeroed global
 // row with atomics, and the work may be split into key-range chunks (P.items) so
 // that one large query (a read set) spreads over many SMs.
-template <bool LOWER, bool UNIQUE, bool SMEM>
+template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE>
 __global__ void __launch_bounds__(512) k_count_batched(CountParams P)
 {
     extern __shared__ uint32_t sm[];
@@ -765,7 +775,7 @@ __global__ void __launch_bounds__(512) k_count_batched(CountParams P)
         if (SMEM) {
             const SmemAcc acc{row0, row0 + nref, row0 + 2 * nref, row0 + 3 * nref};
             const SmemAcc uacc{row1, row1 + nref, row1 + 2 * nref, row1 + 3 * nref};
-            process_query<LOWER, UNIQUE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
+            process_query<LOWER, UNIQUE, WIDE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
         } else {
             const GlobalAcc acc{P.out_ctx + row, P.out_obj + row};
             const GlobalAcc uacc{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr};
@@ -777,7 +787,7 @@ __global__ void __launch_bounds__(512) k_count_batched(CountParams P)
                 cb = b + (uint64_t)(it - (int)P.chunk_prefix[q]) * P.chunk_keys;
                 ce = min(e, cb + (uint64_t)P.chunk_keys);
             }
-            process_query<LOWER, UNIQUE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
+            process_query<LOWER, UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
         }
         __syncthreads();
         if (SMEM) {
@@ -803,7 +813,7 @@ __global__ void __launch_bounds__(512) k_count_batched(CountParams P)
 // global rows with atomics, as in the chunked mode.
 constexpr uint32_t kStripeGrab = 2;
 
-template <bool LOWER, bool UNIQUE>
+template <bool LOWER, bool UNIQUE, bool WIDE>
 __global__ void __launch_bounds__(512) k_count_striped(CountParams P)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -827,7 +837,7 @@ __global__ void __launch_bounds__(512) k_count_striped(CountParams P)
             const GlobalAcc acc{P.out_ctx + row, P.out_obj + row};
             const GlobalAcc uacc{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr};
             const FilterView fv{P.bloom + stripe_words * w.pad, P.bloom_mask, 1, nullptr};
-            process_query<LOWER, UNIQUE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32);
+            process_query<LOWER, UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32);
         }
     }
 }
@@ -2034,9 +2044,11 @@ __global__ void k_allele_sample(const uint32_t *__restrict__ gbeg, uint64_t u, u
     }
 }
 
-// Groups of at least kmin postings as (begin | k << 32), appended in any order.
+// Groups of at least kmin postings as (begin | k << 32), appended in any order; number_at
+// (may be null) receives a group's place in the list at its first posting's.
 __global__ void k_dense_list(const uint32_t *__restrict__ gbeg, uint64_t u, uint32_t kmin,
-                             unsigned long long *__restrict__ list, unsigned int *__restrict__ n_list)
+                             unsigned long long *__restrict__ list, unsigned int *__restrict__ n_list,
+                             uint32_t *__restrict__ number_at)
 {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -2049,8 +2061,11 @@ __global__ void k_dense_list(const uint32_t *__restrict__ gbeg, uint64_t u, uint
         }
         const bool want = k >= kmin;
         const uint32_t at = warp_slot(n_list, want, lane);
-        if (want)
+        if (want) {
             list[at] = (unsigned long long)b | ((unsigned long long)k << 32);
+            if (number_at)
+                number_at[b] = at;
+        }
     }
 }
 
@@ -2623,7 +2638,8 @@ struct kssdgpu_index {
     // wide join scratch: the wide groups, their rows, the Gram matrices, the pair corrections
     DevBuf<unsigned long long> w_list, w_corr;
     DevBuf<unsigned int> w_count;
-    DevBuf<int8_t> w_x;
+    DevBuf<int8_t> w_x, w_y;
+    DevBuf<uint32_t> w_qobj, w_at;          // block join: the queries' objects, group numbers by first posting
     DevBuf<int32_t> w_g;
     bool w_ran = false;                     // the last dense join was a wide join (kssdgpu_self_dense_alleles)
 };
@@ -2825,10 +2841,10 @@ int cell_table(kssdgpu_index *ix, cudaStream_t st, CellTable &t)
     return KSSDGPU_OK;
 }
 
-template <bool LOWER, bool UNIQUE, bool SMEM>
+template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE = false>
 int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStream_t st)
 {
-    auto kern = k_count_batched<LOWER, UNIQUE, SMEM>;
+    auto kern = k_count_batched<LOWER, UNIQUE, SMEM, WIDE>;
     if (smem > 48 * 1024)
         CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
@@ -2847,10 +2863,10 @@ int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStr
     return KSSDGPU_OK;
 }
 
-template <bool LOWER, bool UNIQUE>
+template <bool LOWER, bool UNIQUE, bool WIDE = false>
 int launch_striped(kssdgpu_index *ix, const CountParams &P, cudaStream_t st)
 {
-    auto kern = k_count_striped<LOWER, UNIQUE>;
+    auto kern = k_count_striped<LOWER, UNIQUE, WIDE>;
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, 0));
     const int grid = ix->sms * std::max(per_sm, 1);  // persistent: the item count stays on the device
@@ -2904,6 +2920,125 @@ void build_chunks(const uint64_t *offs, int nq, const int *order, uint64_t chunk
         for (uint64_t c = b; c < e; c += chunk)
             items.push_back(WorkItem{(uint32_t)q, 0u, c, std::min(e, c + chunk)});
     }
+}
+
+uint64_t wide_npad(uint64_t n) { return (n + 15) / 16 * 16; }
+uint64_t wide_pass(const kssdgpu_index *ix) { return std::min<uint64_t>(ix->f_wgroups, kWidePass); }
+
+// Room for `need` more bytes in half of the free device memory, `have` of which the index
+// holds already (no query of the free memory once it holds them all).
+bool dense_fits(uint64_t need, uint64_t have)
+{
+    if (need <= have)
+        return true;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return need <= free_b / 2;
+}
+
+// Launch shape of k_wide_rows: warps of a CTA (as many as its shared memory holds, at most
+// 8) and the CTAs that fill the GPU.
+template <class Kernel>
+cudaError_t wide_rows_shape(const kssdgpu_index *ix, Kernel kern, uint32_t npad, int &warps, int &grid)
+{
+    const size_t per_warp = wide_warp_smem(npad, (uint32_t)ix->nref);
+    warps = (int)std::min<size_t>(8, kWideSmem / per_warp);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(warps * per_warp));
+    int per_sm = 0;
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, warps * per_warp);
+    grid = ix->sms * std::max(1, per_sm);
+    return e;
+}
+
+// Scratch of a wide block join in bytes: the queries' objects, both operands, the
+// products, the corrections.
+uint64_t wide_block_bytes(const kssdgpu_index *ix, uint64_t nq)
+{
+    const uint64_t np = wide_npad((uint64_t)ix->nref), nqp = wide_npad(nq);
+    return 4 * ix->f_wgroups * nqp + (uint64_t)kWideRows * (wide_pass(ix) * (np + nqp) + 4 * nqp * np) +
+           8 * nq * (uint64_t)ix->nref + 4 * ix->n;
+}
+
+// Whether a block of nq queries leaves the wide groups to the tensor cores: by estimated
+// times in ms, the walk's credits at 3.8 ps (200 queries of one species against 1,024
+// genomes: 1.9 G credits in 7.3 ms; half of the wide groups assumed per query), or 0.67 ns
+// over the CTAs that few queries' chunks occupy (one query: 2.2 ms), against the operand
+// rows of both sides, the products, and the pairs to correct.
+bool wide_block_chosen(const kssdgpu_index *ix, int nq, unsigned flags)
+{
+    if (ix->f_conflict || !ix->f_wgroups || ix->nref > (int)kWideMaxRefs || ix->obj_bits >= 32 ||
+        (flags & (KSSDGPU_PLAIN | KSSDGPU_GLOBAL_ACC | KSSDGPU_SMEM_ACC)))
+        return false;
+    const double n = (double)ix->nref, q = (double)nq;
+    const double ctas = q * (1.0 + (double)ix->f_wgroups / ix->count_chunk_keys);
+    const double walk = std::max(3.8e-9, 0.67e-6 / ctas) * 0.5 * q * (double)ix->f_wpostings;
+    const double wide = 0.04 + (double)ix->f_wgroups * (12 * q * n / 2.0e12 + 6 * (n + q) / 4e9) +
+                        7.4e-9 * (double)ix->f_wcorr * 2 * q / n;
+    if (wide >= walk)
+        return false;
+    const uint64_t need = wide_block_bytes(ix, (uint64_t)nq);
+    return need <= kWideBlockBytes &&
+           dense_fits(need, ix->w_x.cap + ix->w_y.cap + 4 * ((uint64_t)ix->w_g.cap + ix->w_qobj.cap + ix->w_at.cap) +
+                                8 * (uint64_t)ix->w_corr.cap);
+}
+
+// Before the counting kernel: the wide groups' list and numbers, the queries' objects.
+int wide_block_begin(kssdgpu_index *ix, int nq, CountParams &P, cudaStream_t st)
+{
+    const uint64_t nqp = wide_npad((uint64_t)nq);
+    CUDA_TRY(ix->w_list.ensure(ix->f_wgroups));
+    CUDA_TRY(ix->w_count.ensure(1));
+    CUDA_TRY(ix->w_at.ensure(ix->n));
+    CUDA_TRY(ix->w_qobj.ensure(ix->f_wgroups * nqp));
+    CUDA_TRY(cudaMemsetAsync(ix->w_count.p, 0, sizeof(unsigned int), st));
+    CUDA_TRY(cudaMemsetAsync(ix->w_qobj.p, 0xFF, ix->f_wgroups * nqp * 4, st));
+    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->wide_min, ix->w_list.p, ix->w_count.p,
+                                                  ix->w_at.p);
+    count_launch();
+    CUDA_TRY(cudaGetLastError());
+    P.wide_obj = ix->w_qobj.p;
+    P.wide_at = ix->w_at.p;
+    P.wide_min = ix->wide_min;
+    P.wide_stride = (uint32_t)nqp;
+    return KSSDGPU_OK;
+}
+
+// After it: per pass of kWidePass groups the operand rows of both sides and the
+// corrections, the six products in one batched GEMM, and the counters added to the rows.
+int wide_block_end(kssdgpu_index *ix, int nq, unsigned long long *oc, unsigned long long *oo, cudaStream_t st)
+{
+    const uint32_t n = (uint32_t)ix->nref, npad = (uint32_t)wide_npad(n), nqp = (uint32_t)wide_npad((uint64_t)nq);
+    const uint64_t pass = wide_pass(ix);
+    const size_t cells = (size_t)nq * n, gs = (size_t)nqp * npad, xs = (size_t)pass * npad, ys = (size_t)pass * nqp;
+    CUDA_TRY(ix->w_corr.ensure(cells));
+    CUDA_TRY(ix->w_x.ensure(kWideRows * xs));
+    CUDA_TRY(ix->w_y.ensure(kWideRows * ys));
+    CUDA_TRY(ix->w_g.ensure(kWideRows * gs));
+    CUDA_TRY(ix->d_ws.ensure(kssd::dense_gemm_s8_workspace((int)nqp, (int)npad, (int)pass, kWideRows)));
+    CUDA_TRY(cudaMemsetAsync(ix->w_corr.p, 0, cells * 8, st));
+    int warps = 0, rows_grid = 0;
+    CUDA_TRY(wide_rows_shape(ix, k_wide_rows<true>, npad, warps, rows_grid));
+    for (uint64_t c0 = 0; c0 < ix->f_wgroups; c0 += pass) {
+        const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
+        const WideBlock Q{ix->w_qobj.p + c0 * nqp, (uint32_t)nq, nqp, ix->w_y.p, ys};
+        k_wide_rows<true><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
+                            warps * wide_warp_smem(npad, n), st>>>(ix->w_list.p + c0, cn, ix->post, n, npad, ix->w_x.p,
+                                                                   xs, ix->w_corr.p, Q);
+        CUDA_TRY(cudaGetLastError());
+        const int grc = kssd::dense_gemm_s8(ix->w_y.p, ix->w_x.p, ix->w_g.p, (int)nqp, (int)npad, (int)cn, kWideRows,
+                                            nqp, npad, npad, (int64_t)ys, (int64_t)xs, (int64_t)gs, ix->d_ws.p, st);
+        if (grc)
+            return fail(KSSDGPU_ERR_CUDA, grc == 1 ? "wide block join: GEMM shape not supported"
+                                                   : "wide block join: GEMM launch failed");
+        k_wide_block<<<grid_for(cells), 256, 0, st>>>(ix->w_g.p, gs, npad, (uint32_t)nq, n, ix->w_corr.p, oc, oo);
+        count_launch(3);
+        CUDA_TRY(cudaGetLastError());
+    }
+    return KSSDGPU_OK;
 }
 
 int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_offs, int nq, int qgid_offset, bool lower,
@@ -2996,6 +3131,12 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
             CUDA_TRY(cudaMemsetAsync(uo, 0, cells * 8, st));
         }
     }
+    const bool wide = !lower && !use_smem && wide_block_chosen(ix, nq, flags);
+    if (wide) {
+        const int rc = wide_block_begin(ix, nq, P, st);
+        if (rc)
+            return rc;
+    }
     if (plain) {
         if (!sizes)
             return fail(KSSDGPU_ERR_ARG, "plain kernel needs host-side query sizes");
@@ -3009,14 +3150,20 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
         return unique ? launch_batched<false, true, true>(ix, P, smem, st)
                       : launch_batched<false, false, true>(ix, P, smem, st);
     }
-    if (striped) {
-        if (lower)
-            return launch_striped<true, false>(ix, P, st);
-        return unique ? launch_striped<false, true>(ix, P, st) : launch_striped<false, false>(ix, P, st);
-    }
-    if (lower)
-        return launch_batched<true, false, false>(ix, P, 0, st);
-    return unique ? launch_batched<false, true, false>(ix, P, 0, st) : launch_batched<false, false, false>(ix, P, 0, st);
+    int rc;
+    if (wide && striped)
+        rc = unique ? launch_striped<false, true, true>(ix, P, st) : launch_striped<false, false, true>(ix, P, st);
+    else if (wide)
+        rc = unique ? launch_batched<false, true, false, true>(ix, P, 0, st)
+                    : launch_batched<false, false, false, true>(ix, P, 0, st);
+    else if (striped)
+        rc = lower ? launch_striped<true, false>(ix, P, st)
+                   : unique ? launch_striped<false, true>(ix, P, st) : launch_striped<false, false>(ix, P, st);
+    else
+        rc = lower ? launch_batched<true, false, false>(ix, P, 0, st)
+                   : unique ? launch_batched<false, true, false>(ix, P, 0, st)
+                            : launch_batched<false, false, false>(ix, P, 0, st);
+    return rc || !wide ? rc : wide_block_end(ix, nq, oc, oo, st);
 }
 
 // A host-buffer count is split into sub-blocks whose copies overlap the counting when
@@ -3962,8 +4109,6 @@ uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 // the rows at or below them (the products are symmetric).
 constexpr uint64_t kWideSquare = 1536, kWideBlock = 512;
 
-uint64_t wide_pass(const kssdgpu_index *ix) { return std::min<uint64_t>(ix->f_wgroups, kWidePass); }
-
 // Device bytes of a wide self join: operand rows, Gram matrices, corrections.
 uint64_t wide_bytes(const kssdgpu_index *ix)
 {
@@ -3997,19 +4142,6 @@ double allele_ms(const kssdgpu_index *ix)
            (double)ix->f_alleles * ((ix->nref >= 700 ? 4.5 : 8.0) * n * n / 2.6e12 + 5 * n / 6e9);
 }
 
-// Room for `need` more bytes in half of the free device memory, `have` of which the index
-// holds already (no query of the free memory once it holds them all).
-bool dense_fits(uint64_t need, uint64_t have)
-{
-    if (need <= have)
-        return true;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return need <= free_b / 2;
-}
 bool wide_fits(const kssdgpu_index *ix)
 {
     return dense_fits(wide_bytes(ix), ix->w_x.cap + 4 * (uint64_t)ix->w_g.cap + 8 * (uint64_t)ix->w_corr.cap);
@@ -4032,7 +4164,7 @@ int dense_alleles_impl(kssdgpu_index *ix, uint32_t S, cudaStream_t st, uint32_t 
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, ix->d_poff.p, ix->d_allele.p, (int)S + 1, st));
     CUDA_TRY(ix->d_tmp.ensure(tb));
     CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned int), st));
-    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, 2, ix->d_list.p, d_count);
+    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, 2, ix->d_list.p, d_count, nullptr);
     // persistent CTAs over the groups: as many as fit on an SM at once (the group's
     // barriers and dependent loads leave one CTA mostly waiting)
     int per_sm_al = 0;
@@ -4086,19 +4218,15 @@ int self_wide_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long long
     CUDA_TRY(ix->d_ws.ensure(ws));
     CUDA_TRY(cudaMemsetAsync(ix->w_count.p, 0, sizeof(unsigned int), st));
     CUDA_TRY(cudaMemsetAsync(ix->w_corr.p, 0, cells * 8, st));
-    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->wide_min, ix->w_list.p, ix->w_count.p);
+    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->wide_min, ix->w_list.p, ix->w_count.p, nullptr);
     count_launch();
-    // warps of a CTA: as many as its shared memory holds, at most 8
-    const size_t per_warp = wide_warp_smem(npad, n);
-    const int warps = (int)std::min<size_t>(8, kWideSmem / per_warp);
-    CUDA_TRY(cudaFuncSetAttribute(k_wide_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(warps * per_warp)));
-    int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_rows, warps * 32, warps * per_warp));
+    int warps = 0, rows_grid = 0;
+    CUDA_TRY(wide_rows_shape(ix, k_wide_rows<false>, npad, warps, rows_grid));
     for (uint64_t c0 = 0; c0 < ix->f_wgroups; c0 += pass) {
         const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
-        const int grid = std::min<int>(ix->sms * std::max(1, per_sm), (int)((cn + warps - 1) / warps));
-        k_wide_rows<<<grid, warps * 32, warps * per_warp, st>>>(ix->w_list.p + c0, cn, ix->post, n, npad, ix->w_x.p, xs,
-                                                               ix->w_corr.p);
+        k_wide_rows<false><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
+                             warps * wide_warp_smem(npad, n), st>>>(ix->w_list.p + c0, cn, ix->post, n, npad,
+                                                                    ix->w_x.p, xs, ix->w_corr.p, WideBlock{});
         count_launch();
         CUDA_TRY(cudaGetLastError());
         for (uint64_t j = 0; j < npad; j += bw) {
@@ -4826,6 +4954,9 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     ix->w_corr.release();
     ix->w_count.release();
     ix->w_x.release();
+    ix->w_y.release();
+    ix->w_qobj.release();
+    ix->w_at.release();
     ix->w_g.release();
     delete ix;
 }

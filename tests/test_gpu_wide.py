@@ -78,3 +78,43 @@ def test_common_alleles_take_the_allele_rows():
     np.testing.assert_array_equal(got[1], want[1])
     assert idx.dense_alleles() == oracle_alleles(keys, 20)
     idx.close()
+
+
+@pytest.mark.parametrize("n,nq,contexts,unique", [(200, 101, 1500, False), (65, 304, 3000, True),
+                                                  (129, 129, 2100, False), (16, 2000, 900, True)])
+def test_wide_block(n, nq, contexts, unique):
+    """A block of queries against an index of wide groups, narrow groups and contexts of one
+    genome; every third query holds some contexts with several objects, one query is empty."""
+    keys, offs = _species(n, contexts, 0.9, 0.03, 20, 300 + n)
+    rng = np.random.default_rng(n)
+    samples = []
+    for i in range(n):  # contexts of few genomes beside the wide ones
+        k = keys[int(offs[i]):int(offs[i + 1])]
+        few = [((1 << 40) + int(c), int(o)) for c, o in zip(rng.integers(0, 60 * n, 40), rng.integers(0, 1 << 20, 40))]
+        samples.append([(int(x) >> 20, int(x) & 0xFFFFF) for x in k] + list(dict(few).items()))
+    keys, offs = samples_to_sketch(samples)
+    queries = []
+    for q in range(nq):
+        s = samples[int(rng.integers(0, n))]
+        pick = np.flatnonzero(rng.random(len(s)) < 0.8)
+        own = [(s[j][0], s[j][1] ^ (int(rng.integers(1, 4)) << 4) if rng.random() < 0.2 else s[j][1]) for j in pick]
+        if q % 3 == 0:
+            own += [(c, o ^ 1) for c, o in own[:50]]
+        queries.append([] if q == 5 else own)
+    qkeys, qoffs = samples_to_sketch(queries)
+    rec = oracle.build_index(keys, offs)
+    idx = kssdgpu.Index.from_records(rec, n)
+    flags = kssdgpu.UNIQUE if unique else 0
+    for more in (0, kssdgpu.IGNORECONFLICT):
+        want = oracle.count_block(rec, n, qkeys, qoffs, unique=unique, ignoreconflict=bool(more))
+        before = kssdgpu.launch_count()
+        walked = idx.count_block(qkeys, qoffs, flags | more | kssdgpu.GLOBAL_ACC)
+        plain = kssdgpu.launch_count() - before
+        for _ in range(2):
+            before = kssdgpu.launch_count()
+            got = idx.count_block(qkeys, qoffs, flags | more)
+            assert kssdgpu.launch_count() - before > plain  # the wide groups went to the tensor cores
+            for g, w, v in zip(got, want, walked):
+                np.testing.assert_array_equal(g, w)
+                np.testing.assert_array_equal(v, w)
+    idx.close()
