@@ -519,6 +519,12 @@ int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, 
                    const uint64_t *samp_recs, int nsamples, const kssdgpu_sketch_params_t *p, uint64_t *keys,
                    uint64_t keys_cap, uint64_t *offs);
 
+/* The same with every record in a buffer of its own: record r is the rec_offs[r + 1] -
+ * rec_offs[r] bytes at recs[r] (no copy of them back to back is needed). */
+int kssdgpu_sketch_records(const char *const *recs, const uint64_t *rec_offs, uint64_t nrec, const uint64_t *samp_recs,
+                           int nsamples, const kssdgpu_sketch_params_t *p, uint64_t *keys, uint64_t keys_cap,
+                           uint64_t *offs);
+
 /* Number of kernels launched by this library so far in this process. */
 uint64_t kssdgpu_launch_count(void);
 

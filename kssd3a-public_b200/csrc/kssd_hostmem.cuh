@@ -1,0 +1,290 @@
+// Host side of device memory: blocks kept between calls, and copies of pageable buffers
+// staged through page-locked chunks by several threads.  Included by kssdgpu.cu inside its
+// namespace.
+#pragma once
+
+// ------------------------------------------------------------------ device blocks
+//
+// An index build takes some twenty device arrays and gives half of them back before it
+// returns.  cudaMalloc and cudaFree of each cost 0.3 to 0.7 ms (1.3 ms at 1 GB, and many
+// times that on a host whose other processes allocate too), which was most of a small
+// index's build: 64 genomes 6.2 ms, of which kernels 0.3.  Freed blocks are kept instead
+// and handed out again for requests they fit.  Kept: at most kPoolKeep bytes a device,
+// blocks that two indexes in a row left unused are given back, and all of them when an
+// allocation fails.  (cudaMallocAsync's pool was measured too: 6 ms per 500 MB that its
+// reservation grows by.)
+constexpr uint64_t kPoolKeep = 2ull << 30;
+
+class DevicePool {
+public:
+    cudaError_t get(void **p, size_t bytes)
+    {
+        *p = nullptr;
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess)
+            return e;
+        // sizes in steps of an eighth of their power of two (at least 512 bytes), so that
+        // requests a little apart use one another's blocks
+        size_t step = 512;
+        while (step * 16 < bytes)
+            step <<= 1;
+        const size_t size = (std::max<size_t>(bytes, 1) + step - 1) / step * step;
+        try {
+            std::lock_guard<std::mutex> lock(mu_);
+            const auto it = idle_.lower_bound({dev, size});
+            if (it != idle_.end() && it->first.first == dev && it->first.second <= size + size / 4) {
+                live_.emplace(it->second.p, Live{it->first.second, dev});
+                *p = it->second.p;
+                idle_bytes_[dev] -= it->first.second;
+                idle_.erase(it);
+                return cudaSuccess;
+            }
+        } catch (const std::bad_alloc &) {
+            return cudaErrorMemoryAllocation;
+        }
+        e = cudaMalloc(p, size);
+        if (e == cudaErrorMemoryAllocation) {  // the kept blocks may be what is missing
+            cudaGetLastError();
+            release(dev, ~0ull);
+            e = cudaMalloc(p, size);
+            if (e == cudaErrorMemoryAllocation && size != bytes) {
+                cudaGetLastError();
+                e = cudaMalloc(p, std::max<size_t>(bytes, 1));
+            }
+        }
+        if (e == cudaSuccess) {
+            try {
+                std::lock_guard<std::mutex> lock(mu_);
+                live_.emplace(*p, Live{size, dev});
+            } catch (const std::bad_alloc &) {
+            }  // unknown to put(): freed there
+        }
+        return e;
+    }
+
+    // p: a block whose device work has ended (the caller synchronized).
+    void put(void *p)
+    {
+        if (!p)
+            return;
+        try {
+            std::lock_guard<std::mutex> lock(mu_);
+            const auto it = live_.find(p);
+            if (it != live_.end()) {
+                const Live b = it->second;
+                live_.erase(it);
+                if (idle_bytes_[b.dev] + b.bytes <= kPoolKeep) {
+                    idle_.emplace(std::make_pair(b.dev, b.bytes), Idle{p, epoch_});
+                    idle_bytes_[b.dev] += b.bytes;
+                    return;
+                }
+            }
+        } catch (const std::bad_alloc &) {
+        }
+        cudaFree(p);
+    }
+
+    // One index less: blocks of its device that two of them in a row did not use go back.
+    void age(int dev)
+    {
+        uint64_t now;
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            now = ++epoch_;
+        }
+        if (now > 2)
+            release(dev, now - 2);
+    }
+
+private:
+    struct Live {
+        size_t bytes;
+        int dev;
+    };
+    struct Idle {
+        void *p;
+        uint64_t epoch;
+    };
+
+    // Gives back the device's blocks kept since before epoch `until`.
+    void release(int dev, uint64_t until)
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (auto it = idle_.lower_bound({dev, 0}); it != idle_.end() && it->first.first == dev;) {
+            if (it->second.epoch < until) {
+                idle_bytes_[dev] -= it->first.second;
+                cudaFree(it->second.p);
+                it = idle_.erase(it);
+            } else {
+                ++it;
+            }
+        }
+    }
+
+    std::mutex mu_;
+    std::unordered_map<void *, Live> live_;
+    std::multimap<std::pair<int, size_t>, Idle> idle_;
+    std::map<int, uint64_t> idle_bytes_;
+    uint64_t epoch_ = 0;
+};
+
+// Never destroyed: at process exit the driver frees what it holds, in whatever order.
+DevicePool &device_pool()
+{
+    static DevicePool *pool = new DevicePool();
+    return *pool;
+}
+
+template <class T>
+cudaError_t pool_malloc(T **p, size_t bytes)
+{
+    return device_pool().get(reinterpret_cast<void **>(p), bytes);
+}
+// As cudaFree: waits for the device first.
+void pool_free(void *p)
+{
+    if (!p)
+        return;
+    cudaDeviceSynchronize();
+    device_pool().put(p);
+}
+// After a synchronization that covers every use of the block.
+void pool_free_idle(void *p) { device_pool().put(p); }
+
+// ------------------------------------------------------------------ staged copies
+//
+// A copy from or to pageable memory goes through the driver's own staging on one thread:
+// 11 GB/s at 98 MB here, 5 GB/s into pages not touched before, against 55 GB/s from
+// page-locked memory.  Copies of at least kStageMin bytes are cut into chunks that several
+// threads move between the caller's buffer and page-locked chunks of their own, the DMA of
+// one under the memcpy of the other.  The chunks (16 MB, page-locked on first use) belong to
+// the process; a second caller at the same time takes the driver's way.
+constexpr size_t kStageMin = 2u << 20, kStageChunk = 1u << 20;
+constexpr int kStageThreads = 8;
+
+class Stager {
+public:
+    // Copies `bytes` between device memory and a host buffer on `st`; chunk(host, off, len)
+    // moves one chunk to (IN) or from the page-locked chunk `host`.  false: not done here
+    // (busy, no memory, no threads).  On return the host buffer is free / filled.
+    template <bool IN, class Chunk>
+    bool run(char *dev_ptr, size_t bytes, cudaStream_t st, const Chunk &chunk, cudaError_t &err)
+    {
+        std::unique_lock<std::mutex> lock(mu_, std::try_to_lock);
+        if (!lock.owns_lock())
+            return false;
+        if (!pinned_ && cudaHostAlloc(&pinned_, kStageThreads * 2 * kStageChunk, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            pinned_ = nullptr;
+            return false;
+        }
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess)
+            return false;
+        const size_t chunks = (bytes + kStageChunk - 1) / kStageChunk;
+        const int threads = (int)std::min<size_t>(
+            {(size_t)kStageThreads, std::max<size_t>(1, std::thread::hardware_concurrency() / 2), (chunks + 1) / 2});
+        std::atomic<size_t> next{0};
+        std::atomic<int> bad{(int)cudaSuccess};
+        auto work = [&](int t) {
+            cudaError_t e = cudaSetDevice(dev);
+            cudaEvent_t ev[2] = {nullptr, nullptr};
+            for (int i = 0; i < 2 && e == cudaSuccess; ++i)
+                e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+            char *buf[2] = {(char *)pinned_ + (size_t)(2 * t) * kStageChunk,
+                            (char *)pinned_ + (size_t)(2 * t + 1) * kStageChunk};
+            size_t off[2] = {0, 0}, len[2] = {0, 0};  // len: a DMA of the slot is under way
+            for (int s = 0; e == cudaSuccess && bad.load() == (int)cudaSuccess; s ^= 1) {
+                if (len[s]) {  // the slot's last DMA
+                    e = cudaEventSynchronize(ev[s]);
+                    if (e == cudaSuccess && !IN)
+                        chunk(buf[s], off[s], len[s]);
+                    len[s] = 0;
+                }
+                const size_t c = e == cudaSuccess ? next.fetch_add(1) : chunks;
+                if (c >= chunks)
+                    break;
+                const size_t o = c * kStageChunk, n = std::min(kStageChunk, bytes - o);
+                if (IN)
+                    chunk(buf[s], o, n);
+                e = IN ? cudaMemcpyAsync(dev_ptr + o, buf[s], n, cudaMemcpyHostToDevice, st)
+                       : cudaMemcpyAsync(buf[s], dev_ptr + o, n, cudaMemcpyDeviceToHost, st);
+                if (e == cudaSuccess)
+                    e = cudaEventRecord(ev[s], st);
+                off[s] = o;
+                len[s] = n;
+            }
+            for (int s = 0; s < 2; ++s)
+                if (len[s]) {
+                    const cudaError_t e2 = cudaEventSynchronize(ev[s]);
+                    if (e2 == cudaSuccess && e == cudaSuccess && !IN)
+                        chunk(buf[s], off[s], len[s]);
+                    if (e == cudaSuccess)
+                        e = e2;
+                }
+            for (int i = 0; i < 2; ++i)
+                if (ev[i])
+                    cudaEventDestroy(ev[i]);
+            if (e != cudaSuccess)
+                bad.store((int)e);
+        };
+        std::vector<std::thread> team;
+        try {
+            team.reserve(threads);
+            for (int t = 1; t < threads; ++t)
+                team.emplace_back(work, t);
+        } catch (const std::exception &) {
+        }  // fewer threads: the others' chunks are this one's
+        work(0);
+        for (std::thread &t : team)
+            t.join();
+        err = (cudaError_t)bad.load();
+        return true;
+    }
+
+private:
+    std::mutex mu_;
+    void *pinned_ = nullptr;
+};
+
+Stager &stager()
+{
+    static Stager *s = new Stager();
+    return *s;
+}
+
+// Ordinary host memory (neither page-locked, managed nor of a device).
+bool host_pageable(const void *p)
+{
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+// Host buffer -> device on `st` (as cudaMemcpyAsync of a pageable buffer: the buffer may be
+// reused on return).
+cudaError_t upload(void *dst, const void *src, size_t bytes, cudaStream_t st)
+{
+    cudaError_t e = cudaSuccess;
+    if (bytes >= kStageMin && host_pageable(src) &&
+        stager().run<true>((char *)dst, bytes, st,
+                           [&](char *host, size_t off, size_t len) { memcpy(host, (const char *)src + off, len); }, e))
+        return e;
+    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st) : cudaSuccess;
+}
+
+// Device -> host buffer behind the work on `st`; a staged copy is complete on return, any
+// other when `st` has been synchronized.
+cudaError_t download(void *dst, const void *src, size_t bytes, cudaStream_t st)
+{
+    cudaError_t e = cudaSuccess;
+    if (bytes >= kStageMin && host_pageable(dst) &&
+        stager().run<false>((char *)const_cast<void *>(src), bytes, st,
+                            [&](char *host, size_t off, size_t len) { memcpy((char *)dst + off, host, len); }, e))
+        return e;
+    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st) : cudaSuccess;
+}

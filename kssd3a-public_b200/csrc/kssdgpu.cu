@@ -21,9 +21,13 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <new>
 #include <numeric>
 #include <string>
+#include <thread>
+#include <unordered_map>
 #include <vector>
 
 using namespace kssd;
@@ -52,6 +56,8 @@ int fail(int code, const std::string &msg)
             return fail(e_ == cudaErrorMemoryAllocation ? KSSDGPU_ERR_NOMEM : KSSDGPU_ERR_CUDA,   \
                         std::string(#expr) + ": " + cudaGetErrorString(e_));                        \
     } while (0)
+
+#include "kssd_hostmem.cuh"
 
 inline void count_launch(uint64_t n = 1) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
@@ -2340,18 +2346,23 @@ struct DevBuf {
         if (n <= cap && p)
             return cudaSuccess;
         if (p)
-            cudaFree(p);
+            pool_free(p);
         p = nullptr;
         cap = 0;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T));
+        cudaError_t e = pool_malloc(&p, std::max<size_t>(n, 1) * sizeof(T));
         if (e == cudaSuccess)
             cap = std::max<size_t>(n, 1);
         return e;
     }
     void release()
     {
-        if (p)
-            cudaFree(p);
+        pool_free(p);
+        p = nullptr;
+        cap = 0;
+    }
+    void release_idle()  // the device's work on it has ended
+    {
+        pool_free_idle(p);
         p = nullptr;
         cap = 0;
     }
@@ -2652,8 +2663,8 @@ namespace {
 // power of two (at most kMaxStripes) that keeps a stripe within stripe_bytes.
 int build_filter(kssdgpu_index *ix, uint64_t stripe_bytes, cudaStream_t st)
 {
-    cudaFree(ix->bloom);
-    cudaFree(ix->bloom_bounds);
+    pool_free(ix->bloom);
+    pool_free(ix->bloom_bounds);
     ix->bloom = nullptr;
     ix->bloom_bounds = nullptr;
     ix->bloom_stripes = 1;
@@ -2672,8 +2683,8 @@ int build_filter(kssdgpu_index *ix, uint64_t stripe_bytes, cudaStream_t st)
         stripes <<= 1;
     }
     const size_t fbytes = (size_t)stripes * blocks * 32;
-    CUDA_TRY(cudaMalloc(&ix->bloom, fbytes));
-    CUDA_TRY(cudaMalloc(&ix->bloom_bounds, (size_t)(stripes + 1) * sizeof(unsigned long long)));
+    CUDA_TRY(pool_malloc(&ix->bloom, fbytes));
+    CUDA_TRY(pool_malloc(&ix->bloom_bounds, (size_t)(stripes + 1) * sizeof(unsigned long long)));
     ix->bloom_stripes = stripes;
     ix->bloom_mask = (uint32_t)(blocks - 1);
     CUDA_TRY(cudaMemsetAsync(ix->bloom, 0, fbytes, st));
@@ -2689,11 +2700,11 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
 {
     const uint64_t n = ix->n;
     uint32_t *gidx = nullptr;
-    CUDA_TRY(cudaMalloc(&gidx, std::max<uint64_t>(n, 1) * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&gidx, std::max<uint64_t>(n, 1) * sizeof(uint32_t)));
     size_t tmp_bytes = 0;
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, head, gidx, (int64_t)n, st));
     void *tmp = nullptr;
-    CUDA_TRY(cudaMalloc(&tmp, std::max<size_t>(tmp_bytes, 1)));
+    CUDA_TRY(pool_malloc(&tmp, std::max<size_t>(tmp_bytes, 1)));
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, head, gidx, (int64_t)n, st));
     count_launch();
     uint32_t last_idx = 0, last_head = 0;
@@ -2703,15 +2714,15 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
     }
     CUDA_TRY(cudaStreamSynchronize(st));
     ix->u = n ? (uint64_t)last_idx + last_head : 0;
-    CUDA_TRY(cudaMalloc(&ix->gkey, std::max<uint64_t>(ix->u, 1) * sizeof(unsigned long long)));
-    CUDA_TRY(cudaMalloc(&ix->gbeg, (ix->u + 1) * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&ix->gkey, std::max<uint64_t>(ix->u, 1) * sizeof(unsigned long long)));
+    CUDA_TRY(pool_malloc(&ix->gbeg, (ix->u + 1) * sizeof(uint32_t)));
     k_scatter_groups<<<grid_for(n), 256, 0, st>>>(head, gidx, ctx_of, n, ix->gkey, ix->gbeg, ix->u);
     count_launch();
     uint64_t cap = 1024;
     while (cap < 2 * ix->u)
         cap <<= 1;
     ix->mask = (uint32_t)(cap - 1);
-    CUDA_TRY(cudaMalloc(&ix->table, cap * sizeof(Slot)));
+    CUDA_TRY(pool_malloc(&ix->table, cap * sizeof(Slot)));
     CUDA_TRY(cudaMemsetAsync(ix->table, 0xFF, cap * sizeof(Slot), st));
     k_table_insert<<<grid_for(ix->u), 256, 0, st>>>(ix->gkey, ix->gbeg, ix->u, ix->post, ix->table, ix->mask,
                                                      ix->err);
@@ -2722,15 +2733,15 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
             return frc;
     }
     CUDA_TRY(cudaStreamSynchronize(st));
-    cudaFree(tmp);
-    cudaFree(gidx);
+    pool_free_idle(tmp);
+    pool_free_idle(gidx);
     int herr = 0;
     CUDA_TRY(cudaMemcpy(&herr, ix->err, sizeof(int), cudaMemcpyDeviceToHost));
     if (!herr && ix->u) {
         // facts of the shared contexts (sizes of the self joins; the dense path's conditions)
         ix->wide_min = wide_min_postings(ix->nref);
         unsigned long long *d = nullptr, h[kStatFacts + 3] = {};
-        CUDA_TRY(cudaMalloc(&d, sizeof h));
+        CUDA_TRY(pool_malloc(&d, sizeof h));
         cudaError_t e = cudaMemsetAsync(d, 0, sizeof h, st);
         if (e == cudaSuccess) {
             k_self_stats<<<std::min(grid_for(ix->u), ix->sms * 8), 256, 0, st>>>(ix->gbeg, ix->u, ix->post,
@@ -2745,7 +2756,7 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof h, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        cudaFree(d);
+        pool_free_idle(d);
         if (e != cudaSuccess)
             return fail(KSSDGPU_ERR_CUDA, std::string("index facts: ") + cudaGetErrorString(e));
         ix->f_groups = h[0];
@@ -2791,13 +2802,13 @@ int new_index(int nref, int obj_bits, int device, uint64_t n, kssdgpu_index **ou
     ix->n = n;
     cudaDeviceGetAttribute(&ix->sms, cudaDevAttrMultiProcessorCount, device);
     cudaDeviceGetAttribute(&ix->l2_bytes, cudaDevAttrL2CacheSize, device);
-    cudaError_t e = cudaMalloc(&ix->err, sizeof(int));
+    cudaError_t e = pool_malloc(&ix->err, sizeof(int));
     if (e == cudaSuccess)
-        e = cudaMalloc(&ix->work, sizeof(unsigned int));
+        e = pool_malloc(&ix->work, sizeof(unsigned int));
     if (e == cudaSuccess)
         e = cudaMemset(ix->err, 0, sizeof(int));
     if (e == cudaSuccess)
-        e = cudaMalloc(&ix->post, std::max<uint64_t>(n, 1) * sizeof(uint64_t));
+        e = pool_malloc(&ix->post, std::max<uint64_t>(n, 1) * sizeof(uint64_t));
     if (e != cudaSuccess) {
         kssdgpu_index_free(ix);
         return fail(KSSDGPU_ERR_NOMEM, std::string("index allocation: ") + cudaGetErrorString(e));
@@ -3311,8 +3322,7 @@ int count_host_impl(kssdgpu_index *ix, const uint64_t *qkeys, const uint64_t *qo
     CUDA_TRY(ix->s_order.ensure((size_t)nq));
     CUDA_TRY(ix->s_items.ensure(items.size()));
     cudaStream_t st = 0;
-    if (nkeys)
-        CUDA_TRY(cudaMemcpyAsync(ix->s_keys.p, qkeys, nkeys * 8, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(upload(ix->s_keys.p, qkeys, nkeys * 8, st));
     CUDA_TRY(cudaMemcpyAsync(ix->s_offs.p, qoffs, ((size_t)nq + 1) * 8, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(ix->s_order.p, order.data(), (size_t)nq * sizeof(int), cudaMemcpyHostToDevice, st));
     if (!items.empty())
@@ -3324,11 +3334,11 @@ int count_host_impl(kssdgpu_index *ix, const uint64_t *qkeys, const uint64_t *qo
                             &sizes, st, items.empty() ? nullptr : ix->s_items.p, (int)items.size());
     if (rc)
         return rc;
-    CUDA_TRY(cudaMemcpyAsync(ctx, oc, cells * 8, cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(obj, oo, cells * 8, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(download(ctx, oc, cells * 8, st));
+    CUDA_TRY(download(obj, oo, cells * 8, st));
     if (unique) {
-        CUDA_TRY(cudaMemcpyAsync(uctx, uc, cells * 8, cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(uobj, uo, cells * 8, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(download(uctx, uc, cells * 8, st));
+        CUDA_TRY(download(uobj, uo, cells * 8, st));
     }
     return check_dev_err(ix, st);
 }
@@ -3624,19 +3634,19 @@ cudaError_t build_compact(kssdgpu_index *ix, uint32_t nitems, uint32_t *ntouched
     uint32_t *v1 = nullptr, *v2 = nullptr, *hd = nullptr, *inc = nullptr;
     void *tmp = nullptr;
     auto cleanup = [&]() {
-        cudaFree(k1); cudaFree(k2); cudaFree(v1); cudaFree(v2); cudaFree(hd); cudaFree(inc); cudaFree(tmp);
+        pool_free(k1); pool_free(k2); pool_free(v1); pool_free(v2); pool_free(hd); pool_free(inc); pool_free(tmp);
     };
     size_t tb1 = 0, tb2 = 0;
-    cudaError_t e = cudaMalloc(&k1, (size_t)nitems * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&k2, (size_t)nitems * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&v1, (size_t)nitems * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&v2, (size_t)nitems * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&hd, (size_t)nitems * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&inc, (size_t)nitems * 4);
+    cudaError_t e = pool_malloc(&k1, (size_t)nitems * 8);
+    if (e == cudaSuccess) e = pool_malloc(&k2, (size_t)nitems * 8);
+    if (e == cudaSuccess) e = pool_malloc(&v1, (size_t)nitems * 4);
+    if (e == cudaSuccess) e = pool_malloc(&v2, (size_t)nitems * 4);
+    if (e == cudaSuccess) e = pool_malloc(&hd, (size_t)nitems * 4);
+    if (e == cudaSuccess) e = pool_malloc(&inc, (size_t)nitems * 4);
     if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb1, k1, k2, v1, v2, nitems, 0, 64, st);
     if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, tb2, hd, inc, nitems, st);
     const size_t tb = std::max<size_t>(std::max(tb1, tb2), 1);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, tb);
+    if (e == cudaSuccess) e = pool_malloc(&tmp, tb);
     if (e == cudaSuccess) {
         k_item_cells<<<grid_for(nitems), 256, 0, st>>>(ix->j_items.p, nitems, ix->j_tile.p, k1, v1);
         count_launch();
@@ -3683,32 +3693,32 @@ cudaError_t set_major_plan(kssdgpu_index *ix, uint32_t n, cudaStream_t st)
     ulonglong2 *chunks0 = nullptr;
     void *tmp = nullptr;
     auto cleanup = [&]() {
-        cudaFree(heads); cudaFree(runs); cudaFree(first); cudaFree(cheads); cudaFree(cpos);
-        cudaFree(skey); cudaFree(skey2); cudaFree(sval); cudaFree(sval2); cudaFree(npairs); cudaFree(ioff);
-        cudaFree(f2d); cudaFree(twords); cudaFree(tword0); cudaFree(chunks0); cudaFree(tmp);
+        pool_free(heads); pool_free(runs); pool_free(first); pool_free(cheads); pool_free(cpos);
+        pool_free(skey); pool_free(skey2); pool_free(sval); pool_free(sval2); pool_free(npairs); pool_free(ioff);
+        pool_free(f2d); pool_free(twords); pool_free(tword0); pool_free(chunks0); pool_free(tmp);
     };
     size_t tb1 = 0, tb2 = 0, tb3 = 0, tb4 = 0;
-    cudaError_t e = cudaMalloc(&heads, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&f2d, (kFlatMax + 1) * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&runs, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&first, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&cheads, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&cpos, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&skey, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&skey2, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&sval, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&sval2, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&npairs, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&ioff, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&chunks0, (size_t)n * sizeof(ulonglong2));
-    if (e == cudaSuccess) e = cudaMalloc(&twords, (size_t)n * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&tword0, (size_t)n * 8);
+    cudaError_t e = pool_malloc(&heads, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&f2d, (kFlatMax + 1) * 4);
+    if (e == cudaSuccess) e = pool_malloc(&runs, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&first, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&cheads, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&cpos, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&skey, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&skey2, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&sval, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&sval2, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&npairs, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&ioff, (size_t)n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&chunks0, (size_t)n * sizeof(ulonglong2));
+    if (e == cudaSuccess) e = pool_malloc(&twords, (size_t)n * 8);
+    if (e == cudaSuccess) e = pool_malloc(&tword0, (size_t)n * 8);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb4, twords, tword0, n, st);
     if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, tb1, heads, runs, n, st);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb2, cheads, cpos, n, st);
     if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb3, skey, skey2, sval, sval2, n, 0, 16, st);
     const size_t tb = std::max<size_t>(std::max(std::max(tb1, tb2), std::max(tb3, tb4)), 1);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, tb);
+    if (e == cudaSuccess) e = pool_malloc(&tmp, tb);
     if (e == cudaSuccess) {
         k_set_heads<<<grid_for(n), 256, 0, st>>>(ix->j_small.p, n, ix->j_post.p, heads);
         count_launch();
@@ -3875,9 +3885,9 @@ cudaError_t tune_join(kssdgpu_index *ix, uint32_t n, cudaStream_t st)
     unsigned long long *oc = nullptr, *oo = nullptr;
     void *flush = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    e = cudaMalloc(&oc, cells * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&oo, cells * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&flush, flush_b);
+    e = pool_malloc(&oc, cells * 8);
+    if (e == cudaSuccess) e = pool_malloc(&oo, cells * 8);
+    if (e == cudaSuccess) e = pool_malloc(&flush, flush_b);
     if (e == cudaSuccess) e = cudaEventCreate(&ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&ev1);
     float best = 1e30f;
@@ -3921,9 +3931,9 @@ cudaError_t tune_join(kssdgpu_index *ix, uint32_t n, cudaStream_t st)
     for (const auto &cand : kChunkCands)
         if (e == cudaSuccess)
             time_plan(cand.size, cand.sorted, flat_at);
-    cudaFree(oc);
-    cudaFree(oo);
-    cudaFree(flush);
+    pool_free(oc);
+    pool_free(oo);
+    pool_free(flush);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (e != cudaSuccess)
@@ -3950,13 +3960,13 @@ int self_plan(kssdgpu_index *ix, cudaStream_t st)
     unsigned long long *tot = nullptr;
     void *tmp = nullptr;
     auto cleanup = [&]() {
-        cudaFree(skey); cudaFree(skey2); cudaFree(sval); cudaFree(sval2);
-        cudaFree(ks); cudaFree(offs); cudaFree(cnt); cudaFree(tot); cudaFree(tmp);
+        pool_free(skey); pool_free(skey2); pool_free(sval); pool_free(sval2);
+        pool_free(ks); pool_free(offs); pool_free(cnt); pool_free(tot); pool_free(tmp);
     };
-    cudaError_t e = cudaMalloc(&skey, cap * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&sval, cap * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&cnt, 3 * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMalloc(&tot, 2 * sizeof(unsigned long long));
+    cudaError_t e = pool_malloc(&skey, cap * 8);
+    if (e == cudaSuccess) e = pool_malloc(&sval, cap * 4);
+    if (e == cudaSuccess) e = pool_malloc(&cnt, 3 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = pool_malloc(&tot, 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(tot, 0, 2 * sizeof(unsigned long long), st);
     if (e != cudaSuccess) {
@@ -3976,14 +3986,14 @@ int self_plan(kssdgpu_index *ix, cudaStream_t st)
     const uint32_t n = e == cudaSuccess ? hc[0] : 0;
     // small groups: sort by (size desc, leading gids), then lay their postings out contiguously
     if (e == cudaSuccess && n) {
-        e = cudaMalloc(&skey2, (size_t)n * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&sval2, (size_t)n * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&ks, (size_t)n * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&offs, (size_t)n * 4);
+        e = pool_malloc(&skey2, (size_t)n * 8);
+        if (e == cudaSuccess) e = pool_malloc(&sval2, (size_t)n * 4);
+        if (e == cudaSuccess) e = pool_malloc(&ks, (size_t)n * 4);
+        if (e == cudaSuccess) e = pool_malloc(&offs, (size_t)n * 4);
         size_t tb = 0, tb2 = 0;
         if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(nullptr, tb, skey, skey2, sval, sval2, n, 0, 64, st);
         if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tb2, ks, offs, n, st);
-        if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max<size_t>(std::max(tb, tb2), 1));
+        if (e == cudaSuccess) e = pool_malloc(&tmp, std::max<size_t>(std::max(tb, tb2), 1));
         if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(tmp, tb, skey, skey2, sval, sval2, n, 0, 64, st);
         count_launch(8);
         if (e == cudaSuccess) {
@@ -4545,12 +4555,12 @@ static int metric_params(int device, const kssdgpu_metric_opt_t *o, kssd::Metric
     HgbDeviceModel &m = g_hgb[device];
     if (m.host_nodes != o->hgb_nodes || m.nodes != o->hgb_nodes_count || m.trees != o->hgb_trees) {
         if (m.d_nodes)
-            cudaFree(m.d_nodes);
+            pool_free(m.d_nodes);
         if (m.d_begin)
-            cudaFree(m.d_begin);
+            pool_free(m.d_begin);
         m = HgbDeviceModel{};
-        CUDA_TRY(cudaMalloc(&m.d_nodes, (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode)));
-        CUDA_TRY(cudaMalloc(&m.d_begin, ((size_t)o->hgb_trees + 1) * sizeof(uint32_t)));
+        CUDA_TRY(pool_malloc(&m.d_nodes, (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode)));
+        CUDA_TRY(pool_malloc(&m.d_begin, ((size_t)o->hgb_trees + 1) * sizeof(uint32_t)));
         CUDA_TRY(cudaMemcpy(m.d_nodes, o->hgb_nodes, (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode),
                             cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(m.d_begin, o->hgb_tree_begin, ((size_t)o->hgb_trees + 1) * sizeof(uint32_t),
@@ -4639,11 +4649,16 @@ uint32_t kssdgpu_sketch_hash_id(const kssdgpu_sketch_params_t *p)
     return h;
 }
 
-int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, uint64_t nrec,
-                   const uint64_t *samp_recs, int nsamples, const kssdgpu_sketch_params_t *p, uint64_t *keys,
-                   uint64_t keys_cap, uint64_t *offs)
+}  // extern "C"
+
+// The two sketch entry points: copy_in(device buffer, stream) uploads the records' bytes
+// back to back (called once, after the arguments have been checked).
+template <class CopyIn>
+static int sketch_impl(const CopyIn &copy_in, bool have_seq, uint64_t seq_len, const uint64_t *rec_offs, uint64_t nrec,
+                       const uint64_t *samp_recs, int nsamples, const kssdgpu_sketch_params_t *p, uint64_t *keys,
+                       uint64_t keys_cap, uint64_t *offs)
 {
-    if (!p || !offs || nsamples < 0 || (nrec && !rec_offs) || (nsamples && !samp_recs) || (seq_len && !seq))
+    if (!p || !offs || nsamples < 0 || (nrec && !rec_offs) || (nsamples && !samp_recs) || (seq_len && !have_seq))
         return fail(KSSDGPU_ERR_ARG, "invalid sketch arguments");
     uint64_t cm = 0, tm = 0;
     int ob = 0;
@@ -4691,19 +4706,21 @@ int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, 
         int *nsel = nullptr;
         ~Bufs()
         {
-            cudaFree(seq); cudaFree(rec); cudaFree(samp); cudaFree(counts); cudaFree(pos); cudaFree(scounts);
-            cudaFree(seg); cudaFree(kept); cudaFree(k0); cudaFree(k1); cudaFree(keep); cudaFree(tmp); cudaFree(nsel);
+            cudaStreamSynchronize(nullptr);  // an error may have left work behind
+            for (void *p : {(void *)seq, (void *)rec, (void *)samp, (void *)counts, (void *)pos, (void *)scounts,
+                            (void *)seg, (void *)kept, (void *)k0, (void *)k1, (void *)keep, tmp, (void *)nsel})
+                pool_free_idle(p);
         }
     } b;
-    CUDA_TRY(cudaMalloc(&b.seq, seq_len));
-    CUDA_TRY(cudaMalloc(&b.rec, (nrec + 1) * sizeof(uint64_t)));
-    CUDA_TRY(cudaMalloc(&b.samp, ((size_t)nsamples + 1) * sizeof(uint64_t)));
-    CUDA_TRY(cudaMalloc(&b.counts, nthreads * sizeof(uint32_t)));
-    CUDA_TRY(cudaMalloc(&b.pos, (nthreads + 1) * sizeof(uint32_t)));
-    CUDA_TRY(cudaMalloc(&b.scounts, ((size_t)nsamples + 1) * sizeof(uint32_t)));
-    CUDA_TRY(cudaMalloc(&b.seg, ((size_t)nsamples + 1) * sizeof(uint32_t)));
-    CUDA_TRY(cudaMalloc(&b.kept, ((size_t)nsamples + 1) * sizeof(uint32_t)));
-    CUDA_TRY(cudaMemcpyAsync(b.seq, seq, seq_len, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(pool_malloc(&b.seq, seq_len));
+    CUDA_TRY(pool_malloc(&b.rec, (nrec + 1) * sizeof(uint64_t)));
+    CUDA_TRY(pool_malloc(&b.samp, ((size_t)nsamples + 1) * sizeof(uint64_t)));
+    CUDA_TRY(pool_malloc(&b.counts, nthreads * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&b.pos, (nthreads + 1) * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&b.scounts, ((size_t)nsamples + 1) * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&b.seg, ((size_t)nsamples + 1) * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&b.kept, ((size_t)nsamples + 1) * sizeof(uint32_t)));
+    CUDA_TRY(copy_in(b.seq, st));
     CUDA_TRY(cudaMemcpyAsync(b.rec, rec_offs, (nrec + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(b.samp, samp_recs, ((size_t)nsamples + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemsetAsync(b.scounts, 0, ((size_t)nsamples + 1) * sizeof(uint32_t), st));
@@ -4716,7 +4733,7 @@ int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, 
     size_t tb0 = 0, tb1 = 0, tb2 = 0, tb3 = 0;
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb0, b.counts, b.pos, (int64_t)nthreads, st));
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb1, b.scounts, b.seg, nsamples + 1, st));
-    CUDA_TRY(cudaMalloc(&b.tmp, std::max(tb0, tb1)));
+    CUDA_TRY(pool_malloc(&b.tmp, std::max(tb0, tb1)));
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(b.tmp, tb0, b.counts, b.pos, (int64_t)nthreads, st));
     CUDA_TRY(cub::DeviceScan::ExclusiveSum(b.tmp, tb1, b.scounts, b.seg, nsamples + 1, st));
     count_launch(2);
@@ -4725,10 +4742,10 @@ int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, 
     CUDA_TRY(cudaStreamSynchronize(st));
     if (total == 0)
         return KSSDGPU_OK;
-    CUDA_TRY(cudaMalloc(&b.k0, (size_t)total * sizeof(unsigned long long)));
-    CUDA_TRY(cudaMalloc(&b.k1, (size_t)total * sizeof(unsigned long long)));
-    CUDA_TRY(cudaMalloc(&b.keep, total));
-    CUDA_TRY(cudaMalloc(&b.nsel, sizeof(int)));
+    CUDA_TRY(pool_malloc(&b.k0, (size_t)total * sizeof(unsigned long long)));
+    CUDA_TRY(pool_malloc(&b.k1, (size_t)total * sizeof(unsigned long long)));
+    CUDA_TRY(pool_malloc(&b.keep, total));
+    CUDA_TRY(pool_malloc(&b.nsel, sizeof(int)));
     k_sketch_scan<true><<<(unsigned)nblocks, kSketchThreads, 0, st>>>(b.seq, seq_len, b.rec, nrec, b.samp, nsamples, g,
                                                                       nullptr, nullptr, b.pos, b.k0);
     count_launch();
@@ -4738,9 +4755,9 @@ int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, 
                                                 b.seg + 1, st));
     CUDA_TRY(cub::DeviceSelect::Flagged(nullptr, tb3, b.k1, b.keep, b.k0, b.nsel, (int64_t)total, st));
     if (std::max(tb2, tb3) > std::max(tb0, tb1)) {
-        cudaFree(b.tmp);
+        pool_free(b.tmp);
         b.tmp = nullptr;
-        CUDA_TRY(cudaMalloc(&b.tmp, std::max(tb2, tb3)));
+        CUDA_TRY(pool_malloc(&b.tmp, std::max(tb2, tb3)));
     }
     CUDA_TRY(cub::DeviceSegmentedSort::SortKeys(b.tmp, tb2, b.k0, b.k1, (int64_t)total, nsamples, b.seg, b.seg + 1,
                                                 st));
@@ -4765,6 +4782,49 @@ int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, 
 }
 
 
+extern "C" {
+
+int kssdgpu_sketch(const char *seq, uint64_t seq_len, const uint64_t *rec_offs, uint64_t nrec,
+                   const uint64_t *samp_recs, int nsamples, const kssdgpu_sketch_params_t *p, uint64_t *keys,
+                   uint64_t keys_cap, uint64_t *offs)
+{
+    return sketch_impl([&](void *d, cudaStream_t st) { return upload(d, seq, seq_len, st); }, seq != nullptr, seq_len,
+                       rec_offs, nrec, samp_recs, nsamples, p, keys, keys_cap, offs);
+}
+
+int kssdgpu_sketch_records(const char *const *recs, const uint64_t *rec_offs, uint64_t nrec, const uint64_t *samp_recs,
+                           int nsamples, const kssdgpu_sketch_params_t *p, uint64_t *keys, uint64_t keys_cap,
+                           uint64_t *offs)
+{
+    const uint64_t seq_len = nrec && rec_offs ? rec_offs[nrec] : 0;
+    auto gather = [&](char *to, size_t off, size_t len) {
+        uint64_t r = (uint64_t)(std::upper_bound(rec_offs, rec_offs + nrec + 1, (uint64_t)off) - rec_offs) - 1;
+        while (len) {
+            const size_t in = off - rec_offs[r], n = std::min<size_t>(len, rec_offs[r + 1] - off);
+            if (n)
+                memcpy(to, recs[r] + in, n);
+            to += n;
+            off += n;
+            len -= n;
+            ++r;
+        }
+    };
+    auto copy_in = [&](void *d, cudaStream_t st) {
+        cudaError_t e = cudaSuccess;
+        if (seq_len >= kStageMin && stager().run<true>((char *)d, seq_len, st, gather, e))
+            return e;
+        for (uint64_t r = 0; r < nrec && e == cudaSuccess; ++r)
+            if (rec_offs[r + 1] > rec_offs[r])
+                e = cudaMemcpyAsync((char *)d + rec_offs[r], recs[r], rec_offs[r + 1] - rec_offs[r],
+                                    cudaMemcpyHostToDevice, st);
+        return e;
+    };
+    for (uint64_t r = 0; r < nrec; ++r)
+        if (recs && rec_offs && rec_offs[r + 1] > rec_offs[r] && !recs[r])
+            return fail(KSSDGPU_ERR_ARG, "null sketch record");
+    return sketch_impl(copy_in, recs != nullptr, seq_len, rec_offs, nrec, samp_recs, nsamples, p, keys, keys_cap, offs);
+}
+
 int kssdgpu_index_from_records(const void *records12, uint64_t n, int nref, int obj_bits, int device,
                                kssdgpu_index_t **out)
 {
@@ -4778,17 +4838,18 @@ int kssdgpu_index_from_records(const void *records12, uint64_t n, int nref, int 
     uint32_t *w = nullptr, *head = nullptr;
     unsigned long long *ctx_of = nullptr;
     auto cleanup = [&]() {
-        cudaFree(w);
-        cudaFree(head);
-        cudaFree(ctx_of);
+        cudaStreamSynchronize(st);  // an error may have left work behind
+        pool_free_idle(w);
+        pool_free_idle(head);
+        pool_free_idle(ctx_of);
     };
-    cudaError_t e = cudaMalloc(&w, std::max<uint64_t>(n, 1) * 12);
+    cudaError_t e = pool_malloc(&w, std::max<uint64_t>(n, 1) * 12);
     if (e == cudaSuccess)
-        e = cudaMalloc(&head, std::max<uint64_t>(n, 1) * 4);
+        e = pool_malloc(&head, std::max<uint64_t>(n, 1) * 4);
     if (e == cudaSuccess)
-        e = cudaMalloc(&ctx_of, std::max<uint64_t>(n, 1) * 8);
+        e = pool_malloc(&ctx_of, std::max<uint64_t>(n, 1) * 8);
     if (e == cudaSuccess && n)
-        e = cudaMemcpyAsync(w, records12, n * 12, cudaMemcpyHostToDevice, st);
+        e = upload(w, records12, n * 12, st);
     if (e != cudaSuccess) {
         cleanup();
         kssdgpu_index_free(ix);
@@ -4828,26 +4889,27 @@ int kssdgpu_index_from_sketch(const uint64_t *keys, const uint64_t *offs, int nr
     uint32_t *sval = nullptr, *sval2 = nullptr, *head = nullptr;
     void *tmp = nullptr;
     auto cleanup = [&]() {
-        cudaFree(dk);
-        cudaFree(doffs);
-        cudaFree(skey);
-        cudaFree(skey2);
-        cudaFree(ctx_of);
-        cudaFree(sval);
-        cudaFree(sval2);
-        cudaFree(head);
-        cudaFree(tmp);
+        cudaStreamSynchronize(st);  // an error may have left work behind
+        pool_free_idle(dk);
+        pool_free_idle(doffs);
+        pool_free_idle(skey);
+        pool_free_idle(skey2);
+        pool_free_idle(ctx_of);
+        pool_free_idle(sval);
+        pool_free_idle(sval2);
+        pool_free_idle(head);
+        pool_free_idle(tmp);
     };
     const uint64_t nn = std::max<uint64_t>(n, 1);
-    cudaError_t e = cudaMalloc(&dk, nn * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&doffs, ((uint64_t)nref + 1) * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&skey, nn * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&skey2, nn * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&sval, nn * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&sval2, nn * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&head, nn * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&ctx_of, nn * 8);
-    if (e == cudaSuccess && n) e = cudaMemcpyAsync(dk, keys, n * 8, cudaMemcpyHostToDevice, st);
+    cudaError_t e = pool_malloc(&dk, nn * 8);
+    if (e == cudaSuccess) e = pool_malloc(&doffs, ((uint64_t)nref + 1) * 8);
+    if (e == cudaSuccess) e = pool_malloc(&skey, nn * 8);
+    if (e == cudaSuccess) e = pool_malloc(&skey2, nn * 8);
+    if (e == cudaSuccess) e = pool_malloc(&sval, nn * 4);
+    if (e == cudaSuccess) e = pool_malloc(&sval2, nn * 4);
+    if (e == cudaSuccess) e = pool_malloc(&head, nn * 4);
+    if (e == cudaSuccess) e = pool_malloc(&ctx_of, nn * 8);
+    if (e == cudaSuccess && n) e = upload(dk, keys, n * 8, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(doffs, offs, ((uint64_t)nref + 1) * 8, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) {
         cleanup();
@@ -4862,7 +4924,7 @@ int kssdgpu_index_from_sketch(const uint64_t *keys, const uint64_t *offs, int nr
         int end_bit = 64;
         size_t tb = 0;
         e = cub::DeviceRadixSort::SortPairs(nullptr, tb, skey, skey2, sval, sval2, (int64_t)n, 0, end_bit, st);
-        if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max<size_t>(tb, 1));
+        if (e == cudaSuccess) e = pool_malloc(&tmp, std::max<size_t>(tb, 1));
         if (e == cudaSuccess)
             e = cub::DeviceRadixSort::SortPairs(tmp, tb, skey, skey2, sval, sval2, (int64_t)n, 0, end_bit, st);
         count_launch(4);
@@ -4889,75 +4951,77 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     if (!ix)
         return;
     cudaSetDevice(ix->device);
-    cudaFree(ix->post);
-    cudaFree(ix->gkey);
-    cudaFree(ix->gbeg);
-    cudaFree(ix->table);
-    cudaFree(ix->bloom);
-    cudaFree(ix->bloom_bounds);
-    cudaFree(ix->err);
-    cudaFree(ix->work);
-    ix->s_keys.release();
-    ix->s_offs.release();
-    ix->s_out.release();
-    ix->s_order.release();
-    ix->s_items.release();
-    ix->s_prefix.release();
-    ix->s_spos.release();
-    ix->s_scnt.release();
-    ix->s_spre.release();
-    ix->s_sitems.release();
+    cudaDeviceSynchronize();
+    pool_free_idle(ix->post);
+    pool_free_idle(ix->gkey);
+    pool_free_idle(ix->gbeg);
+    pool_free_idle(ix->table);
+    pool_free_idle(ix->bloom);
+    pool_free_idle(ix->bloom_bounds);
+    pool_free_idle(ix->err);
+    pool_free_idle(ix->work);
+    ix->s_keys.release_idle();
+    ix->s_offs.release_idle();
+    ix->s_out.release_idle();
+    ix->s_order.release_idle();
+    ix->s_items.release_idle();
+    ix->s_prefix.release_idle();
+    ix->s_spos.release_idle();
+    ix->s_scnt.release_idle();
+    ix->s_spre.release_idle();
+    ix->s_sitems.release_idle();
     for (int i = 0; i < 3; ++i)
         if (ix->pipe_st[i])
             cudaStreamDestroy(ix->pipe_st[i]);
     for (cudaEvent_t e : ix->pipe_ev)
         cudaEventDestroy(e);
     ix->pipe_ev.clear();
-    ix->s_counts.release();
-    ix->s_cubtmp.release();
-    ix->j_small.release();
-    ix->c_key.release();
-    ix->c_acc.release();
-    ix->m_val.release();
-    ix->m_recheck.release();
-    ix->m_nrecheck.release();
-    ix->j_post.release();
-    ix->j_chunks.release();
-    ix->j_items.release();
-    ix->j_tile.release();
-    ix->j_islot.release();
-    ix->j_touched.release();
-    ix->j_cacc.release();
+    ix->s_counts.release_idle();
+    ix->s_cubtmp.release_idle();
+    ix->j_small.release_idle();
+    ix->c_key.release_idle();
+    ix->c_acc.release_idle();
+    ix->m_val.release_idle();
+    ix->m_recheck.release_idle();
+    ix->m_nrecheck.release_idle();
+    ix->j_post.release_idle();
+    ix->j_chunks.release_idle();
+    ix->j_items.release_idle();
+    ix->j_tile.release_idle();
+    ix->j_islot.release_idle();
+    ix->j_touched.release_idle();
+    ix->j_cacc.release_idle();
     if (ix->j_fill_st)
         cudaStreamDestroy(ix->j_fill_st);
     for (cudaEvent_t e : ix->j_fill_ev)
         if (e)
             cudaEventDestroy(e);
-    ix->j_fheads.release();
-    ix->j_big.release();
-    ix->j_conf.release();
-    ix->s_qcnt.release();
-    ix->s_rcnt.release();
-    ix->s_dcount.release();
-    ix->s_dprefix.release();
-    ix->s_hits.release();
-    ix->d_list.release();
-    ix->d_poff.release();
-    ix->d_allele.release();
-    ix->d_aval.release();
-    ix->d_a.release();
-    ix->d_f.release();
-    ix->d_d.release();
-    ix->d_tmp.release();
-    ix->d_ws.release();
-    ix->w_list.release();
-    ix->w_corr.release();
-    ix->w_count.release();
-    ix->w_x.release();
-    ix->w_y.release();
-    ix->w_qobj.release();
-    ix->w_at.release();
-    ix->w_g.release();
+    ix->j_fheads.release_idle();
+    ix->j_big.release_idle();
+    ix->j_conf.release_idle();
+    ix->s_qcnt.release_idle();
+    ix->s_rcnt.release_idle();
+    ix->s_dcount.release_idle();
+    ix->s_dprefix.release_idle();
+    ix->s_hits.release_idle();
+    ix->d_list.release_idle();
+    ix->d_poff.release_idle();
+    ix->d_allele.release_idle();
+    ix->d_aval.release_idle();
+    ix->d_a.release_idle();
+    ix->d_f.release_idle();
+    ix->d_d.release_idle();
+    ix->d_tmp.release_idle();
+    ix->d_ws.release_idle();
+    ix->w_list.release_idle();
+    ix->w_corr.release_idle();
+    ix->w_count.release_idle();
+    ix->w_x.release_idle();
+    ix->w_y.release_idle();
+    ix->w_qobj.release_idle();
+    ix->w_at.release_idle();
+    ix->w_g.release_idle();
+    device_pool().age(ix->device);
     delete ix;
 }
 
@@ -5002,24 +5066,24 @@ int kssdgpu_index_export(const kssdgpu_index_t *cix, void *records12, uint8_t *u
     const uint64_t n = ix->n;
     if (records12 && n) {
         uint32_t *w = nullptr;
-        CUDA_TRY(cudaMalloc(&w, n * 12));
+        CUDA_TRY(pool_malloc(&w, n * 12));
         k_export_records<<<grid_for(ix->u), 256, 0, st>>>(ix->gkey, ix->gbeg, ix->u, ix->post, w);
         count_launch();
-        CUDA_TRY(cudaMemcpyAsync(records12, w, n * 12, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(download(records12, w, n * 12, st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        cudaFree(w);
+        pool_free(w);
     }
     if (unique_bits && n) {
         const uint64_t words = (n + 31) / 32;
         uint32_t *b = nullptr;
-        CUDA_TRY(cudaMalloc(&b, words * 4));
+        CUDA_TRY(pool_malloc(&b, words * 4));
         CUDA_TRY(cudaMemsetAsync(b, 0, words * 4, st));
         k_unique_bits<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->post, b);
         count_launch();
         std::vector<uint32_t> hb(words);
         CUDA_TRY(cudaMemcpyAsync(hb.data(), b, words * 4, cudaMemcpyDeviceToHost, st));
         CUDA_TRY(cudaStreamSynchronize(st));
-        cudaFree(b);
+        pool_free(b);
         std::memcpy(unique_bits, hb.data(), (n + 7) / 8);
     }
     return KSSDGPU_OK;
@@ -5034,7 +5098,7 @@ int kssdgpu_index_ref_ctx_counts(const kssdgpu_index_t *cix, int conflict, int i
     CUDA_TRY(cudaSetDevice(ix->device));
     cudaStream_t st = 0;
     uint32_t *c = nullptr;
-    CUDA_TRY(cudaMalloc(&c, (size_t)ix->nref * 2 * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&c, (size_t)ix->nref * 2 * sizeof(uint32_t)));
     CUDA_TRY(cudaMemsetAsync(c, 0, (size_t)ix->nref * 2 * sizeof(uint32_t), st));
     k_ref_counts<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->post, conflict, ignoreconflict, c, c + ix->nref);
     count_launch();
@@ -5043,7 +5107,7 @@ int kssdgpu_index_ref_ctx_counts(const kssdgpu_index_t *cix, int conflict, int i
     if (unique_out)
         CUDA_TRY(cudaMemcpyAsync(unique_out, c + ix->nref, (size_t)ix->nref * 4, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
-    cudaFree(c);
+    pool_free(c);
     return KSSDGPU_OK;
 }
 
@@ -5338,8 +5402,7 @@ int kssdgpu_count_detail(kssdgpu_index_t *ix, const uint64_t *qry_keys, const ui
     CUDA_TRY(ix->s_dcount.ensure((size_t)nq));
     CUDA_TRY(ix->s_dprefix.ensure((size_t)nq + 1));
     cudaStream_t st = 0;
-    if (nkeys)
-        CUDA_TRY(cudaMemcpyAsync(ix->s_keys.p, qry_keys, nkeys * 8, cudaMemcpyHostToDevice, st));
+    CUDA_TRY(upload(ix->s_keys.p, qry_keys, nkeys * 8, st));
     CUDA_TRY(cudaMemcpyAsync(ix->s_offs.p, qry_offs, ((size_t)nq + 1) * 8, cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(ix->s_order.p, order.data(), (size_t)nq * sizeof(int), cudaMemcpyHostToDevice, st));
     if (!items.empty())
@@ -5382,7 +5445,7 @@ int kssdgpu_count_detail(kssdgpu_index_t *ix, const uint64_t *qry_keys, const ui
     k_detail_write<<<grid, 256, 0, st>>>(oc, oo, uc, uo, nq, nref, F, ix->s_dprefix.p, ix->s_hits.p);
     count_launch();
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(hits, ix->s_hits.p, total * sizeof(kssdgpu_hit_t), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(download(hits, ix->s_hits.p, total * sizeof(kssdgpu_hit_t), st));
     CUDA_TRY(cudaStreamSynchronize(st));
     return KSSDGPU_OK;
 }
@@ -5478,8 +5541,8 @@ int kssdgpu_self_lower(kssdgpu_index_t *ix, unsigned flags, kssdgpu_ctx_mut2_t *
     if (rc)
         return rc;
     if (cells) {
-        CUDA_TRY(cudaMemcpyAsync(ctx_lower, ix->s_out.p, cells * 8, cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(obj_lower, ix->s_out.p + cells, cells * 8, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(download(ctx_lower, ix->s_out.p, cells * 8, st));
+        CUDA_TRY(download(obj_lower, ix->s_out.p + cells, cells * 8, st));
     }
     return check_dev_err(ix, st);
 }
@@ -5504,11 +5567,10 @@ int kssdgpu_self_votes(kssdgpu_index_t *ix, const uint64_t *keys, const uint64_t
     CUDA_TRY(ix->s_keys.ensure(nkeys));
     CUDA_TRY(ix->s_offs.ensure((size_t)n + 1));
     uint32_t *d = nullptr;
-    cudaError_t e = cudaMalloc(&d, cells * 8);
+    cudaError_t e = pool_malloc(&d, cells * 8);
     if (e != cudaSuccess)
         return fail(KSSDGPU_ERR_NOMEM, std::string("vote counters: ") + cudaGetErrorString(e));
-    if (nkeys)
-        e = cudaMemcpyAsync(ix->s_keys.p, keys, nkeys * 8, cudaMemcpyHostToDevice, st);
+    e = upload(ix->s_keys.p, keys, nkeys * 8, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ix->s_offs.p, offs, ((size_t)n + 1) * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, cells * 4, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d + cells, 0xFF, cells * 4, st);
@@ -5518,10 +5580,10 @@ int kssdgpu_self_votes(kssdgpu_index_t *ix, const uint64_t *keys, const uint64_t
         count_launch();
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(votes, d, cells * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(first, d + cells, cells * 4, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = download(votes, d, cells * 4, st);
+    if (e == cudaSuccess) e = download(first, d + cells, cells * 4, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d);
+    pool_free(d);
     if (e != cudaSuccess)
         return fail(KSSDGPU_ERR_CUDA, cudaGetErrorString(e));
     return check_dev_err(ix, st);
@@ -5595,7 +5657,7 @@ int kssdgpu_self_lower_metric(kssdgpu_index_t *ix, unsigned flags, const kssdgpu
     CUDA_TRY(kssd::lower_metric_launch(P, n, ix->s_out.p, ix->s_out.p + cells, ix->s_qcnt.p, ix->s_rcnt.p,
                                        ix->m_val.p, ix->m_recheck.p, recheck_cap, ix->m_nrecheck.p, ix->sms, st));
     count_launch();
-    CUDA_TRY(cudaMemcpyAsync(value_lower, ix->m_val.p, cells * 8, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(download(value_lower, ix->m_val.p, cells * 8, st));
     unsigned long long nre = 0;
     CUDA_TRY(cudaMemcpyAsync(&nre, ix->m_nrecheck.p, sizeof nre, cudaMemcpyDeviceToHost, st));
     rc = check_dev_err(ix, st);  // synchronizes

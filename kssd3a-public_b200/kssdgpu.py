@@ -98,6 +98,8 @@ def gpu_lib() -> C.CDLL:
         lib.kssdgpu_server_destroy.restype = None
         lib.kssdgpu_sketch.argtypes = [C.c_char_p, C.c_uint64, _u64p, C.c_uint64, _u64p, C.c_int,
                                        C.POINTER(_SketchParams), vp, C.c_uint64, _u64p]
+        lib.kssdgpu_sketch_records.argtypes = [C.POINTER(C.c_char_p), _u64p, C.c_uint64, _u64p, C.c_int,
+                                               C.POINTER(_SketchParams), vp, C.c_uint64, _u64p]
         lib.kssdgpu_sketch_hash_id.argtypes = [C.POINTER(_SketchParams)]
         lib.kssdgpu_sketch_hash_id.restype = C.c_uint32
         lib.kssdgpu_lower_metric_dev.argtypes = [C.c_int, C.POINTER(MetricOpt), C.c_int, vp, vp, vp, vp, vp, vp,
@@ -151,19 +153,25 @@ def sketch(samples, klen=32, coden_len=11, hclen=0, holen=0, drfold=8, conflict=
     """Sketches on the device: samples is a list of samples, each a list of records'
     sequence bytes.  Returns (keys, offs) in the comblco / comblco.index layout."""
     recs = [r for smp in samples for r in smp]
-    seq = b"".join(recs)
     rec_offs = np.cumsum([0] + [len(r) for r in recs]).astype(np.uint64)
+    total = int(rec_offs[-1])
     samp = np.cumsum([0] + [len(smp) for smp in samples]).astype(np.uint64)
     prm = _SketchParams(klen, coden_len, hclen, holen, drfold, 1 if conflict else 0)
     offs = np.zeros(len(samples) + 1, dtype=np.uint64)
-    cap = max(1, len(seq) // max(1, 1 << min(drfold, 8)) + 1024)
+    if all(type(r) is bytes for r in recs):  # the library reads the records where they are
+        seq = (C.c_char_p * max(len(recs), 1))(*recs)
+        call = lambda k, cap: gpu_lib().kssdgpu_sketch_records(  # noqa: E731
+            seq, rec_offs, len(recs), samp, len(samples), C.byref(prm), k, cap, offs)
+    else:
+        seq = b"".join(recs)
+        call = lambda k, cap: gpu_lib().kssdgpu_sketch(  # noqa: E731
+            seq, total, rec_offs, len(recs), samp, len(samples), C.byref(prm), k, cap, offs)
+    cap = max(1, total // max(1, 1 << min(drfold, 8)) + 1024)
     keys = np.zeros(cap, dtype=np.uint64)
-    rc = gpu_lib().kssdgpu_sketch(seq, len(seq), rec_offs, len(recs), samp, len(samples), C.byref(prm),
-                                  keys.ctypes.data, cap, offs)
+    rc = call(keys.ctypes.data, cap)
     if rc == 7:  # capacity: offs holds the sizes
         keys = np.zeros(int(offs[-1]), dtype=np.uint64)
-        rc = gpu_lib().kssdgpu_sketch(seq, len(seq), rec_offs, len(recs), samp, len(samples), C.byref(prm),
-                                      keys.ctypes.data if len(keys) else None, len(keys), offs)
+        rc = call(keys.ctypes.data if len(keys) else None, len(keys))
     _check(rc)
     return keys[:int(offs[-1])].copy(), offs
 
