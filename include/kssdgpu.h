@@ -251,10 +251,11 @@ int kssdgpu_self_votes(kssdgpu_index_t *idx, const uint64_t *keys, const uint64_
                        uint32_t sample_step, uint32_t *votes, uint32_t *first);
 /* Device form of kssdgpu_self_lower (outputs in HBM, stream-ordered).
  *
- * Default: nothing cached between calls; the join follows the index's density
- * (kssdgpu_self_choice).  The one-pass scan (KSSDGPU_SELF_SCAN) zero-fills the packed
- * lower triangle (unless KSSDGPU_NO_ZERO), reads every context group's bounds and
- * joins each group of >= 2 postings as it finds it.  The dense join
+ * Default: the join follows the index's shared contexts (kssdgpu_self_choice); no result
+ * is kept between calls.  The join by atomics (KSSDGPU_SELF_SCAN) zero-fills the packed lower
+ * triangle (unless KSSDGPU_NO_ZERO) and joins the index's list of shared contexts, made when
+ * the index was built; an index with conflicts (several objects of one context in a genome)
+ * has no list, and every context group's bounds are read instead.  The dense join
  * (KSSDGPU_SELF_DENSE) computes the counters of the contexts that many genomes share as
  * exact int8 Gram products of the genomes' distances to each context's most frequent
  * object on the tensor cores (int32 accumulation), corrects the pairs that these

@@ -110,7 +110,7 @@ __host__ __device__ __forceinline__ size_t wide_warp_smem(uint32_t npad, uint32_
     return (size_t)npad + ((size_t)nref * 8 + 15) / 16 * 16;
 }
 
-// Operand rows of the groups list[0 .. n_list) (row c of matrix m at X + m * xs + c *
+// Operand rows of the groups 0 .. n_list of list (row c of matrix m at X + m * xs + c *
 // npad), and the corrections of their pairs into corr[cell of (q, r)].  A warp takes a
 // group: one pass over its postings fills a byte map of the genomes' distances in shared
 // memory, from which the rows are written in 16-byte pieces, and lists the genomes away
@@ -131,7 +131,8 @@ struct WideBlock {
 constexpr uint32_t kWideNone = 0xFFFFFFFFu;  // not an object: the block join takes objects below 32 bits
 
 template <bool BLOCK>
-__global__ void __launch_bounds__(256) k_wide_rows(const unsigned long long *__restrict__ list, uint32_t n_list,
+__global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict__ list,
+                                                   const unsigned long long *__restrict__ items, uint32_t n_list,
                                                    const uint64_t *__restrict__ post, uint32_t nref, uint32_t npad,
                                                    int8_t *__restrict__ X, size_t xs,
                                                    unsigned long long *__restrict__ corr, const WideBlock Q)
@@ -142,7 +143,8 @@ __global__ void __launch_bounds__(256) k_wide_rows(const unsigned long long *__r
     unsigned long long *minor = reinterpret_cast<unsigned long long *>(emap + npad);
     const uint4 absent = make_uint4(~0u, ~0u, ~0u, ~0u);
     for (uint32_t s = blockIdx.x * warps + (threadIdx.x >> 5); s < n_list; s += gridDim.x * warps) {
-        const unsigned long long item = list[s];
+        // a group of the index's list, or (BLOCK) a numbered (begin | k << 32)
+        const unsigned long long item = BLOCK ? items[s] : *reinterpret_cast<const unsigned long long *>(list + s);
         const uint32_t b = (uint32_t)item, k = (uint32_t)(item >> 32);
         for (uint32_t i = lane; i < npad / 16; i += 32)
             reinterpret_cast<uint4 *>(emap)[i] = absent;

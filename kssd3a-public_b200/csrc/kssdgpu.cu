@@ -15,6 +15,7 @@
 
 #include <cub/cub.cuh>
 #include <cub/device/device_segmented_sort.cuh>
+#include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
 #include <atomic>
@@ -250,15 +251,6 @@ constexpr int kMaxStripes = 256;
 constexpr uint64_t kStripeChunk = 256;
 constexpr uint64_t kStripeItemsMax = 1ull << 20;
 
-// An open-addressing table of touched counter cells (see table_credit below).
-constexpr uint32_t kCellEmpty = 0xFFFFFFFFu;
-
-struct CellTable {
-    uint32_t *key;            // cell number, kCellEmpty for a free slot (null: no table)
-    unsigned long long *acc;  // per slot: ctx word (num_mut2 << 32 | num_ctx), obj word (section << 32 | diff_obj)
-    int log;                  // 2^log slots
-};
-
 struct CountParams {
     const Slot *table;
     uint32_t mask;
@@ -318,48 +310,7 @@ struct SmemAcc {
     }
 };
 
-// Where a counter array spans far more memory than L2 (the 20,000-genome lower
-// triangle: 3.2 GB), its touched cells lie scattered
-// over the whole span and every add into them is slow -- atomics onto a fixed set of
-// addresses spread over 1.6 GB run at 38 G/s on a B200 against 130 G/s when the same
-// addresses fit in 16 MB -- although the touched cells themselves are few (92,633).
-// The self join's scan then adds into a compact open-addressing table of touched cells
-// instead (2^21 slots by default: a cell
-// number and its two counter words, 40 MB), claimed by the first credit of a cell that
-// finds a free slot among its first kCellTableProbes; a cell whose probes find no room
-// goes to the array directly.  Keys only go from empty to a cell while a kernel runs and
-// every credit of a cell probes the same sequence, so a cell lives in one slot or in the
-// array, never both; k_cell_table_flush adds the slots into the array after the kernel
-// and empties them for the next call.
-constexpr int kCellTableLog = 21;
-constexpr uint32_t kCellTableProbes = 8;
-
-
-// One credit of difference d into the cell's slot; false when its probes find no room.
-__device__ __forceinline__ bool table_credit(const CellTable &T, uint32_t cell, int d)
-{
-    const uint32_t mask = (1u << T.log) - 1;
-    uint32_t s = (cell * 2654435761u) >> (32 - T.log);
-    for (uint32_t p = 0; p < kCellTableProbes; ++p) {
-        uint32_t k = __ldcg(T.key + s);  // from L2: keys are claimed while the kernel runs
-        if (k == kCellEmpty) {
-            const uint32_t old = atomicCAS(T.key + s, kCellEmpty, cell);
-            k = old == kCellEmpty ? cell : old;
-        }
-        if (k == cell) {
-            atomicAdd(T.acc + 2 * (size_t)s, inc_ctx(d));
-            if (d)
-                atomicAdd(T.acc + 2 * (size_t)s + 1, inc_obj(d));
-            return true;
-        }
-        s = (s + 1) & mask;
-    }
-    return false;
-}
-
-// A query's global counter row.  (Through the table of touched cells, the 10,000 x
-// 20,000 block's count measured 2.24 vs 2.18 ms: unlike the self join's, its credits'
-// cost is not the scattered addresses, and the key load per credit adds latency.)
+// A query's global counter row.
 struct GlobalAcc {
     unsigned long long *c, *o;
     __device__ __forceinline__ void add(uint32_t gid, int d) const
@@ -1594,14 +1545,15 @@ __global__ void k_self_conflict_groups(const unsigned long long *__restrict__ li
 
 // ------------------------------------------------------------------ self lower triangle: one-pass scan join
 //
-// The self step from the resident index alone, with nothing prepared beforehand: a
-// persistent grid streams the context-group boundaries (gbeg) tile by tile, queues
-// every group of >= 2 postings in shared memory and joins the queue at once -- one
-// thread per group of at most kScanLaneMax postings, the whole CTA for a larger one.
-// Every pair of gid runs of a group credits cell (higher gid, lower gid) with the
+// The self step of an index with conflicts (several objects of one context in a genome),
+// from its groups alone: a persistent grid streams the context-group boundaries (gbeg) tile
+// by tile, queues every group of >= 2 postings in shared memory and joins the queue at
+// once -- one thread per group of at most kScanLaneMax postings, the whole CTA for a larger
+// one.  Every pair of gid runs of a group credits cell (higher gid, lower gid) with the
 // minimum object difference over the two runs' cross product (the higher gid's run is
 // the query run of count_lower at that context, src/command_ani.h:694-716);
-// --ignoreconflict skips reference (lower-gid) runs of several objects.
+// --ignoreconflict skips reference (lower-gid) runs of several objects.  (Conflict-free
+// indexes join their list of shared groups instead: kssd_shared.cuh.)
 
 constexpr uint32_t kScanThreads = 256;
 #ifndef KSSD_SCAN_PER_THREAD
@@ -1683,65 +1635,6 @@ __device__ __forceinline__ void join_group_cta(const uint64_t *__restrict__ post
     }
 }
 
-// Shared memory of k_self_scan: the tile's queue of shared groups, and (PAIRS) the
-// exclusive prefix of the small groups' pair counts.
-constexpr uint32_t kScanPairRanks = kScanLaneMax * (kScanLaneMax - 1) / 2;  // pairs of the largest small group
-struct ScanSmem {
-    unsigned long long queue[kScanTile];  // groups of 2..kScanLaneMax from the front, larger from the back
-    uint32_t prefix[kScanTile];
-    unsigned short pair[kScanPairRanks];  // (i, j) of every pair rank of a small group: i | j << 8
-};
-
-// One credit into the table, or into the triangle (no table, or no room).
-__device__ __forceinline__ void credit_global(const CellTable &T, unsigned long long *__restrict__ oc,
-                                              unsigned long long *__restrict__ oo, uint32_t qg, uint32_t rg, int d)
-{
-    if (T.key && table_credit(T, (uint32_t)lower_cell(qg, rg), d))
-        return;
-    credit_lower(oc, oo, qg, rg, d);
-}
-
-// The table's cells into the triangle (plain adds: a cell lives in one slot and the join
-// has finished), slots emptied for the next call.
-__global__ void k_cell_table_flush(uint32_t *__restrict__ key, unsigned long long *__restrict__ acc, uint32_t slots,
-                                   unsigned long long *__restrict__ oc, unsigned long long *__restrict__ oo)
-{
-    for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < slots; s += gridDim.x * blockDim.x) {
-        const uint32_t cell = key[s];
-        if (cell == kCellEmpty)
-            continue;
-        const ulonglong2 a = reinterpret_cast<const ulonglong2 *>(acc)[s];
-        oc[cell] += a.x;
-        if (a.y)
-            oo[cell] += a.y;
-        key[s] = kCellEmpty;
-        reinterpret_cast<ulonglong2 *>(acc)[s] = make_ulonglong2(0, 0);
-    }
-}
-
-// The pair (i < j) of rank t among the k(k-1)/2 pairs of a group: j(j-1)/2 <= t.
-__device__ __forceinline__ void pair_of_rank(uint32_t t, uint32_t &i, uint32_t &j)
-{
-    j = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)t)) * 0.5f);
-    while (j * (j - 1) / 2 > t)
-        --j;
-    while ((j + 1) * j / 2 <= t)
-        ++j;
-    i = t - j * (j - 1) / 2;
-}
-
-// The same for the pairs of a large group (ranks up to 2^32, 64-bit arithmetic).
-__device__ __forceinline__ void pair_of_rank_wide(uint32_t t, uint32_t &i, uint32_t &j)
-{
-    uint64_t jj = (uint64_t)((1.0 + sqrt(1.0 + 8.0 * (double)t)) * 0.5);
-    while (jj * (jj - 1) / 2 > t)
-        --jj;
-    while ((jj + 1) * jj / 2 <= t)
-        ++jj;
-    j = (uint32_t)jj;
-    i = (uint32_t)(t - jj * (jj - 1) / 2);
-}
-
 // Bounds of this thread's groups of tile t: groups g0 .. g0 + kScanPerThread - 1
 // (contiguous per thread, so a warp reads one 1 KB span with 16-byte loads), the
 // kScanPerThread + 1 values gbeg[g0 ..]; past the end they repeat gbeg[u] (empty groups).
@@ -1769,51 +1662,19 @@ __device__ __forceinline__ void scan_load_bounds(const uint32_t *__restrict__ gb
 
 // Per tile: every thread holds the bounds of kScanPerThread contiguous groups (loaded
 // while the previous tile was joined), one block scan places the tile's shared groups
-// in the queue.  PAIRS (a conflict-free index: one object per gid run): the small
-// groups' pairs are then dealt out evenly, thread t taking a contiguous range of the
-// tile's pair ranks and loading the postings of kScanPairBatch pairs before it credits
-// them (2: more costs registers and idle predicated slots at ~2 pairs per lane and
-// tile), so every lane runs the same short sequence per pair and no thread walks a
-// whole large group while the others wait; with conflicts every thread walks whole
-// groups (run cross products).  Groups of more than kScanLaneMax postings are taken by
-// the whole CTA.  NARROW: groups of more than kmax postings are left to the caller (a
-// kernel of its own: the comparison costs the join of a 2,000-genome index 7 %).
-#ifndef KSSD_SCAN_PAIR_TABLE
-#define KSSD_SCAN_PAIR_TABLE 1
-#endif
-#ifndef KSSD_SCAN_PAIR_BATCH
-#define KSSD_SCAN_PAIR_BATCH 2
-#endif
-constexpr uint32_t kScanPairBatch = KSSD_SCAN_PAIR_BATCH;
+// in the queue (small ones from its front, larger ones from its back).
 static_assert(kScanPerThread % 4 == 0, "contiguous bounds are loaded 4 at a time");
 
-// four CTAs per SM (64 registers): 2,000 genomes 0.112 vs 0.124 ms per join with three
-#ifndef KSSD_SCAN_MINB
-#define KSSD_SCAN_MINB 4
-#endif
-template <bool PAIRS, bool NARROW>
-__global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(const uint32_t *__restrict__ gbeg, uint64_t u,
-                                                            const uint64_t *__restrict__ post, int ignoreconflict,
-                                                            uint32_t kmax, CellTable table,
-                                                            unsigned long long *__restrict__ oc,
-                                                            unsigned long long *__restrict__ oo)
+__global__ void __launch_bounds__(kScanThreads, 4) k_self_scan(const uint32_t *__restrict__ gbeg, uint64_t u,
+                                                               const uint64_t *__restrict__ post, int ignoreconflict,
+                                                               unsigned long long *__restrict__ oc,
+                                                               unsigned long long *__restrict__ oo)
 {
-    extern __shared__ __align__(16) unsigned char scan_smem[];
-    ScanSmem &S = *reinterpret_cast<ScanSmem *>(scan_smem);
-    using Scan = cub::BlockScan<unsigned long long, kScanThreads>;
+    __shared__ unsigned long long queue[kScanTile];
+    using Scan = cub::BlockScan<uint32_t, kScanThreads>;
     __shared__ typename Scan::TempStorage scan_tmp;
     const uint64_t ntiles = (u + kScanTile - 1) / kScanTile;
     bool waited = false;
-#if KSSD_SCAN_PAIR_TABLE
-    if (PAIRS) {
-        for (uint32_t t = threadIdx.x; t < kScanPairRanks; t += kScanThreads) {
-            uint32_t i, j;
-            pair_of_rank(t, i, j);
-            S.pair[t] = (unsigned short)(i | (j << 8));
-        }
-        // visible to every thread after the first tile's queue barrier
-    }
-#endif
     uint32_t bnd[kScanPerThread + 1];
     if (blockIdx.x < ntiles)
         scan_load_bounds(gbeg, u, blockIdx.x, bnd);
@@ -1822,111 +1683,37 @@ __global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(cons
         uint32_t nxt[kScanPerThread + 1];
         if (t + gridDim.x < ntiles)
             scan_load_bounds(gbeg, u, t + gridDim.x, nxt);
-        // this thread's small groups (bits 0-15), large groups (bits 16-31) and small
-        // pairs (bits 32-63): at most 2,048 x 2 groups and 2,048 x 496 pairs per tile,
-        // so one 64-bit scan carries all three without overflow between the fields
-        uint32_t cnt[kScanPerThread];
-        unsigned long long mine = 0;
+        // this thread's small groups (bits 0-15) and large groups (bits 16-31): at most
+        // 2,048 of each in a tile
+        uint32_t mine = 0;
 #pragma unroll
         for (uint32_t j = 0; j < kScanPerThread; ++j) {
             const uint32_t k = bnd[j + 1] - bnd[j];
-            cnt[j] = k;
-            const bool small = k >= 2 && k <= (NARROW ? min(kScanLaneMax, kmax) : kScanLaneMax);
-            mine += small ? (1ull | ((unsigned long long)(k * (k - 1) / 2) << 32))
-                          : (k > kScanLaneMax && (!NARROW || k <= kmax) ? 0x10000ull : 0ull);
+            mine += k > kScanLaneMax ? 0x10000u : k >= 2 ? 1u : 0u;
         }
-        unsigned long long off, tot;
+        uint32_t off, tot;
         Scan(scan_tmp).ExclusiveSum(mine, off, tot);
-        uint32_t sl = (uint32_t)off & 0xFFFFu, ll = ((uint32_t)off >> 16) & 0xFFFFu;
-        uint32_t poff = (uint32_t)(off >> 32);
+        uint32_t sl = off & 0xFFFFu, ll = off >> 16;
 #pragma unroll
         for (uint32_t j = 0; j < kScanPerThread; ++j) {
-            const uint32_t k = cnt[j];
+            const uint32_t k = bnd[j + 1] - bnd[j];
             const unsigned long long item = (unsigned long long)bnd[j] | ((unsigned long long)k << 32);
-            if (k >= 2 && k <= (NARROW ? min(kScanLaneMax, kmax) : kScanLaneMax)) {
-                S.queue[sl] = item;
-                if (PAIRS) {
-                    S.prefix[sl] = poff;
-                    poff += k * (k - 1) / 2;
-                }
-                ++sl;
-            } else if (k > kScanLaneMax && (!NARROW || k <= kmax)) {
-                S.queue[kScanTile - 1 - ll] = item;
-                ++ll;
-            }
+            if (k > kScanLaneMax)
+                queue[kScanTile - 1 - ll++] = item;
+            else if (k >= 2)
+                queue[sl++] = item;
         }
         __syncthreads();
-        const uint32_t nl = (uint32_t)tot & 0xFFFFu, nc = ((uint32_t)tot >> 16) & 0xFFFFu;
+        const uint32_t nl = tot & 0xFFFFu, nc = tot >> 16;
         if (!waited) {
             pdl_wait_primary();  // the counters' zero fill has finished (no-op without a dependency)
             waited = true;
         }
-        if (PAIRS) {
-            const uint32_t total = (uint32_t)(tot >> 32);
-            const uint32_t p0 = (uint32_t)((uint64_t)total * threadIdx.x / kScanThreads);
-            const uint32_t p1 = (uint32_t)((uint64_t)total * (threadIdx.x + 1) / kScanThreads);
-            if (p0 < p1) {
-                // the group holding pair rank p0: the last q < nl with prefix[q] <= p0
-                uint32_t lo = 0, hi = nl - 1;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi + 1) >> 1;
-                    if (S.prefix[mid] <= p0)
-                        lo = mid;
-                    else
-                        hi = mid - 1;
-                }
-                uint32_t q = lo;
-                for (uint32_t pr = p0; pr < p1; pr += kScanPairBatch) {
-                    uint64_t pi[kScanPairBatch], pj[kScanPairBatch];
-#pragma unroll
-                    for (uint32_t x = 0; x < kScanPairBatch; ++x) {
-                        if (pr + x < p1) {
-                            while (q + 1 < nl && S.prefix[q + 1] <= pr + x)
-                                ++q;
-                            const unsigned long long item = S.queue[q];
-                            uint32_t i, j;
-#if KSSD_SCAN_PAIR_TABLE
-                            const uint32_t ij = S.pair[pr + x - S.prefix[q]];
-                            i = ij & 0xFFu;
-                            j = ij >> 8;
-#else
-                            pair_of_rank(pr + x - S.prefix[q], i, j);
-#endif
-                            pi[x] = __ldg(post + (uint32_t)item + i);
-                            pj[x] = __ldg(post + (uint32_t)item + j);
-                        }
-                    }
-#pragma unroll
-                    for (uint32_t x = 0; x < kScanPairBatch; ++x) {
-                        if (pr + x < p1) {
-                            const int d = min(kMinInit, dna_pop((uint32_t)pi[x] ^ (uint32_t)pj[x]));
-                            credit_global(table, oc, oo, (uint32_t)(pj[x] >> 32), (uint32_t)(pi[x] >> 32), d);
-                        }
-                    }
-                }
-            }
-        } else {
-            for (uint32_t i = threadIdx.x; i < nl; i += kScanThreads) {
-                const unsigned long long item = S.queue[i];
-                join_group_lane(post, (uint32_t)item, (uint32_t)(item >> 32), ignoreconflict, oc, oo);
-            }
-        }
+        for (uint32_t i = threadIdx.x; i < nl; i += kScanThreads)
+            join_group_lane(post, (uint32_t)queue[i], (uint32_t)(queue[i] >> 32), ignoreconflict, oc, oo);
         for (uint32_t i = 0; i < nc; ++i) {
-            const unsigned long long item = S.queue[kScanTile - 1 - i];
-            const uint32_t b = (uint32_t)item, k = (uint32_t)(item >> 32);
-            if (PAIRS && table.key) {
-                // one object per gid: the group's pairs dealt out over the CTA, into the table
-                const uint32_t np = (uint32_t)((uint64_t)k * (k - 1) / 2);  // k < 92,682 genomes
-                for (uint32_t pr = threadIdx.x; pr < np; pr += kScanThreads) {
-                    uint32_t x, y;
-                    pair_of_rank_wide(pr, x, y);
-                    const uint64_t px = __ldg(post + b + x), py = __ldg(post + b + y);
-                    credit_global(table, oc, oo, (uint32_t)(py >> 32), (uint32_t)(px >> 32),
-                                  min(kMinInit, dna_pop((uint32_t)px ^ (uint32_t)py)));
-                }
-            } else {
-                join_group_cta(post, b, k, ignoreconflict, oc, oo);
-            }
+            const unsigned long long item = queue[kScanTile - 1 - i];
+            join_group_cta(post, (uint32_t)item, (uint32_t)(item >> 32), ignoreconflict, oc, oo);
         }
         __syncthreads();  // the queue and the scan storage are reused by the next tile
 #pragma unroll
@@ -1935,12 +1722,15 @@ __global__ void __launch_bounds__(kScanThreads, KSSD_SCAN_MINB) k_self_scan(cons
     }
 }
 
+#include "kssd_shared.cuh"
+
 // Facts of the self join: tot[0..2] groups of >= 2 postings, postings in them, their
 // pairs; tot[3] whether any gid holds several objects of one context (a conflict);
-// tot[4..6] the groups of at least `wide` postings, their postings and pairs.  Sums meet in
-// shared memory first: one atomic per warp and fact onto seven global words made this
+// tot[4..6] the groups of at least `wide` postings, their postings and pairs; tot[7..9]
+// the groups of at most kSharedSmall, their postings and pairs.  Sums meet in
+// shared memory first: one atomic per warp and fact onto the same global words made this
 // kernel wait on those words (an index of 64 small genomes: 100 us for 0.5 MB of bounds).
-constexpr int kStatFacts = 7;
+constexpr int kStatFacts = 10;
 __global__ void __launch_bounds__(256) k_self_stats(const uint32_t *__restrict__ gbeg, uint64_t u,
                                                     const uint64_t *__restrict__ post, uint32_t wide,
                                                     unsigned long long *__restrict__ tot)
@@ -1957,6 +1747,11 @@ __global__ void __launch_bounds__(256) k_self_stats(const uint32_t *__restrict__
             f[0] += 1;
             f[1] += k;
             f[2] += k * (k - 1) / 2;
+            if (k <= kSharedSmall) {
+                f[7] += 1;
+                f[8] += k;
+                f[9] += k * (k - 1) / 2;
+            }
             if (k >= wide) {
                 f[4] += 1;
                 f[5] += k;
@@ -2626,9 +2421,6 @@ struct kssdgpu_index {
     DevBuf<double> m_val;                   // self matrix values (kssdgpu_self_lower_metric)
     DevBuf<kssd::RecheckCell> m_recheck;    // cells the host values
     DevBuf<unsigned long long> m_nrecheck;
-    DevBuf<uint32_t> c_key;                 // scan join: table of touched cells (empty between calls)
-    int c_log = kCellTableLog;              // its 2^c_log slots (KSSDGPU_CELL_TABLE_LOG, read at its allocation)
-    DevBuf<unsigned long long> c_acc;       // scan join: its counter words
     // facts of the index, from one pass at build: shared groups (>= 2 postings), their
     // postings and pairs, whether any gid run holds several objects (a conflict)
     unsigned long long f_groups = 0, f_postings = 0, f_pairs = 0;
@@ -2637,7 +2429,16 @@ struct kssdgpu_index {
     // the wide join corrects one by one (sampled estimate)
     uint32_t wide_min = 2;
     unsigned long long f_wgroups = 0, f_wpostings = 0, f_wpairs = 0, f_wcorr = 0;
-    bool f_conflict = false;
+    unsigned long long f_spairs = 0;        // pairs of the groups of at most kSharedSmall genomes
+    // shared groups of a conflict-free index (kssd_shared.cuh): the list, the blocks of its
+    // small groups (narrow ones: sh_small[0] blocks, all: sh_small[1]), the first large
+    // narrow and the first large wide group
+    SharedGroup *sh_list = nullptr;
+    SharedBlock *sh_blocks = nullptr;
+    uint32_t *sh_place = nullptr, *sh_object = nullptr, *sh_table = nullptr;
+    unsigned char *sh_number = nullptr;
+    uint32_t sh_small[2] = {0, 0}, sh_large[2] = {0, 0};
+    bool f_conflict = false;                // a genome holds several objects of one context
     // dense self join scratch
     DevBuf<unsigned long long> d_list;
     DevBuf<uint32_t> d_poff, d_allele;
@@ -2693,6 +2494,90 @@ int build_filter(kssdgpu_index *ix, uint64_t stripe_bytes, cudaStream_t st)
                                                      reinterpret_cast<uint32_t *>(ix->bloom));
     count_launch(2);
     CUDA_TRY(cudaGetLastError());
+    return KSSDGPU_OK;
+}
+
+// The index's list of shared groups and its blocks (kssd_shared.cuh); small: the small
+// groups, their postings and pairs.  Ends with the stream synchronized.
+int build_shared(kssdgpu_index *ix, const unsigned long long small[3], cudaStream_t st)
+{
+    const uint64_t n = ix->f_groups;
+    if (n >= 0x7FFFFFFFull || small[1] >= 0xFFFFFFFFull || (small[2] >> kBlockLog) >= 0x7FFFFFFFull)
+        return fail(KSSDGPU_ERR_CAPACITY, "too many shared contexts");
+    int gid_bits = 1;
+    while ((1 << gid_bits) < ix->nref)
+        ++gid_bits;
+    // the list: narrow small, narrow large, wide small, wide large groups, of which narrow
+    // large or wide small ones do not exist together
+    const uint64_t narrow = n - ix->f_wgroups, narrow_pairs = ix->f_pairs - ix->f_wpairs;
+    const bool split = ix->wide_min <= kSharedSmall;  // some small groups are wide
+    SharedRun run[2];
+    run[0] = SharedRun{0, (uint32_t)(split ? narrow : small[0]), 0, split ? narrow_pairs : small[2]};
+    const uint32_t blocks0 = (uint32_t)((run[0].pairs + kBlockPairs - 1) >> kBlockLog);
+    // marks of a run are one more than its blocks
+    run[1] = SharedRun{(uint32_t)narrow, (uint32_t)(split ? small[0] - narrow : 0), blocks0 + 1,
+                       split ? small[2] - narrow_pairs : 0};
+    const uint32_t blocks1 = (uint32_t)((run[1].pairs + kBlockPairs - 1) >> kBlockLog);
+    const uint64_t blocks = (uint64_t)blocks0 + 1 + blocks1;  // one between the runs stays empty
+    ix->sh_small[0] = blocks0;
+    ix->sh_small[1] = (uint32_t)blocks;
+    ix->sh_large[0] = (uint32_t)run[0].groups;  // large narrow groups: [run 0's end, narrow)
+    ix->sh_large[1] = (uint32_t)(narrow + run[1].groups);  // large wide groups: [.., n)
+    struct Temps {
+        uint32_t *key = nullptr, *key2 = nullptr, *mark = nullptr;
+        unsigned long long *val = nullptr, *val2 = nullptr;
+        SharedSums *sums = nullptr;
+        unsigned int *count = nullptr;
+        void *tmp = nullptr;
+        cudaStream_t st;
+        ~Temps()
+        {
+            cudaStreamSynchronize(st);
+            for (void *p : {(void *)key, (void *)key2, (void *)mark, (void *)val, (void *)val2, (void *)sums,
+                            (void *)count, tmp})
+                pool_free_idle(p);
+        }
+    } t;
+    t.st = st;
+    CUDA_TRY(pool_malloc(&t.key, n * 4));
+    CUDA_TRY(pool_malloc(&t.key2, n * 4));
+    CUDA_TRY(pool_malloc(&t.mark, (blocks + 2) * 4));
+    CUDA_TRY(pool_malloc(&t.val, n * 8));
+    CUDA_TRY(pool_malloc(&t.val2, n * 8));
+    CUDA_TRY(pool_malloc(&t.sums, n * sizeof(SharedSums)));
+    CUDA_TRY(pool_malloc(&t.count, sizeof(unsigned int)));
+    CUDA_TRY(pool_malloc(&ix->sh_list, n * sizeof(SharedGroup)));
+    CUDA_TRY(pool_malloc(&ix->sh_blocks, blocks * sizeof(SharedBlock)));
+    CUDA_TRY(pool_malloc(&ix->sh_place, n * 4));
+    CUDA_TRY(pool_malloc(&ix->sh_object, std::max<uint64_t>(small[1], 1) * 4));
+    CUDA_TRY(pool_malloc(&ix->sh_number, std::max<uint64_t>(small[1], 1)));  // slots while it is built, too
+    CUDA_TRY(pool_malloc(&ix->sh_table, blocks * kBlockGenomes * 4));
+    const auto sizes = thrust::make_transform_iterator(t.val2, SharedSize{});
+    size_t tb0 = 0, tb1 = 0;
+    CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb0, t.key, t.key2, t.val, t.val2, (int64_t)n, 0, gid_bits + 2,
+                                             st));
+    CUDA_TRY(cub::DeviceScan::ExclusiveScan(nullptr, tb1, sizes, t.sums, SharedAdd{}, SharedSums{0, 0}, (int64_t)n, st));
+    CUDA_TRY(pool_malloc(&t.tmp, std::max(tb0, tb1)));
+    CUDA_TRY(cudaMemsetAsync(t.count, 0, sizeof(unsigned int), st));
+    CUDA_TRY(cudaMemsetAsync(ix->sh_blocks, 0, blocks * sizeof(SharedBlock), st));
+    k_shared_collect<<<(unsigned)std::min<uint64_t>((ix->u + kScanTile - 1) / kScanTile, (uint64_t)ix->sms * 8),
+                       kScanThreads, 0, st>>>(ix->gbeg, ix->u, ix->post, ix->wide_min, gid_bits, t.key, t.val, t.count);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cub::DeviceRadixSort::SortPairs(t.tmp, tb0, t.key, t.key2, t.val, t.val2, (int64_t)n, 0, gid_bits + 2, st));
+    CUDA_TRY(cub::DeviceScan::ExclusiveScan(t.tmp, tb1, sizes, t.sums, SharedAdd{}, SharedSums{0, 0}, (int64_t)n, st));
+    k_shared_list<<<grid_for(n), 256, 0, st>>>(t.val2, (uint32_t)n, ix->sh_list);
+    count_launch(4);
+    CUDA_TRY(cudaGetLastError());
+    for (const SharedRun &r : run) {
+        const uint32_t nb = (uint32_t)((r.pairs + kBlockPairs - 1) >> kBlockLog);
+        if (!nb)
+            continue;
+        k_shared_marks<<<grid_for(r.groups), 256, 0, st>>>(t.sums, r, t.mark);
+        k_shared_blocks<<<nb, 256, 0, st>>>(ix->sh_list, ix->obj_bits <= kPackBits, t.sums, r, t.mark, ix->post, ix->sh_blocks, ix->sh_place,
+                                            ix->sh_object, ix->sh_number, ix->sh_table);
+        count_launch(2);
+        CUDA_TRY(cudaGetLastError());
+    }
     return KSSDGPU_OK;
 }
 
@@ -2766,12 +2651,18 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
         ix->f_wgroups = h[4];
         ix->f_wpostings = h[5];
         ix->f_wpairs = h[6];
+        ix->f_spairs = h[9];
         const unsigned long long *sampled = h + kStatFacts;
         ix->f_alleles = ix->f_postings;
         if (sampled[1]) {
             const double scale = (double)ix->f_postings / (double)sampled[1];
             ix->f_alleles = std::max<unsigned long long>(1, (unsigned long long)((double)sampled[0] * scale));
             ix->f_wcorr = (unsigned long long)((double)sampled[2] * scale);
+        }
+        if (!ix->f_conflict && ix->f_groups) {
+            const int lrc = build_shared(ix, h + 7, st);
+            if (lrc)
+                return lrc;
         }
     }
     if (herr == kDevUnsorted)
@@ -2834,23 +2725,6 @@ int check_dev_err(kssdgpu_index *ix, cudaStream_t st)
 }
 
 uint32_t env_u32(const char *name, uint32_t def, uint32_t lo, uint32_t hi);
-
-// The index's table of touched cells (allocated on first use with 2^KSSDGPU_CELL_TABLE_LOG
-// slots, default 2^21; empty between calls: every kernel that fills it is followed by
-// k_cell_table_flush on the same stream).
-int cell_table(kssdgpu_index *ix, cudaStream_t st, CellTable &t)
-{
-    if (!ix->c_key.p || !ix->c_acc.p) {
-        ix->c_log = (int)env_u32("KSSDGPU_CELL_TABLE_LOG", kCellTableLog, 4, 26);
-        const size_t slots = (size_t)1 << ix->c_log;
-        CUDA_TRY(ix->c_key.ensure(slots));
-        CUDA_TRY(ix->c_acc.ensure(2 * slots));
-        CUDA_TRY(cudaMemsetAsync(ix->c_key.p, 0xFF, slots * 4, st));
-        CUDA_TRY(cudaMemsetAsync(ix->c_acc.p, 0, slots * 16, st));
-    }
-    t = CellTable{ix->c_key.p, ix->c_acc.p, ix->c_log};
-    return KSSDGPU_OK;
-}
 
 template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE = false>
 int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStream_t st)
@@ -3037,8 +2911,8 @@ int wide_block_end(kssdgpu_index *ix, int nq, unsigned long long *oc, unsigned l
         const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
         const WideBlock Q{ix->w_qobj.p + c0 * nqp, (uint32_t)nq, nqp, ix->w_y.p, ys};
         k_wide_rows<true><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
-                            warps * wide_warp_smem(npad, n), st>>>(ix->w_list.p + c0, cn, ix->post, n, npad, ix->w_x.p,
-                                                                   xs, ix->w_corr.p, Q);
+                            warps * wide_warp_smem(npad, n), st>>>(nullptr, ix->w_list.p + c0, cn, ix->post, n, npad,
+                                                                   ix->w_x.p, xs, ix->w_corr.p, Q);
         CUDA_TRY(cudaGetLastError());
         const int grc = kssd::dense_gemm_s8(ix->w_y.p, ix->w_x.p, ix->w_g.p, (int)nqp, (int)npad, (int)cn, kWideRows,
                                             nqp, npad, npad, (int64_t)ys, (int64_t)xs, (int64_t)gs, ix->d_ws.p, st);
@@ -4030,31 +3904,17 @@ int self_plan(kssdgpu_index *ix, cudaStream_t st)
     return KSSDGPU_OK;
 }
 
-// The one-pass self step: zero fill of the dense lower triangle (unless NO_ZERO), then
-// the scan join over the whole index.  When the fill stays in L2 the scan launches
-// programmatically after it and waits for it only before its first atomic, so its
-// first tiles' gbeg loads overlap the fill.
-// kmax: larger groups of a conflict-free index are left out (the wide join takes them).
-constexpr uint32_t kScanAll = 0xFFFFFFFFu;
+// The self step by atomics: zero fill of the dense lower triangle (unless NO_ZERO), then
+// the join of the listed pairs, or with conflicts the scan over the whole index.  When the
+// fill stays in L2 the join launches programmatically after it and waits for it only
+// before its first credit.  narrow: of a conflict-free index the pairs of narrow groups only
+// (the wide join takes the others).
 int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, unsigned long long *oo, cudaStream_t st,
-                   uint32_t kmax = kScanAll)
+                   bool narrow = false)
 {
     const size_t cells = (size_t)ix->nref * (ix->nref - 1) / 2;
     if (!cells)
         return KSSDGPU_OK;
-    // a conflict-free index deals out pairs; with conflicts threads walk whole groups
-    const bool pairs = !ix->f_conflict;
-    // Triangles larger than L2 (and of 32-bit cell numbers: at most 92,681 genomes) add
-    // through the table of touched cells (allocated on first use, kept empty between
-    // calls); with the counters in L2 the table's probes cost more than they save (2,000
-    // genomes: 0.19 vs 0.14 ms per step) and the join adds into the triangle directly.
-    const bool big = cells < (size_t)kCellEmpty && cells * 16 > (size_t)ix->l2_bytes;
-    CellTable table{nullptr, nullptr, 0};
-    if (ix->u && pairs && big) {
-        int rc = cell_table(ix, st, table);
-        if (rc)
-            return rc;
-    }
     bool after_fill = false;
     if (!(flags & KSSDGPU_NO_ZERO)) {
         if ((((uintptr_t)oc | (uintptr_t)oo) & 15) == 0) {
@@ -4067,23 +3927,10 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
             CUDA_TRY(cudaMemsetAsync(oo, 0, cells * 8, st));
         }
     }
-    if (!ix->u)
+    const unsigned long long pairs = ix->f_pairs - (narrow ? ix->f_wpairs : 0);
+    if (!ix->u || !pairs)
         return KSSDGPU_OK;
-    auto kern = !pairs ? k_self_scan<false, false> : kmax == kScanAll ? k_self_scan<true, false> : k_self_scan<true, true>;
-    const size_t smem = sizeof(ScanSmem);
-    if (!ix->scan_grid) {
-        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        CUDA_TRY(cudaFuncSetAttribute(k_self_scan<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int per_sm = 0;
-        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_self_scan<true, false>, kScanThreads, smem));
-        ix->scan_grid = std::max(1, per_sm) * ix->sms;
-    }
-    const uint64_t ntiles = (ix->u + kScanTile - 1) / kScanTile;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)std::min<uint64_t>(ntiles, (uint64_t)ix->scan_grid));
-    cfg.blockDim = dim3(kScanThreads);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -4092,15 +3939,47 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const uint32_t *)ix->gbeg, ix->u, (const uint64_t *)ix->post,
-                                (flags & KSSDGPU_IGNORECONFLICT) ? 1 : 0, kmax, table, oc, oo));
+    const bool pack = ix->obj_bits <= kPackBits;
+    const auto pairs_kernel = pack ? k_self_pairs<true> : k_self_pairs<false>;
+    const size_t pairs_smem = pack ? offsetof(PairSmem, number) : sizeof(PairSmem);
+    if (!ix->scan_grid) {
+        int per_sm = 0;
+        if (ix->f_conflict) {
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_self_scan, kScanThreads, 0));
+        } else {
+            CUDA_TRY(cudaFuncSetAttribute(pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_smem));
+            CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs_kernel, kPairThreads, pairs_smem));
+        }
+        ix->scan_grid = std::max(1, per_sm) * ix->sms;
+    }
+    if (ix->f_conflict) {
+        const uint64_t ntiles = (ix->u + kScanTile - 1) / kScanTile;
+        cfg.gridDim = dim3((unsigned)std::min<uint64_t>(ntiles, (uint64_t)ix->scan_grid));
+        cfg.blockDim = dim3(kScanThreads);
+        CUDA_TRY(cudaLaunchKernelEx(&cfg, k_self_scan, (const uint32_t *)ix->gbeg, ix->u, (const uint64_t *)ix->post,
+                                    (flags & KSSDGPU_IGNORECONFLICT) ? 1 : 0, oc, oo));
+    } else {
+        const uint32_t nblocks = ix->sh_small[narrow ? 0 : 1];
+        if (nblocks) {
+            cfg.gridDim = dim3(std::min<uint32_t>(nblocks, (uint32_t)ix->scan_grid));
+            cfg.blockDim = dim3(kPairThreads);
+            cfg.dynamicSmemBytes = pairs_smem;
+            CUDA_TRY(cudaLaunchKernelEx(&cfg, pairs_kernel, (const SharedBlock *)ix->sh_blocks, nblocks,
+                                        (const SharedGroup *)ix->sh_list, (const uint32_t *)ix->sh_place,
+                                        (const uint32_t *)ix->sh_object, (const unsigned char *)ix->sh_number,
+                                        (const uint32_t *)ix->sh_table, (const uint64_t *)ix->post, oc, oo));
+        }
+        const uint32_t nnarrow = (uint32_t)(ix->f_groups - ix->f_wgroups), n = (uint32_t)ix->f_groups;
+        const uint32_t large[2][2] = {{ix->sh_large[0], nnarrow}, {ix->sh_large[1], narrow ? ix->sh_large[1] : n}};
+        for (const auto &r : large)
+            if (r[1] > r[0]) {
+                k_self_large<<<std::min<uint32_t>(r[1] - r[0], (uint32_t)ix->sms * 32), 256, 0, st>>>(
+                    ix->sh_list + r[0], r[1] - r[0], ix->post, oc, oo);
+                count_launch();
+            }
+    }
     count_launch();
     CUDA_TRY(cudaGetLastError());
-    if (table.key) {
-        k_cell_table_flush<<<ix->sms * 4, 256, 0, st>>>(table.key, table.acc, 1u << table.log, oc, oo);
-        count_launch();
-        CUDA_TRY(cudaGetLastError());
-    }
     return KSSDGPU_OK;
 }
 
@@ -4126,23 +4005,24 @@ uint64_t wide_bytes(const kssdgpu_index *ix)
     return (uint64_t)kWideRows * np * (wide_pass(ix) + 4 * np) + 4ull * ix->nref * (ix->nref - 1);
 }
 
-// Estimated times in ms of the three self joins (B200): the scan's pair credits (6.22 G
-// pairs: 45.8 ms), or where few genomes share much the credits that queue up on one cell
-// (14 ns each, one per warp where a group has fewer pairs than a warp lanes: 30 genomes of
-// one species 232 us, two genomes 8 us); the wide join, whose products run near 2.0 P int8 ops/s (six of n^2 a
-// group), whose corrections cost an atomic each and whose narrow groups are scanned; the
-// join with a row per allele (1,024 genomes of one species, 643,817 alleles: products
-// 1.15 ms, rows 0.54 ms, numbering 0.24 ms).  The first terms are launches and gaps.
+// Estimated times in ms of the three self joins (B200).  By atomics: small groups 3 ps a
+// pair (2,000 genomes of 200 species, 4.85 M pairs: 36 us; 400 genomes in species of 24, 46
+// M pairs: 100 us), large ones 7.4 ps (6.22 G pairs of one species: 45.8 ms) or where few
+// genomes share them the credits that queue up on one cell, 14 ns each.  The wide join's
+// products run near 2.0 P int8 ops/s (six of n^2 a group), its corrections cost an atomic
+// each, its narrow groups are joined by atomics.  A row per allele: 1,024 genomes of one
+// species, 643,817 alleles: products 1.15 ms, rows 0.54 ms, numbering 0.24 ms.  The first
+// terms are launches and gaps.
 double scan_ms(const kssdgpu_index *ix)
 {
     const double cells = std::max(1.0, 0.5 * (double)ix->nref * (double)(ix->nref - 1));
-    const double merged = std::max(1.0, 32.0 * (double)ix->f_groups / std::max(1.0, (double)ix->f_pairs));
-    return std::max(7.4e-9 * (double)ix->f_pairs, 14e-6 * (double)ix->f_pairs / cells / merged);
+    const double large = (double)(ix->f_pairs - ix->f_spairs);
+    return 0.01 + 3e-9 * (double)ix->f_spairs + std::max(7.4e-9 * large, 14e-6 * large / cells);
 }
 double wide_ms(const kssdgpu_index *ix)
 {
     const double n = (double)ix->nref;
-    return 0.02 + 7.4e-9 * (double)(ix->f_pairs - ix->f_wpairs + ix->f_wcorr) +
+    return 0.04 + 3e-9 * (double)(ix->f_pairs - ix->f_wpairs) + 7.4e-9 * (double)ix->f_wcorr +
            (double)ix->f_wgroups * (12 * n * n / 2.0e12 + 6 * n / 4e9);
 }
 double allele_ms(const kssdgpu_index *ix)
@@ -4201,7 +4081,7 @@ int self_wide_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long long
     const uint32_t npad = (uint32_t)dense_npad(ix);
     ix->w_ran = true;
     if (ix->f_groups > ix->f_wgroups) {
-        const int rc = self_scan_impl(ix, 0, oc, oo, st, ix->wide_min - 1);
+        const int rc = self_scan_impl(ix, 0, oc, oo, st, true);
         if (rc)
             return rc;
     } else {
@@ -4215,27 +4095,23 @@ int self_wide_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long long
                                            " bytes exceed half of the free device memory");
     const uint64_t pass = wide_pass(ix);
     const size_t gs = (size_t)npad * npad, xs = (size_t)pass * npad;
-    CUDA_TRY(ix->w_list.ensure(ix->f_wgroups));
-    CUDA_TRY(ix->w_count.ensure(1));
     CUDA_TRY(ix->w_corr.ensure(cells));
     CUDA_TRY(ix->w_x.ensure(kWideRows * xs));
     CUDA_TRY(ix->w_g.ensure(kWideRows * gs));
+    const SharedGroup *list = ix->sh_list + (ix->f_groups - ix->f_wgroups);  // the wide groups
     const uint64_t bw = npad <= kWideSquare ? npad : kWideBlock;
     size_t ws = 0;
     for (uint64_t j = 0; j < npad; j += bw)
         ws = std::max(ws, kssd::dense_gemm_s8_workspace((int)(npad - j), (int)std::min<uint64_t>(bw, npad - j),
                                                         (int)pass, kWideRows));
     CUDA_TRY(ix->d_ws.ensure(ws));
-    CUDA_TRY(cudaMemsetAsync(ix->w_count.p, 0, sizeof(unsigned int), st));
     CUDA_TRY(cudaMemsetAsync(ix->w_corr.p, 0, cells * 8, st));
-    k_dense_list<<<grid_for(ix->u), 256, 0, st>>>(ix->gbeg, ix->u, ix->wide_min, ix->w_list.p, ix->w_count.p, nullptr);
-    count_launch();
     int warps = 0, rows_grid = 0;
     CUDA_TRY(wide_rows_shape(ix, k_wide_rows<false>, npad, warps, rows_grid));
     for (uint64_t c0 = 0; c0 < ix->f_wgroups; c0 += pass) {
         const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
         k_wide_rows<false><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
-                             warps * wide_warp_smem(npad, n), st>>>(ix->w_list.p + c0, cn, ix->post, n, npad,
+                             warps * wide_warp_smem(npad, n), st>>>(list + c0, nullptr, cn, ix->post, n, npad,
                                                                     ix->w_x.p, xs, ix->w_corr.p, WideBlock{});
         count_launch();
         CUDA_TRY(cudaGetLastError());
@@ -4363,7 +4239,7 @@ double self_density(const kssdgpu_index *ix)
 // The rule of the self join: a dense join where the estimates above put it below the
 // scan, on a conflict-free index whose operands fit in half of the free device memory.
 // (A fixed density of 1/2048 sent 64 genomes of eight species, 0.6 M pairs, to the dense
-// join: 290 us of kernels against 12 us by the scan.)
+// join: 290 us of kernels against 12 us by atomics.)
 bool dense_chosen(const kssdgpu_index *ix)
 {
     if (ix->f_conflict || ix->f_pairs == 0 || ix->nref < 2 || (uint32_t)ix->nref > kDenseMaxGroup)
@@ -4959,6 +4835,12 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     pool_free_idle(ix->bloom);
     pool_free_idle(ix->bloom_bounds);
     pool_free_idle(ix->err);
+    pool_free_idle(ix->sh_list);
+    pool_free_idle(ix->sh_blocks);
+    pool_free_idle(ix->sh_place);
+    pool_free_idle(ix->sh_object);
+    pool_free_idle(ix->sh_number);
+    pool_free_idle(ix->sh_table);
     pool_free_idle(ix->work);
     ix->s_keys.release_idle();
     ix->s_offs.release_idle();
@@ -4979,8 +4861,6 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     ix->s_counts.release_idle();
     ix->s_cubtmp.release_idle();
     ix->j_small.release_idle();
-    ix->c_key.release_idle();
-    ix->c_acc.release_idle();
     ix->m_val.release_idle();
     ix->m_recheck.release_idle();
     ix->m_nrecheck.release_idle();
