@@ -246,6 +246,7 @@ int server_launch(kssdgpu_server *s, ServerSlot &sl)
     P.bloom_mask = s->ix->bloom_mask;
     P.bloom_stripes = s->ix->bloom_stripes;
     P.bloom_bounds = s->ix->bloom_bounds;
+    P.conflict_free = !s->ix->f_conflict;
     int rc = (s->cfg.flags & KSSDGPU_UNIQUE) ? launch_batched<false, true, false>(s->ix, P, 0, sl.st)
                                              : launch_batched<false, false, false>(s->ix, P, 0, sl.st);
     if (rc)

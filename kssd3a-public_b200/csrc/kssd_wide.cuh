@@ -26,7 +26,8 @@
 // Measured (B200, whole calls): the self join of 1,024 genomes of one species 1,748 (rows
 // per allele) -> 241 us, of 3,000 genomes of ten species 16.4 -> 3.0 ms; a block of 200
 // queries against 1,024 genomes of their species 6.82 ms (postings walked per query, 1.9 G
-// atomics) -> 0.24 ms, of one query 2.23 -> 0.17 ms.
+// atomics) -> 0.24 ms, of one query 2.23 -> 0.17 ms, of 30 read sets against 500 genomes
+// 975 -> 277 us.
 #pragma once
 
 // Groups of at least this many postings are wide.  A group costs six rows of the products
@@ -119,16 +120,19 @@ __host__ __device__ __forceinline__ size_t wide_warp_smem(uint32_t npad, uint32_
 // pairs) and the corrections' atomics (L2); the rows are 6 n bytes.
 //
 // BLOCK: the pairs are those of a query with the group's genomes instead.  qobj[c * nqpad
-// + q] is the object of query q at group c (kWideNone: it does not hold it), written by
-// the counting kernel; the queries' operand rows go to Y, the corrections to corr[q * nref
-// + r].
+// + q] is the object of query q at group c (kWideNone: it does not hold it; kWideRun: it
+// holds several, from that entry on), written by the counting kernel; the queries' operand
+// rows go to Y, the corrections to corr[q * nref + r].  A query of several objects takes the
+// place of the one nearest to the major object: its difference to a genome there is that
+// one's, and to every other genome the least over the run, so all of them are compared.
 struct WideBlock {
     const uint32_t *qobj;
     uint32_t nq, nqpad;
     int8_t *Y;
     size_t ys;
+    const uint64_t *qkeys, *qoffs;
+    int obj_bits;
 };
-constexpr uint32_t kWideNone = 0xFFFFFFFFu;  // not an object: the block join takes objects below 32 bits
 
 template <bool BLOCK>
 __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict__ list,
@@ -186,11 +190,25 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
                 uint4 oq = make_uint4(kWideNone, kWideNone, kWideNone, kWideNone);
                 if (q < Q.nqpad)
                     oq = __ldcs(reinterpret_cast<const uint4 *>(Q.qobj + (size_t)s * Q.nqpad + q));
-                const uint32_t ob[4] = {oq.x, oq.y, oq.z, oq.w};
+                uint32_t ob[4] = {oq.x, oq.y, oq.z, oq.w}, runs[4] = {0, 0, 0, 0};
                 uint32_t e4 = 0;
 #pragma unroll
-                for (int x = 0; x < 4; ++x)
-                    e4 |= (ob[x] == kWideNone ? 0xFFu : wide_e(ob[x], major)) << (8 * x);
+                for (int x = 0; x < 4; ++x) {
+                    uint32_t ex = 0xFFu;
+                    if (ob[x] != kWideNone && (ob[x] & kWideRun)) {
+                        const uint64_t from = ob[x] & ~kWideRun, end = Q.qoffs[q + x + 1] - Q.qoffs[0];
+                        const uint64_t mask = (1ull << Q.obj_bits) - 1, ctx = __ldg(Q.qkeys + from) >> Q.obj_bits;
+                        for (uint64_t i = from; i < end; ++i, ++runs[x]) {
+                            const uint64_t key = __ldg(Q.qkeys + i);
+                            if (key >> Q.obj_bits != ctx)
+                                break;
+                            ex = min(ex, wide_e((uint32_t)(key & mask), major));
+                        }
+                    } else if (ob[x] != kWideNone) {
+                        ex = wide_e(ob[x], major);
+                    }
+                    e4 |= ex << (8 * x);
+                }
                 if (q < Q.nqpad) {
                     const WideWords w = wide_words(e4);
 #pragma unroll
@@ -200,7 +218,31 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
                     const uint32_t ex = (e4 >> (8 * x)) & 0xFFu;
-                    for (unsigned away = __ballot_sync(0xffffffffu, ex != 0 && ex != 0xFFu); away; away &= away - 1) {
+                    for (unsigned several = __ballot_sync(0xffffffffu, runs[x] != 0); several; several &= several - 1) {
+                        const int src = __ffs(several) - 1;
+                        const uint64_t from = __shfl_sync(0xffffffffu, ob[x], src) & ~kWideRun;
+                        const uint32_t run = __shfl_sync(0xffffffffu, runs[x], src);
+                        const uint32_t ea = __shfl_sync(0xffffffffu, ex, src);
+                        const uint32_t mask = (1u << Q.obj_bits) - 1u;
+                        unsigned long long *row = corr + (size_t)(q0 + 4 * src + x) * nref;
+                        for (uint32_t j = lane; j < nm; j += 32) {
+                            const unsigned long long c = minor[j];
+                            const uint32_t rc = (uint32_t)(c >> 32), er = rc >> kGidBits;
+                            uint32_t d = (uint32_t)kMinInit;
+                            for (uint32_t i = 0; i < run; ++i)
+                                d = min(d, (uint32_t)dna_pop(((uint32_t)__ldg(Q.qkeys + from + i) & mask) ^ (uint32_t)c));
+                            // the products count a difference, two where the run has no object
+                            // at the major one or the genome's is two away, and ea + er of it
+                            const uint32_t two = ea ? 1u : er >= 2 ? 1u : 0u;
+                            const unsigned long long w = (unsigned long long)(two - (d >= 2 ? 1u : 0u)) |
+                                                         ((unsigned long long)(d == 0) << 21) |
+                                                         ((unsigned long long)(ea + er - d) << 42);
+                            if (w)
+                                atomicAdd(row + (rc & ((1u << kGidBits) - 1)), w);
+                        }
+                    }
+                    for (unsigned away = __ballot_sync(0xffffffffu, ex != 0 && ex != 0xFFu && runs[x] == 0); away;
+                         away &= away - 1) {
                         const int src = __ffs(away) - 1;
                         const uint32_t oa = __shfl_sync(0xffffffffu, ob[x], src), ea = __shfl_sync(0xffffffffu, ex, src);
                         unsigned long long *row = corr + (size_t)(q0 + 4 * src + x) * nref;

@@ -295,14 +295,16 @@ struct CountParams {
     int nitems;
     const uint32_t *chunk_prefix;  // global-row mode without items: query q owns the chunk_keys-entry
                                    // chunks [prefix[q], prefix[q+1]) (nq + 1 words), may be null
-    uint32_t chunk_keys;           // entries per chunk in that mode
+    uint32_t chunk_keys;           // entries per chunk in that mode, at most
+    uint32_t chunk_auto;           // chunks a block should give (count_chunk), 0: chunk_keys as it is
     int *err;
     const uint4 *bloom;            // membership filter of the index's contexts, may be null
     uint32_t bloom_mask;           // 32-byte blocks of one stripe of it - 1
     int bloom_stripes;             // its key-range stripes (a power of two)
     const unsigned long long *bloom_bounds;  // first context of each stripe (stripes + 1 words)
     const uint32_t *nitems_dev;    // stripe-major mode: count of P.items (built on the device), may be null
-    // wide groups left to the tensor cores (kssd_wide.cuh), or null: a query's object at a
+    int conflict_free;             // the index holds one object per context and genome
+    // wide groups left to the tensor cores (kssd_wide.cuh): a query's object at a
     // group of at least wide_min postings goes to wide_obj[number * wide_stride + query], the
     // group's number at wide_at[its first posting]
     uint32_t *wide_obj;
@@ -321,6 +323,7 @@ __device__ __forceinline__ unsigned long long inc_obj(int d) { return 1ull | ((u
 // hot cells of similar genomes contend less than on 64-bit words).
 struct SmemAcc {
     uint32_t *nc, *m2, *dobj, *sect;
+    __device__ __forceinline__ void add_spread(uint32_t gid, int d) const { add(gid, d); }
     __device__ __forceinline__ void add(uint32_t gid, int d) const
     {
         atomicAdd(nc + gid, 1u);
@@ -343,6 +346,73 @@ struct GlobalAcc {
             atomicAdd(o + gid, inc_obj(d));
     }
 };
+
+// A warp's own counters of one query's row: a query meets few references (its species), so
+// nearly all its credits fall on a few cells, and L2 atomics onto the same words queue up.  A
+// reference takes the slot its number names, if no other has; the slots go to the row with
+// one atomic per touched word (flush, before a count could pass 16 bits), credits of other
+// references at once.
+constexpr uint32_t kWarpCells = 64;
+constexpr uint64_t kWarpCellEntries = 4096;  // entries between two flushes, at most
+static_assert(kWarpCellEntries * kMinInit < 65536, "packed counts of a warp's cell");
+struct WarpCells {
+    uint32_t ref[kWarpCells];  // kNoRef: free
+    uint32_t ctx[kWarpCells];  // num_ctx | num_mut2_ctx << 16
+    uint32_t obj[kWarpCells];  // diff_obj | diff_obj_section << 16
+};
+constexpr uint32_t kNoRef = 0xFFFFFFFFu;
+
+struct WarpAcc {
+    GlobalAcc row;
+    WarpCells *cells;
+    // lanes on consecutive references: more of them than cells
+    __device__ __forceinline__ void add_spread(uint32_t gid, int d) const { row.add(gid, d); }
+    __device__ __forceinline__ void add(uint32_t gid, int d) const
+    {
+        const uint32_t h = (gid * 2654435761u) >> 26;
+        uint32_t have = *(volatile uint32_t *)&cells->ref[h];
+        if (have == kNoRef) {
+            have = atomicCAS(&cells->ref[h], kNoRef, gid);
+            if (have == kNoRef)
+                have = gid;
+        }
+        if (have == gid) {
+            atomicAdd(&cells->ctx[h], 1u | (d > 1 ? 0x10000u : 0u));
+            if (d)
+                atomicAdd(&cells->obj[h], 1u | ((uint32_t)d << 16));
+        } else {
+            row.add(gid, d);
+        }
+    }
+    __device__ __forceinline__ void clear(uint32_t lane) const
+    {
+        for (uint32_t i = lane; i < kWarpCells; i += 32) {
+            cells->ref[i] = kNoRef;
+            cells->ctx[i] = 0;
+            cells->obj[i] = 0;
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ void flush(uint32_t lane) const
+    {
+        __syncwarp();
+        for (uint32_t i = lane; i < kWarpCells; i += 32) {
+            const uint32_t gid = cells->ref[i];
+            if (gid != kNoRef) {
+                const uint32_t c = cells->ctx[i], o = cells->obj[i];
+                atomicAdd(row.c + gid, (unsigned long long)(c & 0xFFFFu) | ((unsigned long long)(c >> 16) << 32));
+                if (o)
+                    atomicAdd(row.o + gid, (unsigned long long)(o & 0xFFFFu) | ((unsigned long long)(o >> 16) << 32));
+                cells->ref[i] = kNoRef;
+                cells->ctx[i] = 0;
+                cells->obj[i] = 0;
+            }
+        }
+        __syncwarp();
+    }
+};
+__device__ __forceinline__ void flush_acc(const WarpAcc &a, uint32_t lane) { a.flush(lane); }
+__device__ __forceinline__ void flush_acc(const SmemAcc &, uint32_t) {}
 
 // min over the query run's objects x one reference object
 __device__ __forceinline__ int min_diff_obj(uint32_t robj, uint32_t q0, int s, const uint64_t *__restrict__ qrun,
@@ -443,28 +513,27 @@ __device__ __forceinline__ void process_entry(const CountParams &P, uint64_t i, 
 // Membership filter of an index's contexts, cut into key-range stripes: stripe s holds
 // the contexts of [bounds[s], bounds[s+1]) (quantiles of the sorted contexts, so every
 // stripe holds U / S of them) in a power of two of 32-byte blocks, at most 16 MB per
-// stripe and at least 8 bits per context; each context sets 4 bits in one 16-byte half
-// of its block.  A query context whose bits are not all set is not in the index and
+// stripe and at least 8 bits per context; each context sets a bit in each word of one
+// 16-byte half of its block.  A query context whose bits are not all set is not in the index and
 // needs no table probe: for queries of other genomes most contexts are absent (a
 // 10,000 x 20,000 block: 88%), and each absent context would otherwise cost a random
 // table line from HBM.  A filter read at random as a whole does not stay in L2 once it
 // is tens of MB; a count that walks the query keys stripe by stripe keeps only the
 // current stripe's part hot (k_count_striped).
 struct BloomBits {
-    uint32_t block, half, p[4];
+    uint32_t half;  // 16-byte half of a block, of the stripe's halves
+    uint32_t r;     // five bits for each of its four words, from the top
 };
+// One multiplication for the half and one for the bits: the filter is asked for every entry,
+// and hashing took a third of the count's instructions (two rounds of a 64-bit finalizer, bits
+// anywhere in the half: 40 more per entry).
 __device__ __forceinline__ BloomBits bloom_bits(unsigned long long ctx, uint32_t mask)
 {
-    const unsigned long long h = mix64(mix64(ctx) ^ 0x243F6A8885A308D3ull);
-    BloomBits b;
-    b.block = (uint32_t)h & mask;
-    b.half = (uint32_t)(h >> 32) & 1u;
-    b.p[0] = (uint32_t)(h >> 33) & 127u;
-    b.p[1] = (uint32_t)(h >> 40) & 127u;
-    b.p[2] = (uint32_t)(h >> 47) & 127u;
-    b.p[3] = (uint32_t)(h >> 54) & 127u;
-    return b;
+    const unsigned long long p = ctx * 0x9E3779B97F4A7C15ull;
+    const uint32_t r = (uint32_t)(p >> 20) * 0x85EBCA6Bu;
+    return BloomBits{(((uint32_t)(p >> 32) & mask) << 1) | ((r >> 11) & 1u), r};
 }
+__device__ __forceinline__ uint32_t bloom_bit(uint32_t r, int word) { return (r >> (27 - 5 * word)) & 31u; }
 
 // stripe of a context: the largest s < S with bounds[s] <= ctx (bounds[0] = 0)
 __device__ __forceinline__ uint32_t stripe_of(const unsigned long long *__restrict__ bounds, int S,
@@ -479,47 +548,43 @@ __device__ __forceinline__ uint32_t stripe_of(const unsigned long long *__restri
 
 // Filter loads ask L2 to keep their lines (evict_last), so that the streamed query
 // keys and the random table lines do not push the filter out of L2.
-__device__ __forceinline__ uint4 ld_keep_l2(const uint4 *p)
+__device__ __forceinline__ unsigned long long keep_l2_policy()
+{
+    unsigned long long pol;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+    return pol;
+}
+__device__ __forceinline__ uint4 ld_keep_l2(const uint4 *p, unsigned long long policy)
 {
     uint4 r;
-    unsigned long long pol;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
     asm volatile("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-                 : "l"(p), "l"(pol));
+                 : "l"(p), "l"(policy));
     return r;
 }
 
-// f: the context's stripe of the filter
-__device__ __forceinline__ bool bloom_may_hold(const uint4 *__restrict__ f, uint32_t mask, unsigned long long ctx)
+// whether a context's bit is set in each of its half's words
+__device__ __forceinline__ bool bloom_all(const uint4 &w, const BloomBits &b)
 {
-    const BloomBits b = bloom_bits(ctx, mask);
-    const uint4 w = ld_keep_l2(f + 2 * (size_t)b.block + b.half);
-    bool all = true;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t p = b.p[i];  // word by selects (a dynamically indexed array would live in local memory)
-        const uint32_t word = (p & 64) ? ((p & 32) ? w.w : w.z) : ((p & 32) ? w.y : w.x);
-        all &= (word >> (p & 31)) & 1u;
-    }
-    return all;
+    return ((w.x >> bloom_bit(b.r, 0)) & (w.y >> bloom_bit(b.r, 1)) & (w.z >> bloom_bit(b.r, 2)) &
+            (w.w >> bloom_bit(b.r, 3)) & 1u) != 0;
 }
 
 // The filter as one kernel sees it: a whole filter whose stripe is found per context,
-// or (stripes == 1) the one stripe the caller works in.
+// or (stripes == 1) the one stripe the caller works in.  f null: no filter.
 struct FilterView {
     const uint4 *f;
     uint32_t mask;
     int stripes;
     const unsigned long long *bounds;
-    __device__ __forceinline__ bool may_hold(unsigned long long ctx) const
+    unsigned long long policy;  // keep_l2_policy()
+    __device__ __forceinline__ uint4 load(unsigned long long ctx, BloomBits &b) const
     {
-        if (!f)
-            return true;
         const uint4 *base = f;
         if (stripes > 1)
             base += 2 * ((size_t)mask + 1) * stripe_of(bounds, stripes, ctx);
-        return bloom_may_hold(base, mask, ctx);
+        b = bloom_bits(ctx, mask);
+        return ld_keep_l2(base + b.half, policy);
     }
 };
 
@@ -529,11 +594,11 @@ __global__ void k_bloom_insert(const unsigned long long *__restrict__ gkey, uint
     for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < u; g += (uint64_t)gridDim.x * blockDim.x) {
         const unsigned long long ctx = gkey[g];
         const BloomBits b = bloom_bits(ctx, mask);
-        const size_t blk = (size_t)(stripes > 1 ? stripe_of(bounds, stripes, ctx) : 0) * ((size_t)mask + 1) + b.block;
-        uint32_t *half = f + (2 * blk + b.half) * 4;
+        const size_t stripe = stripes > 1 ? stripe_of(bounds, stripes, ctx) : 0;
+        uint32_t *half = f + (2 * stripe * ((size_t)mask + 1) + b.half) * 4;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            atomicOr(half + (b.p[i] >> 5), 1u << (b.p[i] & 31));
+            atomicOr(half + i, 1u << bloom_bit(b.r, i));
     }
 }
 
@@ -590,22 +655,32 @@ __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ p
                                                   int qgid, int ignoreconflict, const Acc &acc, const Acc &uacc,
                                                   uint32_t lane)
 {
-    const uint32_t q0 = (uint32_t)(__ldg(qrun) & objmask);
+    // the query run's first 32 objects, one a lane; the next postings are loaded while these
+    // are compared
+    const uint32_t mine = (int)lane < s ? (uint32_t)(__ldg(qrun + lane) & objmask) : 0u;
+    const uint32_t q0 = __shfl_sync(0xFFFFFFFFu, mine, 0);
     uint32_t owners = 0, sole_gid = 0;
     int sole_d = 0;
     bool sole_mine = false, sole_ok = false;
+    uint64_t next = pb + lane < pe ? __ldg(post + pb + lane) : 0;
     for (uint32_t p0 = pb; p0 < pe; p0 += 32) {
         const uint32_t p = p0 + lane;
         const bool in = p < pe;
-        const uint64_t w = in ? __ldg(post + p) : 0;
+        const uint64_t w = next;
+        next = p + 32 < pe ? __ldg(post + p + 32) : 0;
         const uint32_t gid = (uint32_t)(w >> 32);
         uint32_t pg = __shfl_up_sync(0xFFFFFFFFu, gid, 1);
         if (lane == 0)
             pg = p0 > pb ? (uint32_t)(__ldg(post + p0 - 1) >> 32) : 0xFFFFFFFFu;
         const bool live = in && (!LOWER || (int)gid < qgid);
         const bool head = live && gid != pg;
+        int d = min(kMinInit, dna_pop((uint32_t)w ^ q0));
+        for (int k = 1; k < s; ++k) {
+            const uint32_t o =
+                k < 32 ? __shfl_sync(0xFFFFFFFFu, mine, k) : (uint32_t)(__ldg(qrun + k) & objmask);
+            d = min(d, dna_pop((uint32_t)w ^ o));
+        }
         if (head) {
-            int d = min_diff_obj((uint32_t)w, q0, s, qrun, objmask, kMinInit);
             uint32_t x = p + 1;
             while (x < pe) {
                 const uint64_t w2 = __ldg(post + x);
@@ -616,7 +691,7 @@ __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ p
             }
             const bool counted = !(ignoreconflict && x - p > 1);
             if (counted)
-                acc.add(gid, d);
+                acc.add_spread(gid, d);
             sole_mine = true;
             sole_gid = gid;
             sole_d = d;
@@ -630,78 +705,222 @@ __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ p
         uacc.add(sole_gid, sole_d);
 }
 
+// A query's object at a wide group, as the counting kernels hand it to the block join: the
+// object (at most 30 bits), the first entry of a run of several, or none.
+constexpr uint32_t kWideRun = 0x80000000u, kWideRunMost = 0x7FFFFFFFu, kWideNone = 0xFFFFFFFFu;
+constexpr int kWideObjBits = 30;
+
+// Shared memory of one warp of the counting kernels: entries that passed the filter, and
+// the found contexts whose postings are dealt out over the lanes.
+constexpr uint32_t kProbeLoads = 2;                      // entries of a lane whose loads are in flight together
+constexpr uint32_t kProbeQueue = 32 * kProbeLoads + 31;  // entries waiting: a part of a batch, and a round's
+constexpr uint32_t kPostLoads = 2;  // postings of a lane whose loads are in flight together
+struct ProbeQueue {
+    unsigned long long key[kProbeQueue];
+    uint32_t at[kProbeQueue];  // entry - cb
+    unsigned long long payload[32];
+    uint32_t object[32], start[32];
+};
+
+// One entry per lane below `count`: the hash probe, and the credits of what it finds.  A run
+// of one object on a conflict-free index credits each posting by itself, so the postings of
+// all the warp's found contexts (short groups and inline single postings) are dealt out
+// over the lanes, 32 at a time; walked each by its own lane, the longest group holds up
+// the others.  Runs of several objects and indexes with conflicts are walked by their lane,
+// groups of at least kWarpWalk postings by the warp, or (WIDE) left to the tensor cores.
+template <bool LOWER, bool UNIQUE, bool WIDE, class Acc>
+__device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q, uint32_t first, uint32_t count,
+                                            uint64_t cb, uint64_t e, int qgid, uint64_t objmask, const Acc &acc,
+                                            const Acc &uacc, uint32_t lane)
+{
+    int s = 0;
+    uint64_t i = 0;
+    unsigned long long key = 0, payload = 0;
+    bool single = false, wide = false, flat = false;
+    if (lane < count) {
+        key = Q.key[first + lane];
+        i = cb + Q.at[first + lane];
+        const unsigned long long ctx = key >> P.obj_bits;
+        uint32_t slot = (uint32_t)mix64(ctx) & P.mask;
+        ulonglong2 sl = __ldg(reinterpret_cast<const ulonglong2 *>(P.table + slot));
+        s = 1;
+        while (i + s < e && (__ldg(P.qkeys + i + s) >> P.obj_bits) == ctx)
+            ++s;
+        bool found = false;
+        for (uint32_t probe = 0; probe <= P.mask; ++probe) {
+            if ((sl.x & ~kInlineBit) == ctx) {
+                found = true;
+                break;
+            }
+            if (sl.x == kEmptyCtx)
+                break;
+            slot = (slot + 1) & P.mask;
+            sl = __ldg(reinterpret_cast<const ulonglong2 *>(P.table + slot));
+        }
+        if (found) {
+            payload = sl.y;
+            single = (sl.x & kInlineBit) != 0;
+            const uint32_t pc = (uint32_t)(payload >> 32);
+            if (WIDE && !single && pc >= P.wide_min && (s == 1 || i < kWideRunMost))
+                P.wide_obj[(size_t)__ldg(P.wide_at + (uint32_t)payload) * P.wide_stride +
+                           (uint32_t)(qgid - P.qgid_offset)] =
+                    s == 1 ? (uint32_t)(key & objmask) : kWideRun | (uint32_t)i;
+            else if (!single && pc >= kWarpWalk)
+                wide = true;
+            else if (s == 1 && P.conflict_free)
+                flat = true;
+            else
+                credit_context<LOWER, UNIQUE>(P, i, s, payload, single, qgid, objmask, acc, uacc);
+        }
+    }
+    __syncwarp();
+    const unsigned hits = __ballot_sync(0xFFFFFFFFu, flat);
+    if (hits) {
+        const uint32_t n = flat ? (single ? 1u : (uint32_t)(payload >> 32)) : 0u;
+        uint32_t start = n;  // inclusive sum, then this lane's first posting
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, start, o);
+            if ((int)lane >= o)
+                start += v;
+        }
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, start, 31);
+        start -= n;
+        if (flat) {
+            const uint32_t at = __popc(hits & ((1u << lane) - 1u));
+            Q.payload[at] = payload;
+            Q.object[at] = (uint32_t)(key & objmask);
+            Q.start[at] = start | (single ? 0x80000000u : 0u);
+        }
+        __syncwarp();
+        for (uint32_t p0 = 0; p0 < total; p0 += 32 * kPostLoads) {
+            unsigned long long w[kPostLoads];  // in flight together: a batch of hits is a chain of HBM reads else
+            uint32_t own[kPostLoads];
+            bool one[kPostLoads];
+#pragma unroll
+            for (uint32_t x = 0; x < kPostLoads; ++x) {
+                const uint32_t base = p0 + 32 * x, p = base + lane;
+                // owner of posting p: the last hit that starts at or before it
+                const uint32_t before = __popc(__ballot_sync(0xFFFFFFFFu, flat && start < base));
+                const unsigned heads =
+                    __reduce_or_sync(0xFFFFFFFFu, flat && start - base < 32u ? 1u << (start - base) : 0u);
+                if (p < total) {
+                    own[x] = before + __popc(heads & (0xFFFFFFFFu >> (31 - lane))) - 1;
+                    w[x] = Q.payload[own[x]];
+                    const uint32_t st = Q.start[own[x]];
+                    one[x] = (st >> 31) != 0;
+                    if (!one[x])
+                        w[x] = __ldg(P.post + (uint32_t)w[x] + (p - st));
+                }
+            }
+#pragma unroll
+            for (uint32_t x = 0; x < kPostLoads; ++x) {
+                const uint32_t gid = (uint32_t)(w[x] >> 32);
+                if (p0 + 32 * x + lane < total && (!LOWER || (int)gid < qgid)) {
+                    const int d = min(kMinInit, dna_pop((uint32_t)w[x] ^ Q.object[own[x]]));
+                    acc.add(gid, d);
+                    if (UNIQUE && one[x])  // the context's only owner
+                        uacc.add(gid, d);
+                }
+            }
+        }
+        __syncwarp();
+    }
+    // the warp walks its lanes' long groups together, one after another
+    const uint32_t pb = (uint32_t)payload, pc = (uint32_t)(payload >> 32);
+    for (unsigned m = __ballot_sync(0xFFFFFFFFu, wide); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const uint32_t gb = __shfl_sync(0xFFFFFFFFu, pb, src), gc = __shfl_sync(0xFFFFFFFFu, pc, src);
+        const uint64_t gi = __shfl_sync(0xFFFFFFFFu, i, src);
+        const int gs = __shfl_sync(0xFFFFFFFFu, s, src);
+        walk_context_warp<LOWER, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
+                                         acc, uacc, lane);
+    }
+}
+
 // Entries [cb, ce) of one query (whose entries are [b, e)), taken by the caller's
-// threads t0, t0 + T, ... (t0 % 32 = the lane, T a multiple of 32): every lane of a warp
-// takes one entry per round (the warp's rounds are the same for all its lanes).  Only the
-// first entry of a context run works (src/command_ani.h:498-505); the filter rules out
-// most absent contexts; one hash probe finds the context; the inline single posting is
-// credited at once, short groups are walked by their lane, long ones by the warp, or
-// (WIDE) left to the tensor cores.
+// threads t0, t0 + T, ... (t0 % 32 = the lane, T a multiple of 32): a warp loads
+// kProbeLoads entries a lane and their filter words at a time.  Only the first entry of a
+// context run works (src/command_ani.h:498-505); the filter rules out most absent contexts
+// (88 % of the entries of new assemblies); the others wait in the warp's queue until 32 of
+// them probe the table together, so that no lane idles in the probe and the walk.
 template <bool LOWER, bool UNIQUE, bool WIDE, class Acc>
 __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, uint64_t e, uint64_t cb, uint64_t ce,
                                               int qgid, uint64_t objmask, const Acc &acc, const Acc &uacc,
-                                              const FilterView &fv, uint64_t t0, uint64_t T)
+                                              const FilterView &fv, uint64_t t0, uint64_t T, ProbeQueue &Q)
 {
     const uint32_t lane = (uint32_t)(t0 & 31u);
-    for (uint64_t wb = cb + (t0 - lane); wb < ce; wb += T) {
-        const uint64_t i = wb + lane;
-        int s = 0;
-        unsigned long long ctx = 0;
-        uint32_t slot = 0;
-        if (i < ce) {
-            const uint64_t key = __ldg(P.qkeys + i);
-            ctx = key >> P.obj_bits;
-            const uint64_t prev = i > b ? __ldg(P.qkeys + i - 1) : 0;
-            if (prev > key)
+    uint32_t waiting = 0, seen = 0;
+    for (uint64_t wb = cb + (t0 - lane); wb < ce; wb += kProbeLoads * T) {
+        unsigned long long key[kProbeLoads], prev[kProbeLoads];
+        bool keep[kProbeLoads];
+#pragma unroll
+        for (uint32_t x = 0; x < kProbeLoads; ++x) {
+            const uint64_t i = wb + x * T + lane;
+            key[x] = i < ce ? __ldg(P.qkeys + i) : 0;
+            prev[x] = lane == 0 && i < ce && i > b ? __ldg(P.qkeys + i - 1) : 0;
+        }
+#pragma unroll
+        for (uint32_t x = 0; x < kProbeLoads; ++x) {
+            const uint64_t i = wb + x * T + lane;
+            const unsigned long long below = __shfl_up_sync(0xFFFFFFFFu, key[x], 1);
+            if (lane)
+                prev[x] = below;
+            if (i < ce && prev[x] > key[x])
                 atomicMax(P.err, (int)kDevUnsorted);  // a sample's keys must ascend (comblco order)
-            if (!(i > b && (prev >> P.obj_bits) == ctx) && fv.may_hold(ctx)) {
-                int run = 1;
-                while (i + run < e && (__ldg(P.qkeys + i + run) >> P.obj_bits) == ctx)
-                    ++run;
-                s = run;
-                slot = (uint32_t)mix64(ctx) & P.mask;
-            }
+            keep[x] = i < ce && !(i > b && (prev[x] >> P.obj_bits) == (key[x] >> P.obj_bits));
         }
-        bool wide = false;
-        uint32_t pb = 0, pc = 0;
-        if (s) {
-            ulonglong2 sl = __ldg(reinterpret_cast<const ulonglong2 *>(P.table + slot));
-            uint32_t at = slot;
-            bool found = false;
-            for (uint32_t probe = 0; probe <= P.mask; ++probe) {
-                if ((sl.x & ~kInlineBit) == ctx) {
-                    found = true;
-                    break;
-                }
-                if (sl.x == kEmptyCtx)
-                    break;
-                at = (at + 1) & P.mask;
-                sl = __ldg(reinterpret_cast<const ulonglong2 *>(P.table + at));
-            }
-            if (found) {
-                const bool single = (sl.x & kInlineBit) != 0;
-                pb = (uint32_t)sl.y;
-                pc = (uint32_t)(sl.y >> 32);
-                if (WIDE && !single && s == 1 && pc >= P.wide_min)
-                    P.wide_obj[(size_t)__ldg(P.wide_at + pb) * P.wide_stride + (uint32_t)(qgid - P.qgid_offset)] =
-                        (uint32_t)(__ldg(P.qkeys + i) & objmask);
-                else if (!single && pc >= kWarpWalk)
-                    wide = true;
-                else
-                    credit_context<LOWER, UNIQUE>(P, i, s, sl.y, single, qgid, objmask, acc, uacc);
-            }
+        if (fv.f) {
+            uint4 w[kProbeLoads];
+            BloomBits bits[kProbeLoads];
+#pragma unroll
+            for (uint32_t x = 0; x < kProbeLoads; ++x)
+                if (keep[x])
+                    w[x] = fv.load(key[x] >> P.obj_bits, bits[x]);
+#pragma unroll
+            for (uint32_t x = 0; x < kProbeLoads; ++x)
+                keep[x] = keep[x] && bloom_all(w[x], bits[x]);
         }
-        // the warp walks its lanes' long groups together, one after another
-        for (unsigned m = __ballot_sync(0xFFFFFFFFu, wide); m; m &= m - 1) {
-            const int src = __ffs(m) - 1;
-            const uint32_t gb = __shfl_sync(0xFFFFFFFFu, pb, src), gc = __shfl_sync(0xFFFFFFFFu, pc, src);
-            const uint64_t gi = __shfl_sync(0xFFFFFFFFu, i, src);
-            const int gs = __shfl_sync(0xFFFFFFFFu, s, src);
-            walk_context_warp<LOWER, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
-                                             acc, uacc, lane);
+#pragma unroll
+        for (uint32_t x = 0; x < kProbeLoads; ++x) {
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, keep[x]);
+            if (keep[x]) {
+                const uint32_t at = waiting + __popc(m & ((1u << lane) - 1u));
+                Q.key[at] = key[x];
+                Q.at[at] = (uint32_t)(wb + x * T + lane - cb);
+            }
+            waiting += __popc(m);
+        }
+        __syncwarp();
+        while (waiting >= 32) {
+            waiting -= 32;
+            probe_batch<LOWER, UNIQUE, WIDE>(P, Q, waiting, 32, cb, e, qgid, objmask, acc, uacc, lane);
+        }
+        __syncwarp();
+        seen += 32 * kProbeLoads;
+        if (seen + 32 * kProbeLoads > kWarpCellEntries - 32) {  // those waiting were seen before
+            flush_acc(acc, lane);
+            if (UNIQUE)
+                flush_acc(uacc, lane);
+            seen = 0;
         }
     }
+    if (waiting)
+        probe_batch<LOWER, UNIQUE, WIDE>(P, Q, 0, waiting, cb, e, qgid, objmask, acc, uacc, lane);
+    flush_acc(acc, lane);
+    if (UNIQUE)
+        flush_acc(uacc, lane);
 }
+
+// Entries of a chunk of the chunk-major kernel: at most `most`, fewer when a block of
+// `total` entries would not give `ctas` chunks, at least one round of a CTA's threads.
+__host__ __device__ __forceinline__ uint32_t count_chunk(uint64_t total, uint32_t most, uint32_t ctas)
+{
+    const uint64_t even = (total / ctas + 255) / 256 * 256;
+    return even < 256 ? (most < 256 ? most : 256) : even < most ? (uint32_t)even : most;
+}
+
+constexpr int kCountThreads = 256;
 
 // Batched persistent kernel: CTAs take whole queries from a work counter
 // (largest first); with SMEM the query's reference row is accumulated in shared
@@ -709,14 +928,23 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
 // row with atomics, and the work may be split into key-range chunks (P.items) so
 // that one large query (a read set) spreads over many SMs.
 template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE>
-__global__ void __launch_bounds__(512) k_count_batched(CountParams P)
+__global__ void __launch_bounds__(kCountThreads, 4) k_count_batched(CountParams P)
 {
     extern __shared__ uint32_t sm[];
+    __shared__ ProbeQueue queues[kCountThreads / 32];
+    __shared__ WarpCells cells[SMEM ? 1 : UNIQUE ? 2 : 1][SMEM ? 1 : kCountThreads / 32];
     __shared__ int s_item;
     const uint64_t objmask = (P.obj_bits >= 64) ? ~0ull : ((1ull << P.obj_bits) - 1);
     const uint64_t base = P.qoffs[0];
     const int nref = P.nref;
-    const FilterView fv{P.bloom, P.bloom_mask, P.bloom_stripes, P.bloom_bounds};
+    const FilterView fv{P.bloom, P.bloom_mask, P.bloom_stripes, P.bloom_bounds, keep_l2_policy()};
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t chunk_keys = P.chunk_auto ? count_chunk(P.qoffs[P.nq] - base, P.chunk_keys, P.chunk_auto) : P.chunk_keys;
+    if (!SMEM) {
+        WarpAcc{{}, &cells[0][warp]}.clear(lane);
+        if (UNIQUE)
+            WarpAcc{{}, &cells[UNIQUE][warp]}.clear(lane);
+    }
     for (;;) {
         if (threadIdx.x == 0)
             s_item = (int)atomicAdd(P.work, 1u);
@@ -755,19 +983,22 @@ __global__ void __launch_bounds__(512) k_count_batched(CountParams P)
         if (SMEM) {
             const SmemAcc acc{row0, row0 + nref, row0 + 2 * nref, row0 + 3 * nref};
             const SmemAcc uacc{row1, row1 + nref, row1 + 2 * nref, row1 + 3 * nref};
-            process_query<LOWER, UNIQUE, WIDE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
+            process_query<LOWER, UNIQUE, WIDE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x,
+                                               queues[warp]);
         } else {
-            const GlobalAcc acc{P.out_ctx + row, P.out_obj + row};
-            const GlobalAcc uacc{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr};
+            const WarpAcc acc{{P.out_ctx + row, P.out_obj + row}, &cells[0][warp]};
+            const WarpAcc uacc{{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr},
+                               &cells[UNIQUE && !SMEM][warp]};
             uint64_t cb = b, ce = e;
             if (P.items) {
                 cb = P.items[it].b;
                 ce = P.items[it].e;
             } else if (vchunks) {
-                cb = b + (uint64_t)(it - (int)P.chunk_prefix[q]) * P.chunk_keys;
-                ce = min(e, cb + (uint64_t)P.chunk_keys);
+                cb = b + (uint64_t)(it - (int)P.chunk_prefix[q]) * chunk_keys;
+                ce = min(e, cb + (uint64_t)chunk_keys);
             }
-            process_query<LOWER, UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
+            process_query<LOWER, UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x,
+                                               queues[warp]);
         }
         __syncthreads();
         if (SMEM) {
@@ -788,42 +1019,53 @@ __global__ void __launch_bounds__(512) k_count_batched(CountParams P)
 // Stripe-major global-row kernel: the work items are chunks of one query's entries
 // whose contexts fall in one filter stripe, listed stripe by stripe (k_stripe_expand),
 // so that at any time the SMs probe one stripe of the filter and it stays in L2 while
-// the query keys stream past.  Each warp takes kStripeGrab chunks at a time from the
-// work counter; its lanes stride over a chunk's entries.  Counters go to the zeroed
-// global rows with atomics, as in the chunked mode.
-constexpr uint32_t kStripeGrab = 2;
-
+// the query keys stream past.  Each warp takes a chunk at a time from the work counter
+// (two at a time, or the next one asked for while one is counted: 281 and 269 instead of
+// 252 us for 1,500 queries x 2,000 references, the last chunks wait longer); its lanes
+// stride over the chunk's entries.  Counters go to the zeroed global rows through the
+// warp's own cells, as in the chunked mode.
+//
+// Bound by the latency of dependent reads (filter, table, postings) at 32 warps a SM.
+// Measured (B200, whole calls): 1,500 assemblies x 2,000 references 341 -> 262 us, 40 read
+// sets x 2,000 with unique contexts 357 -> 211 us, 1,500 x 2,000 in species of 24 with
+// unique contexts 972 -> 730 us.
 template <bool LOWER, bool UNIQUE, bool WIDE>
-__global__ void __launch_bounds__(512) k_count_striped(CountParams P)
+__global__ void __launch_bounds__(kCountThreads, 4) k_count_striped(CountParams P)
 {
-    const uint32_t lane = threadIdx.x & 31u;
+    __shared__ ProbeQueue queues[kCountThreads / 32];
+    __shared__ WarpCells cells[UNIQUE ? 2 : 1][kCountThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    WarpAcc{{}, &cells[0][warp]}.clear(lane);
+    if (UNIQUE)
+        WarpAcc{{}, &cells[UNIQUE][warp]}.clear(lane);
     const uint64_t objmask = (P.obj_bits >= 64) ? ~0ull : ((1ull << P.obj_bits) - 1);
     const uint64_t base = P.qoffs[0];
     const uint32_t nitems = *P.nitems_dev;
+    const unsigned long long policy = keep_l2_policy();
     const size_t stripe_words = 2 * ((size_t)P.bloom_mask + 1);  // uint4 per stripe
     for (;;) {
-        uint32_t it0 = 0;
+        uint32_t it = 0;
         if (lane == 0)
-            it0 = atomicAdd(P.work, kStripeGrab);
-        it0 = __shfl_sync(0xFFFFFFFFu, it0, 0);
-        if (it0 >= nitems)
+            it = atomicAdd(P.work, 1u);
+        it = __shfl_sync(0xFFFFFFFFu, it, 0);
+        if (it >= nitems)
             break;
-        const uint32_t it1 = min(nitems, it0 + kStripeGrab);
-        for (uint32_t it = it0; it < it1; ++it) {
-            const WorkItem w = P.items[it];
-            const int q = (int)w.q;
-            const uint64_t b = P.qoffs[q] - base, e = P.qoffs[q + 1] - base;
-            const size_t row = (size_t)q * P.nref;
-            const GlobalAcc acc{P.out_ctx + row, P.out_obj + row};
-            const GlobalAcc uacc{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr};
-            const FilterView fv{P.bloom + stripe_words * w.pad, P.bloom_mask, 1, nullptr};
-            process_query<LOWER, UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32);
-        }
+        const WorkItem w = P.items[it];
+        const int q = (int)w.q;
+        const uint64_t b = P.qoffs[q] - base, e = P.qoffs[q + 1] - base;
+        const size_t row = (size_t)q * P.nref;
+        const WarpAcc acc{{P.out_ctx + row, P.out_obj + row}, &cells[0][warp]};
+        const WarpAcc uacc{{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr},
+                           &cells[UNIQUE][warp]};
+        const FilterView fv{P.bloom + stripe_words * w.pad, P.bloom_mask, 1, nullptr, policy};
+        process_query<LOWER, UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32,
+                                           queues[warp]);
     }
 }
 
 // chunk size of the stripe-major items: kStripeChunk entries, more for blocks so large
-// that the chunks would exceed kStripeItemsMax
+// that the chunks would exceed kStripeItemsMax (1,500 queries x 2,000 references: 252 us
+// with chunks of 256, 264 of 128 and 293 of 512, where the last few hold up the end)
 __device__ __forceinline__ uint64_t stripe_chunk(const uint64_t *__restrict__ qoffs, int nq)
 {
     const uint64_t total = qoffs[nq] - qoffs[0];
@@ -856,28 +1098,38 @@ __global__ void k_stripe_counts(const uint64_t *__restrict__ spos, const uint64_
 }
 
 // the chunks themselves, at their scanned offsets: {query, stripe, begin, end} with
-// offsets relative to the block's first entry
+// offsets relative to the block's first entry.  One thread per chunk (pre[n] of them; its
+// query and stripe by a search of the offsets): a read set has hundreds of chunks in one
+// stripe, which a thread per (query, stripe) wrote one after another (40 read sets: 83 us).
 __global__ void k_stripe_expand(const uint64_t *__restrict__ spos, const uint64_t *__restrict__ qoffs, int nq,
                                 int stripes, const uint32_t *__restrict__ pre, WorkItem *__restrict__ items)
 {
     const uint64_t ck = stripe_chunk(qoffs, nq);
     const uint64_t base = qoffs[0];
     const uint64_t n = (uint64_t)stripes * nq;
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
-        const int st = (int)(t / (uint64_t)nq), q = (int)(t % (uint64_t)nq);
+    const uint32_t total = pre[n];
+    for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < total; o += gridDim.x * blockDim.x) {
+        uint64_t lo = 0, hi = n - 1;  // the last (stripe, query) whose first chunk is at or before o
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi + 1) >> 1;
+            if (__ldg(pre + mid) <= o)
+                lo = mid;
+            else
+                hi = mid - 1;
+        }
+        const int st = (int)(lo / (uint64_t)nq), q = (int)(lo % (uint64_t)nq);
         const uint64_t *sp = spos + (size_t)q * (stripes + 1) + st;
-        const uint64_t b = sp[0] - base, e = sp[1] - base;
-        uint32_t o = pre[t];
-        for (uint64_t c = b; c < e && o < pre[t + 1]; c += ck)
-            items[o++] = WorkItem{(uint32_t)q, (uint32_t)st, c, min(e, c + ck)};
+        const uint64_t c = sp[0] - base + (uint64_t)(o - pre[lo]) * ck;
+        items[o] = WorkItem{(uint32_t)q, (uint32_t)st, c, min(sp[1] - base, c + ck)};
     }
 }
 
 // counts[q] = chunk-entry chunks of query q; prefix[0] = 0 (a scan of counts fills
 // prefix[1..nq])
-__global__ void k_chunk_counts(const uint64_t *__restrict__ qoffs, int nq, uint32_t chunk,
+__global__ void k_chunk_counts(const uint64_t *__restrict__ qoffs, int nq, uint32_t most, uint32_t ctas,
                                uint32_t *__restrict__ counts, uint32_t *__restrict__ prefix)
 {
+    const uint32_t chunk = count_chunk(qoffs[nq] - qoffs[0], most, ctas);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         if (q == 0)
             prefix[0] = 0;
@@ -2756,7 +3008,7 @@ int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStr
     if (smem > 48 * 1024)
         CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCountThreads, smem));
     if (per_sm < 1)
         return fail(KSSDGPU_ERR_CAPACITY, "shared-memory row does not fit one CTA");
     int grid = ix->sms * per_sm;
@@ -2765,7 +3017,7 @@ int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStr
     if (grid > units)
         grid = std::max(units, 1);
     CUDA_TRY(cudaMemsetAsync(P.work, 0, sizeof(unsigned int), st));
-    kern<<<grid, 512, smem, st>>>(P);
+    kern<<<grid, kCountThreads, smem, st>>>(P);
     count_launch();
     CUDA_TRY(cudaGetLastError());
     return KSSDGPU_OK;
@@ -2776,10 +3028,10 @@ int launch_striped(kssdgpu_index *ix, const CountParams &P, cudaStream_t st)
 {
     auto kern = k_count_striped<LOWER, UNIQUE, WIDE>;
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, 0));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCountThreads, 0));
     const int grid = ix->sms * std::max(per_sm, 1);  // persistent: the item count stays on the device
     CUDA_TRY(cudaMemsetAsync(P.work, 0, sizeof(unsigned int), st));
-    kern<<<grid, 512, 0, st>>>(P);
+    kern<<<grid, kCountThreads, 0, st>>>(P);
     count_launch();
     CUDA_TRY(cudaGetLastError());
     return KSSDGPU_OK;
@@ -2878,7 +3130,7 @@ uint64_t wide_block_bytes(const kssdgpu_index *ix, uint64_t nq)
 // rows of both sides, the products, and the pairs to correct.
 bool wide_block_chosen(const kssdgpu_index *ix, int nq, unsigned flags)
 {
-    if (ix->f_conflict || !ix->f_wgroups || ix->nref > (int)kWideMaxRefs || ix->obj_bits >= 32 ||
+    if (ix->f_conflict || !ix->f_wgroups || ix->nref > (int)kWideMaxRefs || ix->obj_bits > kWideObjBits ||
         (flags & (KSSDGPU_PLAIN | KSSDGPU_GLOBAL_ACC | KSSDGPU_SMEM_ACC)))
         return false;
     const double n = (double)ix->nref, q = (double)nq;
@@ -2917,7 +3169,8 @@ int wide_block_begin(kssdgpu_index *ix, int nq, CountParams &P, cudaStream_t st)
 
 // After it: per pass of kWidePass groups the operand rows of both sides and the
 // corrections, the six products in one batched GEMM, and the counters added to the rows.
-int wide_block_end(kssdgpu_index *ix, int nq, unsigned long long *oc, unsigned long long *oo, cudaStream_t st)
+int wide_block_end(kssdgpu_index *ix, int nq, const CountParams &P, unsigned long long *oc, unsigned long long *oo,
+                   cudaStream_t st)
 {
     const uint32_t n = (uint32_t)ix->nref, npad = (uint32_t)wide_npad(n), nqp = (uint32_t)wide_npad((uint64_t)nq);
     const uint64_t pass = wide_pass(ix);
@@ -2932,7 +3185,7 @@ int wide_block_end(kssdgpu_index *ix, int nq, unsigned long long *oc, unsigned l
     CUDA_TRY(wide_rows_shape(ix, k_wide_rows<true>, npad, warps, rows_grid));
     for (uint64_t c0 = 0; c0 < ix->f_wgroups; c0 += pass) {
         const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
-        const WideBlock Q{ix->w_qobj.p + c0 * nqp, (uint32_t)nq, nqp, ix->w_y.p, ys};
+        const WideBlock Q{ix->w_qobj.p + c0 * nqp, (uint32_t)nq, nqp, ix->w_y.p, ys, P.qkeys, P.qoffs, P.obj_bits};
         k_wide_rows<true><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
                             warps * wide_warp_smem(npad, n), st>>>(nullptr, ix->w_list.p + c0, cn, ix->post, n, npad,
                                                                    ix->w_x.p, xs, ix->w_corr.p, Q);
@@ -2981,6 +3234,7 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
     P.bloom_mask = ix->bloom_mask;
     P.bloom_stripes = ix->bloom_stripes;
     P.bloom_bounds = ix->bloom_bounds;
+    P.conflict_free = !ix->f_conflict;
     const size_t cells = (size_t)nq * ix->nref;
     if (nq == 0)
         return KSSDGPU_OK;
@@ -3009,7 +3263,7 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
                                                       ix->s_spos.p);
         k_stripe_counts<<<grid_for(nsq + 1), 256, 0, st>>>(ix->s_spos.p, d_offs, nq, S, ix->s_scnt.p, ix->err);
         CUDA_TRY(cub::DeviceScan::ExclusiveSum(ix->s_cubtmp.p, tb, ix->s_scnt.p, ix->s_spre.p, (int64_t)nsq + 1, st));
-        k_stripe_expand<<<grid_for(nsq), 256, 0, st>>>(ix->s_spos.p, d_offs, nq, S, ix->s_spre.p, ix->s_sitems.p);
+        k_stripe_expand<<<ix->sms * 4, 256, 0, st>>>(ix->s_spos.p, d_offs, nq, S, ix->s_spre.p, ix->s_sitems.p);
         count_launch(4);
         P.items = ix->s_sitems.p;
         P.nitems_dev = ix->s_spre.p + nsq;
@@ -3025,8 +3279,10 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
         size_t tb = 0;
         CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, tb, ix->s_counts.p, ix->s_prefix.p + 1, nq, st));
         CUDA_TRY(ix->s_cubtmp.ensure(tb));
+        P.chunk_auto = (uint32_t)ix->sms * 8;
         k_chunk_counts<<<std::min((nq + 255) / 256, ix->sms * 8), 256, 0, st>>>(d_offs, nq, ix->count_chunk_keys,
-                                                                                ix->s_counts.p, ix->s_prefix.p);
+                                                                                P.chunk_auto, ix->s_counts.p,
+                                                                                ix->s_prefix.p);
         CUDA_TRY(cub::DeviceScan::InclusiveSum(ix->s_cubtmp.p, tb, ix->s_counts.p, ix->s_prefix.p + 1, nq, st));
         count_launch(3);
         P.chunk_prefix = ix->s_prefix.p;
@@ -3071,7 +3327,7 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
         rc = lower ? launch_batched<true, false, false>(ix, P, 0, st)
                    : unique ? launch_batched<false, true, false>(ix, P, 0, st)
                             : launch_batched<false, false, false>(ix, P, 0, st);
-    return rc || !wide ? rc : wide_block_end(ix, nq, oc, oo, st);
+    return rc || !wide ? rc : wide_block_end(ix, nq, P, oc, oo, st);
 }
 
 // A host-buffer count is split into sub-blocks whose copies overlap the counting when
@@ -3210,7 +3466,7 @@ int count_host_impl(kssdgpu_index *ix, const uint64_t *qkeys, const uint64_t *qo
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sizes[a] > sizes[b]; });
     std::vector<WorkItem> items;
     if (!uses_smem_row(ix, flags) && !(flags & KSSDGPU_PLAIN))
-        build_chunks(qoffs, nq, order.data(), ix->count_chunk_keys, items);
+        build_chunks(qoffs, nq, order.data(), count_chunk(nkeys, ix->count_chunk_keys, (uint32_t)ix->sms * 8), items);
     const size_t cells = (size_t)nq * ix->nref;
     const int nout = unique ? 4 : 2;
     CUDA_TRY(ix->s_keys.ensure(nkeys));
@@ -5252,6 +5508,7 @@ int kssdgpu_count_block_noalloc(kssdgpu_index_t *ix, const uint64_t *d_qry_keys,
     P.bloom_mask = ix->bloom_mask;
     P.bloom_stripes = ix->bloom_stripes;
     P.bloom_bounds = ix->bloom_bounds;
+    P.conflict_free = !ix->f_conflict;
     P.order = use_smem ? reinterpret_cast<const int *>(scr + kNoallocHeaderWords) : nullptr;
     P.chunk_prefix = use_smem ? nullptr : scr + kNoallocHeaderWords - 1;
     P.chunk_keys = ix->count_chunk_keys;
@@ -5304,7 +5561,7 @@ int kssdgpu_count_detail(kssdgpu_index_t *ix, const uint64_t *qry_keys, const ui
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sizes[a] > sizes[b]; });
     std::vector<WorkItem> items;
     if (!uses_smem_row(ix, flags))
-        build_chunks(qry_offs, nq, order.data(), ix->count_chunk_keys, items);
+        build_chunks(qry_offs, nq, order.data(), count_chunk(nkeys, ix->count_chunk_keys, (uint32_t)ix->sms * 8), items);
     const int nref = ix->nref;
     const size_t cells = (size_t)nq * nref;
     CUDA_TRY(ix->s_keys.ensure(nkeys));
