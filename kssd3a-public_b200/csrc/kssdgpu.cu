@@ -14,7 +14,6 @@
 #include "kssd_metric.cuh"
 
 #include <cub/cub.cuh>
-#include <cub/device/device_segmented_sort.cuh>
 #include <thrust/iterator/transform_iterator.h>
 
 #include <algorithm>
@@ -2446,8 +2445,42 @@ struct DevBuf {
 // drfold, and becomes ctx << obj_bits | obj by extracting the mask's bits of the k-mer
 // on the chosen strand.  Per sample: sort, dedup, and without conflict mode the contexts
 // holding several objects dropped (src/command_sketch.c:4156-4188, src/kssdlib_sort.c:388-406).
+// A mask's bits packed from the low end (BMI2 pext): each of six steps moves the bits that
+// have a set bit of the step's power of two in their distance (the "compress" of Hacker's
+// Delight, 2nd ed., 7-4); the steps' masks are made once on the host.
+struct BitExtract {
+    unsigned long long mask, move[6];
+};
+BitExtract make_extract(unsigned long long m)
+{
+    BitExtract x;
+    x.mask = m;
+    unsigned long long mk = ~m << 1;  // zeros to the right of each bit
+    for (int i = 0; i < 6; ++i) {
+        unsigned long long mp = mk ^ (mk << 1);  // parallel suffix
+        for (int s = 2; s < 64; s <<= 1)
+            mp ^= mp << s;
+        const unsigned long long mv = mp & m;  // bits to move
+        x.move[i] = mv;
+        m = (m ^ mv) | (mv >> (1 << i));
+        mk &= ~mp;
+    }
+    return x;
+}
+__device__ __forceinline__ unsigned long long extract_bits(unsigned long long v, const BitExtract &x)
+{
+    v &= x.mask;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const unsigned long long t = v & x.move[i];
+        v = (v ^ t) | (t >> (1 << i));
+    }
+    return v;
+}
+
 struct SketchGeom {
     unsigned long long ctxmask, tupmask;
+    BitExtract ctx, obj;
     int klen, obj_bits;
     uint32_t filter;
 };
@@ -2462,35 +2495,20 @@ __host__ __device__ __forceinline__ unsigned long long splitmix64(unsigned long 
     return x ^ (x >> 31);
 }
 
-// bits of x under mask m, packed from the low end (BMI2 pext)
-__device__ __forceinline__ unsigned long long extract_bits(unsigned long long x, unsigned long long m)
+// 2-bit codes of four bases, 0xFF for anything but A/C/G/T in either case
+__device__ __forceinline__ uint32_t base_codes(uint32_t w)
 {
-    unsigned long long r = 0;
-    int k = 0;
-    while (m) {
-        const int b = __ffsll((long long)m) - 1;
-        r |= ((x >> b) & 1ull) << k++;
-        m &= m - 1;
-    }
-    return r;
-}
-
-// 2-bit code of a base, -1 for anything but A/C/G/T in either case
-__device__ __forceinline__ int base_code(unsigned char c)
-{
-    switch (c | 0x20) {
-    case 'a': return 0;
-    case 'c': return 1;
-    case 'g': return 2;
-    case 't': return 3;
-    default: return -1;
-    }
+    const uint32_t l = w | 0x20202020u;
+    const uint32_t ok = __vcmpeq4(l, 0x61616161u) | __vcmpeq4(l, 0x63636363u) | __vcmpeq4(l, 0x67676767u) |
+                        __vcmpeq4(l, 0x74747474u);
+    return (((w >> 1) ^ (w >> 2)) & 0x03030303u) | ~ok;  // a, c, g, t: 0, 1, 2, 3
 }
 
 constexpr int kSketchThreads = 256;
-constexpr int kSketchSpan = 64;                               // k-mer end positions per thread
+constexpr int kSketchSpan = 128;                              // k-mer end positions per thread
 constexpr int kSketchTile = kSketchThreads * kSketchSpan;     // bytes per CTA
 constexpr int kSketchHalo = 32;                               // >= klen - 1 bytes before the tile
+constexpr int kSketchList = 64 + 32;                          // a warp's kept k-mers before they are written
 
 // largest i in [0, n) with a[i] <= v (a[0] <= v)
 __device__ __forceinline__ uint64_t last_le(const uint64_t *__restrict__ a, uint64_t n, uint64_t v)
@@ -2506,108 +2524,184 @@ __device__ __forceinline__ uint64_t last_le(const uint64_t *__restrict__ a, uint
     return lo;
 }
 
-// Pass 1 (WRITE = false): kept k-mers per thread (counts) and per sample; pass 2: the
-// keys, each thread's at out[pos[thread] ...] (byte order, so grouped by sample).
-// Records rec_offs[r]..rec_offs[r+1] of seq; sample s = records samp_recs[s]..samp_recs[s+1].
-template <bool WRITE>
+// Place of the code at tile position p (from -kSketchHalo on): a thread's 128 bytes and 4
+// more, so that the lanes of a warp, each on its own stretch, read 33 words apart and meet
+// in no bank.
+__device__ __forceinline__ int sketch_at(int p)
+{
+    return p + kSketchHalo + ((p + kSketchSpan) / kSketchSpan) * 4;
+}
+
+// The kept k-mers of every record, in any order: key and sample to out_key / out_samp,
+// their number in *count (past cap only counted).  Records rec_offs[r]..rec_offs[r+1] of
+// seq; sample s = records samp_recs[s]..samp_recs[s+1].  A thread rolls the k-mers that end
+// in its 128 positions, all lanes in step; kept ones wait in the warp's list, are turned
+// into keys by all lanes together and go out with one atomic per 64.  The sort behind it
+// makes their order irrelevant, so one pass does: a second one to write what a first had
+// counted, and extracting a key bit by bit in one lane, took 717 us of 1.02 ms at 48 Mbp.
+//
+// Bound by issue (137 M warp instructions, 72 % busy): 202 us at 48 Mbp, where the two passes
+// took 301 and 717.  The whole call (twelve samples from host buffers) 3.5 -> 2.6 ms; the
+// rest is the upload.
 __global__ void __launch_bounds__(kSketchThreads) k_sketch_scan(
     const unsigned char *__restrict__ seq, uint64_t n, const uint64_t *__restrict__ rec_offs, uint64_t nrec,
-    const uint64_t *__restrict__ samp_recs, int nsamples, SketchGeom g, uint32_t *__restrict__ counts,
-    uint32_t *__restrict__ samp_counts, const uint32_t *__restrict__ pos, unsigned long long *__restrict__ out)
+    const uint64_t *__restrict__ samp_recs, int nsamples, const SketchGeom g, unsigned long long *__restrict__ out_key,
+    uint32_t *__restrict__ out_samp, uint64_t cap, unsigned long long *__restrict__ count)
 {
-    __shared__ unsigned char tile[kSketchHalo + kSketchTile];
-    const uint64_t t0 = (uint64_t)blockIdx.x * kSketchTile;
-    // stage the tile and its halo (coalesced bytes; the tile start is 32-byte aligned)
-    for (int i = threadIdx.x; i < kSketchHalo + kSketchTile; i += kSketchThreads) {
-        const int64_t p = (int64_t)t0 - kSketchHalo + i;
-        tile[i] = (p >= 0 && (uint64_t)p < n) ? seq[p] : (unsigned char)'N';
+    __shared__ __align__(16) unsigned char tile[kSketchHalo + kSketchTile + 4 * (kSketchThreads + 2)];
+    __shared__ unsigned long long kept_tuple[kSketchThreads / 32][kSketchList];
+    __shared__ uint32_t kept_rec[kSketchThreads / 32][kSketchList];
+    const int64_t t0 = (int64_t)blockIdx.x * kSketchTile;
+    // stage the codes of the tile and its halo, four bases at a time (the tile's start and the
+    // halo's are multiples of 4 bytes from seq, which is 16-byte aligned)
+    for (int i = 4 * threadIdx.x; i < kSketchHalo + kSketchTile; i += 4 * kSketchThreads) {
+        const int64_t p = t0 - kSketchHalo + i;
+        uint32_t w = 0;  // no base
+        if (p >= 0 && p + 4 <= (int64_t)n) {
+            w = __ldg(reinterpret_cast<const uint32_t *>(seq + p));
+        } else if (p >= 0) {
+            for (int x = 0; x < 4; ++x)
+                if (p + x < (int64_t)n)
+                    w |= (uint32_t)seq[p + x] << (8 * x);
+        }
+        *reinterpret_cast<uint32_t *>(tile + sketch_at(i - kSketchHalo)) = base_codes(w);
     }
     __syncthreads();
-    const uint64_t gt = (uint64_t)blockIdx.x * kSketchThreads + threadIdx.x;
-    const uint64_t p0 = gt * kSketchSpan;
-    uint32_t kept = 0;
-    if (p0 < n && nrec) {
-        const uint64_t p1 = min(n, p0 + kSketchSpan);
-        const int len_mv = 2 * g.klen - 2;
-        uint64_t r = last_le(rec_offs, nrec + 1, p0);   // record holding p0 (or the last empty one before)
-        uint64_t rs = __ldg(rec_offs + r), re = r < nrec ? __ldg(rec_offs + r + 1) : rs;
-        uint64_t p = p0 >= rs + (uint64_t)(g.klen - 1) ? p0 - (g.klen - 1) : rs;
-        unsigned long long tuple = 0, crv = 0;
-        int run = 0;
-        uint32_t wi = 0;
-        const uint32_t wbase = WRITE ? pos[gt] : 0;
-        for (; p < p1; ++p) {
-            while (p >= re && r < nrec) {  // next record: the k-mer state starts over
-                ++r;
-                rs = re;
-                re = r < nrec ? __ldg(rec_offs + r + 1) : rs;
-                run = 0;
-                tuple = crv = 0;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // positions from here on are relative to the tile (the last tile ends with the sequence)
+    const int p0 = (int)threadIdx.x * kSketchSpan;
+    const int p1 = (int)min((int64_t)(p0 + kSketchSpan), (int64_t)n - t0);
+    const int len_mv = 2 * g.klen - 2;
+    uint64_t r = nrec;
+    int rs = 0, re = 0;  // record r, as far as the tile and its halo reach
+    auto local = [&](uint64_t at) {
+        return (int)max((int64_t)-kSketchHalo, min((int64_t)kSketchTile, (int64_t)at - t0));
+    };
+    if (p0 < p1) {
+        r = last_le(rec_offs, nrec + 1, (uint64_t)(t0 + p0));  // record holding p0 (or the last empty one before)
+        rs = local(__ldg(rec_offs + r));
+        re = r < nrec ? local(__ldg(rec_offs + r + 1)) : rs;
+    }
+    const int from = max(p0 - (g.klen - 1), rs);  // the k-mer state starts here
+    unsigned long long tuple = 0, crv = 0;
+    int run = 0;
+    uint32_t waiting = 0;
+    auto flush = [&]() {
+        __syncwarp();
+        unsigned long long base = 0;
+        if (lane == 0)
+            base = atomicAdd(count, (unsigned long long)waiting);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        for (uint32_t i = lane; i < waiting; i += 32) {
+            if (base + i < cap) {
+                const unsigned long long ut = kept_tuple[warp][i];
+                const int sm = (int)last_le(samp_recs, (uint64_t)nsamples + 1, kept_rec[warp][i]);
+                out_key[base + i] = (extract_bits(ut, g.ctx) << g.obj_bits) | extract_bits(ut, g.obj);
+                out_samp[base + i] = (uint32_t)min(sm, nsamples - 1);
             }
-            if (r >= nrec)
-                break;
-            const int v = base_code(tile[kSketchHalo + (int64_t)(p - t0)]);
-            if (v < 0) {
-                run = 0;
-                tuple = crv = 0;
-                continue;
-            }
-            tuple = (tuple << 2) | (unsigned long long)v;
-            crv = (crv >> 2) | ((unsigned long long)(v ^ 3) << len_mv);
-            if (++run < g.klen || p < p0)
-                continue;
+        }
+        __syncwarp();
+        waiting = 0;
+    };
+    const unsigned long long top = 1ull << len_mv;  // a base's low bit at the reverse strand's end
+    const uint32_t top_lo = (uint32_t)top, top_hi = (uint32_t)(top >> 32);
+    auto reset = [&]() {
+        run = 0;
+        tuple = crv = 0;
+    };
+    auto roll = [&](uint32_t v) {
+        tuple = (tuple << 2) | v;
+        // the two bits lie in one half of the word: len_mv is even
+        crv = (crv >> 2) | (((unsigned long long)((v ^ 3u) * top_hi) << 32) | ((v ^ 3u) * top_lo));
+        ++run;
+    };
+    // one position with all its conditions: whether a base was rolled in
+    auto step = [&](int p, uint32_t v) {
+        if (p < from || p >= p1)
+            return false;
+        while (p >= re && r < nrec) {  // next record: the k-mer state starts over
+            ++r;
+            rs = re;
+            re = r < nrec ? local(__ldg(rec_offs + r + 1)) : rs;
+            reset();
+        }
+        if (v > 3 || r >= nrec) {
+            reset();
+            return false;
+        }
+        roll(v);
+        return true;
+    };
+    for (int p = p0 - (g.klen - 1); p < p0; ++p)
+        step(p, tile[sketch_at(p)]);
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(tile + sketch_at(p0));
+    for (int x = 0; x < kSketchSpan; x += 4) {
+        const uint32_t w = words[x / 4];
+        // four bases of one record behind a whole k-mer: nothing to ask at each
+        const bool plain = (w & 0xFCFCFCFCu) == 0 && run >= g.klen && p0 + x + 3 < min(re, p1) && r < nrec;
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const uint32_t v = (w >> (8 * y)) & 0xFFu;
+            bool keep = true;
+            if (plain)
+                roll(v);
+            else
+                keep = step(p0 + x + y, v) && run >= g.klen;
             const unsigned long long tc = tuple & g.ctxmask, rc = crv & g.ctxmask;
             const bool fwd = tc < rc;
-            const unsigned long long uctx = fwd ? tc : rc;
-            if ((uint32_t)splitmix64(uctx) > g.filter)
-                continue;
-            if (WRITE) {
-                const unsigned long long ut = (fwd ? tuple : crv) & g.tupmask;
-                out[wbase + wi++] = (extract_bits(ut, g.ctxmask) << g.obj_bits) |
-                                    extract_bits(ut, g.tupmask & ~g.ctxmask);
-            } else {
-                ++kept;
-                const int sm = (int)last_le(samp_recs, (uint64_t)nsamples + 1, r);
-                atomicAdd(samp_counts + min(sm, nsamples - 1), 1u);
+            keep = keep && (uint32_t)splitmix64(fwd ? tc : rc) <= g.filter;
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
+            if (m) {
+                if (keep) {
+                    const uint32_t at = waiting + __popc(m & ((1u << lane) - 1u));
+                    kept_tuple[warp][at] = (fwd ? tuple : crv) & g.tupmask;
+                    kept_rec[warp][at] = (uint32_t)r;
+                }
+                waiting += __popc(m);
+                if (waiting >= kSketchList - 31)
+                    flush();
             }
         }
     }
-    if (!WRITE && gt < (n + kSketchSpan - 1) / kSketchSpan)
-        counts[gt] = kept;
+    if (waiting)
+        flush();
 }
 
 // keep[i]: key i of its sample's sorted run is the first of its duplicates and (without
-// conflict mode) the only object of its context; kept keys counted per sample
-__global__ void k_sketch_keep(const unsigned long long *__restrict__ k, uint64_t n, const uint32_t *__restrict__ seg,
-                              int nsamples, int obj_bits, int conflict, uint8_t *__restrict__ keep,
-                              uint32_t *__restrict__ kept)
+// conflict mode) the only object of its context; kept keys counted per sample, a warp of
+// one sample with one atomic (one per key queued up on a few words: 124 us for 188,000)
+__global__ void k_sketch_keep(const unsigned long long *__restrict__ k, const uint32_t *__restrict__ samp, uint32_t n,
+                              int obj_bits, int conflict, uint8_t *__restrict__ keep, uint32_t *__restrict__ kept)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        // sample of key i: the last segment starting at or before i that is not empty
-        int lo = 0, hi = nsamples - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (seg[mid] <= i)
-                lo = mid;
-            else
-                hi = mid - 1;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x - lane); i0 < n; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + lane;
+        bool ok = false;
+        uint32_t sm = 0xFFFFFFFFu;
+        if (i < n) {
+            sm = samp[i];
+            const unsigned long long x = k[i], c = x >> obj_bits;
+            const bool after = i > 0 && samp[i - 1] == sm;  // not its sample's first
+            ok = !after || k[i - 1] != x;
+            if (ok && !conflict) {
+                if (after && (k[i - 1] >> obj_bits) == c)
+                    ok = false;
+                uint32_t j = i + 1;
+                while (ok && j < n && samp[j] == sm && k[j] == x)
+                    ++j;
+                if (ok && j < n && samp[j] == sm && (k[j] >> obj_bits) == c)
+                    ok = false;
+            }
+            keep[i] = ok ? 1 : 0;
         }
-        const uint64_t b = seg[lo], e = seg[lo + 1];
-        const unsigned long long x = k[i];
-        bool ok = i == b || k[i - 1] != x;
-        if (ok && !conflict) {
-            const unsigned long long c = x >> obj_bits;
-            if (i > b && (k[i - 1] >> obj_bits) == c)
-                ok = false;
-            uint64_t j = i + 1;
-            while (ok && j < e && k[j] == x)
-                ++j;
-            if (ok && j < e && (k[j] >> obj_bits) == c)
-                ok = false;
+        const uint32_t first = __shfl_sync(0xFFFFFFFFu, sm, 0);
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, ok);
+        if (__all_sync(0xFFFFFFFFu, i >= n || sm == first)) {
+            if (lane == 0 && m)
+                atomicAdd(kept + first, (uint32_t)__popc(m));
+        } else if (ok) {
+            atomicAdd(kept + sm, 1u);
         }
-        keep[i] = ok ? 1 : 0;
-        if (ok)
-            atomicAdd(kept + lo, 1u);
     }
 }
 
@@ -4844,82 +4938,87 @@ static int sketch_impl(const CopyIn &copy_in, bool have_seq, uint64_t seq_len, c
     SketchGeom g;
     g.ctxmask = cm;
     g.tupmask = tm;
+    g.ctx = make_extract(cm);
+    g.obj = make_extract(tm & ~cm);
     g.klen = p->klen;
     g.obj_bits = ob;
     g.filter = p->drfold >= 32 ? 0u : (0xFFFFFFFFu >> p->drfold);
     cudaStream_t st = nullptr;
-    const uint64_t nthreads = (seq_len + kSketchSpan - 1) / kSketchSpan;
     const uint64_t nblocks = (seq_len + kSketchTile - 1) / kSketchTile;
     // device buffers (freed on every path)
     struct Bufs {
         unsigned char *seq = nullptr;
         uint64_t *rec = nullptr, *samp = nullptr;
-        uint32_t *counts = nullptr, *pos = nullptr, *scounts = nullptr, *seg = nullptr, *kept = nullptr;
-        unsigned long long *k0 = nullptr, *k1 = nullptr;
+        uint32_t *s0 = nullptr, *s1 = nullptr, *kept = nullptr;
+        unsigned long long *k0 = nullptr, *k1 = nullptr, *count = nullptr;
         uint8_t *keep = nullptr;
         void *tmp = nullptr;
         int *nsel = nullptr;
         ~Bufs()
         {
             cudaStreamSynchronize(nullptr);  // an error may have left work behind
-            for (void *p : {(void *)seq, (void *)rec, (void *)samp, (void *)counts, (void *)pos, (void *)scounts,
-                            (void *)seg, (void *)kept, (void *)k0, (void *)k1, (void *)keep, tmp, (void *)nsel})
+            for (void *p : {(void *)seq, (void *)rec, (void *)samp, (void *)s0, (void *)s1, (void *)kept,
+                            (void *)k0, (void *)k1, (void *)count, (void *)keep, tmp, (void *)nsel})
                 pool_free_idle(p);
         }
     } b;
     CUDA_TRY(pool_malloc(&b.seq, seq_len));
     CUDA_TRY(pool_malloc(&b.rec, (nrec + 1) * sizeof(uint64_t)));
     CUDA_TRY(pool_malloc(&b.samp, ((size_t)nsamples + 1) * sizeof(uint64_t)));
-    CUDA_TRY(pool_malloc(&b.counts, nthreads * sizeof(uint32_t)));
-    CUDA_TRY(pool_malloc(&b.pos, (nthreads + 1) * sizeof(uint32_t)));
-    CUDA_TRY(pool_malloc(&b.scounts, ((size_t)nsamples + 1) * sizeof(uint32_t)));
-    CUDA_TRY(pool_malloc(&b.seg, ((size_t)nsamples + 1) * sizeof(uint32_t)));
     CUDA_TRY(pool_malloc(&b.kept, ((size_t)nsamples + 1) * sizeof(uint32_t)));
+    CUDA_TRY(pool_malloc(&b.count, sizeof(unsigned long long)));
     CUDA_TRY(copy_in(b.seq, st));
     CUDA_TRY(cudaMemcpyAsync(b.rec, rec_offs, (nrec + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(b.samp, samp_recs, ((size_t)nsamples + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemsetAsync(b.scounts, 0, ((size_t)nsamples + 1) * sizeof(uint32_t), st));
     CUDA_TRY(cudaMemsetAsync(b.kept, 0, ((size_t)nsamples + 1) * sizeof(uint32_t), st));
-    k_sketch_scan<false><<<(unsigned)nblocks, kSketchThreads, 0, st>>>(b.seq, seq_len, b.rec, nrec, b.samp, nsamples, g,
-                                                                       b.counts, b.scounts, nullptr, nullptr);
-    count_launch();
-    CUDA_TRY(cudaGetLastError());
-    // thread offsets and sample segments: exclusive sums (the totals land in the last word)
-    size_t tb0 = 0, tb1 = 0, tb2 = 0, tb3 = 0;
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb0, b.counts, b.pos, (int64_t)nthreads, st));
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb1, b.scounts, b.seg, nsamples + 1, st));
-    CUDA_TRY(pool_malloc(&b.tmp, std::max(tb0, tb1)));
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(b.tmp, tb0, b.counts, b.pos, (int64_t)nthreads, st));
-    CUDA_TRY(cub::DeviceScan::ExclusiveSum(b.tmp, tb1, b.scounts, b.seg, nsamples + 1, st));
-    count_launch(2);
-    uint32_t total = 0;
-    CUDA_TRY(cudaMemcpyAsync(&total, b.seg + nsamples, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    if (total == 0)
+    // the kept k-mers, into room for the expected number and half as many again; a sequence
+    // that keeps more (repeats of a kept k-mer) is scanned again with room for all
+    uint64_t room = std::min<uint64_t>(seq_len, (seq_len >> std::min(p->drfold, 31)) * 3 / 2 + 65536);
+    unsigned long long found = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        CUDA_TRY(pool_malloc(&b.k0, room * sizeof(unsigned long long)));
+        CUDA_TRY(pool_malloc(&b.s0, room * sizeof(uint32_t)));
+        CUDA_TRY(cudaMemsetAsync(b.count, 0, sizeof(unsigned long long), st));
+        k_sketch_scan<<<(unsigned)nblocks, kSketchThreads, 0, st>>>(b.seq, seq_len, b.rec, nrec, b.samp, nsamples, g,
+                                                                    b.k0, b.s0, room, b.count);
+        count_launch();
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaMemcpyAsync(&found, b.count, sizeof found, cudaMemcpyDeviceToHost, st));
+        CUDA_TRY(cudaStreamSynchronize(st));
+        if (found <= room)
+            break;
+        pool_free_idle(b.k0);
+        pool_free_idle(b.s0);
+        b.k0 = nullptr;
+        b.s0 = nullptr;
+        room = found;
+    }
+    if (found == 0)
         return KSSDGPU_OK;
-    CUDA_TRY(pool_malloc(&b.k0, (size_t)total * sizeof(unsigned long long)));
+    const uint32_t total = (uint32_t)found;  // at most the sequence's length
     CUDA_TRY(pool_malloc(&b.k1, (size_t)total * sizeof(unsigned long long)));
+    CUDA_TRY(pool_malloc(&b.s1, (size_t)total * sizeof(uint32_t)));
     CUDA_TRY(pool_malloc(&b.keep, total));
     CUDA_TRY(pool_malloc(&b.nsel, sizeof(int)));
-    k_sketch_scan<true><<<(unsigned)nblocks, kSketchThreads, 0, st>>>(b.seq, seq_len, b.rec, nrec, b.samp, nsamples, g,
-                                                                      nullptr, nullptr, b.pos, b.k0);
-    count_launch();
-    CUDA_TRY(cudaGetLastError());
-    // sort each sample's keys, mark the kept ones, compact
-    CUDA_TRY(cub::DeviceSegmentedSort::SortKeys(nullptr, tb2, b.k0, b.k1, (int64_t)total, nsamples, b.seg,
-                                                b.seg + 1, st));
-    CUDA_TRY(cub::DeviceSelect::Flagged(nullptr, tb3, b.k1, b.keep, b.k0, b.nsel, (int64_t)total, st));
-    if (std::max(tb2, tb3) > std::max(tb0, tb1)) {
-        pool_free(b.tmp);
-        b.tmp = nullptr;
-        CUDA_TRY(pool_malloc(&b.tmp, std::max(tb2, tb3)));
-    }
-    CUDA_TRY(cub::DeviceSegmentedSort::SortKeys(b.tmp, tb2, b.k0, b.k1, (int64_t)total, nsamples, b.seg, b.seg + 1,
-                                                st));
-    k_sketch_keep<<<grid_for(total), 256, 0, st>>>(b.k1, total, b.seg, nsamples, ob, p->conflict ? 1 : 0, b.keep,
+    // by key, then (stable) by sample
+    int sbits = 1;
+    while ((1ll << sbits) < nsamples)
+        ++sbits;
+    cub::DoubleBuffer<unsigned long long> dk(b.k0, b.k1);
+    cub::DoubleBuffer<uint32_t> ds(b.s0, b.s1);
+    const int kbits = std::min(64, 2 * g.klen);
+    size_t tb0 = 0, tb1 = 0, tb2 = 0;
+    CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb0, dk, ds, (int64_t)total, 0, kbits, st));
+    CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb1, ds, dk, (int64_t)total, 0, sbits, st));
+    CUDA_TRY(cub::DeviceSelect::Flagged(nullptr, tb2, b.k1, b.keep, b.k0, b.nsel, (int64_t)total, st));
+    CUDA_TRY(pool_malloc(&b.tmp, std::max(tb0, std::max(tb1, tb2))));
+    CUDA_TRY(cub::DeviceRadixSort::SortPairs(b.tmp, tb0, dk, ds, (int64_t)total, 0, kbits, st));
+    if (nsamples > 1)
+        CUDA_TRY(cub::DeviceRadixSort::SortPairs(b.tmp, tb1, ds, dk, (int64_t)total, 0, sbits, st));
+    k_sketch_keep<<<grid_for(total), 256, 0, st>>>(dk.Current(), ds.Current(), total, ob, p->conflict ? 1 : 0, b.keep,
                                                    b.kept);
-    CUDA_TRY(cub::DeviceSelect::Flagged(b.tmp, tb3, b.k1, b.keep, b.k0, b.nsel, (int64_t)total, st));
-    count_launch(3);
+    CUDA_TRY(cub::DeviceSelect::Flagged(b.tmp, tb2, dk.Current(), b.keep, dk.Alternate(), b.nsel, (int64_t)total, st));
+    count_launch(4);
     int nsel = 0;
     std::vector<uint32_t> kept((size_t)nsamples);
     CUDA_TRY(cudaMemcpyAsync(&nsel, b.nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -4932,7 +5031,7 @@ static int sketch_impl(const CopyIn &copy_in, bool have_seq, uint64_t seq_len, c
     if ((uint64_t)nsel > keys_cap || (nsel && !keys))
         return fail(KSSDGPU_ERR_CAPACITY, "sketch output needs " + std::to_string(nsel) + " keys (offs holds them)");
     if (nsel)
-        CUDA_TRY(cudaMemcpy(keys, b.k0, (size_t)nsel * sizeof(uint64_t), cudaMemcpyDeviceToHost));
+        CUDA_TRY(cudaMemcpy(keys, dk.Alternate(), (size_t)nsel * sizeof(uint64_t), cudaMemcpyDeviceToHost));
     return KSSDGPU_OK;
 }
 
