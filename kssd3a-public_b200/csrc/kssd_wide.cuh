@@ -24,7 +24,7 @@
 // join with a row per allele takes over (dense_chosen compares the two).
 //
 // Measured (B200, whole calls): the self join of 1,024 genomes of one species 1,748 (rows
-// per allele) -> 241 us, of 3,000 genomes of ten species 16.4 -> 3.0 ms; a block of 200
+// per allele) -> 175 us, of 3,000 genomes of ten species 16.4 -> 2.9 ms; a block of 200
 // queries against 1,024 genomes of their species 6.82 ms (postings walked per query, 1.9 G
 // atomics) -> 0.24 ms, of one query 2.23 -> 0.17 ms, of 30 read sets against 500 genomes
 // 975 -> 277 us.
@@ -54,6 +54,9 @@ __device__ __forceinline__ uint32_t wide_e(uint32_t o, uint32_t major)
 {
     return (uint32_t)min(kMinInit, dna_pop(o ^ major));
 }
+
+// the bases at which an object xor the major one differs, as bits 0, 2, 4, ...
+__device__ __forceinline__ uint32_t wide_bases(uint32_t x) { return (x | (x >> 1)) & 0x55555555u; }
 
 // What the products overcount on a pair of genomes with objects a and b, both different
 // from major: their sum of distances for the difference, and one of each threshold.
@@ -104,8 +107,9 @@ __device__ __forceinline__ WideWords wide_words(uint32_t e)
     return x;
 }
 
-// Shared memory of one warp of k_wide_rows: the genomes' distances, then the genomes away
-// from the major object as (gid | e << 20) << 32 | object.
+// Shared memory of one warp of k_wide_rows: the genomes' distances (later the list of those
+// that differ at a base), then the genomes away from the major object as (gid | e << 20) <<
+// 32 | object ^ major.
 __host__ __device__ __forceinline__ size_t wide_warp_smem(uint32_t npad, uint32_t nref)
 {
     return (size_t)npad + ((size_t)nref * 8 + 15) / 16 * 16;
@@ -139,7 +143,8 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
                                                    const unsigned long long *__restrict__ items, uint32_t n_list,
                                                    const uint64_t *__restrict__ post, uint32_t nref, uint32_t npad,
                                                    int8_t *__restrict__ X, size_t xs,
-                                                   unsigned long long *__restrict__ corr, const WideBlock Q)
+                                                   unsigned long long *__restrict__ corr, int bases_only,
+                                                   const WideBlock Q)
 {
     extern __shared__ __align__(16) unsigned char wsm[];
     const uint32_t lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
@@ -172,7 +177,7 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
                 const unsigned away = __ballot_sync(0xffffffffu, e != 0);
                 if (e)
                     minor[nm + __popc(away & ((1u << lane) - 1u))] =
-                        ((unsigned long long)(gid | (e << kGidBits)) << 32) | (uint32_t)p[x];
+                        ((unsigned long long)(gid | (e << kGidBits)) << 32) | ((uint32_t)p[x] ^ major);
                 nm += __popc(away);
             }
         }
@@ -230,7 +235,7 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
                             const uint32_t rc = (uint32_t)(c >> 32), er = rc >> kGidBits;
                             uint32_t d = (uint32_t)kMinInit;
                             for (uint32_t i = 0; i < run; ++i)
-                                d = min(d, (uint32_t)dna_pop(((uint32_t)__ldg(Q.qkeys + from + i) & mask) ^ (uint32_t)c));
+                                d = min(d, (uint32_t)dna_pop(((uint32_t)__ldg(Q.qkeys + from + i) & mask) ^ major ^ (uint32_t)c));
                             // the products count a difference, two where the run has no object
                             // at the major one or the genome's is two away, and ea + er of it
                             const uint32_t two = ea ? 1u : er >= 2 ? 1u : 0u;
@@ -244,7 +249,8 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
                     for (unsigned away = __ballot_sync(0xffffffffu, ex != 0 && ex != 0xFFu && runs[x] == 0); away;
                          away &= away - 1) {
                         const int src = __ffs(away) - 1;
-                        const uint32_t oa = __shfl_sync(0xffffffffu, ob[x], src), ea = __shfl_sync(0xffffffffu, ex, src);
+                        const uint32_t oa = __shfl_sync(0xffffffffu, ob[x], src) ^ major;
+                        const uint32_t ea = __shfl_sync(0xffffffffu, ex, src);
                         unsigned long long *row = corr + (size_t)(q0 + 4 * src + x) * nref;
                         for (uint32_t j = lane; j < nm; j += 32) {
                             const unsigned long long c = minor[j];
@@ -259,9 +265,48 @@ __global__ void __launch_bounds__(256) k_wide_rows(const SharedGroup *__restrict
             __syncwarp();  // the warp's shared memory is reused by its next group
             continue;
         }
-        // pairs (i, j), j < i: kWidePairs genomes i against lanes on consecutive j (postings
-        // ascend by gid, so i is the pair's higher genome)
-        for (uint32_t i0 = 1; i0 < nm; i0 += kWidePairs) {
+        // Only pairs with a base in common among their differences from the major object are
+        // corrected (bases_only: objects too short to pass the cap without one), so for every
+        // base the genomes that differ there are listed and their pairs compared, a pair at its
+        // first common base.  In one species a list holds a tenth of the genomes away, so all
+        // ten lists a tenth of their pairs (1,024 genomes: 139 -> 101 us).
+        uint32_t bases = 0;
+        const bool by_base = bases_only && nm <= npad / 2;  // a list fits
+        if (by_base) {
+            for (uint32_t i = lane; i < nm; i += 32)
+                bases |= wide_bases((uint32_t)minor[i]);
+            bases = __reduce_or_sync(0xffffffffu, bases);
+        }
+        unsigned short *list16 = reinterpret_cast<unsigned short *>(emap);  // the rows are written
+        for (uint32_t left = bases; left; left &= left - 1) {
+            const uint32_t bit = left & (0u - left);
+            uint32_t nb = 0;
+            __syncwarp();
+            for (uint32_t i0 = 0; i0 < nm; i0 += 32) {
+                const uint32_t i = i0 + lane;
+                const bool here = i < nm && (wide_bases((uint32_t)minor[i]) & bit);
+                const unsigned m = __ballot_sync(0xffffffffu, here);
+                if (here)
+                    list16[nb + __popc(m & ((1u << lane) - 1u))] = (unsigned short)i;
+                nb += __popc(m);
+            }
+            __syncwarp();
+            const uint32_t np = nb * (nb - 1) / 2;
+            for (uint32_t t = lane; t < np; t += 32) {
+                uint32_t i, j;
+                pair_of_rank(t, i, j);
+                const unsigned long long a = minor[list16[j]], c = minor[list16[i]];  // j's genome is the higher
+                if (wide_bases((uint32_t)a) & wide_bases((uint32_t)c) & (bit - 1))
+                    continue;
+                const uint32_t qa = (uint32_t)(a >> 32), rc = (uint32_t)(c >> 32);
+                const uint32_t g = qa & ((1u << kGidBits) - 1);
+                const unsigned long long w = wide_correction((uint32_t)a, (uint32_t)c, qa >> kGidBits, rc >> kGidBits);
+                atomicAdd(corr + g * (g - 1) / 2 + (rc & ((1u << kGidBits) - 1)), w);  // g < 2^12
+            }
+        }
+        // else all pairs (i, j), j < i: kWidePairs genomes i against lanes on consecutive j
+        // (postings ascend by gid, so i is the pair's higher genome)
+        for (uint32_t i0 = 1; i0 < nm && !by_base; i0 += kWidePairs) {
             uint32_t oq[kWidePairs], eq[kWidePairs];
             unsigned long long *row[kWidePairs];
 #pragma unroll

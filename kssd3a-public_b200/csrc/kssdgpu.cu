@@ -3282,7 +3282,7 @@ int wide_block_end(kssdgpu_index *ix, int nq, const CountParams &P, unsigned lon
         const WideBlock Q{ix->w_qobj.p + c0 * nqp, (uint32_t)nq, nqp, ix->w_y.p, ys, P.qkeys, P.qoffs, P.obj_bits};
         k_wide_rows<true><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
                             warps * wide_warp_smem(npad, n), st>>>(nullptr, ix->w_list.p + c0, cn, ix->post, n, npad,
-                                                                   ix->w_x.p, xs, ix->w_corr.p, Q);
+                                                                   ix->w_x.p, xs, ix->w_corr.p, 0, Q);
         CUDA_TRY(cudaGetLastError());
         const int grc = kssd::dense_gemm_s8(ix->w_y.p, ix->w_x.p, ix->w_g.p, (int)nqp, (int)npad, (int)cn, kWideRows,
                                             nqp, npad, npad, (int64_t)ys, (int64_t)xs, (int64_t)gs, ix->d_ws.p, st);
@@ -4367,8 +4367,9 @@ uint64_t dense_bytes(const kssdgpu_index *ix, uint64_t kpad)
 uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 
 // Columns of the Gram products one GEMM launch covers: the whole square up to
-// kWideSquare genomes (one launch fills the GPU), else blocks of kWideBlock columns over
-// the rows at or below them (the products are symmetric).
+// kWideSquare genomes (one launch fills the GPU: 1,024 genomes 176 us per join, 181 in two
+// blocks of 512 columns, 209 in four of 256), else blocks of kWideBlock columns over the
+// rows at or below them (the products are symmetric).
 constexpr uint64_t kWideSquare = 1536, kWideBlock = 512;
 
 // Device bytes of a wide self join: operand rows, Gram matrices, corrections.
@@ -4485,7 +4486,8 @@ int self_wide_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long long
         const uint32_t cn = (uint32_t)std::min<uint64_t>(pass, ix->f_wgroups - c0);
         k_wide_rows<false><<<std::min<int>(rows_grid, (int)((cn + warps - 1) / warps)), warps * 32,
                              warps * wide_warp_smem(npad, n), st>>>(list + c0, nullptr, cn, ix->post, n, npad,
-                                                                    ix->w_x.p, xs, ix->w_corr.p, WideBlock{});
+                                                                    ix->w_x.p, xs, ix->w_corr.p,
+                                                                    ix->obj_bits <= 2 * kMinInit, WideBlock{});
         count_launch();
         CUDA_TRY(cudaGetLastError());
         for (uint64_t j = 0; j < npad; j += bw) {
