@@ -92,18 +92,40 @@ __global__ void k_unpack_records(const uint32_t *__restrict__ w, uint64_t n, int
 
 // Sketch keys -> sort keys (ctx << 20 | gid) with obj values; checks that each
 // sample's keys ascend (comblco order), which makes one stable sort by ctxgid
-// produce the reference's (ctxgid, obj) order.
+// produce the reference's (ctxgid, obj) order.  A warp takes kSortSpan keys, whatever
+// samples they belong to (a CTA per sample left 64 small ones on 64 SMs: 20 us; spans of 512
+// keys still measured 15 us, their few warps' reads a serial chain).
+constexpr uint64_t kSortSpan = 128;
 __global__ void k_sketch_to_sortkeys(const uint64_t *__restrict__ keys, const uint64_t *__restrict__ offs, int nref,
                                      int obj_bits, unsigned long long *__restrict__ skey, uint32_t *__restrict__ sval,
                                      int *__restrict__ err)
 {
-    const uint64_t base = offs[0];
+    const uint64_t base = offs[0], n = offs[nref] - base;
     const uint64_t objmask = (obj_bits >= 64) ? ~0ull : ((1ull << obj_bits) - 1);
-    for (int g = blockIdx.x; g < nref; g += gridDim.x) {
-        const uint64_t b = offs[g] - base, e = offs[g + 1] - base;
-        for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; w * kSortSpan < n; w += warps) {
+        const uint64_t b = w * kSortSpan, e = min(n, b + kSortSpan);
+        // sample of the span's first key (the last one that starts at or before it), then step
+        int g = 0;
+        for (int lo = 0, hi = nref - 1; lo <= hi;) {
+            const int mid = (lo + hi) >> 1;
+            if (__ldg(offs + mid) - base <= b) {
+                g = mid;
+                lo = mid + 1;
+            } else {
+                hi = mid - 1;
+            }
+        }
+        uint64_t gb = __ldg(offs + g) - base, ge = __ldg(offs + g + 1) - base;
+        for (uint64_t i = b + lane; i < e; i += 32) {
+            while (i >= ge) {
+                ++g;
+                gb = ge;
+                ge = __ldg(offs + g + 1) - base;
+            }
             const uint64_t k = keys[i];
-            if (i > b && keys[i - 1] > k)
+            if (i > gb && keys[i - 1] > k)
                 atomicMax(err, (int)kDevUnsorted);
             skey[i] = ((k >> obj_bits) << kGidBits) | (uint64_t)g;
             sval[i] = (uint32_t)(k & objmask);
@@ -594,10 +616,12 @@ __global__ void k_bloom_insert(const unsigned long long *__restrict__ gkey, uint
         const unsigned long long ctx = gkey[g];
         const BloomBits b = bloom_bits(ctx, mask);
         const size_t stripe = stripes > 1 ? stripe_of(bounds, stripes, ctx) : 0;
-        uint32_t *half = f + (2 * stripe * ((size_t)mask + 1) + b.half) * 4;
+        // four words in two atomics: they are what the kernel waits for
+        unsigned long long *half =
+            reinterpret_cast<unsigned long long *>(f + (2 * stripe * ((size_t)mask + 1) + b.half) * 4);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            atomicOr(half + i, 1u << bloom_bit(b.r, i));
+        for (int i = 0; i < 2; ++i)
+            atomicOr(half + i, (1ull << bloom_bit(b.r, 2 * i)) | (1ull << (32 + bloom_bit(b.r, 2 * i + 1))));
     }
 }
 
@@ -611,31 +635,37 @@ __global__ void k_stripe_bounds(const unsigned long long *__restrict__ gkey, uin
 
 // spos[q * (S + 1) + s]: the first entry of query q whose context is >= bounds[s]
 // (absolute offsets; s = 0 and s = S are the query's own bounds).  Keys ascend within
-// a query, so each is one binary search.
+// a query; a warp finds a place by 32 probes at a time (a thread's binary search was a
+// chain of 14 HBM reads: 12 us for 1,500 queries).
 __global__ void k_stripe_pos(const uint64_t *__restrict__ qkeys, const uint64_t *__restrict__ qoffs, int nq,
                              int stripes, const unsigned long long *__restrict__ bounds, int obj_bits,
                              uint64_t *__restrict__ spos)
 {
     const uint64_t base = qoffs[0];
     const uint64_t n = (uint64_t)nq * (stripes + 1);
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t t = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; t < n;
+         t += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
         const int q = (int)(t / (uint64_t)(stripes + 1)), s = (int)(t % (uint64_t)(stripes + 1));
         uint64_t lo = qoffs[q], hi = qoffs[q + 1];
         if (s == stripes) {
-            spos[t] = hi;
-            continue;
-        }
-        if (s > 0) {
+            lo = hi;
+        } else if (s > 0) {
             const unsigned long long bound = bounds[s];
             while (lo < hi) {
-                const uint64_t mid = lo + ((hi - lo) >> 1);
-                if ((__ldg(qkeys + (mid - base)) >> obj_bits) < bound)
-                    lo = mid + 1;
-                else
-                    hi = mid;
+                // probes at the ends of 32 equal parts: all before the place lie below the bound
+                const uint64_t part = (hi - lo + 31) / 32, at = lo + (uint64_t)(lane + 1) * part - 1;
+                const bool below = at < hi && (__ldg(qkeys + (at - base)) >> obj_bits) < bound;
+                const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, below));
+                lo += (uint64_t)c * part;
+                if (part == 1)
+                    break;
+                hi = min(hi, lo + part - 1);
             }
+            lo = min(lo, qoffs[q + 1]);
         }
-        spos[t] = lo;
+        if (lane == 0)
+            spos[t] = lo;
     }
 }
 
@@ -2076,7 +2106,11 @@ __global__ void k_allele_sample(const uint32_t *__restrict__ gbeg, uint64_t u, u
                                 const uint64_t *__restrict__ post, uint32_t wide,
                                 unsigned long long *__restrict__ tot)
 {
+    __shared__ unsigned long long sum[3];
     const uint32_t lane = threadIdx.x & 31;
+    if (threadIdx.x < 3)
+        sum[threadIdx.x] = 0;
+    __syncthreads();
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < samples; i += (gridDim.x * blockDim.x) >> 5) {
         const uint64_t g = (uint64_t)i * stride;
         if (g >= u)
@@ -2100,10 +2134,10 @@ __global__ void k_allele_sample(const uint32_t *__restrict__ gbeg, uint64_t u, u
             uint32_t o = 0;
             const uint32_t major = wide_major(post, b, k, lane, o);
             uint32_t hits = 0;  // ordered pairs of the sample
-            for (uint32_t d = 1; d < 32; ++d) {
-                const uint32_t other = (lane + d) & 31u;
-                const uint32_t p = __shfl_sync(0xffffffffu, o, other);
-                if (lane < ns && other < ns && o != major && p != major)
+            for (uint32_t d = 1; d < ns; ++d) {
+                const uint32_t other = lane + d < ns ? lane + d : lane + d - ns;
+                const uint32_t p = __shfl_sync(0xffffffffu, o, (int)(other & 31u));
+                if (lane < ns && o != major && p != major)
                     hits += wide_correction(o, p, major) != 0;
             }
             for (int x = 16; x; x >>= 1)
@@ -2111,12 +2145,15 @@ __global__ void k_allele_sample(const uint32_t *__restrict__ gbeg, uint64_t u, u
             corr = (unsigned long long)((double)hits * k * (k - 1.0) / (2.0 * ns * (ns - 1.0)));
         }
         if (lane == 0) {
-            atomicAdd(tot + 0, (unsigned long long)firsts);
-            atomicAdd(tot + 1, (unsigned long long)k);
+            atomicAdd(&sum[0], (unsigned long long)firsts);
+            atomicAdd(&sum[1], (unsigned long long)k);
             if (corr)
-                atomicAdd(tot + 2, corr);
+                atomicAdd(&sum[2], corr);
         }
     }
+    __syncthreads();
+    if (threadIdx.x < 3 && sum[threadIdx.x])
+        atomicAdd(tot + threadIdx.x, sum[threadIdx.x]);
 }
 
 // Groups of at least kmin postings as (begin | k << 32), appended in any order; number_at
@@ -3003,8 +3040,8 @@ int finish_build(kssdgpu_index *ix, uint32_t *head, unsigned long long *ctx_of, 
             // the dense join's allele count, estimated from up to 65,536 sampled groups
             const uint32_t samples = (uint32_t)std::min<uint64_t>(ix->u, 65536);
             const uint64_t stride = ix->u / samples;
-            k_allele_sample<<<(samples * 32 + 255) / 256, 256, 0, st>>>(ix->gbeg, ix->u, stride, samples, ix->post,
-                                                                       ix->wide_min, d + kStatFacts);
+            k_allele_sample<<<std::min<uint32_t>((samples + 7) / 8, (uint32_t)ix->sms * 8), 256, 0, st>>>(
+                ix->gbeg, ix->u, stride, samples, ix->post, ix->wide_min, d + kStatFacts);
             count_launch(2);
             e = cudaGetLastError();
         }
@@ -3353,8 +3390,8 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
         size_t tb = 0;
         CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, ix->s_scnt.p, ix->s_spre.p, (int64_t)nsq + 1, st));
         CUDA_TRY(ix->s_cubtmp.ensure(tb));
-        k_stripe_pos<<<grid_for(npos), 256, 0, st>>>(d_keys, d_offs, nq, S, ix->bloom_bounds, ix->obj_bits,
-                                                      ix->s_spos.p);
+        k_stripe_pos<<<grid_for(npos * 32), 256, 0, st>>>(d_keys, d_offs, nq, S, ix->bloom_bounds, ix->obj_bits,
+                                                          ix->s_spos.p);
         k_stripe_counts<<<grid_for(nsq + 1), 256, 0, st>>>(ix->s_spos.p, d_offs, nq, S, ix->s_scnt.p, ix->err);
         CUDA_TRY(cub::DeviceScan::ExclusiveSum(ix->s_cubtmp.p, tb, ix->s_scnt.p, ix->s_spre.p, (int64_t)nsq + 1, st));
         k_stripe_expand<<<ix->sms * 4, 256, 0, st>>>(ix->s_spos.p, d_offs, nq, S, ix->s_spre.p, ix->s_sitems.p);
@@ -5174,7 +5211,8 @@ int kssdgpu_index_from_sketch(const uint64_t *keys, const uint64_t *offs, int nr
                     std::string("sketch upload: ") + cudaGetErrorString(e));
     }
     if (n) {
-        k_sketch_to_sortkeys<<<std::min(nref, 148 * 16), 256, 0, st>>>(dk, doffs, nref, obj_bits, skey, sval, ix->err);
+        k_sketch_to_sortkeys<<<grid_for((n + kSortSpan - 1) / kSortSpan * 32), 256, 0, st>>>(dk, doffs, nref, obj_bits,
+                                                                                             skey, sval, ix->err);
         count_launch();
         // stable LSD radix sort on the context alone: the records come sample by sample, so equal
         // contexts keep their gid order, and within a gid the comblco (obj ascending) order.  The
