@@ -432,8 +432,8 @@ struct WarpAcc {
         __syncwarp();
     }
 };
-__device__ __forceinline__ void flush_acc(const WarpAcc &a, uint32_t lane) { a.flush(lane); }
 __device__ __forceinline__ void flush_acc(const SmemAcc &, uint32_t) {}
+__device__ __forceinline__ void flush_acc(const WarpAcc &a, uint32_t lane) { a.flush(lane); }
 
 // min over the query run's objects x one reference object
 __device__ __forceinline__ int min_diff_obj(uint32_t robj, uint32_t q0, int s, const uint64_t *__restrict__ qrun,
@@ -757,7 +757,7 @@ struct ProbeQueue {
 // over the lanes, 32 at a time; walked each by its own lane, the longest group holds up
 // the others.  Runs of several objects and indexes with conflicts are walked by their lane,
 // groups of at least kWarpWalk postings by the warp, or (WIDE) left to the tensor cores.
-template <bool LOWER, bool UNIQUE, bool WIDE, class Acc>
+template <bool UNIQUE, bool WIDE, class Acc>
 __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q, uint32_t first, uint32_t count,
                                             uint64_t cb, uint64_t e, int qgid, uint64_t objmask, const Acc &acc,
                                             const Acc &uacc, uint32_t lane)
@@ -799,7 +799,7 @@ __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q,
             else if (s == 1 && P.conflict_free)
                 flat = true;
             else
-                credit_context<LOWER, UNIQUE>(P, i, s, payload, single, qgid, objmask, acc, uacc);
+                credit_context<false, UNIQUE>(P, i, s, payload, single, qgid, objmask, acc, uacc);
         }
     }
     __syncwarp();
@@ -845,7 +845,7 @@ __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q,
 #pragma unroll
             for (uint32_t x = 0; x < kPostLoads; ++x) {
                 const uint32_t gid = (uint32_t)(w[x] >> 32);
-                if (p0 + 32 * x + lane < total && (!LOWER || (int)gid < qgid)) {
+                if (p0 + 32 * x + lane < total) {
                     const int d = min(kMinInit, dna_pop((uint32_t)w[x] ^ Q.object[own[x]]));
                     acc.add(gid, d);
                     if (UNIQUE && one[x])  // the context's only owner
@@ -862,7 +862,7 @@ __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q,
         const uint32_t gb = __shfl_sync(0xFFFFFFFFu, pb, src), gc = __shfl_sync(0xFFFFFFFFu, pc, src);
         const uint64_t gi = __shfl_sync(0xFFFFFFFFu, i, src);
         const int gs = __shfl_sync(0xFFFFFFFFu, s, src);
-        walk_context_warp<LOWER, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
+        walk_context_warp<false, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
                                          acc, uacc, lane);
     }
 }
@@ -873,7 +873,7 @@ __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q,
 // context run works (src/command_ani.h:498-505); the filter rules out most absent contexts
 // (88 % of the entries of new assemblies); the others wait in the warp's queue until 32 of
 // them probe the table together, so that no lane idles in the probe and the walk.
-template <bool LOWER, bool UNIQUE, bool WIDE, class Acc>
+template <bool UNIQUE, bool WIDE, class Acc>
 __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, uint64_t e, uint64_t cb, uint64_t ce,
                                               int qgid, uint64_t objmask, const Acc &acc, const Acc &uacc,
                                               const FilterView &fv, uint64_t t0, uint64_t T, ProbeQueue &Q)
@@ -923,7 +923,7 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
         __syncwarp();
         while (waiting >= 32) {
             waiting -= 32;
-            probe_batch<LOWER, UNIQUE, WIDE>(P, Q, waiting, 32, cb, e, qgid, objmask, acc, uacc, lane);
+            probe_batch<UNIQUE, WIDE>(P, Q, waiting, 32, cb, e, qgid, objmask, acc, uacc, lane);
         }
         __syncwarp();
         seen += 32 * kProbeLoads;
@@ -935,7 +935,72 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
         }
     }
     if (waiting)
-        probe_batch<LOWER, UNIQUE, WIDE>(P, Q, 0, waiting, cb, e, qgid, objmask, acc, uacc, lane);
+        probe_batch<UNIQUE, WIDE>(P, Q, 0, waiting, cb, e, qgid, objmask, acc, uacc, lane);
+    flush_acc(acc, lane);
+    if (UNIQUE)
+        flush_acc(uacc, lane);
+}
+
+// The same entries, an entry a lane and round, for shared-memory rows and lower blocks.  A
+// lower block is a part of an index's own genomes: every key is found and most credit
+// nothing (a context's only owner is the query itself), so a full warp in the probe is worth
+// less than the warps in flight that the queue's registers and shared memory cost; so are
+// the cheap credits of a row in shared memory.  Measured (B200, 2,000 genomes against
+// themselves, lower, queue -> this): global rows stripe by stripe 1,383 -> 1,201 us, in
+// chunks without the filter 1,264 -> 1,079, shared rows 1,869 -> 1,410; 500 of them as an
+// ordinary block, global rows: 464 -> 402 the other way.
+template <bool LOWER, bool UNIQUE, class Acc>
+__device__ __forceinline__ void process_query_row(const CountParams &P, uint64_t b, uint64_t e, uint64_t cb,
+                                                  uint64_t ce, int qgid, uint64_t objmask, const Acc &acc,
+                                                  const Acc &uacc, const FilterView &fv, uint64_t t0, uint64_t T)
+{
+    const uint32_t lane = (uint32_t)(t0 & 31u);
+    uint32_t seen = 0;
+    for (uint64_t wb = cb + (t0 - lane); wb < ce; wb += T) {
+        if ((seen += 32) > kWarpCellEntries) {
+            flush_acc(acc, lane);
+            if (UNIQUE)
+                flush_acc(uacc, lane);
+            seen = 32;
+        }
+        const uint64_t i = wb + lane;
+        int s = 0;
+        unsigned long long payload = 0;
+        bool wide = false;
+        if (i < ce) {
+            const unsigned long long key = __ldg(P.qkeys + i), ctx = key >> P.obj_bits;
+            const unsigned long long prev = i > b ? __ldg(P.qkeys + i - 1) : 0;
+            if (prev > key)
+                atomicMax(P.err, (int)kDevUnsorted);  // a sample's keys must ascend (comblco order)
+            bool keep = !(i > b && (prev >> P.obj_bits) == ctx);
+            if (keep && fv.f) {
+                BloomBits bits;
+                const uint4 w = fv.load(ctx, bits);
+                keep = bloom_all(w, bits);
+            }
+            if (keep) {
+                s = 1;
+                while (i + s < e && (__ldg(P.qkeys + i + s) >> P.obj_bits) == ctx)
+                    ++s;
+                bool single;
+                if (table_lookup(P.table, P.mask, ctx, payload, single)) {
+                    if (!single && (uint32_t)(payload >> 32) >= kWarpWalk)
+                        wide = true;
+                    else
+                        credit_context<LOWER, UNIQUE>(P, i, s, payload, single, qgid, objmask, acc, uacc);
+                }
+            }
+        }
+        const uint32_t pb = (uint32_t)payload, pc = (uint32_t)(payload >> 32);
+        for (unsigned m = __ballot_sync(0xFFFFFFFFu, wide); m; m &= m - 1) {
+            const int src = __ffs(m) - 1;
+            const uint32_t gb = __shfl_sync(0xFFFFFFFFu, pb, src), gc = __shfl_sync(0xFFFFFFFFu, pc, src);
+            const uint64_t gi = __shfl_sync(0xFFFFFFFFu, i, src);
+            const int gs = __shfl_sync(0xFFFFFFFFu, s, src);
+            walk_context_warp<LOWER, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
+                                             acc, uacc, lane);
+        }
+    }
     flush_acc(acc, lane);
     if (UNIQUE)
         flush_acc(uacc, lane);
@@ -950,17 +1015,23 @@ __host__ __device__ __forceinline__ uint32_t count_chunk(uint64_t total, uint32_
 }
 
 constexpr int kCountThreads = 256;
+constexpr int kRowThreads = 512;  // of a CTA with a shared-memory row, four a SM where the rows allow
 
 // Batched persistent kernel: CTAs take whole queries from a work counter
 // (largest first); with SMEM the query's reference row is accumulated in shared
 // memory and written once, coalesced; without, counters go to the zeroed global
 // row with atomics, and the work may be split into key-range chunks (P.items) so
 // that one large query (a read set) spreads over many SMs.
+// Five CTAs a SM in the global rows, for all that some registers spill: 500 of 1,000
+// genomes in species of 24 637 -> 571 us, 500 of 2,000 without the filter 379 -> 347 (six:
+// 563 and 327, but 2 to 4 % more where species are long).
 template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE>
-__global__ void __launch_bounds__(kCountThreads, 4) k_count_batched(CountParams P)
+__global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 : LOWER ? 6 : 5) k_count_batched(CountParams P)
 {
+    static_assert(!(WIDE && (SMEM || LOWER)), "wide groups leave ordinary blocks in global rows only");
     extern __shared__ uint32_t sm[];
-    __shared__ ProbeQueue queues[kCountThreads / 32];
+    constexpr bool kRow = SMEM || LOWER;
+    __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
     __shared__ WarpCells cells[SMEM ? 1 : UNIQUE ? 2 : 1][SMEM ? 1 : kCountThreads / 32];
     __shared__ int s_item;
     const uint64_t objmask = (P.obj_bits >= 64) ? ~0ull : ((1ull << P.obj_bits) - 1);
@@ -1012,8 +1083,7 @@ __global__ void __launch_bounds__(kCountThreads, 4) k_count_batched(CountParams 
         if (SMEM) {
             const SmemAcc acc{row0, row0 + nref, row0 + 2 * nref, row0 + 3 * nref};
             const SmemAcc uacc{row1, row1 + nref, row1 + 2 * nref, row1 + 3 * nref};
-            process_query<LOWER, UNIQUE, WIDE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x,
-                                               queues[warp]);
+            process_query_row<LOWER, UNIQUE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
         } else {
             const WarpAcc acc{{P.out_ctx + row, P.out_obj + row}, &cells[0][warp]};
             const WarpAcc uacc{{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr},
@@ -1026,8 +1096,11 @@ __global__ void __launch_bounds__(kCountThreads, 4) k_count_batched(CountParams 
                 cb = b + (uint64_t)(it - (int)P.chunk_prefix[q]) * chunk_keys;
                 ce = min(e, cb + (uint64_t)chunk_keys);
             }
-            process_query<LOWER, UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x,
-                                               queues[warp]);
+            if constexpr (kRow)
+                process_query_row<LOWER, UNIQUE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
+            else
+                process_query<UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x,
+                                                   blockDim.x, queues[warp]);
         }
         __syncthreads();
         if (SMEM) {
@@ -1054,14 +1127,17 @@ __global__ void __launch_bounds__(kCountThreads, 4) k_count_batched(CountParams 
 // stride over the chunk's entries.  Counters go to the zeroed global rows through the
 // warp's own cells, as in the chunked mode.
 //
-// Bound by the latency of dependent reads (filter, table, postings) at 32 warps a SM.
+// Bound by the latency of dependent reads (filter, table, postings) at 32 warps a SM (40:
+// 288 instead of 257 us for the 1,500 queries, the cache's share of the SM is smaller).
 // Measured (B200, whole calls): 1,500 assemblies x 2,000 references 341 -> 262 us, 40 read
 // sets x 2,000 with unique contexts 357 -> 211 us, 1,500 x 2,000 in species of 24 with
 // unique contexts 972 -> 730 us.
 template <bool LOWER, bool UNIQUE, bool WIDE>
-__global__ void __launch_bounds__(kCountThreads, 4) k_count_striped(CountParams P)
+__global__ void __launch_bounds__(kCountThreads, LOWER ? 6 : 4) k_count_striped(CountParams P)
 {
-    __shared__ ProbeQueue queues[kCountThreads / 32];
+    constexpr bool kRow = LOWER;
+    static_assert(!(WIDE && LOWER), "wide groups leave ordinary blocks only");
+    __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
     __shared__ WarpCells cells[UNIQUE ? 2 : 1][kCountThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     WarpAcc{{}, &cells[0][warp]}.clear(lane);
@@ -1087,8 +1163,11 @@ __global__ void __launch_bounds__(kCountThreads, 4) k_count_striped(CountParams 
         const WarpAcc uacc{{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr},
                            &cells[UNIQUE][warp]};
         const FilterView fv{P.bloom + stripe_words * w.pad, P.bloom_mask, 1, nullptr, policy};
-        process_query<LOWER, UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32,
-                                           queues[warp]);
+        if constexpr (kRow)
+            process_query_row<LOWER, UNIQUE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32);
+        else
+            process_query<UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32,
+                                               queues[warp]);
     }
 }
 
@@ -3136,10 +3215,11 @@ template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE = false>
 int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStream_t st)
 {
     auto kern = k_count_batched<LOWER, UNIQUE, SMEM, WIDE>;
-    if (smem > 48 * 1024)
+    constexpr int threads = SMEM ? kRowThreads : kCountThreads;
+    if (smem)  // its limit counts the kernel's own shared memory too
         CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCountThreads, smem));
+    CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     if (per_sm < 1)
         return fail(KSSDGPU_ERR_CAPACITY, "shared-memory row does not fit one CTA");
     int grid = ix->sms * per_sm;
@@ -3148,7 +3228,7 @@ int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStr
     if (grid > units)
         grid = std::max(units, 1);
     CUDA_TRY(cudaMemsetAsync(P.work, 0, sizeof(unsigned int), st));
-    kern<<<grid, kCountThreads, smem, st>>>(P);
+    kern<<<grid, threads, smem, st>>>(P);
     count_launch();
     CUDA_TRY(cudaGetLastError());
     return KSSDGPU_OK;
