@@ -676,9 +676,13 @@ __global__ void k_stripe_pos(const uint64_t *__restrict__ qkeys, const uint64_t 
 // unique-context rule.  Same credits as walk_context (src/command_ani.h:515-575): LOWER
 // stops at gid >= qgid, --ignoreconflict skips reference runs of several objects, the
 // sole owner is credited when its run counted.
+// NEIGHBOURS: a posting's neighbours come from the lanes beside, not from memory.  Measured
+// (B200, 128 queries x 512 references of one species, forced global rows): 3,738 -> 3,263
+// us; not where the probe queue counts unique contexts, whose registers are all in use (40
+// read sets x 2,000 references 203 -> 213 us).
 constexpr uint32_t kWarpWalk = 32;
 
-template <bool LOWER, bool UNIQUE, class Acc>
+template <bool LOWER, bool UNIQUE, bool NEIGHBOURS, class Acc>
 __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ post, uint32_t pb, uint32_t pe,
                                                   const uint64_t *__restrict__ qrun, int s, uint64_t objmask,
                                                   int qgid, int ignoreconflict, const Acc &acc, const Acc &uacc,
@@ -692,15 +696,25 @@ __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ p
     int sole_d = 0;
     bool sole_mine = false, sole_ok = false;
     uint64_t next = pb + lane < pe ? __ldg(post + pb + lane) : 0;
+    uint32_t last = 0xFFFFFFFFu;  // gid of the posting before these
     for (uint32_t p0 = pb; p0 < pe; p0 += 32) {
         const uint32_t p = p0 + lane;
         const bool in = p < pe;
         const uint64_t w = next;
         next = p + 32 < pe ? __ldg(post + p + 32) : 0;
         const uint32_t gid = (uint32_t)(w >> 32);
-        uint32_t pg = __shfl_up_sync(0xFFFFFFFFu, gid, 1);
-        if (lane == 0)
+        uint32_t pg = __shfl_up_sync(0xFFFFFFFFu, gid, 1), ng = gid;
+        if (NEIGHBOURS) {
+            ng = __shfl_down_sync(0xFFFFFFFFu, gid, 1);
+            const uint32_t after = __shfl_sync(0xFFFFFFFFu, (uint32_t)(next >> 32), 0);
+            if (lane == 0)
+                pg = last;
+            if (lane == 31)
+                ng = after;
+            last = __shfl_sync(0xFFFFFFFFu, gid, 31);
+        } else if (lane == 0) {
             pg = p0 > pb ? (uint32_t)(__ldg(post + p0 - 1) >> 32) : 0xFFFFFFFFu;
+        }
         const bool live = in && (!LOWER || (int)gid < qgid);
         const bool head = live && gid != pg;
         int d = min(kMinInit, dna_pop((uint32_t)w ^ q0));
@@ -711,7 +725,7 @@ __device__ __forceinline__ void walk_context_warp(const uint64_t *__restrict__ p
         }
         if (head) {
             uint32_t x = p + 1;
-            while (x < pe) {
+            while (ng == gid && x < pe) {  // a run of several objects: seldom
                 const uint64_t w2 = __ldg(post + x);
                 if ((uint32_t)(w2 >> 32) != gid)
                     break;
@@ -862,7 +876,7 @@ __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q,
         const uint32_t gb = __shfl_sync(0xFFFFFFFFu, pb, src), gc = __shfl_sync(0xFFFFFFFFu, pc, src);
         const uint64_t gi = __shfl_sync(0xFFFFFFFFu, i, src);
         const int gs = __shfl_sync(0xFFFFFFFFu, s, src);
-        walk_context_warp<false, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
+        walk_context_warp<false, UNIQUE, !UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
                                          acc, uacc, lane);
     }
 }
@@ -941,7 +955,8 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
         flush_acc(uacc, lane);
 }
 
-// The same entries, an entry a lane and round, for shared-memory rows and lower blocks.  A
+// The same entries, an entry a lane and round (LANES), for shared-memory rows, lower blocks
+// and long walks (walks_long).  A
 // lower block is a part of an index's own genomes: every key is found and most credit
 // nothing (a context's only owner is the query itself), so a full warp in the probe is worth
 // less than the warps in flight that the queue's registers and shared memory cost; so are
@@ -997,7 +1012,7 @@ __device__ __forceinline__ void process_query_row(const CountParams &P, uint64_t
             const uint32_t gb = __shfl_sync(0xFFFFFFFFu, pb, src), gc = __shfl_sync(0xFFFFFFFFu, pc, src);
             const uint64_t gi = __shfl_sync(0xFFFFFFFFu, i, src);
             const int gs = __shfl_sync(0xFFFFFFFFu, s, src);
-            walk_context_warp<LOWER, UNIQUE>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
+            walk_context_warp<LOWER, UNIQUE, true>(P.post, gb, gb + gc, P.qkeys + gi, gs, objmask, qgid, P.ignoreconflict,
                                              acc, uacc, lane);
         }
     }
@@ -1025,12 +1040,12 @@ constexpr int kRowThreads = 512;  // of a CTA with a shared-memory row, four a S
 // Five CTAs a SM in the global rows, for all that some registers spill: 500 of 1,000
 // genomes in species of 24 637 -> 571 us, 500 of 2,000 without the filter 379 -> 347 (six:
 // 563 and 327, but 2 to 4 % more where species are long).
-template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE>
-__global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 : LOWER ? 6 : 5) k_count_batched(CountParams P)
+template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE, bool LANES>
+__global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 : LANES ? 6 : 5) k_count_batched(CountParams P)
 {
-    static_assert(!(WIDE && (SMEM || LOWER)), "wide groups leave ordinary blocks in global rows only");
+    static_assert(!(WIDE && (SMEM || LANES)) && (LANES || !LOWER), "wide groups leave ordinary blocks in global rows only");
     extern __shared__ uint32_t sm[];
-    constexpr bool kRow = SMEM || LOWER;
+    constexpr bool kRow = SMEM || LANES;
     __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
     __shared__ WarpCells cells[SMEM ? 1 : UNIQUE ? 2 : 1][SMEM ? 1 : kCountThreads / 32];
     __shared__ int s_item;
@@ -1132,11 +1147,11 @@ __global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 :
 // Measured (B200, whole calls): 1,500 assemblies x 2,000 references 341 -> 262 us, 40 read
 // sets x 2,000 with unique contexts 357 -> 211 us, 1,500 x 2,000 in species of 24 with
 // unique contexts 972 -> 730 us.
-template <bool LOWER, bool UNIQUE, bool WIDE>
-__global__ void __launch_bounds__(kCountThreads, LOWER ? 6 : 4) k_count_striped(CountParams P)
+template <bool LOWER, bool UNIQUE, bool WIDE, bool LANES>
+__global__ void __launch_bounds__(kCountThreads, LANES ? 6 : 4) k_count_striped(CountParams P)
 {
-    constexpr bool kRow = LOWER;
-    static_assert(!(WIDE && LOWER), "wide groups leave ordinary blocks only");
+    constexpr bool kRow = LANES;
+    static_assert(!(WIDE && LANES) && (LANES || !LOWER), "wide groups leave ordinary blocks only");
     __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
     __shared__ WarpCells cells[UNIQUE ? 2 : 1][kCountThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -3211,10 +3226,10 @@ int check_dev_err(kssdgpu_index *ix, cudaStream_t st)
 
 uint32_t env_u32(const char *name, uint32_t def, uint32_t lo, uint32_t hi);
 
-template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE = false>
+template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE = false, bool LANES = LOWER>
 int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStream_t st)
 {
-    auto kern = k_count_batched<LOWER, UNIQUE, SMEM, WIDE>;
+    auto kern = k_count_batched<LOWER, UNIQUE, SMEM, WIDE, LANES>;
     constexpr int threads = SMEM ? kRowThreads : kCountThreads;
     if (smem)  // its limit counts the kernel's own shared memory too
         CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -3234,10 +3249,10 @@ int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStr
     return KSSDGPU_OK;
 }
 
-template <bool LOWER, bool UNIQUE, bool WIDE = false>
+template <bool LOWER, bool UNIQUE, bool WIDE = false, bool LANES = LOWER>
 int launch_striped(kssdgpu_index *ix, const CountParams &P, cudaStream_t st)
 {
-    auto kern = k_count_striped<LOWER, UNIQUE, WIDE>;
+    auto kern = k_count_striped<LOWER, UNIQUE, WIDE, LANES>;
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCountThreads, 0));
     const int grid = ix->sms * std::max(per_sm, 1);  // persistent: the item count stays on the device
@@ -3278,6 +3293,18 @@ bool uses_smem_row(const kssdgpu_index *ix, unsigned flags)
     if (flags & (KSSDGPU_PLAIN | KSSDGPU_GLOBAL_ACC))
         return false;
     return smem_row_fits(ix, flags) && ((flags & KSSDGPU_SMEM_ACC) || ix->count_smem);
+}
+
+// Ordinary blocks whose found contexts are mostly walked one by one, by their lane (runs of
+// several objects, conflicts) or by the warp (long groups that are not left to the tensor
+// cores), gain little from postings dealt out over the lanes and take an entry a lane, at 48
+// warps a SM.  Measured (B200, indexes with conflicts, queue -> this): 500 queries x 2,000
+// references 478 -> 395 us, 500 x 1,000 in species of 24 985 -> 860, 128 x 512 of one species
+// 4,450 -> 3,830; without conflicts the queue wins (one species apart): 500 x 2,000 464 (an
+// entry a lane) -> 402.
+bool walks_long(const kssdgpu_index *ix)
+{
+    return ix->f_conflict || (ix->f_groups && ix->f_postings >= (unsigned long long)kWarpWalk * ix->f_groups);
 }
 
 // Key-range chunks of at most `chunk` entries for the global-row kernel, the queries
@@ -3531,6 +3558,11 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
     else if (wide)
         rc = unique ? launch_batched<false, true, false, true>(ix, P, 0, st)
                     : launch_batched<false, false, false, true>(ix, P, 0, st);
+    else if (!lower && walks_long(ix))
+        rc = striped ? (unique ? launch_striped<false, true, false, true>(ix, P, st)
+                               : launch_striped<false, false, false, true>(ix, P, st))
+                     : (unique ? launch_batched<false, true, false, false, true>(ix, P, 0, st)
+                               : launch_batched<false, false, false, false, true>(ix, P, 0, st));
     else if (striped)
         rc = lower ? launch_striped<true, false>(ix, P, st)
                    : unique ? launch_striped<false, true>(ix, P, st) : launch_striped<false, false>(ix, P, st);
