@@ -12,9 +12,9 @@ genome-pairs = n^2 matrix cells per step.
 
 Arms:
   ours (default)   value: one self step from the resident index per timed step --
-                   zero fill of the dense lower triangle plus the one-pass scan join
-                   (every context group's bounds read, every shared context joined;
-                   nothing cached between steps); e2e: the reference-facing C-ABI call
+                   zero fill of the dense lower triangle plus the join over the
+                   index's list of shared contexts (made when the index is built, every
+                   shared context joined in every step; no result cached between steps); e2e: the reference-facing C-ABI call
                    kssdgpu_count_lower with HOST buffers (query keys H2D, dense
                    counters D2H) every step, pinned in one call, and as the reference's
                    drivers call it (64-query blocks, pageable buffers); beside it the
@@ -160,11 +160,11 @@ def probe_model_bytes(n_keys, postings_walked, cells):
     return 8 * n_keys + 12 * postings_walked + 16 * cells
 
 
-def scan_join_bytes(contexts, shared_postings, touched):
-    """Distinct bytes of the one-pass scan join: every context group's bounds (4 B per
-    group + 1), the postings of groups of >= 2 (8 B each) and the touched counter cells
-    read and written once (2 x 16 B)."""
-    return 4 * (contexts + 1) + 8 * shared_postings + 2 * 16 * touched
+def join_bytes(groups, shared_postings, touched):
+    """Distinct bytes of the self join over the index's list of shared contexts: a word per
+    group of >= 2 postings, a word per posting in them (the object beside the genome's
+    number in its block) and the touched counter cells read and written once (2 x 16 B)."""
+    return 4 * groups + 4 * shared_postings + 2 * 16 * touched
 
 
 def lower_equals_dense(lower_c, lower_o, dense_c, dense_o, n, rows=1024):
@@ -289,7 +289,7 @@ def run_reference(args, rank, world):
 
 
 def leg_north_star(args, timer, dev, stream, peak):
-    """The 20,000-genome all-vs-all: the self step (fill + scan join) vs the batched
+    """The 20,000-genome all-vs-all: the self step (fill + join) vs the batched
     probe kernel vs the plain per-query kernel on the same counters (parity checked on
     the device), and the cached-plan join (first call = plan + join)."""
     import torch
@@ -334,14 +334,14 @@ def leg_north_star(args, timer, dev, stream, peak):
     same_probe = lower_equals_dense(lc, lo, dc, do, n)
     ms_plain = timer(lambda: idx.count_plain_dev(d_keys, d_offs, sk.offs, dc, do, lower=True, stream=stream), 1, 1)
     same_plain = lower_equals_dense(lc, lo, dc, do, n)
-    scan_bytes = scan_join_bytes(info["contexts"], facts["postings"], touched)
+    scan_bytes = join_bytes(facts["groups"], facts["postings"], touched)
     step_bytes = scan_bytes + 16 * cells
     model = probe_model_bytes(int(sk.offs[-1]), facts["pairs"], cells)
     out = {
         "workload": f"self-ani-matrix-{n}-genomes", "genomes": n, "entries": int(sk.offs[-1]),
         "unique_contexts": info["contexts"], "generate_s": gen_s, "index_build_s": build_s,
         "self_step": {"ms": ms_step, "genome_pairs_s": n * n / (ms_step / 1e3),
-                      "what": "zero fill of the dense lower triangle + one-pass scan join, nothing cached",
+                      "what": "zero fill of the dense lower triangle + join over the list of shared contexts, no result cached",
                       "roofline": {"bound": "hbm", "bytes": step_bytes, "achieved": step_bytes / ms_step / 1e6,
                                    "frac": step_bytes / ms_step / 1e6 / peak},
                       "probe_model_frac": model / ms_step / 1e6 / peak},
@@ -471,8 +471,8 @@ def leg_reads(args, timer, dev, stream, idx, ref):
 
 def leg_dense(args, timer, dev, stream, peak_tc):
     """One species: --dense-genomes genomes of one cluster at 0.1-2% substitutions (most
-    contexts shared by most genomes): the dense tensor-core self join vs the one-pass
-    scan on the same counters."""
+    contexts shared by most genomes): the dense tensor-core self join vs the join by
+    atomics on the same counters."""
     import torch
     import kssdgpu
     n = args.dense_genomes
@@ -775,7 +775,7 @@ def run_ours(args, rank, world, local_rank):
     def plain_step():
         idx.count_plain_dev(d_keys, d_offs, sk.offs, d_c, d_o, lower=True, stream=stream)
 
-    # ---- parity on the benchmark's own inputs: scan join == batched probe == plain == cached-plan join
+    # ---- parity on the benchmark's own inputs: self join == batched probe == plain == cached-plan join
     probe_step()
     idx.sync(stream)
     self_step()
@@ -802,7 +802,7 @@ def run_ours(args, rank, world, local_rank):
     self_step()
     torch.cuda.synchronize()
     launches_per_step = kssdgpu.launch_count() - launches0
-    # the step (zero fill + scan join, the join launched programmatically after the
+    # the step (zero fill + join, the join launched programmatically after the
     # fill) captured once into a CUDA graph and replayed: no host gap between the two
     # launches inside the timed region; direct launches are timed beside it
     ms_direct = timer(self_step, args.steps, args.warmup)
@@ -842,19 +842,19 @@ def run_ours(args, rank, world, local_rank):
     launches_timed = launches_per_step * args.steps
     value = replica_value(world, n * n, ms_step / 1e3)
 
-    # ---- the dominant kernel alone: the scan join, counters zeroed outside the events
+    # ---- the dominant kernel alone: the join, counters zeroed outside the events
     zero = lambda: (d_lc.zero_(), d_lo.zero_())  # noqa: E731
     ms_scan = timer(lambda: self_step(kssdgpu.NO_ZERO), args.steps, 2, pre=zero)
-    scan_bytes = scan_join_bytes(info["contexts"], facts["postings"], touched)
+    scan_bytes = join_bytes(facts["groups"], facts["postings"], touched)
     step_bytes = scan_bytes + 16 * lower_cells
     model_bytes = probe_model_bytes(int(sk.offs[-1]), facts["pairs"], lower_cells)
     achieved = scan_bytes / (ms_scan / 1e3) / 1e9
     traffic = None
-    tfile = os.path.join(ROOT, "profiles", "k_self_scan_traffic.json")
+    tfile = os.path.join(ROOT, "profiles", "k_self_pairs_traffic.json")
     if os.path.exists(tfile):
         try:
             t = json.load(open(tfile))
-            if t.get("workload_genomes") == n:  # the ncu capture of this workload's scan-join launch
+            if t.get("workload_genomes") == n:  # the ncu capture of this workload's join launch
                 traffic = t.get("bytes_per_launch")
         except Exception:
             traffic = None
@@ -969,8 +969,8 @@ def run_ours(args, rank, world, local_rank):
             "config": {"workload": WORKLOAD["name"], "genomes": n, "entries": int(sk.offs[-1]),
                        "unique_contexts": info["contexts"], "matrix_cells": n * n,
                        "lower_pairs": lower_cells,
-                       "path": "self step from the resident index: zero fill + one-pass scan join "
-                               "(kssdgpu_self_lower_dev), nothing cached between steps",
+                       "path": "self step from the resident index: zero fill + join over its list of shared "
+                               "contexts (kssdgpu_self_lower_dev), no result cached between steps",
                        "l2": "flushed (256 MB write) before every timed step",
                        "launch": launch_mode, "ms_per_step_direct_launches": ms_direct,
                        "parallelism": f"replicas x{world}" if world > 1 else "1 GPU"},
@@ -984,16 +984,16 @@ def run_ours(args, rank, world, local_rank):
                                              "(as the reference's drivers call the counting function)"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": peak_kind,
-                         "kernel": "k_self_scan (one-pass scan join)", "ms_per_launch": ms_scan,
+                         "kernel": "k_self_pairs (join over the shared contexts)", "ms_per_launch": ms_scan,
                          "algorithmic_bytes": scan_bytes,
-                         "bytes_model": "4 B per context group + 1 (bounds) + 8 B per posting of a group of >= 2 "
-                                        "+ 2 x 16 B per touched lower cell",
+                         "bytes_model": "4 B per shared context + 4 B per posting of one + 2 x 16 B per touched "
+                                        "lower cell",
                          "touched_cells": touched, "shared_groups": facts["groups"],
                          "shared_postings": facts["postings"], "pairs": facts["pairs"]},
             "step_roofline": {"bound": "hbm", "algorithmic_bytes": step_bytes,
                               "achieved": step_bytes / (ms_step / 1e3) / 1e9,
                               "frac": step_bytes / (ms_step / 1e3) / 1e9 / peak,
-                              "what": "zero fill of the dense lower triangle (16 B per cell) + scan join",
+                              "what": "zero fill of the dense lower triangle (16 B per cell) + join",
                               "probe_model_bytes": model_bytes,
                               "probe_model_frac": model_bytes / (ms_step / 1e3) / 1e9 / peak},
             "kernels": {

@@ -48,8 +48,8 @@ extern "C" {
 #define KSSDGPU_SMEM_ACC 0x20u      /* force shared-memory accumulator rows (KSSDGPU_ERR_CAPACITY when a
                                        row of the index's references does not fit) */
 #define KSSDGPU_SELF_PLAN 0x40u     /* self lower triangle: join over the index's cached set-major plan
-                                       (built and kept on first use) instead of the one-pass scan */
-#define KSSDGPU_SELF_SCAN 0x80u     /* self lower triangle: the one-pass scan join, whatever the density */
+                                       (built and kept on first use) instead of the list of shared contexts */
+#define KSSDGPU_SELF_SCAN 0x80u     /* self lower triangle: the join by atomics, whatever the density */
 #define KSSDGPU_SELF_DENSE 0x100u   /* self lower triangle: the dense tensor-core join, whatever the
                                        density (conflict-free indexes only) */
 
@@ -357,13 +357,13 @@ int kssdgpu_self_plan_info(kssdgpu_index_t *idx, uint64_t *groups, uint64_t *pos
 /*
  * Which join kssdgpu_self_lower(_dev) takes for these flags (KSSDGPU_PATH_*), and the
  * index's shared-context density: pairs of postings of shared contexts / (nref^2 x
- * alleles of shared contexts), the ratio of the scan's counter updates to the dense
+ * alleles of shared contexts), the ratio of that join's counter updates to the dense
  * GEMM's multiply-adds up to a constant (the allele count -- distinct objects per
  * shared context -- is estimated at index build from up to 65,536 sampled context
  * groups).  Without a path flag the dense tensor-core join is taken when the index is
  * conflict-free, its estimated time (from the shared contexts' sizes and pairs) is below
- * the scan's and its operands fit in half of the free device memory; else the one-pass
- * scan.  No reference counterpart.
+ * the join by atomics' and its operands fit in half of the free device memory; else the
+ * join by atomics (KSSDGPU_PATH_SCAN).  No reference counterpart.
  */
 #define KSSDGPU_PATH_SCAN 0
 #define KSSDGPU_PATH_DENSE 1
