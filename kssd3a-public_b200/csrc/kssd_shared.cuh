@@ -380,6 +380,10 @@ __global__ void __launch_bounds__(kPairThreads, PACK ? 5 : 4) k_self_pairs(const
         }
         __syncthreads();  // the block's tables are reused by the next
     }
+    // A CTA without a block waits too: the next kernel on the stream is ordered behind this one
+    // alone, and must not start while the fill still runs.
+    if (!waited)
+        pdl_wait_primary();
 }
 
 // Large groups, one CTA each: a warp takes every eighth genome j, its lanes consecutive

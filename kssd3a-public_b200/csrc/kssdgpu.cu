@@ -3020,7 +3020,7 @@ int build_shared(kssdgpu_index *ix, const unsigned long long small[3], cudaStrea
     const uint32_t blocks1 = (uint32_t)((run[1].pairs + kBlockPairs - 1) >> kBlockLog);
     const uint64_t blocks = (uint64_t)blocks0 + 1 + blocks1;  // one between the runs stays empty
     ix->sh_small[0] = blocks0;
-    ix->sh_small[1] = (uint32_t)blocks;
+    ix->sh_small[1] = small[0] ? (uint32_t)blocks : 0;  // no launch for the empty one alone
     ix->sh_large[0] = (uint32_t)run[0].groups;  // large narrow groups: [run 0's end, narrow)
     ix->sh_large[1] = (uint32_t)(narrow + run[1].groups);  // large wide groups: [.., n)
     struct Temps {
@@ -4480,6 +4480,7 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
         cfg.blockDim = dim3(kScanThreads);
         CUDA_TRY(cudaLaunchKernelEx(&cfg, k_self_scan, (const uint32_t *)ix->gbeg, ix->u, (const uint64_t *)ix->post,
                                     (flags & KSSDGPU_IGNORECONFLICT) ? 1 : 0, oc, oo));
+        count_launch();
     } else {
         const uint32_t nblocks = ix->sh_small[narrow ? 0 : 1];
         if (nblocks) {
@@ -4490,6 +4491,7 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
                                         (const SharedGroup *)ix->sh_list, (const uint32_t *)ix->sh_place,
                                         (const uint32_t *)ix->sh_object, (const unsigned char *)ix->sh_number,
                                         (const uint32_t *)ix->sh_table, (const uint64_t *)ix->post, oc, oo));
+            count_launch();
         }
         const uint32_t nnarrow = (uint32_t)(ix->f_groups - ix->f_wgroups), n = (uint32_t)ix->f_groups;
         const uint32_t large[2][2] = {{ix->sh_large[0], nnarrow}, {ix->sh_large[1], narrow ? ix->sh_large[1] : n}};
@@ -4500,7 +4502,6 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
                 count_launch();
             }
     }
-    count_launch();
     CUDA_TRY(cudaGetLastError());
     return KSSDGPU_OK;
 }
