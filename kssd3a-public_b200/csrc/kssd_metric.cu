@@ -210,7 +210,7 @@ __device__ __forceinline__ HgbNode load_node(const uint4 *nodes, uint32_t i)
 
 // Walks kWays trees side by side, t0, t0 + step, ...: every round loads one node of each,
 // and those loads are independent.  leaf[k] receives the leaf's node number (of a tree
-// below P.ntrees).  Returns true when a feature of `unc` came within kTol of a threshold
+// below P.ntrees), a number below P.nnodes in any case.  Returns true when a feature of `unc` came within kTol of a threshold
 // on a path, or a walk did not end on a leaf (a malformed model): another leaf is
 // possible, the cell is left to the host.
 template <bool SHARED, int kWays>
@@ -251,6 +251,10 @@ __device__ __forceinline__ bool walk_trees(const MetricParams &P, const uint4 *n
             }
         }
     }
+#pragma unroll
+    for (int k = 0; k < kWays; ++k)
+        if ((open >> k) & 1u)  // the last step's node was not looked at: it may lie past the model
+            leaf[k] = 0;
     return bad || open;
 }
 
