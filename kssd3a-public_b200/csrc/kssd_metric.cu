@@ -169,7 +169,6 @@ constexpr bool kCalibrate = KSSD_NUM_CODENS >= 11;
 // The calibration trees' features of a cell (refaf_hgb_predict_ani,
 // src/model_refaf_hgb.h:7593-7628): x[0..10], and the mask of those derived from log /
 // log1p or from an inexact raw ANI, whose thresholds are compared with a tolerance.
-constexpr int kFeatures = 11;
 __device__ uint32_t hgb_features(const MetricParams &P, double raw_ani, bool raw_unc, double ref_af, const Feat &f,
                                  double *x, int stride)
 {

@@ -15,6 +15,7 @@ struct HgbNode {
     unsigned short left, right;
 };
 static_assert(sizeof(HgbNode) == 16, "calibration node records are 16 bytes");
+constexpr int kFeatures = 11;  // features a split may name; the kernel does not check the numbers
 
 // the options a matrix value reads (a subset of the reference's ani_opt_t)
 struct MetricParams {

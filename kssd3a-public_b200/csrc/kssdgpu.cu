@@ -4962,8 +4962,20 @@ static int metric_params(int device, const kssdgpu_metric_opt_t *o, kssd::Metric
         m = HgbDeviceModel{};
         CUDA_TRY(pool_malloc(&m.d_nodes, (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode)));
         CUDA_TRY(pool_malloc(&m.d_begin, ((size_t)o->hgb_trees + 1) * sizeof(uint32_t)));
-        CUDA_TRY(cudaMemcpy(m.d_nodes, o->hgb_nodes, (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode),
-                            cudaMemcpyHostToDevice));
+        // a split on a feature that there is not becomes one onto itself: its walk does not end
+        // on a leaf, so the cell is left to the host, and the kernel need not ask at each step
+        const kssd::HgbNode *nodes = static_cast<const kssd::HgbNode *>(o->hgb_nodes);
+        std::vector<kssd::HgbNode> sound;
+        for (uint32_t t = 0; t < o->hgb_trees; ++t)
+            for (uint32_t i = o->hgb_tree_begin[t]; i < o->hgb_tree_begin[t + 1]; ++i)
+                if (!(nodes[i].flags & 1u) && (nodes[i].feature < 0 || nodes[i].feature >= kssd::kFeatures)) {
+                    if (sound.empty())
+                        sound.assign(nodes, nodes + o->hgb_nodes_count);
+                    sound[i].feature = 0;
+                    sound[i].left = sound[i].right = (unsigned short)(i - o->hgb_tree_begin[t]);
+                }
+        CUDA_TRY(cudaMemcpy(m.d_nodes, sound.empty() ? nodes : sound.data(),
+                            (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode), cudaMemcpyHostToDevice));
         CUDA_TRY(cudaMemcpy(m.d_begin, o->hgb_tree_begin, ((size_t)o->hgb_trees + 1) * sizeof(uint32_t),
                             cudaMemcpyHostToDevice));
         m.host_nodes = o->hgb_nodes;

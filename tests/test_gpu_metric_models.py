@@ -1,5 +1,6 @@
 """The matrix-value kernel on calibration models whose walks do not end on a leaf: a cycle, a
-child past the model, more levels than a walk takes, and such a level's child past the model.
+child past the model, more levels than a walk takes, such a level's child past the model, and splits
+on features that there are not.
 Every cell that takes the trees is left to the host, the others are valued as ever; few such
 cells (the warp walks the trees of one together) and many (a thread walks its own)."""
 import ctypes as C
@@ -37,6 +38,8 @@ MODELS = {
     "past": [_split(60000)],
     "deep": _chain(70, [_leaf(0.125)]),
     "deep_past": _chain(64, [_split(60000)]),
+    "feature": [_split(1), (2.0, 11, 0, 2, 2, 0), _leaf(0.125)],
+    "no_feature": [(2.0, -100, 0, 1, 1, 0), _leaf(0.125)],
 }
 
 
