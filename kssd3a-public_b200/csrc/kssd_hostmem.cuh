@@ -9,125 +9,54 @@
 // returns.  cudaMalloc and cudaFree of each cost 0.3 to 0.7 ms (1.3 ms at 1 GB, and many
 // times that on a host whose other processes allocate too), which was most of a small
 // index's build: 64 genomes 6.2 ms, of which kernels 0.3.  Freed blocks are kept instead
-// and handed out again for requests they fit.  Kept: at most kPoolKeep bytes a device,
+// and handed out again for requests they fit (kssd_pool.h).  Kept: at most kPoolKeep bytes a device,
 // blocks that two indexes in a row left unused are given back, and all of them when an
 // allocation fails.  (cudaMallocAsync's pool was measured too: 6 ms per 500 MB that its
 // reservation grows by.)
 constexpr uint64_t kPoolKeep = 2ull << 30;
 
-class DevicePool {
-public:
-    cudaError_t get(void **p, size_t bytes)
-    {
-        *p = nullptr;
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess)
-            return e;
-        // sizes in steps of an eighth of their power of two (at least 512 bytes), so that
-        // requests a little apart use one another's blocks
-        size_t step = 512;
-        while (step * 16 < bytes)
-            step <<= 1;
-        const size_t size = (std::max<size_t>(bytes, 1) + step - 1) / step * step;
-        try {
-            std::lock_guard<std::mutex> lock(mu_);
-            const auto it = idle_.lower_bound({dev, size});
-            if (it != idle_.end() && it->first.first == dev && it->first.second <= size + size / 4) {
-                live_.emplace(it->second.p, Live{it->first.second, dev});
-                *p = it->second.p;
-                idle_bytes_[dev] -= it->first.second;
-                idle_.erase(it);
-                return cudaSuccess;
-            }
-        } catch (const std::bad_alloc &) {
-            return cudaErrorMemoryAllocation;
-        }
-        e = cudaMalloc(p, size);
-        if (e == cudaErrorMemoryAllocation) {  // the kept blocks may be what is missing
+// Id of the calling thread's context, 0 where there is none.
+uint64_t context_id()
+{
+    using GetId = int (*)(void *, unsigned long long *);
+    static const GetId get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            release(dev, ~0ull);
-            e = cudaMalloc(p, size);
-            if (e == cudaErrorMemoryAllocation && size != bytes) {
-                cudaGetLastError();
-                e = cudaMalloc(p, std::max<size_t>(bytes, 1));
-            }
+            f = nullptr;
         }
-        if (e == cudaSuccess) {
-            try {
-                std::lock_guard<std::mutex> lock(mu_);
-                live_.emplace(*p, Live{size, dev});
-            } catch (const std::bad_alloc &) {
-            }  // unknown to put(): freed there
+        return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    if (!get)
+        return 0;
+    if (get(nullptr, &id) != 0) {  // no context yet, or one that is gone
+        if (cudaFree(nullptr) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
         }
+        if (get(nullptr, &id) != 0)
+            return 0;
+    }
+    return id;
+}
+
+struct CudaMemory {
+    using Error = cudaError_t;
+    static constexpr cudaError_t kOk = cudaSuccess, kNoMemory = cudaErrorMemoryAllocation;
+    static uint64_t context() { return context_id(); }
+    static cudaError_t alloc(void **p, size_t bytes)
+    {
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation)
+            cudaGetLastError();
         return e;
     }
-
-    // p: a block whose device work has ended (the caller synchronized).
-    void put(void *p)
-    {
-        if (!p)
-            return;
-        try {
-            std::lock_guard<std::mutex> lock(mu_);
-            const auto it = live_.find(p);
-            if (it != live_.end()) {
-                const Live b = it->second;
-                live_.erase(it);
-                if (idle_bytes_[b.dev] + b.bytes <= kPoolKeep) {
-                    idle_.emplace(std::make_pair(b.dev, b.bytes), Idle{p, epoch_});
-                    idle_bytes_[b.dev] += b.bytes;
-                    return;
-                }
-            }
-        } catch (const std::bad_alloc &) {
-        }
-        cudaFree(p);
-    }
-
-    // One index less: blocks of its device that two of them in a row did not use go back.
-    void age(int dev)
-    {
-        uint64_t now;
-        {
-            std::lock_guard<std::mutex> lock(mu_);
-            now = ++epoch_;
-        }
-        if (now > 2)
-            release(dev, now - 2);
-    }
-
-private:
-    struct Live {
-        size_t bytes;
-        int dev;
-    };
-    struct Idle {
-        void *p;
-        uint64_t epoch;
-    };
-
-    // Gives back the device's blocks kept since before epoch `until`.
-    void release(int dev, uint64_t until)
-    {
-        std::lock_guard<std::mutex> lock(mu_);
-        for (auto it = idle_.lower_bound({dev, 0}); it != idle_.end() && it->first.first == dev;) {
-            if (it->second.epoch < until) {
-                idle_bytes_[dev] -= it->first.second;
-                cudaFree(it->second.p);
-                it = idle_.erase(it);
-            } else {
-                ++it;
-            }
-        }
-    }
-
-    std::mutex mu_;
-    std::unordered_map<void *, Live> live_;
-    std::multimap<std::pair<int, size_t>, Idle> idle_;
-    std::map<int, uint64_t> idle_bytes_;
-    uint64_t epoch_ = 0;
+    static void release(void *p) { cudaFree(p); }
 };
+using DevicePool = BlockPool<CudaMemory, kPoolKeep>;
 
 // Never destroyed: at process exit the driver frees what it holds, in whatever order.
 DevicePool &device_pool()
@@ -158,8 +87,9 @@ void pool_free_idle(void *p) { device_pool().put(p); }
 // 11 GB/s at 98 MB here, 5 GB/s into pages not touched before, against 55 GB/s from
 // page-locked memory.  Copies of at least kStageMin bytes are cut into chunks that several
 // threads move between the caller's buffer and page-locked chunks of their own, the DMA of
-// one under the memcpy of the other.  The chunks (16 MB, page-locked on first use) belong to
-// the process; a second caller at the same time takes the driver's way.
+// one under the memcpy of the other.  The chunks (16 MB a context, page-locked on first use)
+// are kept and are that context's alone, which frees them when it is reset; a second caller at
+// the same time takes the driver's way.
 constexpr size_t kStageMin = 2u << 20, kStageChunk = 1u << 20;
 constexpr int kStageThreads = 8;
 
@@ -174,17 +104,15 @@ public:
         std::unique_lock<std::mutex> lock(mu_, std::try_to_lock);
         if (!lock.owns_lock())
             return false;
-        if (!pinned_ && cudaHostAlloc(&pinned_, kStageThreads * 2 * kStageChunk, cudaHostAllocPortable) != cudaSuccess) {
-            cudaGetLastError();
-            pinned_ = nullptr;
-            return false;
-        }
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess)
             return false;
-        const size_t chunks = (bytes + kStageChunk - 1) / kStageChunk;
+        char *pinned = chunks(context_id());
+        if (!pinned)
+            return false;
+        const size_t nchunks = (bytes + kStageChunk - 1) / kStageChunk;
         const int threads = (int)std::min<size_t>(
-            {(size_t)kStageThreads, std::max<size_t>(1, std::thread::hardware_concurrency() / 2), (chunks + 1) / 2});
+            {(size_t)kStageThreads, std::max<size_t>(1, std::thread::hardware_concurrency() / 2), (nchunks + 1) / 2});
         std::atomic<size_t> next{0};
         std::atomic<int> bad{(int)cudaSuccess};
         auto work = [&](int t) {
@@ -192,8 +120,7 @@ public:
             cudaEvent_t ev[2] = {nullptr, nullptr};
             for (int i = 0; i < 2 && e == cudaSuccess; ++i)
                 e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-            char *buf[2] = {(char *)pinned_ + (size_t)(2 * t) * kStageChunk,
-                            (char *)pinned_ + (size_t)(2 * t + 1) * kStageChunk};
+            char *buf[2] = {pinned + (size_t)(2 * t) * kStageChunk, pinned + (size_t)(2 * t + 1) * kStageChunk};
             size_t off[2] = {0, 0}, len[2] = {0, 0};  // len: a DMA of the slot is under way
             for (int s = 0; e == cudaSuccess && bad.load() == (int)cudaSuccess; s ^= 1) {
                 if (len[s]) {  // the slot's last DMA
@@ -202,8 +129,8 @@ public:
                         chunk(buf[s], off[s], len[s]);
                     len[s] = 0;
                 }
-                const size_t c = e == cudaSuccess ? next.fetch_add(1) : chunks;
-                if (c >= chunks)
+                const size_t c = e == cudaSuccess ? next.fetch_add(1) : nchunks;
+                if (c >= nchunks)
                     break;
                 const size_t o = c * kStageChunk, n = std::min(kStageChunk, bytes - o);
                 if (IN)
@@ -244,8 +171,25 @@ public:
     }
 
 private:
+    // The context's page-locked chunks, null where there are none.
+    char *chunks(uint64_t context)
+    {
+        if (!context)
+            return nullptr;
+        try {
+            void *&p = pinned_[context];
+            if (!p && cudaHostAlloc(&p, kStageThreads * 2 * kStageChunk, cudaHostAllocDefault) != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+            }
+            return static_cast<char *>(p);
+        } catch (const std::bad_alloc &) {
+            return nullptr;
+        }
+    }
+
     std::mutex mu_;
-    void *pinned_ = nullptr;
+    std::map<uint64_t, void *> pinned_;
 };
 
 Stager &stager()

@@ -12,6 +12,7 @@
 #include "kssdgpu.h"
 #include "kssd_dev.cuh"
 #include "kssd_metric.cuh"
+#include "kssd_pool.h"
 
 #include <cub/cub.cuh>
 #include <thrust/iterator/transform_iterator.h>
@@ -2850,6 +2851,7 @@ int grid_for(uint64_t n, int block = 256)
 
 struct kssdgpu_index {
     int device = 0;
+    uint64_t context = 0;  // that its memory belongs to
     int nref = 0;
     int obj_bits = 20;
     uint64_t n = 0;
@@ -3188,6 +3190,7 @@ int new_index(int nref, int obj_bits, int device, uint64_t n, kssdgpu_index **ou
     CUDA_TRY(cudaSetDevice(device));
     auto *ix = new kssdgpu_index();
     ix->device = device;
+    ix->context = context_id();
     ix->nref = nref;
     ix->obj_bits = obj_bits;
     ix->n = n;
@@ -4916,6 +4919,7 @@ int noalloc_scratch(int device, unsigned int **out)
 // Device copies of the calibration trees, one per device, replaced when a call passes
 // another model.
 struct HgbDeviceModel {
+    uint64_t context = 0;  // that they were made in
     const void *host_nodes = nullptr;
     uint32_t nodes = 0, trees = 0;
     kssd::HgbNode *d_nodes = nullptr;
@@ -4954,12 +4958,16 @@ static int metric_params(int device, const kssdgpu_metric_opt_t *o, kssd::Metric
     if ((int)g_hgb.size() <= device)
         g_hgb.resize(device + 1);
     HgbDeviceModel &m = g_hgb[device];
+    const uint64_t context = context_id();
+    if (m.context != context)
+        m = HgbDeviceModel{};  // cudaDeviceReset has freed them
     if (m.host_nodes != o->hgb_nodes || m.nodes != o->hgb_nodes_count || m.trees != o->hgb_trees) {
         if (m.d_nodes)
             pool_free(m.d_nodes);
         if (m.d_begin)
             pool_free(m.d_begin);
         m = HgbDeviceModel{};
+        m.context = context;
         CUDA_TRY(pool_malloc(&m.d_nodes, (size_t)o->hgb_nodes_count * sizeof(kssd::HgbNode)));
         CUDA_TRY(pool_malloc(&m.d_begin, ((size_t)o->hgb_trees + 1) * sizeof(uint32_t)));
         // a split on a feature that there is not becomes one onto itself: its walk does not end
@@ -5372,6 +5380,10 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     if (!ix)
         return;
     cudaSetDevice(ix->device);
+    if (ix->context != context_id()) {  // cudaDeviceReset has freed its memory and streams
+        delete ix;
+        return;
+    }
     cudaDeviceSynchronize();
     pool_free_idle(ix->post);
     pool_free_idle(ix->gkey);
@@ -5446,7 +5458,7 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     ix->w_qobj.release_idle();
     ix->w_at.release_idle();
     ix->w_g.release_idle();
-    device_pool().age(ix->device);
+    device_pool().age();
     delete ix;
 }
 
