@@ -634,7 +634,9 @@ cudaError_t lower_metric_launch(const MetricParams &P, int n, const unsigned lon
     const bool slots = metric_smem(Q.ntrees, Q.nnodes, shared) <= kMetricSmem && Q.nnodes <= 65536;
     const size_t smem = metric_smem(slots ? Q.ntrees : 0, Q.nnodes, shared);
     auto kern = shared ? k_lower_metric<true> : k_lower_metric<false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit is the context's: the same for every call, so that no thread lowers it before
+    // another one's launch
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMetricSmem);
     if (e != cudaSuccess)
         return e;
     kern<<<grid, kMetricThreads, smem, st>>>(Q, cells, rounds, slots ? kWarpCells : 0, lc, lo, qcnt, rcnt, out, recheck, cap, nrecheck);

@@ -3229,13 +3229,24 @@ int check_dev_err(kssdgpu_index *ix, cudaStream_t st)
 
 uint32_t env_u32(const char *name, uint32_t def, uint32_t lo, uint32_t hi);
 
+// Raises a kernel's limit on dynamic shared memory (which counts its static share too) to the
+// most that any call asks of it.  The limit is the context's, not the call's: set to what one
+// call needs, a thread lowers it between another thread's setting and its launch.
+template <class Kernel>
+cudaError_t allow_smem(Kernel kern, size_t most)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
+constexpr size_t kSmemRowLimit = 112 * 1024;  // a shared-memory row, at most
+
 template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE = false, bool LANES = LOWER>
 int launch_batched(kssdgpu_index *ix, const CountParams &P, size_t smem, cudaStream_t st)
 {
     auto kern = k_count_batched<LOWER, UNIQUE, SMEM, WIDE, LANES>;
     constexpr int threads = SMEM ? kRowThreads : kCountThreads;
-    if (smem)  // its limit counts the kernel's own shared memory too
-        CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem)
+        CUDA_TRY(allow_smem(kern, kSmemRowLimit));
     int per_sm = 0;
     CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
     if (per_sm < 1)
@@ -3281,8 +3292,6 @@ int launch_plain(kssdgpu_index *ix, const CountParams &P, const std::vector<uint
 }
 
 // shared-memory row budget: four 32-bit counters per reference (eight with unique)
-constexpr size_t kSmemRowLimit = 112 * 1024;
-
 bool smem_row_fits(const kssdgpu_index *ix, unsigned flags)
 {
     return (size_t)ix->nref * sizeof(unsigned long long) * ((flags & KSSDGPU_UNIQUE) ? 4 : 2) <= kSmemRowLimit;
@@ -3347,7 +3356,7 @@ cudaError_t wide_rows_shape(const kssdgpu_index *ix, Kernel kern, uint32_t npad,
 {
     const size_t per_warp = wide_warp_smem(npad, (uint32_t)ix->nref);
     warps = (int)std::min<size_t>(8, kWideSmem / per_warp);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(warps * per_warp));
+    cudaError_t e = allow_smem(kern, kWideSmem);
     int per_sm = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * 32, warps * per_warp);
@@ -4472,7 +4481,7 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
         if (ix->f_conflict) {
             CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_self_scan, kScanThreads, 0));
         } else {
-            CUDA_TRY(cudaFuncSetAttribute(pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pairs_smem));
+            CUDA_TRY(allow_smem(pairs_kernel, pairs_smem));  // one size a kernel
             CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pairs_kernel, kPairThreads, pairs_smem));
         }
         ix->scan_grid = std::max(1, per_sm) * ix->sms;
@@ -4571,7 +4580,7 @@ int dense_alleles_impl(kssdgpu_index *ix, uint32_t S, cudaStream_t st, uint32_t 
 {
     const int n = ix->nref;
     const size_t group_smem = dense_group_smem((uint32_t)n);
-    CUDA_TRY(cudaFuncSetAttribute(k_dense_alleles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)group_smem));
+    CUDA_TRY(allow_smem(k_dense_alleles, dense_group_smem(kDenseMaxGroup)));
     CUDA_TRY(ix->d_list.ensure(S));
     CUDA_TRY(ix->d_poff.ensure((size_t)S + 1));   // alleles per group, then the fill counter
     CUDA_TRY(ix->d_allele.ensure((size_t)S + 1)); // first allele row of every group
@@ -4693,7 +4702,7 @@ int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long lon
     ix->w_ran = false;
     const uint32_t npad = (uint32_t)dense_npad(ix);
     const size_t rows_smem = dense_rows_smem(npad);
-    CUDA_TRY(cudaFuncSetAttribute(k_dense_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem));
+    CUDA_TRY(allow_smem(k_dense_rows, dense_rows_smem(kDenseMaxGroup)));
     // 1. the shared groups, their allele counts and first allele rows
     uint32_t alleles = 0;
     const int arc = dense_alleles_impl(ix, S, st, alleles);
@@ -5541,7 +5550,7 @@ int kssdgpu_index_ref_ctx_counts(const kssdgpu_index_t *cix, int conflict, int i
     if (local <= kRefLocalBytes) {
         // one CTA per SM, two of them where their sums fit beside one another
         const int ctas = (int)std::min<uint64_t>((ix->u + 1023) / 1024, (uint64_t)ix->sms * (2 * local <= kRefLocalBytes ? 2 : 1));
-        CUDA_TRY(cudaFuncSetAttribute(k_ref_counts<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)local));
+        CUDA_TRY(allow_smem(k_ref_counts<true>, kRefLocalBytes));
         k_ref_counts<true><<<std::max(1, ctas), 1024, local, st>>>(ix->gbeg, ix->u, ix->post, conflict, ignoreconflict,
                                                                    ix->nref, c, c + ix->nref);
     } else {
