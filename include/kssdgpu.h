@@ -161,7 +161,9 @@ int kssdgpu_count_lower(kssdgpu_index_t *idx, const uint64_t *qry_keys, const ui
  * cudaStream_t or NULL for the legacy stream).  d_qry_offs are absolute offsets as
  * above; outputs are device arrays of nq*nref cells.  Asynchronous: the counters
  * are complete when the stream reaches this point; errors detected on the device
- * are reported by the next kssdgpu_sync(idx, stream).
+ * are reported by the next kssdgpu_sync(idx, stream).  A captured call counts every
+ * context by its postings (not on the tensor cores) and needs the scratch that an earlier
+ * call for as many queries left.
  */
 int kssdgpu_count_block_dev(kssdgpu_index_t *idx, const uint64_t *d_qry_keys,
                             const uint64_t *d_qry_offs, int nq, int qry_gid_offset, int lower,
@@ -263,6 +265,8 @@ int kssdgpu_self_votes(kssdgpu_index_t *idx, const uint64_t *keys, const uint64_
  * context's distinct objects (alleles) and takes one operand row per allele instead,
  * which synchronizes the stream once (for the allele count).  It writes every cell of the
  * triangle and needs a conflict-free index (KSSDGPU_ERR_ARG otherwise).
+ * While the stream is captured the default is the join by atomics: the dense join works in
+ * scratch of the index, which a later call may move.
  *
  * With KSSDGPU_SELF_PLAN: the first call builds a set-major plan of the index's
  * shared contexts (kept on the handle; later calls only join over it).  Where the

@@ -3349,6 +3349,19 @@ bool dense_fits(uint64_t need, uint64_t have)
     return need <= free_b / 2;
 }
 
+// Whether `st` is being captured.  The joins through scratch that grows with the call are not
+// chosen then: it could not be allocated, and a graph would hold its address while a later,
+// larger call moves it.
+bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 // Launch shape of k_wide_rows: warps of a CTA (as many as its shared memory holds, at most
 // 8) and the CTAs that fill the GPU.
 template <class Kernel>
@@ -3545,7 +3558,7 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
             CUDA_TRY(cudaMemsetAsync(uo, 0, cells * 8, st));
         }
     }
-    const bool wide = !lower && !use_smem && wide_block_chosen(ix, nq, flags);
+    const bool wide = !lower && !use_smem && wide_block_chosen(ix, nq, flags) && !capturing(st);
     if (wide) {
         const int rc = wide_block_begin(ix, nq, P, st);
         if (rc)
@@ -4795,7 +4808,8 @@ int self_lower_dev_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *o
 {
     if (flags & KSSDGPU_SELF_DENSE)
         return self_dense_impl(ix, oc, oo, st);
-    if (!(flags & (KSSDGPU_SELF_PLAN | KSSDGPU_SELF_SCAN)) && !(flags & KSSDGPU_NO_ZERO) && dense_chosen(ix))
+    if (!(flags & (KSSDGPU_SELF_PLAN | KSSDGPU_SELF_SCAN)) && !(flags & KSSDGPU_NO_ZERO) && !capturing(st) &&
+        dense_chosen(ix))
         return self_dense_impl(ix, oc, oo, st);
     if (!(flags & KSSDGPU_SELF_PLAN))
         return self_scan_impl(ix, flags, oc, oo, st);
