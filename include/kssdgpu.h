@@ -73,6 +73,11 @@ const char *kssdgpu_last_error(void);
  * files, so context creation overlaps the I/O. */
 int kssdgpu_init(int device);
 
+/* Gives back the device memory and the page-locked host memory that the library keeps for later
+ * calls on `device`: at most 2 GiB of blocks that indexes, calls and sketches returned, and 16 MB
+ * of chunks for host copies.  Memory in use stays. */
+int kssdgpu_trim(int device);
+
 /*
  * Device-resident CSR from the reference's inverted index records
  * (sortedcomb_ctxgid64obj32: n packed 12-byte {uint64 ctx<<20|gid; uint32 obj},
@@ -94,6 +99,10 @@ int kssdgpu_index_from_sketch(const uint64_t *keys, const uint64_t *offs, int nr
                               int device, kssdgpu_index_t **out);
 
 void kssdgpu_index_free(kssdgpu_index_t *idx);
+/* Releases the scratch that calls on the index have grown (a block of one species: up to 8 GiB);
+ * the next calls make what they need again.  Waits for the device.  The blocks are kept for later
+ * calls within kssdgpu_trim's bound. */
+int kssdgpu_index_trim(kssdgpu_index_t *idx);
 
 /* Calls on one index handle share its per-index device scratch (plans, work lists,
  * compact counters): do not make them from several host threads at once, and do

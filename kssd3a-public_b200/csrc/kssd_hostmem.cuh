@@ -9,10 +9,11 @@
 // returns.  cudaMalloc and cudaFree of each cost 0.3 to 0.7 ms (1.3 ms at 1 GB, and many
 // times that on a host whose other processes allocate too), which was most of a small
 // index's build: 64 genomes 6.2 ms, of which kernels 0.3.  Freed blocks are kept instead
-// and handed out again for requests they fit (kssd_pool.h).  Kept: at most kPoolKeep bytes a device,
-// blocks that two indexes in a row left unused are given back, and all of them when an
-// allocation fails.  (cudaMallocAsync's pool was measured too: 6 ms per 500 MB that its
-// reservation grows by.)
+// and handed out again for requests they fit (kssd_pool.h).  Kept: at most kPoolKeep bytes a
+// device; blocks that eight indexes or sketches in a row left unused are given back, all of them
+// when an allocation fails and by kssdgpu_trim, and the rest of the library counts them as free
+// memory.  (cudaMallocAsync's pool was measured too: 6 ms per 500 MB that its reservation grows
+// by.)
 constexpr uint64_t kPoolKeep = 2ull << 30;
 
 // Id of the calling thread's context, 0 where there is none.
@@ -80,6 +81,27 @@ void pool_free(void *p)
 }
 // After a synchronization that covers every use of the block.
 void pool_free_idle(void *p) { device_pool().put(p); }
+
+// Free device memory, the kept blocks (given up for any request) among it.
+cudaError_t free_memory(uint64_t &bytes)
+{
+    size_t free_b = 0, total_b = 0;
+    const cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+    bytes = e == cudaSuccess ? free_b + device_pool().idle_bytes() : 0;
+    return e;
+}
+
+// A block of exactly this size that is not kept (cudaFree it).
+template <class T>
+cudaError_t exact_malloc(T **p, size_t bytes)
+{
+    cudaError_t e = CudaMemory::alloc(reinterpret_cast<void **>(p), bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        device_pool().trim();
+        e = CudaMemory::alloc(reinterpret_cast<void **>(p), bytes);
+    }
+    return e;
+}
 
 // ------------------------------------------------------------------ staged copies
 //
@@ -168,6 +190,17 @@ public:
             t.join();
         err = (cudaError_t)bad.load();
         return true;
+    }
+
+    // Gives back the current context's chunks (none are in use while this holds the lock).
+    void trim()
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        const auto it = pinned_.find(context_id());
+        if (it != pinned_.end()) {
+            cudaFreeHost(it->second);
+            pinned_.erase(it);
+        }
     }
 
 private:

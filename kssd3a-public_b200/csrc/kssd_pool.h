@@ -91,7 +91,8 @@ public:
             Memory::release(p);
     }
 
-    // One index less: blocks of the current context that two of them in a row did not use go back.
+    // One index or sketch less: blocks of the current context that kAges of them in a row did
+    // not use go back.
     void age()
     {
         const uint64_t id = Memory::context();
@@ -102,9 +103,23 @@ public:
         } catch (const std::bad_alloc &) {
             return;
         }
-        if (now > 2)
-            release(id, now - 2);
+        if (now > kAges)
+            release(id, now - kAges);
     }
+
+    // Gives back all idle blocks of the current context.
+    void trim() { release(Memory::context(), ~0ull); }
+
+    // Their bytes.
+    uint64_t idle_bytes()
+    {
+        const uint64_t id = Memory::context();
+        std::lock_guard<std::mutex> lock(mu_);
+        const auto it = context_.find(id);
+        return it == context_.end() ? 0 : it->second.idle;
+    }
+
+    static constexpr uint64_t kAges = 8;
 
 private:
     struct Live {

@@ -149,22 +149,22 @@ int server_slot_alloc(kssdgpu_server *s, ServerSlot &sl)
     const auto &c = s->cfg;
     const size_t cells = (size_t)c.max_batch_queries * s->ix->nref;
     const bool uq = (c.flags & KSSDGPU_UNIQUE) != 0;
-    CUDA_TRY(cudaMalloc(&sl.d_keys, std::max<uint64_t>(c.max_batch_keys, 1) * 8));
-    CUDA_TRY(cudaMalloc(&sl.d_offs, ((size_t)c.max_batch_queries + 1) * 8));
-    CUDA_TRY(cudaMalloc(&sl.d_items, server_item_cap(c) * sizeof(WorkItem)));
-    CUDA_TRY(cudaMalloc(&sl.d_rc, cells * 8));
-    CUDA_TRY(cudaMalloc(&sl.d_ro, cells * 8));
+    CUDA_TRY(exact_malloc(&sl.d_keys, std::max<uint64_t>(c.max_batch_keys, 1) * 8));
+    CUDA_TRY(exact_malloc(&sl.d_offs, ((size_t)c.max_batch_queries + 1) * 8));
+    CUDA_TRY(exact_malloc(&sl.d_items, server_item_cap(c) * sizeof(WorkItem)));
+    CUDA_TRY(exact_malloc(&sl.d_rc, cells * 8));
+    CUDA_TRY(exact_malloc(&sl.d_ro, cells * 8));
     CUDA_TRY(cudaMemset(sl.d_rc, 0, cells * 8));
     CUDA_TRY(cudaMemset(sl.d_ro, 0, cells * 8));
     if (uq) {
-        CUDA_TRY(cudaMalloc(&sl.d_urc, cells * 8));
-        CUDA_TRY(cudaMalloc(&sl.d_uro, cells * 8));
+        CUDA_TRY(exact_malloc(&sl.d_urc, cells * 8));
+        CUDA_TRY(exact_malloc(&sl.d_uro, cells * 8));
         CUDA_TRY(cudaMemset(sl.d_urc, 0, cells * 8));
         CUDA_TRY(cudaMemset(sl.d_uro, 0, cells * 8));
     }
-    CUDA_TRY(cudaMalloc(&sl.d_hits, (size_t)s->hit_cap * sizeof(kssdgpu_hit_t)));
-    CUDA_TRY(cudaMalloc(&sl.d_count, sizeof(unsigned int)));
-    CUDA_TRY(cudaMalloc(&sl.d_work, sizeof(unsigned int)));
+    CUDA_TRY(exact_malloc(&sl.d_hits, (size_t)s->hit_cap * sizeof(kssdgpu_hit_t)));
+    CUDA_TRY(exact_malloc(&sl.d_count, sizeof(unsigned int)));
+    CUDA_TRY(exact_malloc(&sl.d_work, sizeof(unsigned int)));
     CUDA_TRY(cudaMallocHost(&sl.h_keys, std::max<uint64_t>(c.max_batch_keys, 1) * 8));
     CUDA_TRY(cudaMallocHost(&sl.h_offs, ((size_t)c.max_batch_queries + 1) * 8));
     CUDA_TRY(cudaMallocHost(&sl.h_items, server_item_cap(c) * sizeof(WorkItem)));
@@ -416,9 +416,8 @@ int kssdgpu_server_create(kssdgpu_index_t *ix, const kssdgpu_server_config_t *cf
     const uint64_t per_slot = server_slot_bytes(*cfg, ix->nref, hit_cap);
     uint64_t budget = cfg->device_budget;
     if (!budget) {
-        size_t free_b = 0, total_b = 0;
-        CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-        budget = free_b / 2;
+        CUDA_TRY(free_memory(budget));
+        budget /= 2;
     }
     const uint64_t fit = budget / std::max<uint64_t>(per_slot, 1);
     const int want = cfg->slots ? cfg->slots : 4;

@@ -2555,12 +2555,6 @@ struct DevBuf {
             cap = std::max<size_t>(n, 1);
         return e;
     }
-    void release()
-    {
-        pool_free(p);
-        p = nullptr;
-        cap = 0;
-    }
     void release_idle()  // the device's work on it has ended
     {
         pool_free_idle(p);
@@ -3341,8 +3335,8 @@ bool dense_fits(uint64_t need, uint64_t have)
 {
     if (need <= have)
         return true;
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    uint64_t free_b = 0;
+    if (free_memory(free_b) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -4299,8 +4293,8 @@ cudaError_t tune_join(kssdgpu_index *ix, uint32_t n, cudaStream_t st)
     int l2 = 0;
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ix->device);
     const size_t flush_b = std::max<size_t>(2 * (size_t)std::max(l2, 0), 64u << 20);
-    size_t free_b = 0, total_b = 0;
-    cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+    uint64_t free_b = 0;
+    cudaError_t e = free_memory(free_b);
     if (e != cudaSuccess || cells * 16 + flush_b > free_b / 4)
         return set_major_plan(ix, n, st);
     unsigned long long *oc = nullptr, *oo = nullptr;
@@ -4726,8 +4720,8 @@ int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long lon
     const int grid = ix->sms * std::max(1, per_sm_rows);
     ix->d_alleles = alleles;
     const uint64_t kpad = round_up(std::max<uint32_t>(alleles, 1), 128);
-    size_t free_b = 0, total_b = 0;
-    CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
+    uint64_t free_b = 0;
+    CUDA_TRY(free_memory(free_b));
     if (dense_bytes(ix, kpad) > free_b / 2)
         return fail(KSSDGPU_ERR_NOMEM, "dense self join: operands of " + std::to_string(dense_bytes(ix, kpad)) +
                                            " bytes exceed half of the free device memory");
@@ -5155,6 +5149,7 @@ static int sketch_impl(const CopyIn &copy_in, bool have_seq, uint64_t seq_len, c
             for (void *p : {(void *)seq, (void *)rec, (void *)samp, (void *)s0, (void *)s1, (void *)kept,
                             (void *)k0, (void *)k1, (void *)count, (void *)keep, tmp, (void *)nsel})
                 pool_free_idle(p);
+            device_pool().age();
         }
     } b;
     CUDA_TRY(pool_malloc(&b.seq, seq_len));
@@ -5398,6 +5393,67 @@ int kssdgpu_index_from_sketch(const uint64_t *keys, const uint64_t *offs, int nr
     return KSSDGPU_OK;
 }
 
+// Everything that an index's calls allocated, after a synchronization.
+static void release_scratch(kssdgpu_index *ix)
+{
+    ix->s_keys.release_idle();
+    ix->s_offs.release_idle();
+    ix->s_out.release_idle();
+    ix->s_order.release_idle();
+    ix->s_items.release_idle();
+    ix->s_prefix.release_idle();
+    ix->s_spos.release_idle();
+    ix->s_scnt.release_idle();
+    ix->s_spre.release_idle();
+    ix->s_sitems.release_idle();
+    ix->s_counts.release_idle();
+    ix->s_cubtmp.release_idle();
+    ix->m_val.release_idle();
+    ix->m_recheck.release_idle();
+    ix->m_nrecheck.release_idle();
+    ix->s_qcnt.release_idle();
+    ix->s_rcnt.release_idle();
+    ix->s_dcount.release_idle();
+    ix->s_dprefix.release_idle();
+    ix->s_hits.release_idle();
+    ix->d_list.release_idle();
+    ix->d_poff.release_idle();
+    ix->d_allele.release_idle();
+    ix->d_aval.release_idle();
+    ix->d_a.release_idle();
+    ix->d_f.release_idle();
+    ix->d_d.release_idle();
+    ix->d_tmp.release_idle();
+    ix->d_ws.release_idle();
+    ix->w_list.release_idle();
+    ix->w_corr.release_idle();
+    ix->w_count.release_idle();
+    ix->w_x.release_idle();
+    ix->w_y.release_idle();
+    ix->w_qobj.release_idle();
+    ix->w_at.release_idle();
+    ix->w_g.release_idle();
+}
+
+int kssdgpu_index_trim(kssdgpu_index_t *ix)
+{
+    if (!ix)
+        return fail(KSSDGPU_ERR_ARG, "null index");
+    CUDA_TRY(cudaSetDevice(ix->device));
+    CUDA_TRY(cudaDeviceSynchronize());
+    release_scratch(ix);
+    return KSSDGPU_OK;
+}
+
+int kssdgpu_trim(int device)
+{
+    CUDA_TRY(cudaSetDevice(device));
+    CUDA_TRY(cudaFree(nullptr));
+    device_pool().trim();
+    stager().trim();
+    return KSSDGPU_OK;
+}
+
 void kssdgpu_index_free(kssdgpu_index_t *ix)
 {
     if (!ix)
@@ -5422,28 +5478,8 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     pool_free_idle(ix->sh_number);
     pool_free_idle(ix->sh_table);
     pool_free_idle(ix->work);
-    ix->s_keys.release_idle();
-    ix->s_offs.release_idle();
-    ix->s_out.release_idle();
-    ix->s_order.release_idle();
-    ix->s_items.release_idle();
-    ix->s_prefix.release_idle();
-    ix->s_spos.release_idle();
-    ix->s_scnt.release_idle();
-    ix->s_spre.release_idle();
-    ix->s_sitems.release_idle();
-    for (int i = 0; i < 3; ++i)
-        if (ix->pipe_st[i])
-            cudaStreamDestroy(ix->pipe_st[i]);
-    for (cudaEvent_t e : ix->pipe_ev)
-        cudaEventDestroy(e);
-    ix->pipe_ev.clear();
-    ix->s_counts.release_idle();
-    ix->s_cubtmp.release_idle();
+    release_scratch(ix);
     ix->j_small.release_idle();
-    ix->m_val.release_idle();
-    ix->m_recheck.release_idle();
-    ix->m_nrecheck.release_idle();
     ix->j_post.release_idle();
     ix->j_chunks.release_idle();
     ix->j_items.release_idle();
@@ -5451,36 +5487,20 @@ void kssdgpu_index_free(kssdgpu_index_t *ix)
     ix->j_islot.release_idle();
     ix->j_touched.release_idle();
     ix->j_cacc.release_idle();
+    ix->j_fheads.release_idle();
+    ix->j_big.release_idle();
+    ix->j_conf.release_idle();
+    for (int i = 0; i < 3; ++i)
+        if (ix->pipe_st[i])
+            cudaStreamDestroy(ix->pipe_st[i]);
+    for (cudaEvent_t e : ix->pipe_ev)
+        cudaEventDestroy(e);
+    ix->pipe_ev.clear();
     if (ix->j_fill_st)
         cudaStreamDestroy(ix->j_fill_st);
     for (cudaEvent_t e : ix->j_fill_ev)
         if (e)
             cudaEventDestroy(e);
-    ix->j_fheads.release_idle();
-    ix->j_big.release_idle();
-    ix->j_conf.release_idle();
-    ix->s_qcnt.release_idle();
-    ix->s_rcnt.release_idle();
-    ix->s_dcount.release_idle();
-    ix->s_dprefix.release_idle();
-    ix->s_hits.release_idle();
-    ix->d_list.release_idle();
-    ix->d_poff.release_idle();
-    ix->d_allele.release_idle();
-    ix->d_aval.release_idle();
-    ix->d_a.release_idle();
-    ix->d_f.release_idle();
-    ix->d_d.release_idle();
-    ix->d_tmp.release_idle();
-    ix->d_ws.release_idle();
-    ix->w_list.release_idle();
-    ix->w_corr.release_idle();
-    ix->w_count.release_idle();
-    ix->w_x.release_idle();
-    ix->w_y.release_idle();
-    ix->w_qobj.release_idle();
-    ix->w_at.release_idle();
-    ix->w_g.release_idle();
     device_pool().age();
     delete ix;
 }

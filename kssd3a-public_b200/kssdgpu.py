@@ -88,6 +88,8 @@ def gpu_lib() -> C.CDLL:
         lib.kssdgpu_count_plain_dev.argtypes = [vp, vp, vp, _u64p, C.c_int, C.c_int, C.c_int, C.c_uint,
                                                 vp, vp, vp, vp, vp]
         lib.kssdgpu_init.argtypes = [C.c_int]
+        lib.kssdgpu_trim.argtypes = [C.c_int]
+        lib.kssdgpu_index_trim.argtypes = [vp]
         lib.kssdgpu_server_create.argtypes = [vp, C.POINTER(_ServerConfig), C.POINTER(vp)]
         lib.kssdgpu_server_submit.argtypes = [vp, vp, C.c_uint64, C.POINTER(C.c_uint64)]
         lib.kssdgpu_server_wait.argtypes = [vp, C.c_uint64, C.c_int, C.POINTER(C.c_uint32), C.POINTER(C.c_double)]
@@ -246,6 +248,11 @@ def bind_synth(lib: C.CDLL) -> C.CDLL:
 def _check(rc: int):
     if rc != 0:
         raise KssdGpuError(rc, gpu_lib().kssdgpu_last_error().decode(errors="replace"))
+
+
+def trim(device: int = 0):
+    """Gives back the memory that the library keeps for later calls on the device."""
+    _check(gpu_lib().kssdgpu_trim(device))
 
 
 def launch_count() -> int:
@@ -422,6 +429,10 @@ class Index:
             self.close()
         except Exception:
             pass
+
+    def trim(self):
+        """Releases the scratch that this index's calls have grown (the next calls make it again)."""
+        _check(gpu_lib().kssdgpu_index_trim(self._h))
 
     @property
     def handle(self):

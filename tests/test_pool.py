@@ -82,15 +82,23 @@ int main()
     pool.put(b);
     pool.put(c);
     CHECK(Fake::frees == 1);
-    // unused for more than two ages: given back; of other contexts nothing
-    for (int i = 0; i < 4; ++i)
+    // unused for more than kAges ages: given back; of other contexts nothing
+    CHECK(pool.idle_bytes() >= 60000);
+    for (uint64_t i = 0; i <= pool.kAges; ++i) {
+        CHECK(Fake::frees == 1);
         pool.age();
-    CHECK(Fake::frees == 2 && Fake::held.empty());
+    }
+    CHECK(Fake::frees == 2 && Fake::held.empty() && pool.idle_bytes() == 0);
+    // at once
+    CHECK(pool.get(&c, 30000) == 0);
+    pool.put(c);
+    pool.trim();
+    CHECK(Fake::frees == 3 && Fake::held.empty() && pool.idle_bytes() == 0);
     // memory short: the idle blocks go first
     CHECK(pool.get(&a, 40000) == 0);
     pool.put(a);
     Fake::room = 50000;
-    CHECK(pool.get(&b, 45000) == 0 && Fake::frees == 3);
+    CHECK(pool.get(&b, 45000) == 0 && Fake::frees == 4);
     CHECK(pool.get(&c, 20000) == Fake::kNoMemory);
     // no context: plain allocations
     pool.put(b);
