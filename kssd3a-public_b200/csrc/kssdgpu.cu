@@ -2926,9 +2926,9 @@ struct kssdgpu_index {
     uint32_t wide_min = 2;
     unsigned long long f_wgroups = 0, f_wpostings = 0, f_wpairs = 0, f_wcorr = 0;
     unsigned long long f_spairs = 0;        // pairs of the groups of at most kSharedSmall genomes
-    // shared groups of a conflict-free index (kssd_shared.cuh): the list, the blocks of its
-    // small groups (narrow ones: sh_small[0] blocks, all: sh_small[1]), the first large
-    // narrow and the first large wide group
+    // shared groups of a conflict-free index (kssd_shared.cuh; null where memory was short): the
+    // list, the blocks of its small groups (narrow ones: sh_small[0] blocks, all: sh_small[1]),
+    // the first large narrow and the first large wide group
     SharedGroup *sh_list = nullptr;
     SharedBlock *sh_blocks = nullptr;
     uint32_t *sh_place = nullptr, *sh_object = nullptr, *sh_table = nullptr;
@@ -2994,12 +2994,13 @@ int build_filter(kssdgpu_index *ix, uint64_t stripe_bytes, cudaStream_t st)
 }
 
 // The index's list of shared groups and its blocks (kssd_shared.cuh); small: the small
-// groups, their postings and pairs.  Ends with the stream synchronized.
+// groups, their postings and pairs.  Ends with the stream synchronized.  An index whose list
+// does not fit in memory goes without one: its self join reads all groups' bounds.
 int build_shared(kssdgpu_index *ix, const unsigned long long small[3], cudaStream_t st)
 {
     const uint64_t n = ix->f_groups;
     if (n >= 0x7FFFFFFFull || small[1] >= 0xFFFFFFFFull || (small[2] >> kBlockLog) >= 0x7FFFFFFFull)
-        return fail(KSSDGPU_ERR_CAPACITY, "too many shared contexts");
+        return KSSDGPU_OK;
     int gid_bits = 1;
     while ((1 << gid_bits) < ix->nref)
         ++gid_bits;
@@ -3035,25 +3036,39 @@ int build_shared(kssdgpu_index *ix, const unsigned long long small[3], cudaStrea
         }
     } t;
     t.st = st;
-    CUDA_TRY(pool_malloc(&t.key, n * 4));
-    CUDA_TRY(pool_malloc(&t.key2, n * 4));
-    CUDA_TRY(pool_malloc(&t.mark, (blocks + 2) * 4));
-    CUDA_TRY(pool_malloc(&t.val, n * 8));
-    CUDA_TRY(pool_malloc(&t.val2, n * 8));
-    CUDA_TRY(pool_malloc(&t.sums, n * sizeof(SharedSums)));
-    CUDA_TRY(pool_malloc(&t.count, sizeof(unsigned int)));
-    CUDA_TRY(pool_malloc(&ix->sh_list, n * sizeof(SharedGroup)));
-    CUDA_TRY(pool_malloc(&ix->sh_blocks, blocks * sizeof(SharedBlock)));
-    CUDA_TRY(pool_malloc(&ix->sh_place, n * 4));
-    CUDA_TRY(pool_malloc(&ix->sh_object, std::max<uint64_t>(small[1], 1) * 4));
-    CUDA_TRY(pool_malloc(&ix->sh_number, std::max<uint64_t>(small[1], 1)));  // slots while it is built, too
-    CUDA_TRY(pool_malloc(&ix->sh_table, blocks * kBlockGenomes * 4));
-    const auto sizes = thrust::make_transform_iterator(t.val2, SharedSize{});
+    const auto no_sizes = thrust::make_transform_iterator((const unsigned long long *)nullptr, SharedSize{});
     size_t tb0 = 0, tb1 = 0;
     CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb0, t.key, t.key2, t.val, t.val2, (int64_t)n, 0, gid_bits + 2,
                                              st));
-    CUDA_TRY(cub::DeviceScan::ExclusiveScan(nullptr, tb1, sizes, t.sums, SharedAdd{}, SharedSums{0, 0}, (int64_t)n, st));
-    CUDA_TRY(pool_malloc(&t.tmp, std::max(tb0, tb1)));
+    CUDA_TRY(cub::DeviceScan::ExclusiveScan(nullptr, tb1, no_sizes, t.sums, SharedAdd{}, SharedSums{0, 0}, (int64_t)n, st));
+    const uint64_t np = std::max<uint64_t>(small[1], 1);
+    cudaError_t e = pool_malloc(&t.key, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&t.key2, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&t.mark, (blocks + 2) * 4);
+    if (e == cudaSuccess) e = pool_malloc(&t.val, n * 8);
+    if (e == cudaSuccess) e = pool_malloc(&t.val2, n * 8);
+    if (e == cudaSuccess) e = pool_malloc(&t.sums, n * sizeof(SharedSums));
+    if (e == cudaSuccess) e = pool_malloc(&t.count, sizeof(unsigned int));
+    if (e == cudaSuccess) e = pool_malloc(&t.tmp, std::max(tb0, tb1));
+    if (e == cudaSuccess) e = pool_malloc(&ix->sh_list, n * sizeof(SharedGroup));
+    if (e == cudaSuccess) e = pool_malloc(&ix->sh_blocks, blocks * sizeof(SharedBlock));
+    if (e == cudaSuccess) e = pool_malloc(&ix->sh_place, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(&ix->sh_object, np * 4);
+    if (e == cudaSuccess) e = pool_malloc(&ix->sh_number, np);  // slots while it is built, too
+    if (e == cudaSuccess) e = pool_malloc(&ix->sh_table, blocks * kBlockGenomes * 4);
+    if (e != cudaSuccess) {
+        for (void *p : {(void *)ix->sh_list, (void *)ix->sh_blocks, (void *)ix->sh_place, (void *)ix->sh_object,
+                        (void *)ix->sh_number, (void *)ix->sh_table})
+            pool_free_idle(p);  // nothing has run on them
+        ix->sh_list = nullptr;
+        ix->sh_blocks = nullptr;
+        ix->sh_place = ix->sh_object = ix->sh_table = nullptr;
+        ix->sh_number = nullptr;
+        if (e == cudaErrorMemoryAllocation)
+            return KSSDGPU_OK;
+        return fail(KSSDGPU_ERR_CUDA, std::string("list of shared contexts: ") + cudaGetErrorString(e));
+    }
+    const auto sizes = thrust::make_transform_iterator((const unsigned long long *)t.val2, SharedSize{});
     CUDA_TRY(cudaMemsetAsync(t.count, 0, sizeof(unsigned int), st));
     CUDA_TRY(cudaMemsetAsync(ix->sh_blocks, 0, blocks * sizeof(SharedBlock), st));
     k_shared_collect<<<(unsigned)std::min<uint64_t>((ix->u + kScanTile - 1) / kScanTile, (uint64_t)ix->sms * 8),
@@ -4483,9 +4498,10 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
     const bool pack = ix->obj_bits <= kPackBits;
     const auto pairs_kernel = pack ? k_self_pairs<true> : k_self_pairs<false>;
     const size_t pairs_smem = pack ? offsetof(PairSmem, number) : sizeof(PairSmem);
+    const bool listed = ix->sh_list != nullptr;  // not with conflicts
     if (!ix->scan_grid) {
         int per_sm = 0;
-        if (ix->f_conflict) {
+        if (!listed) {
             CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_self_scan, kScanThreads, 0));
         } else {
             CUDA_TRY(allow_smem(pairs_kernel, pairs_smem));  // one size a kernel
@@ -4493,7 +4509,7 @@ int self_scan_impl(kssdgpu_index *ix, unsigned flags, unsigned long long *oc, un
         }
         ix->scan_grid = std::max(1, per_sm) * ix->sms;
     }
-    if (ix->f_conflict) {
+    if (!listed) {
         const uint64_t ntiles = (ix->u + kScanTile - 1) / kScanTile;
         cfg.gridDim = dim3((unsigned)std::min<uint64_t>(ntiles, (uint64_t)ix->scan_grid));
         cfg.blockDim = dim3(kScanThreads);
@@ -4704,7 +4720,7 @@ int self_dense_impl(kssdgpu_index *ix, unsigned long long *oc, unsigned long lon
         CUDA_TRY(cudaMemsetAsync(oo, 0, cells * 8, st));
         return KSSDGPU_OK;
     }
-    if (wide_ms(ix) <= allele_ms(ix))
+    if (ix->sh_list && wide_ms(ix) <= allele_ms(ix))
         return self_wide_impl(ix, oc, oo, st);
     ix->w_ran = false;
     const uint32_t npad = (uint32_t)dense_npad(ix);
@@ -4788,7 +4804,7 @@ bool dense_chosen(const kssdgpu_index *ix)
 {
     if (ix->f_conflict || ix->f_pairs == 0 || ix->nref < 2 || (uint32_t)ix->nref > kDenseMaxGroup)
         return false;
-    const double wide = wide_ms(ix), allele = allele_ms(ix);
+    const double allele = allele_ms(ix), wide = ix->sh_list ? wide_ms(ix) : 2 * allele;  // it needs the list
     if (std::min(wide, allele) >= scan_ms(ix))
         return false;
     if (wide <= allele)
