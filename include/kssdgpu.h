@@ -192,6 +192,9 @@ int kssdgpu_sync(kssdgpu_index_t *idx, void *stream);
  * rules out needs no table probe; with several stripes and global rows the count runs
  * stripe by stripe, see kssdgpu_index_filter); the fastest becomes the index's
  * setting for later batched counts without KSSDGPU_SMEM_ACC / KSSDGPU_GLOBAL_ACC.
+ * The global rows are timed as later calls run: where a block leaves the contexts that many
+ * references share to the tensor cores, so do they, and a later block that does takes no shared
+ * rows whatever the setting.
  * Synchronizes the device; the outputs hold the block's counters afterwards.  Without
  * a call: global rows (in 4,096-entry chunks, or stripe by stripe), filter on.  No
  * reference counterpart (the CPU path has no tunables).

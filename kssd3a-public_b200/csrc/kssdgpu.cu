@@ -3515,7 +3515,9 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
     if ((flags & KSSDGPU_SMEM_ACC) && !plain && !(flags & KSSDGPU_GLOBAL_ACC) && !smem_row_fits(ix, flags))
         return fail(KSSDGPU_ERR_CAPACITY, "shared-memory accumulator rows requested, but a row of " +
                                               std::to_string(ix->nref) + " references does not fit");
-    const bool use_smem = uses_smem_row(ix, flags);
+    // the tensor cores before the tuned rows: those were timed against walks of every posting
+    const bool wide = !lower && wide_block_chosen(ix, nq, flags) && !capturing(st);
+    const bool use_smem = !wide && uses_smem_row(ix, flags);
     P.chunk_keys = ix->count_chunk_keys;
     // stripe-major items when the filter is on and striped (global rows)
     const bool striped = !use_smem && !plain && !d_items && P.bloom && ix->count_striped && ix->bloom_stripes > 1 &&
@@ -3567,7 +3569,6 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
             CUDA_TRY(cudaMemsetAsync(uo, 0, cells * 8, st));
         }
     }
-    const bool wide = !lower && !use_smem && wide_block_chosen(ix, nq, flags) && !capturing(st);
     if (wide) {
         const int rc = wide_block_begin(ix, nq, P, st);
         if (rc)
@@ -5685,7 +5686,8 @@ int kssdgpu_count_tune(kssdgpu_index_t *ix, const uint64_t *d_qry_keys, const ui
         ix->count_chunk_keys = c.chunk;
         ix->count_striped = c.striped;
         ix->count_filter = filter;
-        const unsigned f = base | (c.smem ? KSSDGPU_SMEM_ACC : KSSDGPU_GLOBAL_ACC);
+        // as later calls run: global rows by the setting, so that wide groups go the way they go then
+        const unsigned f = base | (c.smem ? KSSDGPU_SMEM_ACC : 0u);
         t_min = 1e30f;
         for (int r = 0; r < 4 && rc == KSSDGPU_OK; ++r) {
             ce = cudaEventRecord(ev0, 0);
