@@ -10,10 +10,9 @@
 // times that on a host whose other processes allocate too), which was most of a small
 // index's build: 64 genomes 6.2 ms, of which kernels 0.3.  Freed blocks are kept instead
 // and handed out again for requests they fit (kssd_pool.h).  Kept: at most kPoolKeep bytes a
-// device; blocks that eight indexes or sketches in a row left unused are given back, all of them
-// when an allocation fails and by kssdgpu_trim, and the rest of the library counts them as free
-// memory.  (cudaMallocAsync's pool was measured too: 6 ms per 500 MB that its reservation grows
-// by.)
+// device; blocks that two indexes in a row left unused are given back, all of them when an
+// allocation fails and by kssdgpu_trim, and the rest of the library counts them as free memory.
+// (cudaMallocAsync's pool was measured too: 6 ms per 500 MB that its reservation grows by.)
 constexpr uint64_t kPoolKeep = 2ull << 30;
 
 // Id of the calling thread's context, 0 where there is none.

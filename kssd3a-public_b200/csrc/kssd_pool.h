@@ -91,8 +91,9 @@ public:
             Memory::release(p);
     }
 
-    // One index or sketch less: blocks of the current context that kAges of them in a row did
-    // not use go back.
+    // One index less: blocks of the current context that kAges of them in a row did not use go
+    // back (kept for longer, they take the place of blocks that are of use: 2 GiB hold the arrays
+    // of one or two indexes).
     void age()
     {
         const uint64_t id = Memory::context();
@@ -119,7 +120,7 @@ public:
         return it == context_.end() ? 0 : it->second.idle;
     }
 
-    static constexpr uint64_t kAges = 8;
+    static constexpr uint64_t kAges = 2;
 
 private:
     struct Live {

@@ -5175,7 +5175,6 @@ static int sketch_impl(const CopyIn &copy_in, bool have_seq, uint64_t seq_len, c
             for (void *p : {(void *)seq, (void *)rec, (void *)samp, (void *)s0, (void *)s1, (void *)kept,
                             (void *)k0, (void *)k1, (void *)count, (void *)keep, tmp, (void *)nsel})
                 pool_free_idle(p);
-            device_pool().age();
         }
     } b;
     CUDA_TRY(pool_malloc(&b.seq, seq_len));
