@@ -361,6 +361,7 @@ struct SmemAcc {
 // A query's global counter row.
 struct GlobalAcc {
     unsigned long long *c, *o;
+    __device__ __forceinline__ void add_spread(uint32_t gid, int d) const { add(gid, d); }
     __device__ __forceinline__ void add(uint32_t gid, int d) const
     {
         atomicAdd(c + gid, inc_ctx(d));
@@ -433,8 +434,6 @@ struct WarpAcc {
         __syncwarp();
     }
 };
-__device__ __forceinline__ void flush_acc(const SmemAcc &, uint32_t) {}
-__device__ __forceinline__ void flush_acc(const WarpAcc &a, uint32_t lane) { a.flush(lane); }
 
 // min over the query run's objects x one reference object
 __device__ __forceinline__ int min_diff_obj(uint32_t robj, uint32_t q0, int s, const uint64_t *__restrict__ qrun,
@@ -888,9 +887,9 @@ __device__ __forceinline__ void probe_batch(const CountParams &P, ProbeQueue &Q,
 // context run works (src/command_ani.h:498-505); the filter rules out most absent contexts
 // (88 % of the entries of new assemblies); the others wait in the warp's queue until 32 of
 // them probe the table together, so that no lane idles in the probe and the walk.
-template <bool UNIQUE, bool WIDE, class Acc>
+template <bool UNIQUE, bool WIDE>
 __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, uint64_t e, uint64_t cb, uint64_t ce,
-                                              int qgid, uint64_t objmask, const Acc &acc, const Acc &uacc,
+                                              int qgid, uint64_t objmask, const WarpAcc &acc, const WarpAcc &uacc,
                                               const FilterView &fv, uint64_t t0, uint64_t T, ProbeQueue &Q)
 {
     const uint32_t lane = (uint32_t)(t0 & 31u);
@@ -943,42 +942,37 @@ __device__ __forceinline__ void process_query(const CountParams &P, uint64_t b, 
         __syncwarp();
         seen += 32 * kProbeLoads;
         if (seen + 32 * kProbeLoads > kWarpCellEntries - 32) {  // those waiting were seen before
-            flush_acc(acc, lane);
+            acc.flush(lane);
             if (UNIQUE)
-                flush_acc(uacc, lane);
+                uacc.flush(lane);
             seen = 0;
         }
     }
     if (waiting)
         probe_batch<UNIQUE, WIDE>(P, Q, 0, waiting, cb, e, qgid, objmask, acc, uacc, lane);
-    flush_acc(acc, lane);
+    acc.flush(lane);
     if (UNIQUE)
-        flush_acc(uacc, lane);
+        uacc.flush(lane);
 }
 
 // The same entries, an entry a lane and round (LANES), for shared-memory rows, lower blocks
-// and long walks (walks_long).  A
+// and long walks (walks_long), credited to the row at once.  A
 // lower block is a part of an index's own genomes: every key is found and most credit
 // nothing (a context's only owner is the query itself), so a full warp in the probe is worth
 // less than the warps in flight that the queue's registers and shared memory cost; so are
 // the cheap credits of a row in shared memory.  Measured (B200, 2,000 genomes against
 // themselves, lower, queue -> this): global rows stripe by stripe 1,383 -> 1,201 us, in
 // chunks without the filter 1,264 -> 1,079, shared rows 1,869 -> 1,410; 500 of them as an
-// ordinary block, global rows: 464 -> 402 the other way.
+// ordinary block, global rows: 464 -> 402 the other way.  Counters of the warp's own do not pay
+// here (conflicts, 500 queries x 1,000 references in species of 24, unique contexts: 202 us,
+// 192 without them at as many warps).
 template <bool LOWER, bool UNIQUE, class Acc>
 __device__ __forceinline__ void process_query_row(const CountParams &P, uint64_t b, uint64_t e, uint64_t cb,
                                                   uint64_t ce, int qgid, uint64_t objmask, const Acc &acc,
                                                   const Acc &uacc, const FilterView &fv, uint64_t t0, uint64_t T)
 {
     const uint32_t lane = (uint32_t)(t0 & 31u);
-    uint32_t seen = 0;
     for (uint64_t wb = cb + (t0 - lane); wb < ce; wb += T) {
-        if ((seen += 32) > kWarpCellEntries) {
-            flush_acc(acc, lane);
-            if (UNIQUE)
-                flush_acc(uacc, lane);
-            seen = 32;
-        }
         const uint64_t i = wb + lane;
         int s = 0;
         unsigned long long payload = 0;
@@ -1017,9 +1011,6 @@ __device__ __forceinline__ void process_query_row(const CountParams &P, uint64_t
                                              acc, uacc, lane);
         }
     }
-    flush_acc(acc, lane);
-    if (UNIQUE)
-        flush_acc(uacc, lane);
 }
 
 // Entries of a chunk of the chunk-major kernel: at most `most`, fewer when a block of
@@ -1044,15 +1035,17 @@ constexpr int kRowThreads = 512;  // of a CTA with a shared-memory row, four a S
 // that one large query (a read set) spreads over many SMs.
 // Five CTAs a SM in the global rows, for all that some registers spill: 500 of 1,000
 // genomes in species of 24 637 -> 571 us, 500 of 2,000 without the filter 379 -> 347 (six:
-// 563 and 327, but 2 to 4 % more where species are long).
+// 563 and 327, but 2 to 4 % more where species are long).  An entry a lane: eight, at 32
+// registers; the block above with conflicts 192 (six) -> 176 us (230 with four), 20 read sets
+// against it 210 -> 190, 16 queries 48 -> 53.
 template <bool LOWER, bool UNIQUE, bool SMEM, bool WIDE, bool LANES>
-__global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 : LANES ? 6 : 5) k_count_batched(CountParams P)
+__global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 : LANES ? 8 : 5) k_count_batched(CountParams P)
 {
     static_assert(!(WIDE && (SMEM || LANES)) && (LANES || !LOWER), "wide groups leave ordinary blocks in global rows only");
     extern __shared__ uint32_t sm[];
     constexpr bool kRow = SMEM || LANES;
     __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
-    __shared__ WarpCells cells[SMEM ? 1 : UNIQUE ? 2 : 1][SMEM ? 1 : kCountThreads / 32];
+    __shared__ WarpCells cells[!kRow && UNIQUE ? 2 : 1][kRow ? 1 : kCountThreads / 32];
     __shared__ int s_item;
     const uint64_t objmask = (P.obj_bits >= 64) ? ~0ull : ((1ull << P.obj_bits) - 1);
     const uint64_t base = P.qoffs[0];
@@ -1060,7 +1053,7 @@ __global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 :
     const FilterView fv{P.bloom, P.bloom_mask, P.bloom_stripes, P.bloom_bounds, keep_l2_policy()};
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t chunk_keys = P.chunk_auto ? count_chunk(P.qoffs[P.nq] - base, P.chunk_keys, P.chunk_auto) : P.chunk_keys;
-    if (!SMEM) {
+    if constexpr (!kRow) {
         WarpAcc{{}, &cells[0][warp]}.clear(lane);
         if (UNIQUE)
             WarpAcc{{}, &cells[UNIQUE][warp]}.clear(lane);
@@ -1105,9 +1098,8 @@ __global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 :
             const SmemAcc uacc{row1, row1 + nref, row1 + 2 * nref, row1 + 3 * nref};
             process_query_row<LOWER, UNIQUE>(P, b, e, b, e, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
         } else {
-            const WarpAcc acc{{P.out_ctx + row, P.out_obj + row}, &cells[0][warp]};
-            const WarpAcc uacc{{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr},
-                               &cells[UNIQUE && !SMEM][warp]};
+            const GlobalAcc acc{P.out_ctx + row, P.out_obj + row};
+            const GlobalAcc uacc{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr};
             uint64_t cb = b, ce = e;
             if (P.items) {
                 cb = P.items[it].b;
@@ -1119,8 +1111,9 @@ __global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 :
             if constexpr (kRow)
                 process_query_row<LOWER, UNIQUE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x, blockDim.x);
             else
-                process_query<UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, acc, uacc, fv, threadIdx.x,
-                                                   blockDim.x, queues[warp]);
+                process_query<UNIQUE, WIDE>(P, b, e, cb, ce, qgid, objmask, WarpAcc{acc, &cells[0][warp]},
+                                            WarpAcc{uacc, &cells[UNIQUE][warp]}, fv, threadIdx.x, blockDim.x,
+                                            queues[warp]);
         }
         __syncthreads();
         if (SMEM) {
@@ -1158,11 +1151,13 @@ __global__ void __launch_bounds__(kCountThreads, LANES ? 6 : 4) k_count_striped(
     constexpr bool kRow = LANES;
     static_assert(!(WIDE && LANES) && (LANES || !LOWER), "wide groups leave ordinary blocks only");
     __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
-    __shared__ WarpCells cells[UNIQUE ? 2 : 1][kCountThreads / 32];
+    __shared__ WarpCells cells[!kRow && UNIQUE ? 2 : 1][kRow ? 1 : kCountThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    WarpAcc{{}, &cells[0][warp]}.clear(lane);
-    if (UNIQUE)
-        WarpAcc{{}, &cells[UNIQUE][warp]}.clear(lane);
+    if constexpr (!kRow) {
+        WarpAcc{{}, &cells[0][warp]}.clear(lane);
+        if (UNIQUE)
+            WarpAcc{{}, &cells[UNIQUE][warp]}.clear(lane);
+    }
     const uint64_t objmask = (P.obj_bits >= 64) ? ~0ull : ((1ull << P.obj_bits) - 1);
     const uint64_t base = P.qoffs[0];
     const uint32_t nitems = *P.nitems_dev;
@@ -1179,15 +1174,14 @@ __global__ void __launch_bounds__(kCountThreads, LANES ? 6 : 4) k_count_striped(
         const int q = (int)w.q;
         const uint64_t b = P.qoffs[q] - base, e = P.qoffs[q + 1] - base;
         const size_t row = (size_t)q * P.nref;
-        const WarpAcc acc{{P.out_ctx + row, P.out_obj + row}, &cells[0][warp]};
-        const WarpAcc uacc{{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr},
-                           &cells[UNIQUE][warp]};
+        const GlobalAcc acc{P.out_ctx + row, P.out_obj + row};
+        const GlobalAcc uacc{UNIQUE ? P.out_uctx + row : nullptr, UNIQUE ? P.out_uobj + row : nullptr};
         const FilterView fv{P.bloom + stripe_words * w.pad, P.bloom_mask, 1, nullptr, policy};
         if constexpr (kRow)
             process_query_row<LOWER, UNIQUE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32);
         else
-            process_query<UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, acc, uacc, fv, lane, 32,
-                                               queues[warp]);
+            process_query<UNIQUE, WIDE>(P, b, e, w.b, w.e, P.qgid_offset + q, objmask, WarpAcc{acc, &cells[0][warp]},
+                                        WarpAcc{uacc, &cells[UNIQUE][warp]}, fv, lane, 32, queues[warp]);
     }
 }
 
