@@ -247,8 +247,7 @@ int server_launch(kssdgpu_server *s, ServerSlot &sl)
     P.bloom_stripes = s->ix->bloom_stripes;
     P.bloom_bounds = s->ix->bloom_bounds;
     P.conflict_free = !s->ix->f_conflict;
-    int rc = (s->cfg.flags & KSSDGPU_UNIQUE) ? launch_batched<false, true, false>(s->ix, P, 0, sl.st)
-                                             : launch_batched<false, false, false>(s->ix, P, 0, sl.st);
+    int rc = launch_rows(s->ix, P, (s->cfg.flags & KSSDGPU_UNIQUE) != 0, sl.st);
     if (rc)
         return rc;
     k_server_compact<<<std::min(nq, s->ix->sms * 8), 256, 0, sl.st>>>(sl.d_rc, sl.d_ro, sl.d_urc, sl.d_uro, nq,

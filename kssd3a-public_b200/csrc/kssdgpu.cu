@@ -3316,11 +3316,13 @@ bool uses_smem_row(const kssdgpu_index *ix, unsigned flags)
 
 // Ordinary blocks whose found contexts are mostly walked one by one, by their lane (runs of
 // several objects, conflicts) or by the warp (long groups that are not left to the tensor
-// cores), gain little from postings dealt out over the lanes and take an entry a lane, at 48
-// warps a SM.  Measured (B200, indexes with conflicts, queue -> this): 500 queries x 2,000
-// references 478 -> 395 us, 500 x 1,000 in species of 24 985 -> 860, 128 x 512 of one species
-// 4,450 -> 3,830; without conflicts the queue wins (one species apart): 500 x 2,000 464 (an
-// entry a lane) -> 402.
+// cores), gain little from postings dealt out over the lanes and take an entry a lane, at 48 to
+// 64 warps a SM, whoever counts them.  Measured (B200, indexes with conflicts, queue -> this, a
+// block / without allocation): 500 queries x 2,000 references 181 -> 174 / 162 -> 136 us, with
+// unique contexts 195 -> 192 / 183 -> 148; 500 x 1,000 in species of 24 203 -> 176 / 195 -> 169;
+// 128 x 512 of one species 2,756 -> 2,360 / 2,744 -> 2,341; the other way 20 read sets against
+// species of 24 182 -> 190 / 177 -> 183.  Without conflicts the queue wins (one species apart):
+// 500 x 2,000 464 (an entry a lane) -> 402.
 bool walks_long(const kssdgpu_index *ix)
 {
     return ix->f_conflict || (ix->f_groups && ix->f_postings >= (unsigned long long)kWarpWalk * ix->f_groups);
@@ -3328,6 +3330,16 @@ bool walks_long(const kssdgpu_index *ix)
 
 // Chunks that a block in global rows should give, whoever counts it.
 uint32_t chunk_goal(const kssdgpu_index *ix) { return (uint32_t)ix->sms * kSmChunks; }
+
+// An ordinary block in global rows, its wide groups walked like the others (every caller of the
+// chunk-major kernel: blocks, the no-allocation count, the server).
+int launch_rows(kssdgpu_index *ix, const CountParams &P, bool unique, cudaStream_t st)
+{
+    if (walks_long(ix))
+        return unique ? launch_batched<false, true, false, false, true>(ix, P, 0, st)
+                      : launch_batched<false, false, false, false, true>(ix, P, 0, st);
+    return unique ? launch_batched<false, true, false>(ix, P, 0, st) : launch_batched<false, false, false>(ix, P, 0, st);
+}
 
 // Key-range chunks of at most `chunk` entries for the global-row kernel, the queries
 // taken in the given order (offsets relative or absolute).
@@ -3594,18 +3606,14 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
     else if (wide)
         rc = unique ? launch_batched<false, true, false, true>(ix, P, 0, st)
                     : launch_batched<false, false, false, true>(ix, P, 0, st);
-    else if (!lower && walks_long(ix))
-        rc = striped ? (unique ? launch_striped<false, true, false, true>(ix, P, st)
-                               : launch_striped<false, false, false, true>(ix, P, st))
-                     : (unique ? launch_batched<false, true, false, false, true>(ix, P, 0, st)
-                               : launch_batched<false, false, false, false, true>(ix, P, 0, st));
+    else if (!lower && striped && walks_long(ix))
+        rc = unique ? launch_striped<false, true, false, true>(ix, P, st)
+                    : launch_striped<false, false, false, true>(ix, P, st);
     else if (striped)
         rc = lower ? launch_striped<true, false>(ix, P, st)
                    : unique ? launch_striped<false, true>(ix, P, st) : launch_striped<false, false>(ix, P, st);
     else
-        rc = lower ? launch_batched<true, false, false>(ix, P, 0, st)
-                   : unique ? launch_batched<false, true, false>(ix, P, 0, st)
-                            : launch_batched<false, false, false>(ix, P, 0, st);
+        rc = lower ? launch_batched<true, false, false>(ix, P, 0, st) : launch_rows(ix, P, unique, st);
     return rc || !wide ? rc : wide_block_end(ix, nq, P, oc, oo, st);
 }
 
@@ -5871,7 +5879,7 @@ int kssdgpu_count_block_noalloc(kssdgpu_index_t *ix, const uint64_t *d_qry_keys,
     }
     if (lower)
         return launch_batched<true, false, false>(ix, P, 0, st);
-    return unique ? launch_batched<false, true, false>(ix, P, 0, st) : launch_batched<false, false, false>(ix, P, 0, st);
+    return launch_rows(ix, P, unique, st);
 }
 
 int kssdgpu_count_detail(kssdgpu_index_t *ix, const uint64_t *qry_keys, const uint64_t *qry_offs, int nq,
