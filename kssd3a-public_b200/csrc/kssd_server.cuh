@@ -121,10 +121,16 @@ struct kssdgpu_server {
 
 namespace {
 
+// Chunks that a batch gives at least, where its entries suffice: eight a SM (chunks of 4,096
+// entries whatever the batch, which fills few SMs: one request to an index of 512 genomes of one
+// species 2,870 us, so 310; more chunks are more items to copy, and the kernel is not what other
+// requests wait for).
+constexpr uint32_t kServerChunks = 1184;
+
 // chunks of a full batch: every query may end in a partial chunk
 size_t server_item_cap(const kssdgpu_server_config_t &c)
 {
-    return (size_t)(c.max_batch_keys / kChunkKeys) + (size_t)c.max_batch_queries + 1;
+    return std::max<size_t>(c.max_batch_keys / kChunkKeys, kServerChunks) + (size_t)c.max_batch_queries + 1;
 }
 
 // Device bytes one slot reserves: keys, offsets, work items, dense counter rows
@@ -203,7 +209,10 @@ void server_slot_free(ServerSlot &sl)
 int server_launch(kssdgpu_server *s, ServerSlot &sl)
 {
     const int nq = (int)sl.batch.size();
-    uint64_t nk = 0;
+    uint64_t nk = 0, total = 0;
+    for (const auto &r : sl.batch)
+        total += r->keys.size();
+    const uint64_t chunk = count_chunk(total, (uint32_t)kChunkKeys, kServerChunks);
     size_t nitems = 0;
     sl.h_offs[0] = 0;
     for (int i = 0; i < nq; ++i) {
@@ -211,8 +220,8 @@ int server_launch(kssdgpu_server *s, ServerSlot &sl)
         if (!k.empty())
             std::memcpy(sl.h_keys + nk, k.data(), k.size() * 8);
         // key-range chunks: a large request spreads over many SMs
-        for (uint64_t c = nk; c < nk + k.size(); c += kChunkKeys)
-            sl.h_items[nitems++] = WorkItem{(uint32_t)i, 0u, c, std::min<uint64_t>(nk + k.size(), c + kChunkKeys)};
+        for (uint64_t c = nk; c < nk + k.size(); c += chunk)
+            sl.h_items[nitems++] = WorkItem{(uint32_t)i, 0u, c, std::min<uint64_t>(nk + k.size(), c + chunk)};
         nk += k.size();
         sl.h_offs[i + 1] = nk;
     }
