@@ -1131,12 +1131,25 @@ __global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 :
     }
 }
 
+// Chunks that a warp takes at a time.  With many stripes a query's part of one is little more
+// than a chunk (10,000 queries x 20,000 references, 32 stripes: 266 entries, a chunk of 256 and a
+// rest) and taking costs as much as counting, so chunks of one stripe and neighbouring queries go
+// together, up to `most`, where every warp is left at least eight takes.  Measured (B200, one /
+// two / three / four at a time, us): 10,000 x 20,000 2,812 / 2,160 / 1,976 / 1,975, 4,000 x 20,000
+// 1,114 / 921 / 931 / 949, 10,000 x 6,000 (8 stripes) 1,541 / 1,389 / 1,413 / 1,448, 10,000 x
+// 2,000 (2 stripes) 1,291 / 1,302 / 1,331 / 1,366; with fewer takes left 1,500 x 2,000 269 -> 291.
+// An entry a lane: 10,000 x 20,000 2,844 / 2,213 / - / 2,257; lower 20,000 12,390 / 12,750.
+__device__ __forceinline__ uint32_t stripe_take(uint32_t nitems, uint32_t parts, uint32_t warps, uint32_t most)
+{
+    const uint32_t want = nitems < 2 * parts ? 4 : nitems < 8 * (uint64_t)parts ? 2 : 1;
+    return max(1u, min(min(want, most), nitems / (warps * 8)));
+}
+
 // Stripe-major global-row kernel: the work items are chunks of one query's entries
 // whose contexts fall in one filter stripe, listed stripe by stripe (k_stripe_expand),
 // so that at any time the SMs probe one stripe of the filter and it stays in L2 while
-// the query keys stream past.  Each warp takes a chunk at a time from the work counter
-// (two at a time, or the next one asked for while one is counted: 281 and 269 instead of
-// 252 us for 1,500 queries x 2,000 references, the last chunks wait longer); its lanes
+// the query keys stream past.  Each warp takes one chunk or several (stripe_take) at a time
+// from the work counter; its lanes
 // stride over the chunk's entries.  Counters go to the zeroed global rows through the
 // warp's own cells, as in the chunked mode.
 //
@@ -1163,13 +1176,17 @@ __global__ void __launch_bounds__(kCountThreads, LANES ? 6 : 4) k_count_striped(
     const uint32_t nitems = *P.nitems_dev;
     const unsigned long long policy = keep_l2_policy();
     const size_t stripe_words = 2 * ((size_t)P.bloom_mask + 1);  // uint4 per stripe
-    for (;;) {
-        uint32_t it = 0;
-        if (lane == 0)
-            it = atomicAdd(P.work, 1u);
-        it = __shfl_sync(0xFFFFFFFFu, it, 0);
-        if (it >= nitems)
-            break;
+    const uint32_t take = stripe_take(nitems, (uint32_t)P.nq * (uint32_t)P.bloom_stripes,
+                                      gridDim.x * (kCountThreads / 32), LOWER ? 1 : LANES ? 2 : 4);
+    for (uint32_t it = 0, end = 0;; ++it) {
+        if (it == end) {
+            if (lane == 0)
+                it = atomicAdd(P.work, take);
+            it = __shfl_sync(0xFFFFFFFFu, it, 0);
+            if (it >= nitems)
+                break;
+            end = min(nitems, it + take);
+        }
         const WorkItem w = P.items[it];
         const int q = (int)w.q;
         const uint64_t b = P.qoffs[q] - base, e = P.qoffs[q + 1] - base;
