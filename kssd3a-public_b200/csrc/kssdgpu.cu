@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <numeric>
@@ -5297,15 +5298,17 @@ int kssdgpu_sketch_records(const char *const *recs, const uint64_t *rec_offs, ui
             ++r;
         }
     };
+    // short sequences, and all where the chunks are in use: joined here (a copy a record cost 2 us
+    // each, 10,000 records of 150 bases 21 ms, so 1.5)
     auto copy_in = [&](void *d, cudaStream_t st) {
         cudaError_t e = cudaSuccess;
         if (seq_len >= kStageMin && stager().run<true>((char *)d, seq_len, st, gather, e))
             return e;
-        for (uint64_t r = 0; r < nrec && e == cudaSuccess; ++r)
-            if (rec_offs[r + 1] > rec_offs[r])
-                e = cudaMemcpyAsync((char *)d + rec_offs[r], recs[r], rec_offs[r + 1] - rec_offs[r],
-                                    cudaMemcpyHostToDevice, st);
-        return e;
+        const std::unique_ptr<char[]> joined(new (std::nothrow) char[seq_len]);
+        if (!joined)
+            return cudaErrorMemoryAllocation;
+        gather(joined.get(), 0, seq_len);
+        return cudaMemcpy(d, joined.get(), seq_len, cudaMemcpyHostToDevice);
     };
     for (uint64_t r = 0; r < nrec; ++r)
         if (recs && rec_offs && rec_offs[r + 1] > rec_offs[r] && !recs[r])
