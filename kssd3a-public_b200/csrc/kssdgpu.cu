@@ -1166,6 +1166,11 @@ __global__ void __launch_bounds__(kCountThreads, LANES ? 6 : 4) k_count_striped(
     static_assert(!(WIDE && LANES) && (LANES || !LOWER), "wide groups leave ordinary blocks only");
     __shared__ ProbeQueue queues[kRow ? 1 : kCountThreads / 32];
     __shared__ WarpCells cells[!kRow && UNIQUE ? 2 : 1][kRow ? 1 : kCountThreads / 32];
+    // the warp's chunks at hand: in registers, they would be spilled
+    struct Take {
+        uint32_t at, end, size;
+    };
+    __shared__ Take takes[kCountThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if constexpr (!kRow) {
         WarpAcc{{}, &cells[0][warp]}.clear(lane);
@@ -1177,17 +1182,26 @@ __global__ void __launch_bounds__(kCountThreads, LANES ? 6 : 4) k_count_striped(
     const uint32_t nitems = *P.nitems_dev;
     const unsigned long long policy = keep_l2_policy();
     const size_t stripe_words = 2 * ((size_t)P.bloom_mask + 1);  // uint4 per stripe
-    const uint32_t take = stripe_take(nitems, (uint32_t)P.nq * (uint32_t)P.bloom_stripes,
-                                      gridDim.x * (kCountThreads / 32), LOWER ? 1 : LANES ? 2 : 4);
-    for (uint32_t it = 0, end = 0;; ++it) {
-        if (it == end) {
-            if (lane == 0)
-                it = atomicAdd(P.work, take);
-            it = __shfl_sync(0xFFFFFFFFu, it, 0);
-            if (it >= nitems)
-                break;
-            end = min(nitems, it + take);
+    if (lane == 0) {
+        Take &t = takes[warp];
+        t.at = t.end = 0;
+        t.size = stripe_take(nitems, (uint32_t)P.nq * (uint32_t)P.bloom_stripes, gridDim.x * (kCountThreads / 32),
+                             LOWER ? 1 : LANES ? 2 : 4);
+    }
+    for (;;) {
+        uint32_t it = 0;
+        if (lane == 0) {
+            Take &t = takes[warp];
+            it = t.at;
+            if (it == t.end) {
+                it = atomicAdd(P.work, t.size);
+                t.end = it + t.size;
+            }
+            t.at = it + 1;
         }
+        it = __shfl_sync(0xFFFFFFFFu, it, 0);
+        if (it >= nitems)
+            break;
         const WorkItem w = P.items[it];
         const int q = (int)w.q;
         const uint64_t b = P.qoffs[q] - base, e = P.qoffs[q + 1] - base;
