@@ -212,7 +212,7 @@ int server_launch(kssdgpu_server *s, ServerSlot &sl)
     uint64_t nk = 0, total = 0;
     for (const auto &r : sl.batch)
         total += r->keys.size();
-    const uint64_t chunk = count_chunk(total, (uint32_t)kChunkKeys, kServerChunks);
+    const uint64_t chunk = count_chunk(total, nq, (uint32_t)kChunkKeys, ChunkGoal{kServerChunks, kServerChunks});
     size_t nitems = 0;
     sl.h_offs[0] = 0;
     for (int i = 0; i < nq; ++i) {

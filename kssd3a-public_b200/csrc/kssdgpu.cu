@@ -297,6 +297,14 @@ constexpr int kMaxStripes = 256;
 constexpr uint64_t kStripeChunk = 256;
 constexpr uint64_t kStripeItemsMax = 1ull << 20;
 
+// Chunks that a block in global rows should give: of ordinary queries, and of queries of
+// kLargeQuery entries on average.
+struct ChunkGoal {
+    uint32_t small, large;
+};
+constexpr uint32_t kSmChunks = 32, kSmLarge = 5;  // a SM (chunk_goal)
+constexpr uint64_t kLargeQuery = 32768;           // assemblies hold 2,000 to 50,000, read sets 90,000 and more
+
 struct CountParams {
     const Slot *table;
     uint32_t mask;
@@ -319,7 +327,7 @@ struct CountParams {
     const uint32_t *chunk_prefix;  // global-row mode without items: query q owns the chunk_keys-entry
                                    // chunks [prefix[q], prefix[q+1]) (nq + 1 words), may be null
     uint32_t chunk_keys;           // entries per chunk in that mode, at most
-    uint32_t chunk_auto;           // chunks that a block should give (count_chunk)
+    ChunkGoal chunk_goal;          // chunks that a block should give (count_chunk)
     int *err;
     const uint4 *bloom;            // membership filter of the index's contexts, may be null
     uint32_t bloom_mask;           // 32-byte blocks of one stripe of it - 1
@@ -1015,13 +1023,10 @@ __device__ __forceinline__ void process_query_row(const CountParams &P, uint64_t
 }
 
 // Entries of a chunk of the chunk-major kernel: at most `most`, fewer when a block of
-// `total` entries would not give `chunks` of them, at least one round of a CTA's threads.
-// kSmChunks a SM: five or six for each CTA, so that the last ones hold up the end little (500
-// queries x 1,000 references in species of 24, conflicts, unique contexts: 265 us with 8, 219 with
-// 16, 202 with 32, 208 with 64; without conflicts 187, 162, 159 and 177).
-constexpr uint32_t kSmChunks = 32;
-__host__ __device__ __forceinline__ uint32_t count_chunk(uint64_t total, uint32_t most, uint32_t chunks)
+// `total` entries would not give `goal` chunks, at least one round of a CTA's threads.
+__host__ __device__ __forceinline__ uint32_t count_chunk(uint64_t total, int nq, uint32_t most, const ChunkGoal &goal)
 {
+    const uint32_t chunks = total >= (uint64_t)nq * kLargeQuery ? goal.large : goal.small;
     const uint64_t even = (total / chunks + 255) / 256 * 256;
     return even < 256 ? (most < 256 ? most : 256) : even < most ? (uint32_t)even : most;
 }
@@ -1053,7 +1058,8 @@ __global__ void __launch_bounds__(SMEM ? kRowThreads : kCountThreads, SMEM ? 4 :
     const int nref = P.nref;
     const FilterView fv{P.bloom, P.bloom_mask, P.bloom_stripes, P.bloom_bounds, keep_l2_policy()};
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t chunk_keys = P.chunk_auto ? count_chunk(P.qoffs[P.nq] - base, P.chunk_keys, P.chunk_auto) : P.chunk_keys;
+    const uint32_t chunk_keys =
+        P.chunk_goal.small ? count_chunk(P.qoffs[P.nq] - base, P.nq, P.chunk_keys, P.chunk_goal) : P.chunk_keys;
     if constexpr (!kRow) {
         WarpAcc{{}, &cells[0][warp]}.clear(lane);
         if (UNIQUE)
@@ -1280,10 +1286,10 @@ __global__ void k_stripe_expand(const uint64_t *__restrict__ spos, const uint64_
 
 // counts[q] = chunk-entry chunks of query q; prefix[0] = 0 (a scan of counts fills
 // prefix[1..nq])
-__global__ void k_chunk_counts(const uint64_t *__restrict__ qoffs, int nq, uint32_t most, uint32_t chunks,
+__global__ void k_chunk_counts(const uint64_t *__restrict__ qoffs, int nq, uint32_t most, ChunkGoal goal,
                                uint32_t *__restrict__ counts, uint32_t *__restrict__ prefix)
 {
-    const uint32_t chunk = count_chunk(qoffs[nq] - qoffs[0], most, chunks);
+    const uint32_t chunk = count_chunk(qoffs[nq] - qoffs[0], nq, most, goal);
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         if (q == 0)
             prefix[0] = 0;
@@ -2884,7 +2890,7 @@ struct kssdgpu_index {
     unsigned long long *gkey = nullptr;
     uint32_t *gbeg = nullptr;
     Slot *table = nullptr;
-    uint4 *bloom = nullptr;                 // membership filter of the contexts (see bloom_may_hold)
+    uint4 *bloom = nullptr;                 // membership filter of the contexts (see BloomBits)
     uint32_t bloom_mask = 0;                // 32-byte blocks per stripe - 1
     int bloom_stripes = 1;                  // key-range stripes of the filter
     unsigned long long *bloom_bounds = nullptr;  // first context of each stripe (stripes + 1 words)
@@ -3360,8 +3366,19 @@ bool walks_long(const kssdgpu_index *ix)
     return ix->f_conflict || (ix->f_groups && ix->f_postings >= (unsigned long long)kWarpWalk * ix->f_groups);
 }
 
-// Chunks that a block in global rows should give, whoever counts it.
-uint32_t chunk_goal(const kssdgpu_index *ix) { return (uint32_t)ix->sms * kSmChunks; }
+// Chunks that a block in global rows should give, whoever counts it.  Ordinary queries: kSmChunks
+// a SM, five or six for each CTA, so that the last ones hold up the end little (500 queries x 1,000
+// references in species of 24, conflicts, unique contexts: 265 us with 8, 219 with 16, 202 with 32,
+// 208 with 64; without conflicts 187, 162, 159 and 177).  Large queries (read sets) give chunks that
+// cost alike, so one for each CTA is enough, and each costs 6 us beside its entries: 9 read sets x
+// 532 references 93 us with 32 a SM, 76 with 8, 73 with 5; 3 x 150 51, 43, 39; 20 x 700 148, 130,
+// 130 (assemblies the other way, 500 x 1,000 171, 220, 226).  An entry a lane (lower blocks,
+// walks_long) takes kSmChunks of both: 9 read sets x 700 with conflicts 95, 101, 115.
+ChunkGoal chunk_goal(const kssdgpu_index *ix, bool lower, bool wide)
+{
+    const uint32_t sms = (uint32_t)ix->sms;
+    return ChunkGoal{sms * kSmChunks, sms * (!wide && (lower || walks_long(ix)) ? kSmChunks : kSmLarge)};
+}
 
 // An ordinary block in global rows, its wide groups walked like the others (every caller of the
 // chunk-major kernel: blocks, the no-allocation count, the server).
@@ -3598,9 +3615,9 @@ int count_dev_impl(kssdgpu_index *ix, const uint64_t *d_keys, const uint64_t *d_
         size_t tb = 0;
         CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, tb, ix->s_counts.p, ix->s_prefix.p + 1, nq, st));
         CUDA_TRY(ix->s_cubtmp.ensure(tb));
-        P.chunk_auto = chunk_goal(ix);
+        P.chunk_goal = chunk_goal(ix, lower, wide);
         k_chunk_counts<<<std::min((nq + 255) / 256, ix->sms * 8), 256, 0, st>>>(d_offs, nq, ix->count_chunk_keys,
-                                                                                P.chunk_auto, ix->s_counts.p,
+                                                                                P.chunk_goal, ix->s_counts.p,
                                                                                 ix->s_prefix.p);
         CUDA_TRY(cub::DeviceScan::InclusiveSum(ix->s_cubtmp.p, tb, ix->s_counts.p, ix->s_prefix.p + 1, nq, st));
         count_launch(3);
@@ -3689,6 +3706,7 @@ int count_host_pipelined(kssdgpu_index *ix, const uint64_t *qkeys, const uint64_
     const int np = (int)cut.size() - 1;
     // per sub-block query order (largest first) and key-range chunks, relative to it
     const bool smem = uses_smem_row(ix, flags);
+    const ChunkGoal goal = chunk_goal(ix, lower, !lower && wide_block_chosen(ix, nq / np, flags));
     std::vector<int> order_all(nq);
     std::vector<WorkItem> items_all;
     std::vector<size_t> item_off(np + 1, 0);
@@ -3700,7 +3718,7 @@ int count_host_pipelined(kssdgpu_index *ix, const uint64_t *qkeys, const uint64_
         if (!smem) {
             std::vector<WorkItem> it;
             build_chunks(qoffs + q0, nb, ord,
-                         count_chunk(qoffs[q0 + nb] - qoffs[q0], ix->count_chunk_keys, chunk_goal(ix)), it);
+                         count_chunk(qoffs[q0 + nb] - qoffs[q0], nb, ix->count_chunk_keys, goal), it);
             items_all.insert(items_all.end(), it.begin(), it.end());
         }
         item_off[p + 1] = items_all.size();
@@ -3785,8 +3803,9 @@ int count_host_impl(kssdgpu_index *ix, const uint64_t *qkeys, const uint64_t *qo
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sizes[a] > sizes[b]; });
     std::vector<WorkItem> items;
+    const ChunkGoal goal = chunk_goal(ix, lower, !lower && wide_block_chosen(ix, nq, flags));
     if (!uses_smem_row(ix, flags) && !(flags & KSSDGPU_PLAIN))
-        build_chunks(qoffs, nq, order.data(), count_chunk(nkeys, ix->count_chunk_keys, chunk_goal(ix)), items);
+        build_chunks(qoffs, nq, order.data(), count_chunk(nkeys, nq, ix->count_chunk_keys, goal), items);
     const size_t cells = (size_t)nq * ix->nref;
     const int nout = unique ? 4 : 2;
     CUDA_TRY(ix->s_keys.ensure(nkeys));
@@ -4942,10 +4961,10 @@ __global__ void k_noalloc_scatter(const uint64_t *__restrict__ offs, int nq, uns
 // prefix[0] = 0, prefix[q + 1] = prefix[q] + ceil(size(q) / count_chunk(..)): the key-range
 // chunks of the global-row kernel, in one CTA (nq <= KSSDGPU_NOALLOC_MAX_QUERIES).
 __global__ void __launch_bounds__(1024) k_noalloc_prefix(const uint64_t *__restrict__ offs, int nq, uint32_t most,
-                                                         uint32_t chunks, unsigned int *__restrict__ prefix)
+                                                         ChunkGoal goal, unsigned int *__restrict__ prefix)
 {
     __shared__ unsigned int part[1024];
-    const uint32_t chunk = count_chunk(offs[nq] - offs[0], most, chunks);
+    const uint32_t chunk = count_chunk(offs[nq] - offs[0], nq, most, goal);
     const int per = (nq + 1023) / 1024;
     const int q0 = min(nq, (int)threadIdx.x * per), q1 = min(nq, q0 + per);
     unsigned int sum = 0;
@@ -5864,7 +5883,7 @@ int kssdgpu_count_block_noalloc(kssdgpu_index_t *ix, const uint64_t *d_qry_keys,
         k_noalloc_scatter<<<grid, 256, 0, st>>>(d_qry_offs, nq, scr);
         count_launch(3);
     } else {
-        k_noalloc_prefix<<<1, 1024, 0, st>>>(d_qry_offs, nq, ix->count_chunk_keys, chunk_goal(ix),
+        k_noalloc_prefix<<<1, 1024, 0, st>>>(d_qry_offs, nq, ix->count_chunk_keys, chunk_goal(ix, lower != 0, false),
                                              scr + kNoallocHeaderWords - 1);
         count_launch();
     }
@@ -5894,7 +5913,7 @@ int kssdgpu_count_block_noalloc(kssdgpu_index_t *ix, const uint64_t *d_qry_keys,
     P.order = use_smem ? reinterpret_cast<const int *>(scr + kNoallocHeaderWords) : nullptr;
     P.chunk_prefix = use_smem ? nullptr : scr + kNoallocHeaderWords - 1;
     P.chunk_keys = ix->count_chunk_keys;
-    P.chunk_auto = chunk_goal(ix);
+    P.chunk_goal = chunk_goal(ix, lower != 0, false);
     const size_t cells = (size_t)nq * ix->nref;
     const size_t smem = (size_t)ix->nref * sizeof(unsigned long long) * (unique ? 4 : 2);
     if (!use_smem && !(flags & KSSDGPU_NO_ZERO)) {
@@ -5943,8 +5962,9 @@ int kssdgpu_count_detail(kssdgpu_index_t *ix, const uint64_t *qry_keys, const ui
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return sizes[a] > sizes[b]; });
     std::vector<WorkItem> items;
+    const ChunkGoal goal = chunk_goal(ix, false, wide_block_chosen(ix, nq, flags));
     if (!uses_smem_row(ix, flags))
-        build_chunks(qry_offs, nq, order.data(), count_chunk(nkeys, ix->count_chunk_keys, chunk_goal(ix)), items);
+        build_chunks(qry_offs, nq, order.data(), count_chunk(nkeys, nq, ix->count_chunk_keys, goal), items);
     const int nref = ix->nref;
     const size_t cells = (size_t)nq * nref;
     CUDA_TRY(ix->s_keys.ensure(nkeys));
