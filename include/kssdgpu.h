@@ -441,7 +441,9 @@ int kssdgpu_count_plain_dev(kssdgpu_index_t *idx, const uint64_t *d_qry_keys, co
  *     call kssdgpu_init(device) first so that the address is looked up again;
  *   - every call shares the one array (it keeps the last call's contents and is
  *     cleared where needed on each call), so calls that overlap on the GPU (other
- *     streams, other threads) race: serialise them.
+ *     streams, other threads) race: serialise them;
+ *   - every context is counted by its postings: the tensor cores that
+ *     kssdgpu_count_block_dev leaves contexts of many references to need scratch.
  */
 #define KSSDGPU_NOALLOC_MAX_QUERIES 65536
 #define KSSDGPU_NOALLOC_SCRATCH_BYTES (512 + 4 * KSSDGPU_NOALLOC_MAX_QUERIES)
@@ -463,7 +465,8 @@ int kssdgpu_count_block_noalloc(kssdgpu_index_t *idx, const uint64_t *d_qry_keys
  * join the next free slot.  A batch whose nonzero cells overflow max_hits is split:
  * its requests re-run one per batch, and only a request that overflows alone fails
  * (KSSDGPU_ERR_CAPACITY).  Query keys that do not ascend are rejected at submit
- * (KSSDGPU_ERR_UNSORTED).
+ * (KSSDGPU_ERR_UNSORTED).  Batches count every context by its postings, not on the
+ * tensor cores: on an index of one species a request walks hundreds of them per key.
  */
 typedef struct kssdgpu_hit {
     uint32_t query; /* 0 in results (each request is one query) */

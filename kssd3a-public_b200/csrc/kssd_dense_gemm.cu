@@ -42,9 +42,9 @@ using Mainloop = typename cutlass::gemm::collective::CollectiveBuilder<
     cutlass::layout::RowMajor, 16, int32_t, TileShape, ClusterShape,
     cutlass::gemm::collective::StageCountAutoCarveout<static_cast<int>(sizeof(typename Epilogue::SharedStorage))>,
     cutlass::gemm::KernelTmaWarpSpecialized1SmSm100>::CollectiveOp;
-// stream-K scheduler: the output has few 128 x 128 tiles (n x 4n for n of hundreds to
-// thousands of genomes) against a deep K, so the K loop of each tile is split across SMs
-// (by stream-K, or by an even split-K for the smallest outputs: make_args)
+// stream-K scheduler: the output has few 128 x 128 tiles (six products of n x n, or one of
+// n x 4n, for n of hundreds to thousands of genomes) against a deep K, so the K loop of
+// each tile is split across SMs (by stream-K, or by an even split-K for the smallest outputs: make_args)
 using Kernel =
     cutlass::gemm::kernel::GemmUniversal<Shape<int, int, int, int>, Mainloop, Epilogue, cutlass::gemm::StreamKScheduler>;
 using Gemm = cutlass::gemm::device::GemmUniversalAdapter<Kernel>;
@@ -76,8 +76,8 @@ typename Gemm::Arguments make_args(const int8_t *A, const int8_t *B, int32_t *D,
     typename Gemm::Arguments args{cutlass::gemm::GemmUniversalMode::kGemm, {M, N, K, batch}, {A, sa, B, sb},
                                   {{1, 0}, D, sc, D, sd}};
 #if KSSD_GEMM_SCHED
-    // Fewer output tiles than SMs (up to about 770 genomes): split K evenly over
-    // floor(SMs / tiles) CTAs per tile, all resident at once, so the CTAs that share a
+    // Fewer output tiles than SMs (six products of up to 512 genomes, n x 4n of up to about
+    // 770): split K evenly over floor(SMs / tiles) CTAs per tile, all resident at once, so the CTAs that share a
     // K range read the same operand slices at about the same time (L2 hits instead of
     // re-streaming); the int32 partial sums are exact in any order.  Measured on the
     // 512-genome dense join: 1.01-1.14 ms per step against 1.15-1.22 ms with stream-K.
